@@ -5,10 +5,16 @@
 // tiled attention (ShaderTiledMHAN, poly/wgpu_shaders.go:1112-1388).
 //
 // Shape of the kernel
-//   * One cluster per KV head; the S CTAs of a cluster split the positions 0..pos into S contiguous slices.  A CTA
-//     brings its K and V rows into shared memory with ONE bulk async copy each (the ring is head-major, so a slice is
+//   * One cluster per KV head and sequence; the S CTAs of a cluster split the positions 0..pos into S contiguous slices.
+//     A CTA brings its K and V rows into shared memory with ONE bulk async copy each (the ring is head-major, so a slice is
 //     one contiguous block) and serves all query heads of the GQA group from them: every K/V element is converted
-//     to float64 once and used by every head of the group.
+//     to float64 once and used by every head of the group.  A slice that does not fit goes through in chunks with a running
+//     softmax: the next K rows travel behind softmax and weighted V, the next V rows behind the next scores.
+//   * S: one sequence takes the largest cluster of which the device holds one per KV head; a pass of several takes the
+//     largest of which it holds one per (sequence, KV head), down to single CTAs (eight sequences x eight KV heads: pairs).
+//   * Bound: float64 issue and the float32 -> float64 conversions (16 lanes a clock) behind one another's latencies.  Measured:
+//     five KV heads, context 1040, MaxSeqLen 4096: 10.9 us where the split kernel took 14.1 (no cluster held such a ring before);
+//     eight sequences x eight KV heads at context 2048, pairs of CTAs: 58 us (2.3 TB/s) where one streaming CTA each took 101.
 //   * Scores: a warp owns a position at a time, a lane four dimensions of it (the query slices live in registers);
 //     sixteen (position, head) sums are reduced across the warp together so that the shuffle count per position stays small.
 //   * The S partial results (max, sum, weighted V) never touch global memory: every CTA stores its partials straight
@@ -85,20 +91,20 @@ __device__ __forceinline__ int halving_index(int lane) {
 }
 
 // LEAN: one token of one sequence, no phase trace (what a decode step launches); the code of the other forms is left out.
-// (Fixing the head dimension at compile time as well measured no better.)
-template <int G, bool LEAN = false>
+// (Fixing the head dimension at compile time as well measured no better.)  ONE: a slice always fits in one chunk.
+template <int G, bool LEAN, bool ONE>
 __global__ void __launch_bounds__(kAcThreads, 1) lb_attention_cluster_kernel(const LbAttnParams p) {
     extern __shared__ __align__(128) uint8_t smem_raw[];
     __shared__ __align__(8) uint64_t bars[2];
     __shared__ double s_red[kAcWarps], s_red2[kAcWarps];  // per-warp maxima, per-warp sums (separate: no barrier between the two reductions)
-    __shared__ double s_m[G], s_l[G];        // this CTA's maximum and sum per head
+    __shared__ double s_m[G], s_l[G], s_alpha[G];  // this CTA's running maximum and sum per head, factor of what came before the chunk
     __shared__ double s_gw[kAcMaxS * G];     // combine: weight of every (slice, head)
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const int hd = p.hd, half = hd >> 1, kvh = blockIdx.y;
     const int n = LEAN ? 0 : blockIdx.z;  // token of the pass; with seq_stride > 0 every token is a sequence of its own
     const size_t seq_off = LEAN ? 0 : (size_t)n * (size_t)p.seq_stride;
     const uint32_t rank = cluster_ctarank(), S = cluster_nctarank();
-    const int cmax = p.max_chunk;  // positions one CTA holds at most
+    const int cmax = p.max_chunk;  // positions one CTA holds at a time
     const int dps = hd / (int)S;   // output dimensions every CTA combines
     float* kt = reinterpret_cast<float*>(smem_raw);            // [cmax, hd]
     float* vt = kt + (size_t)cmax * hd;                        // [cmax, hd]
@@ -126,13 +132,16 @@ __global__ void __launch_bounds__(kAcThreads, 1) lb_attention_cluster_kernel(con
     const int cnt = k1 > k0 ? k1 - k0 : 0;
     const float* kbase = p.cache_k + seq_off + (size_t)kvh * p.msl * hd;
     const float* vbase = p.cache_v + seq_off + (size_t)kvh * p.msl * hd;
+    auto fetch = [&](int which, int c0) {  // the K (0) or V (1) rows of the chunk that starts at c0; one thread
+        const uint32_t bytes = (uint32_t)(cnt - c0 < cmax ? cnt - c0 : cmax) * hd * 4;
+        lb_mbar_expect_tx(&bars[which], bytes);
+        lb_bulk_g2s_stream(which ? vt : kt, (which ? vbase : kbase) + (size_t)(k0 + c0) * hd, bytes, &bars[which], lb_policy_evict_first());
+    };
     if (cnt > 0 && lane == 0) {
         if (warp == 0) {
-            lb_mbar_expect_tx(&bars[0], (uint32_t)cnt * hd * 4);
-            lb_bulk_g2s_stream(kt, kbase + (size_t)k0 * hd, (uint32_t)cnt * hd * 4, &bars[0], lb_policy_evict_first());
+            fetch(0, 0);
         } else if (warp == 1) {
-            lb_mbar_expect_tx(&bars[1], (uint32_t)cnt * hd * 4);
-            lb_bulk_g2s_stream(vt, vbase + (size_t)k0 * hd, (uint32_t)cnt * hd * 4, &bars[1], lb_policy_evict_first());
+            fetch(1, 0);
         } else if (warp == 2 && p.next_k) {  // the next block's rows of the same positions, into L2
             l2_prefetch(p.next_k + ((size_t)kvh * p.msl + k0) * hd, (uint32_t)cnt * hd * 4);
             l2_prefetch(p.next_v + ((size_t)kvh * p.msl + k0) * hd, (uint32_t)cnt * hd * 4);
@@ -153,110 +162,138 @@ __global__ void __launch_bounds__(kAcThreads, 1) lb_attention_cluster_kernel(con
         sq[g * hd + d] = __dsub_rn(__dmul_rn(v0, c), __dmul_rn(v1, sn));
         sq[g * hd + d + half] = __dadd_rn(__dmul_rn(v0, sn), __dmul_rn(v1, c));
     }
+    if (tid < G) {
+        s_m[tid] = -1e300;
+        s_l[tid] = 0.0;
+    }
     bool failed = false;
-    if (cnt > 0 && !lb_mbar_wait_bounded(&bars[0], 0)) failed = true;
-    if (cnt > 0 && last >= k0 && last < k1) {
-        // the newest position belongs to this slice: its ring row is not written yet; rotate the row the QKV projection
-        // left in k_new into the tile and into the ring (threads 0..hd/2-1 hold the sine and cosine of their pair)
-        if (tid < half) {
+    const double scale = __ddiv_rn(1.0, sqrt((double)hd));
+    const bool lane_on = 4 * lane < hd;
+    double acc[G][4];
+#pragma unroll
+    for (int g = 0; g < G; ++g)
+#pragma unroll
+        for (int c = 0; c < 4; ++c) acc[g][c] = 0.0;
+    const int vi = halving_index<16>(lane);  // scores: this lane finishes value vi = pp * G + g
+    // (ONE: the body runs once even for an empty slice, with no rows)
+    for (int c0 = 0, chunk = 0; ONE ? chunk == 0 : c0 < cnt; c0 += cmax, ++chunk) {
+        const int rows = ONE ? cnt : cnt - c0 < cmax ? cnt - c0 : cmax;
+        const bool more = !ONE && c0 + cmax < cnt;
+        if (rows > 0 && !failed && !lb_mbar_wait_bounded(&bars[0], (uint32_t)(chunk & 1))) failed = true;
+        if (last >= k0 + c0 && last < k0 + c0 + rows && tid < half) {
+            // the newest position belongs to this chunk: its ring row is not written yet; rotate the row the QKV projection
+            // left in k_new into the tile and into the ring (threads 0..hd/2-1 hold the sine and cosine of their pair)
             const float* knew = p.k_new + (size_t)n * p.kv_heads * hd + (size_t)kvh * hd;
             const double v0 = (double)knew[tid], v1 = (double)knew[tid + half];
             const float r0 = (float)__dsub_rn(__dmul_rn(v0, rc), __dmul_rn(v1, rsn));
             const float r1 = (float)__dadd_rn(__dmul_rn(v0, rsn), __dmul_rn(v1, rc));
-            float* trow = kt + (size_t)(last - k0) * hd;
+            float* trow = kt + (size_t)(last - k0 - c0) * hd;
             trow[tid] = r0;
             trow[tid + half] = r1;
             float* grow = p.cache_k_w + seq_off + ((size_t)kvh * p.msl + (size_t)(last % p.msl)) * hd;
             grow[tid] = r0;
             grow[tid + half] = r1;
         }
-    }
-    __syncthreads();
+        __syncthreads();  // the newest row is in the tile; every warp is done with the weights and V rows of the chunk before
+        if (!ONE && chunk > 0 && tid == 0 && !failed) {
+            asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+            fetch(1, c0);
+        }
 
-    // ---- scores: warp = position, lane = four dimensions; PP positions x G heads = 16 sums are reduced together ----
-    const double scale = __ddiv_rn(1.0, sqrt((double)hd));
-    const bool lane_on = 4 * lane < hd;
-    {
-        constexpr int PP = 16 / G;
-        double qv[G][4];
+        // ---- scores: warp = position, lane = four dimensions; PP positions x G heads = 16 sums are reduced together ----
+        {
+            constexpr int PP = 16 / G;
+            double qv[G][4];
 #pragma unroll
-        for (int g = 0; g < G; ++g)
+            for (int g = 0; g < G; ++g)
 #pragma unroll
-            for (int c = 0; c < 4; ++c) qv[g][c] = lane_on ? sq[g * hd + 4 * lane + c] : 0.0;
-        const int vi = halving_index<16>(lane);  // this lane finishes value vi = pp * G + g
-        for (int j0 = warp * PP; j0 < cnt; j0 += kAcWarps * PP) {
-            double acc[16];
+                for (int c = 0; c < 4; ++c) qv[g][c] = lane_on ? sq[g * hd + 4 * lane + c] : 0.0;
+            for (int j0 = warp * PP; j0 < rows; j0 += kAcWarps * PP) {
+                double sums[16];
 #pragma unroll
-            for (int pp = 0; pp < PP; ++pp) {
-                float4 kv = make_float4(0.f, 0.f, 0.f, 0.f);
-                if (lane_on && j0 + pp < cnt) kv = *reinterpret_cast<const float4*>(kt + (size_t)(j0 + pp) * hd + 4 * lane);
-                const double k0d = (double)kv.x, k1d = (double)kv.y, k2d = (double)kv.z, k3d = (double)kv.w;
+                for (int pp = 0; pp < PP; ++pp) {
+                    float4 kv = make_float4(0.f, 0.f, 0.f, 0.f);
+                    if (lane_on && j0 + pp < rows) kv = *reinterpret_cast<const float4*>(kt + (size_t)(j0 + pp) * hd + 4 * lane);
+                    const double k0d = (double)kv.x, k1d = (double)kv.y, k2d = (double)kv.z, k3d = (double)kv.w;
+#pragma unroll
+                    for (int g = 0; g < G; ++g) {
+                        double a = __dmul_rn(qv[g][0], k0d);
+                        a = fma(qv[g][1], k1d, a);
+                        a = fma(qv[g][2], k2d, a);
+                        a = fma(qv[g][3], k3d, a);
+                        sums[pp * G + g] = a;
+                    }
+                }
+                warp_reduce_halving<16>(sums, lane);
+                const int pp = vi / G, g = vi - pp * G;
+                if ((lane & 1) == 0 && j0 + pp < rows) sc[g * cmax + j0 + pp] = __dmul_rn(sums[0], scale);
+            }
+        }
+        __syncthreads();  // scores complete, the K rows are free
+        if (more && tid == 0 && !failed) {
+            asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+            fetch(0, c0 + cmax);
+        }
+        if (!LEAN) lb_trace(p.trace, 3);
+
+        // ---- running softmax, per head: the warps w with w % G == g share head g ----
+        {
+            constexpr int WPG = kAcWarps / G;  // warps per head
+            const int g = warp % G, wq = warp / G;
+            double mx = -1e300;
+            for (int j = wq * 32 + lane; j < rows; j += WPG * 32) mx = fmax(mx, sc[g * cmax + j]);
+#pragma unroll
+            for (int o = 16; o > 0; o >>= 1) mx = fmax(mx, __shfl_xor_sync(0xffffffffu, mx, o));
+            if (lane == 0) s_red[warp] = mx;
+            __syncthreads();
+            mx = s_red[g];
+#pragma unroll
+            for (int w = 1; w < WPG; ++w) mx = fmax(mx, s_red[g + w * G]);
+            const double m_old = s_m[g];
+            mx = fmax(mx, m_old);
+            double sum = 0.0;
+            for (int j = wq * 32 + lane; j < rows; j += WPG * 32) {
+                const double e = exp(__dsub_rn(sc[g * cmax + j], mx));
+                sc[g * cmax + j] = e;
+                sum = __dadd_rn(sum, e);
+            }
+            sum = lb_warp_sum(sum);
+            if (lane == 0) s_red2[warp] = sum;
+            __syncthreads();  // (everyone has read the old maximum)
+            if (wq == 0 && lane == 0) {  // every warp of head g holds the same maximum
+                double l = 0.0;
+                for (int w = 0; w < WPG; ++w) l += s_red2[g + w * G];
+                if (!ONE && chunk > 0) {
+                    const double alpha = exp(__dsub_rn(m_old, mx));
+                    s_alpha[g] = alpha;
+                    l = __dadd_rn(__dmul_rn(s_l[g], alpha), l);
+                }
+                s_l[g] = l;
+                s_m[g] = mx;
+            }
+        }
+        if (rows > 0 && !failed && !lb_mbar_wait_bounded(&bars[1], (uint32_t)(chunk & 1))) failed = true;
+        __syncthreads();
+
+        // ---- weighted V: warp = position, lane = four dimensions, all heads of the group from one converted row ----
+        if (!ONE && chunk > 0) {
+#pragma unroll
+            for (int g = 0; g < G; ++g)
+#pragma unroll
+                for (int c = 0; c < 4; ++c) acc[g][c] = __dmul_rn(acc[g][c], s_alpha[g]);
+        }
+        if (lane_on) {
+            for (int j = warp; j < rows; j += kAcWarps) {
+                const float4 vv = *reinterpret_cast<const float4*>(vt + (size_t)j * hd + 4 * lane);
+                const double v0 = (double)vv.x, v1 = (double)vv.y, v2 = (double)vv.z, v3 = (double)vv.w;
 #pragma unroll
                 for (int g = 0; g < G; ++g) {
-                    double a = __dmul_rn(qv[g][0], k0d);
-                    a = fma(qv[g][1], k1d, a);
-                    a = fma(qv[g][2], k2d, a);
-                    a = fma(qv[g][3], k3d, a);
-                    acc[pp * G + g] = a;
+                    const double w = sc[g * cmax + j];
+                    acc[g][0] = fma(w, v0, acc[g][0]);
+                    acc[g][1] = fma(w, v1, acc[g][1]);
+                    acc[g][2] = fma(w, v2, acc[g][2]);
+                    acc[g][3] = fma(w, v3, acc[g][3]);
                 }
-            }
-            warp_reduce_halving<16>(acc, lane);
-            const int pp = vi / G, g = vi - pp * G;
-            if ((lane & 1) == 0 && j0 + pp < cnt) sc[g * cmax + j0 + pp] = __dmul_rn(acc[0], scale);
-        }
-    }
-    __syncthreads();
-    if (!LEAN) lb_trace(p.trace, 3);
-
-    // ---- softmax over this slice, per head: the warps w with w % G == g share head g ----
-    {
-        constexpr int WPG = kAcWarps / G;  // warps per head
-        const int g = warp % G, wq = warp / G;
-        double mx = -1e300;
-        for (int j = wq * 32 + lane; j < cnt; j += WPG * 32) mx = fmax(mx, sc[g * cmax + j]);
-#pragma unroll
-        for (int o = 16; o > 0; o >>= 1) mx = fmax(mx, __shfl_xor_sync(0xffffffffu, mx, o));
-        if (lane == 0) s_red[warp] = mx;
-        __syncthreads();
-        mx = s_red[g];
-#pragma unroll
-        for (int w = 1; w < WPG; ++w) mx = fmax(mx, s_red[g + w * G]);
-        double sum = 0.0;
-        for (int j = wq * 32 + lane; j < cnt; j += WPG * 32) {
-            const double e = exp(__dsub_rn(sc[g * cmax + j], mx));
-            sc[g * cmax + j] = e;
-            sum = __dadd_rn(sum, e);
-        }
-        sum = lb_warp_sum(sum);
-        if (lane == 0) s_red2[warp] = sum;
-        __syncthreads();
-        if (tid < G) {
-            double l = 0.0;
-            for (int w = 0; w < WPG; ++w) l += s_red2[tid + w * G];
-            s_l[tid] = l;
-        }
-        if (wq == 0 && lane == 0) s_m[g] = mx;  // every warp of head g holds the same maximum
-    }
-    if (cnt > 0 && !lb_mbar_wait_bounded(&bars[1], 0)) failed = true;
-    __syncthreads();
-
-    // ---- weighted V: warp = position, lane = four dimensions, all heads of the group from one converted row ----
-    double acc[G][4];
-#pragma unroll
-    for (int g = 0; g < G; ++g)
-#pragma unroll
-        for (int c = 0; c < 4; ++c) acc[g][c] = 0.0;
-    if (lane_on) {
-        for (int j = warp; j < cnt; j += kAcWarps) {
-            const float4 vv = *reinterpret_cast<const float4*>(vt + (size_t)j * hd + 4 * lane);
-            const double v0 = (double)vv.x, v1 = (double)vv.y, v2 = (double)vv.z, v3 = (double)vv.w;
-#pragma unroll
-            for (int g = 0; g < G; ++g) {
-                const double w = sc[g * cmax + j];
-                acc[g][0] = fma(w, v0, acc[g][0]);
-                acc[g][1] = fma(w, v1, acc[g][1]);
-                acc[g][2] = fma(w, v2, acc[g][2]);
-                acc[g][3] = fma(w, v3, acc[g][3]);
             }
         }
     }
@@ -316,233 +353,40 @@ __global__ void __launch_bounds__(kAcThreads, 1) lb_attention_cluster_kernel(con
     if (!LEAN) lb_trace(p.trace, 5);
 }
 
-// ------------------------------------------------------------------------------------------------------------------
-// The throughput form for a pass of several sequences (one new token each): ONE CTA per (sequence, KV head) streams the
-// sequence's whole context through double-buffered 64-position tiles (one bulk copy per K and per V tile) and keeps a
-// running softmax, all query heads of the GQA group served from the same tiles.  A pass of eight sequences launches
-// kv_heads x 8 such CTAs, which fit the device at once; the cluster kernel above would need sixteen CTAs for each of them
-// and run in waves.  q arrives rotated and the newest K row is already in the ring (lb_rope_kernel ran before).
-// Arithmetic as above; the running softmax rescales by exp(m_old - m_new) per tile (float64).
-constexpr int kAsThreads = 256;
-constexpr int kAsWarps = kAsThreads / 32;
-constexpr int kAsTile = 64;  // positions per tile
+constexpr size_t kAcSmem = 200 * 1024;
+constexpr int kAcChunk = 128;  // positions of a chunk when a slice does not fit at once
 
 template <int G>
-__global__ void __launch_bounds__(kAsThreads, 1) lb_attention_stream_kernel(const LbAttnParams p) {
-    static_assert(G == 4 || G == 8, "group sizes the score reduction is laid out for");
-    extern __shared__ __align__(128) uint8_t smem_raw[];
-    __shared__ __align__(8) uint64_t bars[4];  // [stage][K, V]
-    __shared__ double s_red[kAsWarps], s_red2[kAsWarps];
-    __shared__ double s_m[G], s_l[G], s_alpha[2][G];
-    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-    const int hd = p.hd, kvh = blockIdx.x, n = blockIdx.y;
-    const size_t seq_off = (size_t)n * (size_t)(p.seq_stride > 0 ? p.seq_stride : 0);
-    const size_t tile_elems = (size_t)kAsTile * hd;
-    float* kt = reinterpret_cast<float*>(smem_raw);                 // [2][64, hd]
-    float* vt = kt + 2 * tile_elems;                                // [2][64, hd]
-    double* sq = reinterpret_cast<double*>(vt + 2 * tile_elems);    // [G, hd] queries
-    double* sc = sq + G * hd;                                       // [2][G, 64] scores, then weights, per tile parity
-    double* red = reinterpret_cast<double*>(smem_raw);              // after the last tile: [warps, G, hd] over the tiles
-    if (tid == 0) {
-        for (int i = 0; i < 4; ++i) lb_mbar_init(&bars[i], 1);
-        lb_fence_mbar_init();
-    }
-    __syncthreads();
-    lb_pdl_launch_dependents();
-    lb_pdl_wait();
-    const int last = p.seq_stride > 0 ? p.pos_ptr[n] : *p.pos_ptr + n;  // the token's position; it attends to 0..last
-    const int total = last + 1;
-    const int ntiles = (total + kAsTile - 1) / kAsTile;
-    const float* kbase = p.cache_k + seq_off + (size_t)kvh * p.msl * hd;
-    const float* vbase = p.cache_v + seq_off + (size_t)kvh * p.msl * hd;
-    const uint64_t pol = lb_policy_evict_first();
-    auto rows_of = [&](int t) { return total - t * kAsTile < kAsTile ? total - t * kAsTile : kAsTile; };
-    auto issue = [&](int t) {  // one thread
-        const int st = t & 1, rows = rows_of(t);
-        lb_mbar_expect_tx(&bars[2 * st], (uint32_t)rows * hd * 4);
-        lb_bulk_g2s_stream(kt + st * tile_elems, kbase + (size_t)t * kAsTile * hd, (uint32_t)rows * hd * 4, &bars[2 * st], pol);
-        lb_mbar_expect_tx(&bars[2 * st + 1], (uint32_t)rows * hd * 4);
-        lb_bulk_g2s_stream(vt + st * tile_elems, vbase + (size_t)t * kAsTile * hd, (uint32_t)rows * hd * 4, &bars[2 * st + 1], pol);
-    };
-    if (tid == 0) {
-        issue(0);
-        if (ntiles > 1) issue(1);
-    }
-    for (int idx = tid; idx < G * hd; idx += kAsThreads) sq[idx] = p.q[(size_t)n * p.heads * hd + (size_t)kvh * G * hd + idx];
-    if (tid < G) {
-        s_m[tid] = -1e300;
-        s_l[tid] = 0.0;
-    }
-    __syncthreads();
-    const double scale = __ddiv_rn(1.0, sqrt((double)hd));
-    const bool lane_on = 4 * lane < hd;
-    constexpr int PP = 16 / G;           // positions whose G sums are reduced together
-    constexpr int WPG = kAsWarps / G < 1 ? 1 : kAsWarps / G;  // warps that share a head in the softmax (G = 8: one)
-    double qv[G][4];
-#pragma unroll
-    for (int g = 0; g < G; ++g)
-#pragma unroll
-        for (int c = 0; c < 4; ++c) qv[g][c] = lane_on ? sq[g * hd + 4 * lane + c] : 0.0;
-    const int vi = halving_index<16>(lane);
-    double o[G][4];
-#pragma unroll
-    for (int g = 0; g < G; ++g)
-#pragma unroll
-        for (int c = 0; c < 4; ++c) o[g][c] = 0.0;
-    bool failed = false;
-    for (int t = 0; t < ntiles; ++t) {
-        const int st = t & 1, rows = rows_of(t);
-        const uint32_t ph = (uint32_t)((t >> 1) & 1);
-        const float* ktile = kt + st * tile_elems;
-        const float* vtile = vt + st * tile_elems;
-        double* sct = sc + (size_t)st * G * kAsTile;
-        if (!failed && !lb_mbar_wait_bounded(&bars[2 * st], ph)) failed = true;
-        // ---- scores of the tile: warp = eight positions, lane = four dimensions ----
-        for (int j0 = warp * (kAsTile / kAsWarps); j0 < (warp + 1) * (kAsTile / kAsWarps); j0 += PP) {
-            double acc[16];
-#pragma unroll
-            for (int pp = 0; pp < PP; ++pp) {
-                float4 kv = make_float4(0.f, 0.f, 0.f, 0.f);
-                if (lane_on && j0 + pp < rows) kv = *reinterpret_cast<const float4*>(ktile + (size_t)(j0 + pp) * hd + 4 * lane);
-                const double k0d = (double)kv.x, k1d = (double)kv.y, k2d = (double)kv.z, k3d = (double)kv.w;
-#pragma unroll
-                for (int g = 0; g < G; ++g) {
-                    double a = __dmul_rn(qv[g][0], k0d);
-                    a = fma(qv[g][1], k1d, a);
-                    a = fma(qv[g][2], k2d, a);
-                    a = fma(qv[g][3], k3d, a);
-                    acc[pp * G + g] = a;
-                }
-            }
-            warp_reduce_halving<16>(acc, lane);
-            const int pp = vi / G, g = vi - pp * G;
-            if ((lane & 1) == 0) sct[g * kAsTile + j0 + pp] = j0 + pp < rows ? __dmul_rn(acc[0], scale) : -1e300;  // absent positions: weight 0
-        }
-        __syncthreads();  // scores complete; every warp is past the weighted sum of tile t - 1
-        if (tid == 0 && t >= 1 && t + 1 < ntiles) issue(t + 1);  // into the buffers tile t - 1 has just left
-        // ---- running softmax, per head ----
-        {
-            const int g = warp % G, wq = warp / G;
-            double mx = -1e300;
-            for (int j = wq * 32 + lane; j < kAsTile; j += WPG * 32) mx = fmax(mx, sct[g * kAsTile + j]);
-#pragma unroll
-            for (int off = 16; off > 0; off >>= 1) mx = fmax(mx, __shfl_xor_sync(0xffffffffu, mx, off));
-            if (lane == 0) s_red[warp] = mx;
-            __syncthreads();
-            mx = s_red[g];
-#pragma unroll
-            for (int w = 1; w < WPG; ++w) mx = fmax(mx, s_red[g + w * G]);
-            const double m_old = s_m[g];
-            const double m_new = fmax(m_old, mx);
-            double sum = 0.0;
-            for (int j = wq * 32 + lane; j < kAsTile; j += WPG * 32) {
-                const double e = j < rows ? exp(__dsub_rn(sct[g * kAsTile + j], m_new)) : 0.0;
-                sct[g * kAsTile + j] = e;
-                sum = __dadd_rn(sum, e);
-            }
-            sum = lb_warp_sum(sum);
-            if (lane == 0) s_red2[warp] = sum;
-            __syncthreads();  // weights and per-warp sums visible; everyone has read the old maximum
-            if (wq == 0 && lane == 0) {
-                double l = 0.0;
-                for (int w = 0; w < WPG; ++w) l += s_red2[g + w * G];
-                const double alpha = exp(__dsub_rn(m_old, m_new));  // 0 for the first tile (m_old = -1e300)
-                s_alpha[st][g] = alpha;
-                s_l[g] = __dadd_rn(__dmul_rn(s_l[g], alpha), l);
-                s_m[g] = m_new;
-            }
-        }
-        if (!failed && !lb_mbar_wait_bounded(&bars[2 * st + 1], ph)) failed = true;
-        __syncthreads();  // rescale factors visible
-        // ---- weighted V: warp = every eighth position, lane = four dimensions ----
-#pragma unroll
-        for (int g = 0; g < G; ++g) {
-            const double al = s_alpha[st][g];
-#pragma unroll
-            for (int c = 0; c < 4; ++c) o[g][c] = __dmul_rn(o[g][c], al);
-        }
-        if (lane_on) {
-            for (int j = warp; j < rows; j += kAsWarps) {
-                const float4 vv = *reinterpret_cast<const float4*>(vtile + (size_t)j * hd + 4 * lane);
-                const double v0 = (double)vv.x, v1 = (double)vv.y, v2 = (double)vv.z, v3 = (double)vv.w;
-#pragma unroll
-                for (int g = 0; g < G; ++g) {
-                    const double w = sct[g * kAsTile + j];
-                    o[g][0] = fma(w, v0, o[g][0]);
-                    o[g][1] = fma(w, v1, o[g][1]);
-                    o[g][2] = fma(w, v2, o[g][2]);
-                    o[g][3] = fma(w, v3, o[g][3]);
-                }
-            }
-        }
-    }
-    if (failed && tid == 0) atomicExch(p.status, 1);
-    __syncthreads();  // every warp is done with the tiles: the reduction buffer takes their place
-    if (lane_on) {
-#pragma unroll
-        for (int g = 0; g < G; ++g)
-            *reinterpret_cast<double4*>(red + ((size_t)warp * G + g) * hd + 4 * lane) = make_double4(o[g][0], o[g][1], o[g][2], o[g][3]);
-    }
-    __syncthreads();
-    for (int idx = tid; idx < G * hd; idx += kAsThreads) {
-        const int g = idx / hd, d = idx - g * hd;
-        double v = 0.0;
-#pragma unroll
-        for (int w = 0; w < kAsWarps; ++w) v += red[((size_t)w * G + g) * hd + d];  // fixed order: the same bits on every replay
-        p.out[(size_t)n * p.heads * hd + (size_t)(kvh * G + g) * hd + d] = __ddiv_rn(v, s_l[g]);
-    }
-}
-
-template <int G>
-int launch_stream_attention(loom_b200_ctx* ctx, const LbAttnParams& p) {
-    const size_t smem = (size_t)4 * kAsTile * p.hd * sizeof(float) + (size_t)G * p.hd * 8 + (size_t)2 * G * kAsTile * 8;
-    auto kern = lb_attention_stream_kernel<G>;
-    const unsigned bit = 1u << (G == 4 ? 13 : 14);  // (bits 0-7: the cluster kernel, 8-12: the streaming head, 16, 20-27: others)
-    if (!(ctx->func_attr_mask2 & bit)) {
-        LB_CUDA(ctx, cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024));
-        ctx->func_attr_mask2 |= bit;
-    }
-    cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3(p.kv_heads, p.M);
-    cfg.blockDim = dim3(kAsThreads);
-    cfg.dynamicSmemBytes = smem;
-    cfg.stream = ctx->stream;
-    cudaLaunchAttribute attr[1];
-    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    attr[0].val.programmaticStreamSerializationAllowed = 1;
-    cfg.attrs = attr;
-    cfg.numAttrs = ctx->opt_pdl ? 1 : 0;
-    LB_CUDA(ctx, cudaLaunchKernelEx(&cfg, kern, p));
-    ctx->launches++;
-    return 0;
-}
-
-template <int G>
-size_t cluster_smem(const LbAttnParams& p, int S, int* tile_bytes) {
-    const int cmax = (p.msl + S - 1) / S;
-    size_t tiles = (size_t)2 * cmax * p.hd * sizeof(float);
+size_t cluster_smem(const LbAttnParams& p, int S, int rows, int* tile_bytes) {
+    size_t tiles = (size_t)2 * rows * p.hd * sizeof(float);
     const size_t red = (size_t)kAcWarps * G * p.hd * sizeof(double);
     if (red > tiles) tiles = red;
     tiles = (tiles + 127) & ~(size_t)127;
     *tile_bytes = (int)tiles;
     const int dps = p.hd / S;
-    return tiles + (size_t)G * p.hd * 8 + (size_t)G * cmax * 8 + (size_t)S * G * (dps + 2) * 8;
+    return tiles + (size_t)G * p.hd * 8 + (size_t)G * rows * 8 + (size_t)S * G * (dps + 2) * 8;
 }
 
 template <int G>
 int launch_cluster(loom_b200_ctx* ctx, LbAttnParams p, int S, bool probe_only, int* active_clusters) {
     int tile_bytes = 0;
-    const size_t smem = cluster_smem<G>(p, S, &tile_bytes);
-    if (smem > 200 * 1024) return LOOM_B200_ERR_UNSUPPORTED;
-    p.tile = tile_bytes;
     p.max_chunk = (p.msl + S - 1) / S;
+    size_t smem = cluster_smem<G>(p, S, p.max_chunk, &tile_bytes);
+    const bool one = smem <= kAcSmem;
+    if (!one) {
+        p.max_chunk = kAcChunk;
+        smem = cluster_smem<G>(p, S, kAcChunk, &tile_bytes);
+    }
+    p.tile = tile_bytes;
     const bool lean = !probe_only && !p.trace && p.M == 1 && p.seq_stride <= 0;
-    auto kern = lean ? lb_attention_cluster_kernel<G, true> : lb_attention_cluster_kernel<G, false>;
-    const unsigned bit = 1u << ((G == 1 ? 0 : G == 2 ? 1 : G == 4 ? 2 : 3) + (lean ? 4 : 0));  // one bit per instantiation, per context (= per device)
-    if (!(ctx->func_attr_mask2 & bit)) {
-        LB_CUDA(ctx, cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024));
+    auto kern = lean ? (one ? lb_attention_cluster_kernel<G, true, true> : lb_attention_cluster_kernel<G, true, false>)
+                     : (one ? lb_attention_cluster_kernel<G, false, true> : lb_attention_cluster_kernel<G, false, false>);
+    // one bit per instantiation, per context (= per device)
+    const unsigned bit = 1u << ((G == 1 ? 0 : G == 2 ? 1 : G == 4 ? 2 : 3) + (lean ? 4 : 0) + (one ? 0 : 16));
+    if (!(ctx->func_attr_mask3 & bit)) {
+        LB_CUDA(ctx, cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kAcSmem));
         LB_CUDA(ctx, cudaFuncSetAttribute(kern, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
-        ctx->func_attr_mask2 |= bit;
+        ctx->func_attr_mask3 |= bit;
     }
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(S, p.kv_heads, p.M);
@@ -586,25 +430,23 @@ int dispatch_cluster(loom_b200_ctx* ctx, const LbAttnParams& p, int S, bool prob
 
 }  // namespace
 
-int lb_attention_cluster_size(loom_b200_ctx* ctx, const LbAttnParams& p, bool one_wave) {
+int lb_attention_cluster_size(loom_b200_ctx* ctx, const LbAttnParams& p, int sequences) {
     if ((p.M != 1 && p.seq_stride <= 0) || !p.rope_div || !p.k_new || !p.cache_k_w) return 0;
     if (p.kv_heads <= 0 || p.heads % p.kv_heads != 0) return 0;
     const int G = p.heads / p.kv_heads;
     if (G != 1 && G != 2 && G != 4 && G != 8) return 0;
     if (p.hd % 16 != 0 || p.hd > 128 || p.hd < 16) return 0;
-    // the largest cluster size the device can launch for this shape
+    // the largest cluster size of which the device holds one per KV head and sequence at once
     const int smax = ctx->opt_attn_cluster >= 2 && ctx->opt_attn_cluster < kAcMaxS ? ctx->opt_attn_cluster : kAcMaxS;  // option: 1 = the largest that fits, 2..16 = at most that
+    const int clusters = p.kv_heads * (sequences > 0 ? sequences : 1);
     for (int S = kAcMaxS; S >= 2; S >>= 1) {
         if (S > smax) continue;
         if (p.hd % S != 0) continue;
         int active = 0;
         if (dispatch_cluster(ctx, p, S, true, &active) != 0) continue;
-        // One sequence: only when every KV head's cluster is resident at once (one wave) -- in waves the split kernel is the
-        // faster one (measured at 8 KV heads: 511 against 464 tok/s).  Several sequences launch many clusters anyway and
-        // take whatever size the device can launch: the clusters do not depend on one another.
-        if (one_wave ? (active >= p.kv_heads || (S == 2 && active >= 1)) : active >= 1) return S;
+        if (active >= clusters || (sequences == 0 && S == 2 && active >= 1)) return S;
     }
-    return 0;
+    return sequences > 0 ? 1 : 0;  // more (sequence, KV head) pairs than pairs of SMs: single CTAs, in waves
 }
 
 int lb_launch_attention_cluster(loom_b200_ctx* ctx, const LbAttnParams& pin, int S) {
@@ -614,19 +456,4 @@ int lb_launch_attention_cluster(loom_b200_ctx* ctx, const LbAttnParams& pin, int
     int rc = dispatch_cluster(ctx, p, S, false, nullptr);
     if (rc == LOOM_B200_ERR_UNSUPPORTED) return lb_fail(ctx, rc, "attention (cluster): shape not supported");
     return rc;
-}
-
-// A pass of several sequences through the streaming kernel: head dimension 128 (tiles of 64 x 512 B), four or eight query
-// heads per KV head, plain attention (q rotated, the newest K row already in the ring).
-bool lb_attention_stream_supported(const loom_b200_ctx* ctx, const LbAttnParams& p) {
-    if (!ctx->opt_attn_stream || p.hd != 128 || p.kv_heads <= 0 || p.heads % p.kv_heads != 0) return false;
-    const int G = p.heads / p.kv_heads;
-    return G == 4 || G == 8;
-}
-
-int lb_launch_attention_stream(loom_b200_ctx* ctx, const LbAttnParams& pin) {
-    LbAttnParams p = pin;
-    p.status = ctx->status_dev;
-    p.trace = nullptr;
-    return p.heads / p.kv_heads == 4 ? launch_stream_attention<4>(ctx, p) : launch_stream_attention<8>(ctx, p);
 }

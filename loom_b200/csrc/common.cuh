@@ -70,7 +70,8 @@ struct loom_b200_ctx {
     void* argmax_scratch = nullptr;  // per-CTA partial maxima of the greedy argmax
     void* head_scratch = nullptr;    // per-CTA partial maxima and arrival counter of the LM head's greedy tail
     unsigned func_attr_mask = 0;  // kernels whose shared-memory limit was raised on this device
-    unsigned func_attr_mask2 = 0; // the same for the cluster attention instantiations
+    unsigned func_attr_mask2 = 0; // the same for the streaming head
+    unsigned func_attr_mask3 = 0; // the same for the cluster attention instantiations
     int opt_head_stream = 1;      // the LM head streams its rows through shared memory with bulk copies (0 = warp-per-row loads)
     int opt_attn_cluster = 1;     // one-token decoder steps run the attention as a thread-block cluster per KV head (0: off, 1: the largest cluster that fits, 2..16: at most that many CTAs)
     // tuning knobs (loom_b200_ctx_set_option; initial values from LOOM_B200_* environment variables)
@@ -90,7 +91,6 @@ struct loom_b200_ctx {
     int opt_gemm_tile = 0;         // tokens per CTA of the GEMM: 0 = choose, 128 or 256 = force
     int opt_prefill_gemm = 1;      // prompts of 32+ tokens run their projections as token-block GEMMs
     bool gemm_codes_fresh = false;  // a matrix's pre-expanded codes were built since the last GEMM launch
-    int opt_attn_stream = 1;       // a pass of several sequences runs the attention as one streaming CTA per (sequence, KV head)
     int opt_gemv_lean = 1;         // decode-step launches use the GEMV instantiations without the stream-K and general-prologue code
     int opt_tp_fused = 1;          // row-parallel projections under a peer-memory group: the GEMV's epilogue exchanges the partial sums (0: a finalize kernel does)
     int opt_quant_regs = 1;        // the GEMM's quantizer keeps a token's row in registers (0: staged in shared memory)

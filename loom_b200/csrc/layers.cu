@@ -104,9 +104,10 @@ void lb_mha_release(loom_b200_mha* m) {
         if (p) cudaFree(p);
 }
 
-// CTAs per KV head of the cluster attention for this layer's shape (0 = not usable); decided once
-static int mha_cluster_size(loom_b200_mha* m, bool lanes = false) {
-    int& slot = lanes ? m->attn_cluster_lanes : m->attn_cluster;
+// CTAs per (sequence, KV head) of the cluster attention for this layer's shape (0 = not usable); decided once per number of
+// sequences (0: the one sequence of a single-sequence step)
+static int mha_cluster_size(loom_b200_mha* m, int sequences = 0) {
+    int& slot = m->attn_cluster[sequences];
     if (slot < 0) {
         LbAttnParams t = {};
         t.M = 1;
@@ -117,34 +118,16 @@ static int mha_cluster_size(loom_b200_mha* m, bool lanes = false) {
         t.rope_div = m->rope_div;
         t.k_new = m->k_new;
         t.cache_k_w = m->cache_k;
-        slot = m->ctx->opt_attn_cluster ? lb_attention_cluster_size(m->ctx, t, !lanes) : 0;
+        slot = m->ctx->opt_attn_cluster ? lb_attention_cluster_size(m->ctx, t, sequences) : 0;
     }
     return slot;
-}
-
-// A pass of M sequences: the streaming kernel (one CTA per sequence and KV head) when that many CTAs fill a good part of
-// the device or nothing else takes the shape; with few of them (tensor-parallel slices, few sequences) the cluster kernel's
-// sixteen CTAs per (sequence, KV head) are faster (measured at the 8B shape: 64 CTAs 15.4 against 15.7 ms per step on one
-// GPU, 32 CTAs 14.4 against 11.6 ms on two).
-static bool mha_lanes_stream(loom_b200_mha* m, int M) {
-    LbAttnParams t = {};
-    t.heads = m->heads;
-    t.kv_heads = m->kv_heads;
-    t.hd = m->head_dim;
-    if (!lb_attention_stream_supported(m->ctx, t)) return false;
-    return m->kv_heads * M >= 48 || mha_cluster_size(m, true) == 0;
 }
 
 static bool mha_folds_rope(loom_b200_mha* m, const LbMhaStepArgs& a) {
     // one token of one sequence: RoPE goes into the attention kernel; one token of each of several sequences: only the
     // cluster kernel knows that layout, otherwise RoPE runs as a launch of its own
     if (!a.fold_rope || m->q_norm || m->k_norm || !m->ctx->opt_fold_rope || m->head_dim % 8 != 0) return false;
-    if (a.lanes_pos) {
-        // several sequences: the streaming kernel takes rotated queries and a complete ring (RoPE as a launch of its own)
-        if (mha_lanes_stream(m, a.M)) return false;
-        return mha_cluster_size(m, true) > 0;
-    }
-    return a.M == 1;
+    return a.lanes_pos ? mha_cluster_size(m, a.M) > 0 : a.M == 1;
 }
 
 int lb_mha_qkv_dev(loom_b200_mha* m, const LbMhaStepArgs& a) {
@@ -235,13 +218,12 @@ int lb_mha_attn_dev(loom_b200_mha* m, const LbMhaStepArgs& a) {
         t.rope_div = m->rope_div;
         t.k_new = m->k_new;
         t.cache_k_w = a.lanes_pos ? m->cache_k_base + (size_t)a.lane0 * m->ring_elems : m->cache_k;
-        if (mha_cluster_size(m, a.lanes_pos != nullptr) > 0) {
+        if (const int cluster = mha_cluster_size(m, a.lanes_pos ? a.M : 0)) {
             t.next_k = a.lanes_pos ? nullptr : m->next_k;  // (the prefetch follows one sequence's rings)
             t.next_v = a.lanes_pos ? nullptr : m->next_v;
-            return lb_launch_attention_cluster(ctx, t, mha_cluster_size(m, a.lanes_pos != nullptr));
+            return lb_launch_attention_cluster(ctx, t, cluster);
         }
     }
-    if (a.lanes_pos && !fold_rope && mha_lanes_stream(m, a.M)) return lb_launch_attention_stream(ctx, t);
     return lb_launch_attention(ctx, t);
 }
 
