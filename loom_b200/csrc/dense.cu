@@ -9,6 +9,7 @@ namespace {
 constexpr int kGemvThreads = 256;
 constexpr int kGemvWarps = kGemvThreads / 32;
 constexpr size_t kGemvSmemX = 200 * 1024;
+constexpr int kGemvSmemHalf = 103 * 1024;  // dynamic part of a CTA when two share an SM (228 KB, 1 KB reserved and up to 9.3 KB static each)
 
 // one thread per 16-byte chunk of the source rows
 template <typename WT>
@@ -101,31 +102,25 @@ struct GemvAcc<float> {
     }
 };
 
-// the token columns of a chunk when they live in global memory as rows (routed experts, second product)
+// the same for rows of (token, choice) pairs (routed experts, second product): xw points at the chunks that the lanes of this
+// warp fetched, lane (g, t) the one of token g, zeros where the token did not choose the expert
 template <typename WT>
-__device__ __forceinline__ void step_pairs(GemvAcc<WT>& acc, const uint4& w0, const uint4& w1, const uint8_t* pairs, size_t row_bytes,
-                                           const int* pair, int chunk, int M, int g);
+__device__ __forceinline__ void step_pairs(GemvAcc<WT>& acc, const uint4& w0, const uint4& w1, const uint4* xw, int M, int lane);
 template <>
-__device__ __forceinline__ void step_pairs<__nv_bfloat16>(GemvAcc<__nv_bfloat16>& acc, const uint4& w0, const uint4& w1, const uint8_t* pairs,
-                                                          size_t row_bytes, const int* pair, int chunk, int M, int g) {
-    const int pr = g < M ? pair[g] : -1;
-    uint4 x = make_uint4(0, 0, 0, 0);
-    if (pr >= 0) x = *reinterpret_cast<const uint4*>(pairs + (size_t)pr * row_bytes + (size_t)chunk * 16);
+__device__ __forceinline__ void step_pairs<__nv_bfloat16>(GemvAcc<__nv_bfloat16>& acc, const uint4& w0, const uint4& w1, const uint4* xw, int M, int lane) {
+    const uint4 x = xw[lane];
     mma_bf16(acc.d, w0.x, w1.x, w0.y, w1.y, x.x, x.y);
     mma_bf16(acc.d, w0.z, w1.z, w0.w, w1.w, x.z, x.w);
 }
 template <>
-__device__ __forceinline__ void step_pairs<float>(GemvAcc<float>& acc, const uint4& w0, const uint4& w1, const uint8_t* pairs, size_t row_bytes,
-                                                  const int* pair, int chunk, int M, int g) {
+__device__ __forceinline__ void step_pairs<float>(GemvAcc<float>& acc, const uint4& w0, const uint4& w1, const uint4* xw, int M, int lane) {
     float p[4], q[4], x[4];
     lb_unpack_chunk<float>(w0, p);
     lb_unpack_chunk<float>(w1, q);
 #pragma unroll
     for (int m = 0; m < 8; ++m) {
         if (m >= M) break;
-        const int pr = pair[m];
-        if (pr < 0) continue;
-        lb_unpack_chunk<float>(*reinterpret_cast<const uint4*>(pairs + (size_t)pr * row_bytes + (size_t)chunk * 16), x);
+        lb_unpack_chunk<float>(xw[m * 4 + (lane & 3)], x);
 #pragma unroll
         for (int i = 0; i < 4; ++i) {
             acc.a[0][m] = fmaf(p[i], x[i], acc.a[0][m]);
@@ -134,34 +129,41 @@ __device__ __forceinline__ void step_pairs<float>(GemvAcc<float>& acc, const uin
     }
 }
 
-template <int NB>
-struct GemvBatch {
-    uint4 a[NB][2], b[NB][2];  // [slice][chunk t / t+4], rows g / g+8
-};
-
-// loads NB K slices (first, first + stride, ...; those below n) of a 16-row strip: lane (g, t) takes chunks t, t+4 of rows g, g+8
-template <int NB>
-__device__ __forceinline__ void load_batch(GemvBatch<NB>& w, const uint8_t* strip, int first, int stride, int n, int g, int t) {
-#pragma unroll
-    for (int u = 0; u < NB; ++u) {
-        const int s = first + u * stride;
-        if (s < n) {
-            const uint8_t* p = strip + (size_t)s * kImgBlock + (size_t)t * 128 + (size_t)g * 16;
-            w.a[u][0] = ldg_stream(p);
-            w.a[u][1] = ldg_stream(p + 512);
-            w.b[u][0] = ldg_stream(p + 1024);
-            w.b[u][1] = ldg_stream(p + 1536);
-        }
+// ---- the weight ring: every warp copies the chunks it will multiply itself (16 bytes a lane and copy, so no barrier of the
+// block is needed between the copies and their use), `depth` K slices ahead.  One batch in registers and one in flight (32 KB an
+// SM) left the routed products at half of HBM's rate: a step of eight sequences over 32 experts of 4096 x 1792 (four layers) took
+// 1.53 ms, 1.27 ms with the ring (100 KB an SM); a one-sequence step with gated feed-forwards of 6912 572 and 533 us.  Products
+// whose 16-row strips are fewer than the CTAs that fit are bound by the chain of their input rows, not by this. ----
+constexpr int kRingUnit = kGemvThreads * 16;  // bytes of one 16-byte chunk per thread
+constexpr int kRingMax = 8;
+__device__ __forceinline__ void ring_copy(uint32_t dst, const uint8_t* src) {
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst), "l"(src) : "memory");
+}
+__device__ __forceinline__ void ring_copy_or_zero(uint32_t dst, const uint8_t* src, bool ok) {
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(dst), "l"(src), "r"(ok ? 16 : 0) : "memory");
+}
+__device__ __forceinline__ void ring_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
+// the oldest of `depth` groups has arrived
+__device__ __forceinline__ void ring_wait(int depth) {
+    switch (depth) {
+        case 8: asm volatile("cp.async.wait_group 7;" ::: "memory"); break;
+        case 7: asm volatile("cp.async.wait_group 6;" ::: "memory"); break;
+        case 6: asm volatile("cp.async.wait_group 5;" ::: "memory"); break;
+        case 5: asm volatile("cp.async.wait_group 4;" ::: "memory"); break;
+        case 4: asm volatile("cp.async.wait_group 3;" ::: "memory"); break;
+        case 3: asm volatile("cp.async.wait_group 2;" ::: "memory"); break;
+        case 2: asm volatile("cp.async.wait_group 1;" ::: "memory"); break;
+        default: asm volatile("cp.async.wait_group 0;" ::: "memory"); break;
     }
 }
 
 // KW warps share a strip of 16 rows by K slices, 8/KW strips run side by side in a CTA.
 template <typename WT, int PRO, int EPI>
-__global__ void __launch_bounds__(kGemvThreads, 2) lb_dense_gemv_kernel(const LbDenseGemv p, int Mp_launch, int KW, bool vec) {
+__global__ void __launch_bounds__(kGemvThreads, 2) lb_dense_gemv_kernel(const LbDenseGemv p, int Mp_launch, int KW, bool vec, int ring_off, int depth) {
     extern __shared__ __align__(16) uint8_t smem[];
     constexpr int C = LbElem<WT>::kChunk;
     constexpr bool kDual = EPI == LB_DEPI_GLU || EPI == LB_DEPI_SILU;
-    constexpr int NB = kDual ? 1 : 2;
+    constexpr int kUnits = kDual ? 8 : PRO == LB_DPRO_PAIRS ? 6 : 4;  // 16-byte chunks of a thread per K slice
     __shared__ float red[kGemvWarps][128];
     __shared__ float red2[kDual ? kGemvWarps : 1][128];
     __shared__ float s_stat[kGemvWarps];
@@ -176,15 +178,63 @@ __global__ void __launch_bounds__(kGemvThreads, 2) lb_dense_gemv_kernel(const Lb
     uint4* xs = reinterpret_cast<uint4*>(smem);  // [chunk][Mp]
     const uint8_t *w1 = p.w, *w2 = p.w2;
 
-    // the weights do not depend on earlier launches: the first batch is requested before the dependency wait
-    GemvBatch<NB> cur, cur2;
     int strip = (int)blockIdx.x * SP + sp;
+    const int step = (int)gridDim.x * SP;
     auto strip_ptr = [&](const uint8_t* base, int st) { return base + (size_t)(st >> 3) * p.slices * kImgBlock + (size_t)(st & 7) * 2048; };
+    const size_t lane_off = (size_t)t * 128 + (size_t)g * 16;  // lane (g, t) takes chunks t, t+4 of rows g, g+8
+
+    // The lanes of a warp copy 512 consecutive bytes in order (a line whose bytes land in four places costs four writes: the
+    // 656 MB head took 172 us that way) and read them across: the chunk of lane (g, t) lies at t * 8 + (g ^ 2t), which is free
+    // of bank conflicts both ways.
+    const uint8_t* ring = smem + ring_off + (size_t)warp * 512;
+    const int at_read = t * 8 + (g ^ (2 * t));
+    const uint32_t ring_x = lb_smem_u32(ring) + (uint32_t)lane * 16;
+    const uint32_t ring_s = lb_smem_u32(ring) + (uint32_t)((lane & 24) + ((lane & 7) ^ (2 * (lane >> 3)))) * 16;
+    // the ring's head: the strip and slice the next copy takes, over all strips of this warp (routed second product: K runs over
+    // the experts of the list one after the other)
+    int* s_route = reinterpret_cast<int*>(smem);  // PAIRS: experts of the list, then their pairs
+    int nact = 1, head_strip = strip, head_sl = kw, head_at = 0, head_slot = 0;
+    auto fetch = [&]() {
+        if (head_strip < strips) {
+            const uint32_t dst = ring_s + (uint32_t)(head_slot * kUnits * kRingUnit);
+            const size_t group = PRO == LB_DPRO_PAIRS ? (size_t)s_route[head_at] * p.group_bytes : 0;
+            const size_t off = (size_t)head_sl * kImgBlock + (size_t)lane * 16;
+            const uint8_t* q = strip_ptr(w1 + group, head_strip) + off;
+            ring_copy(dst, q);
+            ring_copy(dst + kRingUnit, q + 512);
+            ring_copy(dst + 2 * kRingUnit, q + 1024);
+            ring_copy(dst + 3 * kRingUnit, q + 1536);
+            if (kDual) {
+                const uint8_t* q2 = strip_ptr(w2, head_strip) + off;
+                ring_copy(dst + 4 * kRingUnit, q2);
+                ring_copy(dst + 5 * kRingUnit, q2 + 512);
+                ring_copy(dst + 6 * kRingUnit, q2 + 1024);
+                ring_copy(dst + 7 * kRingUnit, q2 + 1536);
+            }
+            if (PRO == LB_DPRO_PAIRS) {
+                const int pr = s_route[kMaxLanesPerPass * kMaxTop + head_at * kMaxLanesPerPass + g];
+                const uint8_t* x = p.pairs + (size_t)(pr < 0 ? 0 : pr) * p.ldp * sizeof(WT) + (size_t)(head_sl * 8 + t) * 16;
+                const uint32_t dx = ring_x + (uint32_t)(head_slot * kUnits * kRingUnit);
+                ring_copy_or_zero(dx + 4 * kRingUnit, x, pr >= 0);
+                ring_copy_or_zero(dx + 5 * kRingUnit, x + 64, pr >= 0);
+            }
+            head_sl += KW;
+            if (head_sl >= p.slices) {
+                head_sl -= p.slices;
+                if (++head_at == nact) {
+                    head_at = 0;
+                    head_sl = kw;
+                    head_strip += step;
+                }
+            }
+        }
+        ring_commit();
+        head_slot = head_slot + 1 == depth ? 0 : head_slot + 1;
+    };
+    // the weights do not depend on earlier launches: the ring is filled before the dependency wait
     constexpr bool kEarly = PRO != LB_DPRO_MOE && PRO != LB_DPRO_PAIRS && !kStage;
-    if (kEarly && strip < strips) {
-        load_batch(cur, strip_ptr(w1, strip), kw, KW, p.slices, g, t);
-        if (kDual) load_batch(cur2, strip_ptr(w2, strip), kw, KW, p.slices, g, t);
-    }
+    if (kEarly)
+        for (int i = 0; i < depth; ++i) fetch();
     lb_pdl_launch_dependents();
     lb_pdl_wait();
 
@@ -260,10 +310,7 @@ __global__ void __launch_bounds__(kGemvThreads, 2) lb_dense_gemv_kernel(const Lb
                 }
             s_n = n;
         }
-        if (strip < strips) {
-            load_batch(cur, strip_ptr(w1, strip), kw, KW, p.slices, g, t);
-            load_batch(cur2, strip_ptr(w2, strip), kw, KW, p.slices, g, t);
-        }
+        for (int i = 0; i < depth; ++i) fetch();
         __syncthreads();
         M = s_n;
         Mp = 1;
@@ -384,65 +431,56 @@ __global__ void __launch_bounds__(kGemvThreads, 2) lb_dense_gemv_kernel(const Lb
 
     if (kStage) return;
 
-    const int nact = PRO == LB_DPRO_PAIRS ? p.list->n : 1;
+    if (PRO == LB_DPRO_PAIRS) {
+        nact = p.list->n;
+        for (int i = tid; i < nact; i += kGemvThreads) s_route[i] = p.list->expert[i];
+        for (int i = tid; i < nact * kMaxLanesPerPass; i += kGemvThreads) {
+            const int m = i % kMaxLanesPerPass;
+            s_route[kMaxLanesPerPass * kMaxTop + i] = m < p.M ? p.list->pair[i / kMaxLanesPerPass][m] : -1;
+        }
+        __syncthreads();
+        for (int i = 0; i < depth; ++i) fetch();
+    }
 
-    for (; strip - sp < strips; strip += (int)gridDim.x * SP) {
+    int slot = 0;
+    for (; strip - sp < strips; strip += step) {
         GemvAcc<WT> acc, acc2;
         acc.zero();
         if (kDual) acc2.zero();
         if (strip < strips) {
-            if (PRO != LB_DPRO_PAIRS) {
-                const uint8_t* s1 = strip_ptr(w1, strip);
-                const uint8_t* s2 = kDual ? strip_ptr(w2, strip) : nullptr;
-                const int next = strip + (int)gridDim.x * SP;
-                for (int s = kw; s < p.slices; s += NB * KW) {
-                    GemvBatch<NB> now = cur, now2;
-                    if (kDual) now2 = cur2;
-                    if (s + NB * KW < p.slices) {
-                        load_batch(cur, s1, s + NB * KW, KW, p.slices, g, t);
-                        if (kDual) load_batch(cur2, s2, s + NB * KW, KW, p.slices, g, t);
-                    } else if (next < strips) {  // the next strip's first batch travels while this strip's sums meet
-                        load_batch(cur, strip_ptr(w1, next), kw, KW, p.slices, g, t);
-                        if (kDual) load_batch(cur2, strip_ptr(w2, next), kw, KW, p.slices, g, t);
-                    }
+            const int total = nact * p.slices;
+            const uint8_t *d1 = strip_ptr(w1, strip) + lane_off, *d2 = kDual ? strip_ptr(w2, strip) + lane_off : nullptr;
+            for (int s = kw; s < total; s += KW) {
+                uint4 w[8];
+                const uint4* rs = reinterpret_cast<const uint4*>(ring + (size_t)slot * kUnits * kRingUnit);
+                if (PRO == LB_DPRO_PAIRS || depth > 0) {
+                    ring_wait(depth);
+                    __syncwarp();  // a lane reads what other lanes fetched
 #pragma unroll
-                    for (int u = 0; u < NB; ++u) {
-                        const int sl = s + u * KW;
-                        if (sl < p.slices) {
-                            const uint4* x0 = xs + (size_t)(sl * 8 + t) * Mp;
-                            acc.step(now.a[u][0], now.b[u][0], x0, Mp, M, g);
-                            acc.step(now.a[u][1], now.b[u][1], x0 + 4 * Mp, Mp, M, g);
-                            if (kDual) {
-                                acc2.step(now2.a[u][0], now2.b[u][0], x0, Mp, M, g);
-                                acc2.step(now2.a[u][1], now2.b[u][1], x0 + 4 * Mp, Mp, M, g);
-                            }
-                        }
+                    for (int u = 0; u < (kDual ? 8 : 4); ++u) w[u] = rs[u * kGemvThreads + at_read];
+                } else {  // the input rows leave no room for a ring
+#pragma unroll
+                    for (int u = 0; u < 4; ++u) {
+                        w[u] = ldg_stream(d1 + (size_t)s * kImgBlock + u * 512);
+                        if (kDual) w[4 + u] = ldg_stream(d2 + (size_t)s * kImgBlock + u * 512);
                     }
                 }
-            } else {
-                // K runs over the experts of the list one after the other
-                const int total = nact * p.slices;
-                const size_t row_bytes = (size_t)p.ldp * sizeof(WT);
-                for (int s = kw; s < total; s += 4 * KW) {
-                    uint4 wa[4][2], wb[4][2];
-                    int at[4], sl[4];
-#pragma unroll
-                    for (int u = 0; u < 4; ++u) {
-                        const int i = s + u * KW < total ? s + u * KW : s;
-                        at[u] = i / p.slices;
-                        sl[u] = i - at[u] * p.slices;
-                        const uint8_t* q = strip_ptr(w1 + (size_t)p.list->expert[at[u]] * p.group_bytes, strip) + (size_t)sl[u] * kImgBlock + (size_t)t * 128 + (size_t)g * 16;
-                        wa[u][0] = ldg_stream(q);
-                        wa[u][1] = ldg_stream(q + 512);
-                        wb[u][0] = ldg_stream(q + 1024);
-                        wb[u][1] = ldg_stream(q + 1536);
+                if (PRO == LB_DPRO_PAIRS) {
+                    step_pairs<WT>(acc, w[0], w[2], rs + 4 * kGemvThreads, p.M, lane);
+                    step_pairs<WT>(acc, w[1], w[3], rs + 5 * kGemvThreads, p.M, lane);
+                } else {
+                    const uint4* x0 = xs + (size_t)(s * 8 + t) * Mp;
+                    acc.step(w[0], w[2], x0, Mp, M, g);
+                    acc.step(w[1], w[3], x0 + 4 * Mp, Mp, M, g);
+                    if (kDual) {
+                        acc2.step(w[4], w[6], x0, Mp, M, g);
+                        acc2.step(w[5], w[7], x0 + 4 * Mp, Mp, M, g);
                     }
-#pragma unroll
-                    for (int u = 0; u < 4; ++u) {
-                        if (s + u * KW >= total) break;
-                        step_pairs<WT>(acc, wa[u][0], wb[u][0], p.pairs, row_bytes, p.list->pair[at[u]], sl[u] * 8 + t, p.M, g);
-                        step_pairs<WT>(acc, wa[u][1], wb[u][1], p.pairs, row_bytes, p.list->pair[at[u]], sl[u] * 8 + t + 4, p.M, g);
-                    }
+                }
+                if (PRO == LB_DPRO_PAIRS || depth > 0) {
+                    slot = slot + 1 == depth ? 0 : slot + 1;
+                    __syncwarp();  // every lane has read the slot that is filled again
+                    fetch();
                 }
             }
         }
@@ -496,7 +534,18 @@ int gemv_launch(loom_b200_ctx* ctx, const LbDenseGemv& pin) {
     if (PRO == LB_DPRO_MOE) smem += (size_t)p.M * p.experts * 4 + (size_t)p.M * p.top * 4;
     if (PRO == LB_DPRO_GATED) smem = rows_smem + (size_t)Mp * (p.K / p.head_dim) * 4;
     if (smem > kGemvSmemX + 16 * 1024) return lb_fail(ctx, LOOM_B200_ERR_UNSUPPORTED, "dense_gemv: %d tokens of %d columns need %zu B of shared memory", p.M, p.K, smem);
-    if (smem > 48 * 1024) LB_BIG_SMEM(ctx, (lb_dense_gemv_kernel<WT, PRO, EPI>), kGemvSmemX + 16 * 1024);
+    // the weight ring takes what the input rows leave: of half an SM's shared memory if that is room for two slices, else of all
+    constexpr bool kPairs = PRO == LB_DPRO_PAIRS;
+    constexpr int kSlot = (EPI == LB_DEPI_GLU || EPI == LB_DEPI_SILU ? 8 : kPairs ? 6 : 4) * kRingUnit;
+    int depth = 0;
+    const int ring_off = kPairs ? kMaxLanesPerPass * kMaxTop * (1 + kMaxLanesPerPass) * 4 : lb_round_up((int)smem, 16);
+    if (EPI != LB_DEPI_STAGE) {
+        const int room = ring_off + 2 * kSlot <= kGemvSmemHalf ? kGemvSmemHalf : (int)kGemvSmemX + 16 * 1024;
+        depth = room > ring_off ? (room - ring_off) / kSlot : 0;
+        if (depth > kRingMax) depth = kRingMax;
+        smem = (size_t)ring_off + (size_t)depth * kSlot;
+    }
+    if (smem > 36 * 1024) LB_BIG_SMEM(ctx, (lb_dense_gemv_kernel<WT, PRO, EPI>), kGemvSmemX + 16 * 1024);
     int gx = lb_ceil_div(strips, SP), gy = 1, share = cap;
     if (EPI == LB_DEPI_STAGE) {
         gx = share = p.M;
@@ -506,7 +555,7 @@ int gemv_launch(loom_b200_ctx* ctx, const LbDenseGemv& pin) {
         if (share < 1) share = 1;
     }
     if (gx > share) gx = lb_ceil_div(gx, lb_ceil_div(gx, share));  // equal numbers of strips per CTA
-    LB_LAUNCH(ctx, (lb_dense_gemv_kernel<WT, PRO, EPI>), dim3(gx, gy), dim3(kGemvThreads), smem, p, Mp, KW, vec);
+    LB_LAUNCH(ctx, (lb_dense_gemv_kernel<WT, PRO, EPI>), dim3(gx, gy), dim3(kGemvThreads), smem, p, Mp, KW, vec, ring_off, depth);
     return 0;
 }
 
