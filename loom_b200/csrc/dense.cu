@@ -235,7 +235,17 @@ __global__ void __launch_bounds__(kGemvThreads, 2) lb_dense_gemv_kernel(const Lb
     constexpr bool kEarly = PRO != LB_DPRO_MOE && PRO != LB_DPRO_PAIRS && !kStage;
     if (kEarly)
         for (int i = 0; i < depth; ++i) fetch();
-    lb_pdl_launch_dependents();
+    // nor do the vectors of the prologue, which a layer's weights have pushed out of the L2 cache since the last token
+    if (kEarly || kStage) {
+        auto prefetch = [&](const float* v, int n) {
+            if (v)
+                for (int i = tid * 32; i < n; i += kGemvThreads * 32) asm volatile("prefetch.global.L2 [%0];" ::"l"(v + i));
+        };
+        if (PRO == LB_DPRO_NORM || PRO == LB_DPRO_MOE) prefetch(p.gain_w, p.K);
+        if (PRO == LB_DPRO_GATED) prefetch(p.head_w, p.K);
+        if (PRO == LB_DPRO_CONV) prefetch(p.conv_w, p.taps * p.ring_ld);
+    }
+    if (kStage) lb_pdl_launch_dependents();
     lb_pdl_wait();
 
     if (PRO == LB_DPRO_MOE) {
@@ -318,32 +328,104 @@ __global__ void __launch_bounds__(kGemvThreads, 2) lb_dense_gemv_kernel(const Lb
     }
 
     if (PRO == LB_DPRO_STAGED) {
-        for (int i = tid; i < chunks * Mp; i += kGemvThreads) xs[i] = p.staged[i];
+        const int n = chunks * Mp;
+        for (int i0 = tid; i0 < n; i0 += 8 * kGemvThreads) {
+            uint4 v[8];
+#pragma unroll
+            for (int i = 0; i < 8; ++i)
+                if (i0 + i * kGemvThreads < n) v[i] = p.staged[i0 + i * kGemvThreads];
+#pragma unroll
+            for (int i = 0; i < 8; ++i)
+                if (i0 + i * kGemvThreads < n) xs[i0 + i * kGemvThreads] = v[i];
+        }
         __syncthreads();
     } else if (PRO != LB_DPRO_PAIRS) {
-        // ---- input rows: 8/Mp warps per token ----
+        // ---- input rows: 8/Mp warps per token.  This is on the critical path of every step (the weights are on their way), so a
+        // thread asks for all it needs of R chunks at once -- the row, the gate, the convolution's history -- and keeps the row in
+        // registers over the meeting of the sums; only columns beyond those are read again. ----
         const int WPT = kGemvWarps / Mp, m = warp / WPT, wt = warp % WPT, lt = wt * 32 + lane, nt = WPT * 32;
         const bool live = m < M;
         const int tok = !live ? 0 : kStage ? (int)blockIdx.x : PRO == LB_DPRO_MOE ? s_tok[m] : m;
+        int pos = 0;
+        if (PRO == LB_DPRO_CONV && live) pos = p.pos[tok];
         const int src = p.row_idx ? p.row_idx[tok] : tok;
         const float* xr = p.x + (size_t)src * p.ldx;
+        const float* gate_row = PRO == LB_DPRO_GATED ? p.gate + (size_t)tok * p.gate_ld : nullptr;
+        float* conv_ring = PRO == LB_DPRO_CONV ? p.conv_ring + (size_t)(p.lane0 + tok) * p.taps * p.ring_ld : nullptr;
+        constexpr bool kNormed = PRO == LB_DPRO_NORM || PRO == LB_DPRO_CONV || PRO == LB_DPRO_MOE;
+        constexpr int R = PRO == LB_DPRO_CONV || PRO == LB_DPRO_GATED ? 2 : 4;
+        constexpr bool kSide = PRO == LB_DPRO_CONV || PRO == LB_DPRO_GATED;
+        float xc[R][C], side[kSide ? R : 1][C];
+        auto load = [&](int base, bool with_side) {
+#pragma unroll
+            for (int i = 0; i < R; ++i) {
+                const int c = base + i * nt, k0 = c * C;
+#pragma unroll
+                for (int j = 0; j < C; ++j) xc[i][j] = 0.f;
+                if (live && c < chunks && k0 < p.K) lb_load_cols<C>(xr, k0, p.K, vec, xc[i]);
+            }
+            if (PRO == LB_DPRO_GATED && with_side) {
+#pragma unroll
+                for (int i = 0; i < R; ++i) {
+                    const int c = base + i * nt, k0 = c * C;
+                    if (live && c < chunks && k0 < p.K) lb_load_cols<C>(gate_row, k0, p.K, vec, side[i]);
+                }
+            }
+            if (PRO == LB_DPRO_CONV && with_side) {  // what the earlier positions add
+#pragma unroll
+                for (int i = 0; i < R; ++i) {
+                    const int c = base + i * nt, k0 = c * C;
+#pragma unroll
+                    for (int j = 0; j < C; ++j) side[i][j] = 0.f;
+                    if (!live || c >= chunks || k0 >= p.K) continue;
+                    for (int j0 = 0; j0 + 1 < p.taps; j0 += 3) {  // tap j looks back taps - 1 - j positions
+                        float w[3][C], y[3][C];
+#pragma unroll
+                        for (int j = 0; j < 3; ++j) {
+                            const int ps = pos - (p.taps - 1) + j0 + j;
+                            if (j0 + j + 1 < p.taps && ps >= 0) {
+                                lb_load_cols<C>(p.conv_w + (size_t)(j0 + j) * p.ring_ld, k0, p.K, vec, w[j]);
+                                lb_load_cols<C>(conv_ring + (size_t)(ps % p.taps) * p.ring_ld, k0, p.K, vec, y[j]);
+                            }
+                        }
+#pragma unroll
+                        for (int j = 0; j < 3; ++j)
+                            if (j0 + j + 1 < p.taps && pos - (p.taps - 1) + j0 + j >= 0)
+#pragma unroll
+                                for (int e = 0; e < C; ++e) side[i][e] = fmaf(w[j][e], y[j][e], side[i][e]);
+                    }
+                }
+            }
+        };
+        load(lt, true);
         float rstd = 0.f, gain = 1.f;
         float* s_head = nullptr;
-        int heads = 0;
-        if (PRO == LB_DPRO_NORM || PRO == LB_DPRO_CONV || PRO == LB_DPRO_MOE) {
+        // a head of the gated form is one run of lanes of a warp: its sum needs no second reading of the row
+        const int per_head = PRO == LB_DPRO_GATED ? p.head_dim / C : 0;
+        const bool in_warp = PRO == LB_DPRO_GATED && p.head_dim % C == 0 && per_head <= 32 && (per_head & (per_head - 1)) == 0;
+        if (kNormed) {
+            if (p.gain) gain = *p.gain;
             float ss = 0.f;
+#pragma unroll
+            for (int i = 0; i < R; ++i)
+#pragma unroll
+                for (int j = 0; j < C; ++j) ss = fmaf(xc[i][j], xc[i][j], ss);
             if (live)
-                for (int k = lt; k < p.K; k += nt) ss = fmaf(xr[k], xr[k], ss);
+                for (int c = lt + R * nt; c * C < p.K; c += nt) {
+                    float f[C];
+                    lb_load_cols<C>(xr, c * C, p.K, vec, f);
+#pragma unroll
+                    for (int j = 0; j < C; ++j) ss = fmaf(f[j], f[j], ss);
+                }
             ss = lb_warp_sumf(ss);
             if (lane == 0) s_stat[warp] = ss;
             __syncthreads();
             float tot = 0.f;
             for (int i = 0; i < WPT; ++i) tot += s_stat[m * WPT + i];
             rstd = __fdiv_rn(1.f, sqrtf(__fadd_rn(__fdiv_rn(tot, (float)p.K), p.eps)));
-            if (p.gain) gain = *p.gain;
         }
-        if (PRO == LB_DPRO_GATED) {
-            heads = p.K / p.head_dim;
+        if (PRO == LB_DPRO_GATED && !in_warp) {
+            const int heads = p.K / p.head_dim;
             s_head = reinterpret_cast<float*>(smem + (size_t)chunks * Mp * 16) + (size_t)m * heads;
             if (live)
                 for (int h = wt; h < heads; h += WPT) {
@@ -357,74 +439,69 @@ __global__ void __launch_bounds__(kGemvThreads, 2) lb_dense_gemv_kernel(const Lb
                 }
             __syncthreads();
         }
-        const int seq = p.lane0 + tok;
-        int pos = 0;
-        if (PRO == LB_DPRO_CONV && live) pos = p.pos[tok];
-        for (int c = lt; c < chunks; c += nt) {
-            float f[C];
-            const int k0 = c * C;
-            if (live && k0 < p.K) {
-                lb_load_cols<C>(xr, k0, p.K, vec, f);
-                if (PRO == LB_DPRO_NORM || PRO == LB_DPRO_CONV || PRO == LB_DPRO_MOE) {
+        for (int base = lt; base - lane < chunks; base += R * nt) {  // (uniform over a warp: its lanes sum heads together)
+            if (base != lt) load(base, true);
 #pragma unroll
-                    for (int i = 0; i < C; ++i) f[i] = f[i] * rstd * gain;
-                    if (p.gain_w) {
+            for (int i = 0; i < R; ++i) {
+                const int c = base + i * nt, k0 = c * C;
+                float (&f)[C] = xc[i];
+                float head_rstd = 0.f;
+                if (PRO == LB_DPRO_GATED && in_warp) {
+                    float ss = 0.f;
+#pragma unroll
+                    for (int j = 0; j < C; ++j) ss = fmaf(f[j], f[j], ss);
+                    for (int o = per_head >> 1; o > 0; o >>= 1) ss += __shfl_xor_sync(0xffffffffu, ss, o);
+                    head_rstd = __fdiv_rn(1.f, sqrtf(__fadd_rn(__fdiv_rn(ss, (float)p.head_dim), p.eps)));
+                }
+                if (c >= chunks) continue;
+                if (live && k0 < p.K) {
+                    if (kNormed) {
+#pragma unroll
+                        for (int j = 0; j < C; ++j) f[j] = f[j] * rstd * gain;
+                        if (p.gain_w) {
+                            float w[C];
+                            lb_load_cols<C>(p.gain_w, k0, p.K, vec, w);
+#pragma unroll
+                            for (int j = 0; j < C; ++j) f[j] *= w[j];
+                        }
+                        if (PRO == LB_DPRO_NORM && p.x_out && (kStage || blockIdx.x == 0)) {
+#pragma unroll
+                            for (int j = 0; j < C; ++j)
+                                if (k0 + j < p.K) p.x_out[(size_t)tok * p.ldx + k0 + j] = f[j];
+                        }
+                    }
+                    if (PRO == LB_DPRO_MOE) {
+#pragma unroll
+                        for (int j = 0; j < C; ++j) f[j] *= s_w[m];
+                    }
+                    if (PRO == LB_DPRO_GATED) {
+                        float hw[C];
+                        lb_load_cols<C>(p.head_w, k0, p.K, vec, hw);
+#pragma unroll
+                        for (int j = 0; j < C; ++j) {
+                            const float hs = in_warp ? head_rstd : k0 + j < p.K ? s_head[(k0 + j) / p.head_dim] : 0.f;
+                            if (k0 + j < p.K) f[j] = f[j] * hs * hw[j] * (p.gate_sigmoid ? lb_sigmoidf(side[i][j]) : lb_siluf(side[i][j]));
+                        }
+                    }
+                    if (PRO == LB_DPRO_CONV) {
                         float w[C];
-                        lb_load_cols<C>(p.gain_w, k0, p.K, vec, w);
+                        lb_load_cols<C>(p.conv_w + (size_t)(p.taps - 1) * p.ring_ld, k0, p.K, vec, w);
+                        float* slot = conv_ring + (size_t)(pos % p.taps) * p.ring_ld + k0;  // no CTA of this launch reads this slot
 #pragma unroll
-                        for (int i = 0; i < C; ++i) f[i] *= w[i];
+                        for (int j = 0; j < C; ++j) {
+                            if ((kStage || blockIdx.x == 0) && k0 + j < p.K) slot[j] = f[j];
+                            f[j] += fmaf(w[j], f[j], side[i][j]);
+                        }
                     }
-                    if (PRO == LB_DPRO_NORM && p.x_out && (kStage || blockIdx.x == 0)) {
+                } else {
 #pragma unroll
-                        for (int i = 0; i < C; ++i)
-                            if (k0 + i < p.K) p.x_out[(size_t)tok * p.ldx + k0 + i] = f[i];
-                    }
+                    for (int j = 0; j < C; ++j) f[j] = 0.f;
                 }
-                if (PRO == LB_DPRO_MOE) {
-#pragma unroll
-                    for (int i = 0; i < C; ++i) f[i] *= s_w[m];
-                }
-                if (PRO == LB_DPRO_GATED) {
-                    float gt[C], hw[C];
-                    lb_load_cols<C>(p.gate + (size_t)tok * p.gate_ld, k0, p.K, vec, gt);
-                    lb_load_cols<C>(p.head_w, k0, p.K, vec, hw);
-#pragma unroll
-                    for (int i = 0; i < C; ++i) {
-                        const int k = k0 + i, h = k / p.head_dim;
-                        if (k < p.K) f[i] = f[i] * s_head[h] * hw[i] * (p.gate_sigmoid ? lb_sigmoidf(gt[i]) : lb_siluf(gt[i]));
-                    }
-                }
-                if (PRO == LB_DPRO_CONV) {
-                    float* ring = p.conv_ring + (size_t)seq * p.taps * p.ring_ld;
-                    float a[C], w[C], y[C];
-#pragma unroll
-                    for (int i = 0; i < C; ++i) a[i] = 0.f;
-                    for (int j = 0; j + 1 < p.taps; ++j) {  // tap j looks back taps - 1 - j positions
-                        const int ps = pos - (p.taps - 1) + j;
-                        if (ps < 0) continue;
-                        lb_load_cols<C>(p.conv_w + (size_t)j * p.ring_ld, k0, p.K, vec, w);
-                        lb_load_cols<C>(ring + (size_t)(ps % p.taps) * p.ring_ld, k0, p.K, vec, y);
-#pragma unroll
-                        for (int i = 0; i < C; ++i) a[i] = fmaf(w[i], y[i], a[i]);
-                    }
-                    lb_load_cols<C>(p.conv_w + (size_t)(p.taps - 1) * p.ring_ld, k0, p.K, vec, w);
-                    float* slot = ring + (size_t)(pos % p.taps) * p.ring_ld + k0;  // no CTA of this launch reads this slot
-#pragma unroll
-                    for (int i = 0; i < C; ++i) {
-                        a[i] = fmaf(w[i], f[i], a[i]);
-                        if ((kStage || blockIdx.x == 0) && k0 + i < p.K) slot[i] = f[i];
-                        f[i] += a[i];
-                    }
-                }
-            } else {
-#pragma unroll
-                for (int i = 0; i < C; ++i) f[i] = 0.f;
+                if (kStage)
+                    p.staged[(size_t)c * Mp_launch + tok] = lb_pack_chunk<WT>(f);
+                else
+                    xs[(size_t)c * Mp + m] = lb_pack_chunk<WT>(f);
             }
-            if (kStage) {
-                p.staged[(size_t)c * Mp_launch + tok] = lb_pack_chunk<WT>(f);
-                continue;
-            }
-            xs[(size_t)c * Mp + m] = lb_pack_chunk<WT>(f);
         }
         __syncthreads();
     }
@@ -442,8 +519,17 @@ __global__ void __launch_bounds__(kGemvThreads, 2) lb_dense_gemv_kernel(const Lb
         for (int i = 0; i < depth; ++i) fetch();
     }
 
+    // The next launch may start once this one's input rows are made, not before: its CTAs fetch weights as soon as they sit on an SM,
+    // in front of this launch's own.  One sequence, Zitupel of 2560: 538 us a step so, 561 when told at the start, 564 after the
+    // products, 580 at the end; two float32 sequences 219, 232, 222, 218.
+    lb_pdl_launch_dependents();
     int slot = 0;
     for (; strip - sp < strips; strip += step) {
+        // the residual rows are asked for before the products (two strips at most a CTA: one element a thread)
+        float before = 0.f;
+        const int brow = (strip - sp + (tid >> 7)) * 16 + ((tid & 127) >> 3);
+        const bool early_res = EPI == LB_DEPI_RESID && SP <= 2;
+        if (early_res && tid < SP * 128 && (tid & 7) < M && brow < p.rows) before = (p.res ? p.res : p.out)[(size_t)(tid & 7) * p.ldo + brow];
         GemvAcc<WT> acc, acc2;
         acc.zero();
         if (kDual) acc2.zero();
@@ -500,7 +586,7 @@ __global__ void __launch_bounds__(kGemvThreads, 2) lb_dense_gemv_kernel(const Lb
             if (EPI == LB_DEPI_F32) p.out[(size_t)m * p.ldo + row] = v;
             if (EPI == LB_DEPI_RESID) {
                 const size_t at = (size_t)m * p.ldo + row;
-                p.out[at] = fmaf(p.mult, v, p.res_mult * (p.res ? p.res : p.out)[at]);
+                p.out[at] = fmaf(p.mult, v, p.res_mult * (early_res ? before : (p.res ? p.res : p.out)[at]));
             }
             if (EPI == LB_DEPI_GELU) p.out[(size_t)m * p.ldo + row] = lb_gelu_erff(v);
             if (EPI == LB_DEPI_SILU) p.out[(size_t)m * p.ldo + row] = lb_siluf(v) * u;
