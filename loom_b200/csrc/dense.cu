@@ -683,80 +683,190 @@ int gemv_dispatch(loom_b200_ctx* ctx, int pro, int epi, const LbDenseGemv& p) {
 }
 
 // ---- token-block GEMM with plain fused multiply-adds (32-bit floats) -------------------------------------------
+//
+// Bound by the multiply-adds (74 TFLOP/s) once the loads are hidden: K slices arrive by asynchronous copies, two ahead, in the
+// image's own order; a thread owns 8 tokens x 4 rows and multiplies two columns at a time (packed multiply-adds on register pairs
+// as they were loaded), 12 shared-memory reads of one wavefront each for 64 of them.  Few tiles are split over K by the CTAs of a
+// cluster, which meet in shared memory in the order of K.  The former kernel (2 x 8 per thread, one slice at a time between two
+// barriers) took 159 us for 333 tokens x 1024 rows x 2816 columns, this one 69 us (gate and up of 2816 together 145 and 127 us).
 
-constexpr int kSimtTile = 64;
+constexpr int kSimtTile = 64, kSimtThreads = 128, kSimtStages = 3, kSimtHalf = kSimtTile * 128, kSimtLd = kSimtTile + 4;
 
+__device__ __forceinline__ uint32_t simt_rank() {
+    uint32_t r;
+    asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(r));
+    return r;
+}
+__device__ __forceinline__ float4 simt_peer(uint32_t addr, uint32_t rank) {
+    uint32_t a;
+    float4 v;
+    asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(a) : "r"(addr), "r"(rank));
+    asm volatile("ld.shared::cluster.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "r"(a) : "memory");
+    return v;
+}
+// a 16-byte chunk as pairs of floats
+template <typename WT>
+__device__ __forceinline__ void simt_pairs(const uint8_t* p, uint64_t* f);
+template <>
+__device__ __forceinline__ void simt_pairs<float>(const uint8_t* p, uint64_t* f) {
+    const ulonglong2 v = *reinterpret_cast<const ulonglong2*>(p);
+    f[0] = v.x;
+    f[1] = v.y;
+}
+template <>
+__device__ __forceinline__ void simt_pairs<__nv_bfloat16>(const uint8_t* p, uint64_t* f) {
+    float v[8];
+    lb_unpack_chunk<__nv_bfloat16>(*reinterpret_cast<const uint4*>(p), v);
+#pragma unroll
+    for (int i = 0; i < 4; ++i) f[i] = lb_pack2(v[2 * i], v[2 * i + 1]);
+}
+
+// grid: (row tiles x S, token tiles), clusters of S CTAs along x
 template <typename WT, int EPI>
-__global__ void __launch_bounds__(256) lb_dense_gemm_simt_kernel(const LbDenseGemm p) {
-    constexpr int C = LbElem<WT>::kChunk;
+__global__ void __launch_bounds__(kSimtThreads, EPI == LB_DEPI_GLU || EPI == LB_DEPI_SILU ? 2 : 3) lb_dense_gemm_simt_kernel(const LbDenseGemm p, int S) {
+    constexpr int P = LbElem<WT>::kChunk / 2;
     constexpr bool kDual = EPI == LB_DEPI_GLU || EPI == LB_DEPI_SILU;
-    __shared__ __align__(16) uint8_t sa[8192], sb[8192], sb2[kDual ? 8192 : 16];
+    constexpr int kParts = kDual ? 3 : 2;
+    extern __shared__ __align__(16) uint8_t smem[];
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    const uint32_t rank = S > 1 ? simt_rank() : 0;
+    const int row0 = (int)(blockIdx.x / S) * kSimtTile, tok0 = blockIdx.y * kSimtTile;
     lb_pdl_launch_dependents();
     lb_pdl_wait();
-    const int tid = threadIdx.x, tl = tid & 31, rg = tid >> 5;
-    const int row0 = blockIdx.x * kSimtTile, tok0 = blockIdx.y * kSimtTile;
     const uint8_t *w = p.w, *w2 = p.w2;
     if (p.nblocks) {
-        if (tok0 / kImgRows >= *p.nblocks) return;
+        if (tok0 / kImgRows >= *p.nblocks) return;  // (the whole cluster)
         const size_t off = (size_t)p.block_group[tok0 / kImgRows] * p.group_bytes;
         w += off;
         w2 += kDual ? off : 0;
     }
-    float acc[2][8], acc2[2][8];
-#pragma unroll
-    for (int i = 0; i < 2; ++i)
-#pragma unroll
-        for (int j = 0; j < 8; ++j) acc[i][j] = acc2[i][j] = 0.f;
     const size_t abase = (size_t)(tok0 >> 7) * p.slices * kImgBlock + (size_t)((tok0 & 127) >> 3) * 1024;
     const size_t bbase = (size_t)(row0 >> 7) * p.slices * kImgBlock + (size_t)((row0 & 127) >> 3) * 1024;
-    for (int s = 0; s < p.slices; ++s) {
-        __syncthreads();
-        for (int i = tid; i < 512; i += 256) {
-            reinterpret_cast<uint4*>(sa)[i] = *reinterpret_cast<const uint4*>(p.x + abase + (size_t)s * kImgBlock + (size_t)i * 16);
-            reinterpret_cast<uint4*>(sb)[i] = *reinterpret_cast<const uint4*>(w + bbase + (size_t)s * kImgBlock + (size_t)i * 16);
-            if (kDual) reinterpret_cast<uint4*>(sb2)[i] = *reinterpret_cast<const uint4*>(w2 + bbase + (size_t)s * kImgBlock + (size_t)i * 16);
+    const int first = p.slices * (int)rank / S, last = p.slices * ((int)rank + 1) / S;
+    const uint32_t base = lb_smem_u32(smem);
+    auto fetch = [&](int s) {
+        if (s < last) {
+            const uint32_t dst = base + (uint32_t)((s - first) % kSimtStages * kParts * kSimtHalf);
+            const size_t off = (size_t)s * kImgBlock;
+#pragma unroll
+            for (int i = 0; i < kSimtHalf / 16 / kSimtThreads; ++i) {
+                const int at = (tid + i * kSimtThreads) * 16;
+                ring_copy(dst + at, p.x + abase + off + at);
+                ring_copy(dst + kSimtHalf + at, w + bbase + off + at);
+                if (kDual) ring_copy(dst + 2 * kSimtHalf + at, w2 + bbase + off + at);
+            }
         }
-        __syncthreads();
+        ring_commit();
+    };
+    // tokens tq + 8 i, rows rq + 8 j + 32 (warp / 2)
+    const int tq = (lane >> 3) + 4 * (warp & 1), rq = lane & 7, rh = warp >> 1;
+    uint64_t acc[8][4], acc2[kDual ? 8 : 1][4];
+#pragma unroll
+    for (int i = 0; i < 8; ++i)
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+            acc[i][j] = 0;
+            if (kDual) acc2[i][j] = 0;
+        }
+    for (int i = 0; i < kSimtStages - 1; ++i) fetch(first + i);
+    for (int s = first; s < last; ++s) {
+        asm volatile("cp.async.wait_group %0;" ::"n"(kSimtStages - 2) : "memory");
+        __syncthreads();  // slice s is there for everyone, and everyone is done with the slot that is filled next
+        fetch(s + kSimtStages - 1);
+        const uint8_t* sa = smem + (s - first) % kSimtStages * kParts * kSimtHalf;
+        const uint8_t* xa = sa + tq * 16;
+        const uint8_t* wa = sa + kSimtHalf + rh * 4096 + rq * 16;
+#pragma unroll 2
         for (int c = 0; c < 8; ++c) {
-            float a0[C], a1[C], b[C];
-            lb_unpack_chunk<WT>(*reinterpret_cast<const uint4*>(sa + (tl >> 3) * 1024 + c * 128 + (tl & 7) * 16), a0);
-            lb_unpack_chunk<WT>(*reinterpret_cast<const uint4*>(sa + ((tl >> 3) + 4) * 1024 + c * 128 + (tl & 7) * 16), a1);
+            uint64_t a[8][P], b[4][P];
 #pragma unroll
-            for (int j = 0; j < 8; ++j) {
-                lb_unpack_chunk<WT>(*reinterpret_cast<const uint4*>(sb + rg * 1024 + c * 128 + j * 16), b);
+            for (int i = 0; i < 8; ++i) simt_pairs<WT>(xa + i * 1024 + c * 128, a[i]);
 #pragma unroll
-                for (int i = 0; i < C; ++i) {
-                    acc[0][j] = fmaf(a0[i], b[i], acc[0][j]);
-                    acc[1][j] = fmaf(a1[i], b[i], acc[1][j]);
-                }
-                if (kDual) {
-                    lb_unpack_chunk<WT>(*reinterpret_cast<const uint4*>(sb2 + rg * 1024 + c * 128 + j * 16), b);
+            for (int j = 0; j < 4; ++j) simt_pairs<WT>(wa + j * 1024 + c * 128, b[j]);
 #pragma unroll
-                    for (int i = 0; i < C; ++i) {
-                        acc2[0][j] = fmaf(a0[i], b[i], acc2[0][j]);
-                        acc2[1][j] = fmaf(a1[i], b[i], acc2[1][j]);
-                    }
-                }
+            for (int h = 0; h < P; ++h)
+#pragma unroll
+                for (int i = 0; i < 8; ++i)
+#pragma unroll
+                    for (int j = 0; j < 4; ++j) acc[i][j] = lb_fma2(a[i][h], b[j][h], acc[i][j]);
+            if (kDual) {
+#pragma unroll
+                for (int j = 0; j < 4; ++j) simt_pairs<WT>(wa + kSimtHalf + j * 1024 + c * 128, b[j]);
+#pragma unroll
+                for (int h = 0; h < P; ++h)
+#pragma unroll
+                    for (int i = 0; i < 8; ++i)
+#pragma unroll
+                        for (int j = 0; j < 4; ++j) acc2[i][j] = lb_fma2(a[i][h], b[j][h], acc2[i][j]);
             }
         }
     }
+    asm volatile("cp.async.wait_group 0;" ::: "memory");
+    __syncthreads();
+    // the sums go through shared memory: eight consecutive rows of a token are one thread's to write
+    float* tile = reinterpret_cast<float*>(smem);  // [64 tokens][64 rows], a second one for the second product
 #pragma unroll
-    for (int i = 0; i < 2; ++i) {
-        const int tok = tok0 + tl + 32 * i, r = row0 + rg * 8;
+    for (int i = 0; i < 8; ++i)
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+            const int at = (tq + 8 * i) * kSimtLd + rq + 8 * j + 32 * rh;
+            float lo, hi;
+            lb_unpack2(acc[i][j], lo, hi);
+            tile[at] = lo + hi;
+            if (kDual) {
+                lb_unpack2(acc2[i][j], lo, hi);
+                tile[kSimtTile * kSimtLd + at] = lo + hi;
+            }
+        }
+    if (S > 1)
+        asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
+    else
+        __syncthreads();
+    const int per = 512 / S;  // (token, eight rows) pairs of a CTA
+    for (int idx = (int)rank * per + tid; idx < ((int)rank + 1) * per; idx += kSimtThreads) {
+        const int tk = idx >> 3, r8 = (idx & 7) * 8;
+        float v[8], u[8];
+#pragma unroll
+        for (int d = 0; d < (kDual ? 2 : 1); ++d) {
+            float* f = d ? u : v;
+            const uint32_t at = base + (uint32_t)(d * kSimtTile * kSimtLd + tk * kSimtLd + r8) * 4;
+#pragma unroll
+            for (int j = 0; j < 8; ++j) f[j] = 0.f;
+            for (int q = 0; q < S; ++q) {
+                float4 lo, hi;
+                if (S > 1) {
+                    lo = simt_peer(at, (uint32_t)q);
+                    hi = simt_peer(at + 16, (uint32_t)q);
+                } else {
+                    const float4* o = reinterpret_cast<const float4*>(tile + d * kSimtTile * kSimtLd + tk * kSimtLd + r8);
+                    lo = o[0];
+                    hi = o[1];
+                }
+                f[0] += lo.x;
+                f[1] += lo.y;
+                f[2] += lo.z;
+                f[3] += lo.w;
+                f[4] += hi.x;
+                f[5] += hi.y;
+                f[6] += hi.z;
+                f[7] += hi.w;
+            }
+        }
+        const int tok = tok0 + tk, r = row0 + r8;
         if (!p.nblocks && tok >= p.tokens) continue;
         if (EPI == LB_DEPI_F32 || EPI == LB_DEPI_RESID) {
             if (r >= p.ldo) continue;
             float* o = p.out + (size_t)tok * p.ldo + r;
 #pragma unroll
-            for (int j = 0; j < 8; ++j) o[j] = EPI == LB_DEPI_F32 ? acc[i][j] : fmaf(p.mult, acc[i][j], p.res_mult * o[j]);
+            for (int j = 0; j < 8; ++j) o[j] = EPI == LB_DEPI_F32 ? v[j] : fmaf(p.mult, v[j], p.res_mult * o[j]);
         } else {
             float f[8];
 #pragma unroll
             for (int j = 0; j < 8; ++j) {
-                f[j] = acc[i][j];
-                if (EPI == LB_DEPI_GELU) f[j] = lb_gelu_erff(acc[i][j]);
-                if (EPI == LB_DEPI_GLU) f[j] = lb_clamped_glu(acc[i][j], acc2[i][j], p.limit);
-                if (EPI == LB_DEPI_SILU) f[j] = lb_siluf(acc[i][j]) * acc2[i][j];
+                f[j] = v[j];
+                if (EPI == LB_DEPI_GELU) f[j] = lb_gelu_erff(v[j]);
+                if (EPI == LB_DEPI_GLU) f[j] = lb_clamped_glu(v[j], u[j], p.limit);
+                if (EPI == LB_DEPI_SILU) f[j] = lb_siluf(v[j]) * u[j];
             }
             if (EPI == LB_DEPI_HEADS) {
                 if (r < p.rows) *reinterpret_cast<uint4*>(p.img + lb_heads_chunk(tok, r, p.heads, p.head_dim, p.head_chunks)) = lb_pack_chunk<__nv_bfloat16>(f);
@@ -765,27 +875,57 @@ __global__ void __launch_bounds__(256) lb_dense_gemm_simt_kernel(const LbDenseGe
             }
         }
     }
+    if (S > 1)  // a neighbour may still read this CTA's sums
+        asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
+}
+
+template <typename WT, int EPI>
+int gemm_simt_launch(loom_b200_ctx* ctx, const LbDenseGemm& p) {
+    constexpr bool kDual = EPI == LB_DEPI_GLU || EPI == LB_DEPI_SILU;
+    constexpr size_t kSmem = (size_t)kSimtStages * (kDual ? 3 : 2) * kSimtHalf;
+    static_assert(kSmem >= (kDual ? 2 : 1) * kSimtTile * kSimtLd * sizeof(float), "the sums fit the stages");
+    // rows: every 64-row tile that holds a row or a column of the output image's padding
+    const int tiles = lb_ceil_div(p.rows, kSimtTile), blocks = p.nblocks ? p.max_blocks * 2 : lb_ceil_div(p.tokens, kSimtTile);
+    // CTAs that share a tile: as many as the SMs hold at once (two or three CTAs each), four slices each at least
+    int S = 1;
+    while (S < 8 && (long long)tiles * blocks * S * 2 <= (kDual ? 2ll : 3ll) * ctx->sm_count && p.slices / (S * 2) >= 4) S *= 2;
+    LB_BIG_SMEM(ctx, (lb_dense_gemm_simt_kernel<WT, EPI>), kSmem);
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(tiles * S, blocks);
+    cfg.blockDim = dim3(kSimtThreads);
+    cfg.dynamicSmemBytes = kSmem;
+    cfg.stream = ctx->stream;
+    cudaLaunchAttribute attr[2];
+    int n = 0;
+    if (S > 1) {
+        attr[n].id = cudaLaunchAttributeClusterDimension;
+        attr[n].val.clusterDim.x = S;
+        attr[n].val.clusterDim.y = attr[n].val.clusterDim.z = 1;
+        ++n;
+    }
+    if (ctx->opt_pdl) {
+        attr[n].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+        attr[n].val.programmaticStreamSerializationAllowed = 1;
+        ++n;
+    }
+    cfg.attrs = attr;
+    cfg.numAttrs = n;
+    LB_CUDA(ctx, cudaLaunchKernelEx(&cfg, lb_dense_gemm_simt_kernel<WT, EPI>, p, S));
+    ctx->launches++;
+    return 0;
 }
 
 template <typename WT>
 int gemm_simt(loom_b200_ctx* ctx, int epi, const LbDenseGemm& p) {
-    // rows: every 64-row tile that holds a row or a column of the output image's padding
-    const int rows = lb_round_up(p.rows, kSimtTile);
-    const int blocks = p.nblocks ? p.max_blocks * 2 : lb_ceil_div(p.tokens, kSimtTile);
-    const dim3 grid(rows / kSimtTile, blocks);
-#define LB_CASE(E)                                                                           \
-    if (epi == E) {                                                                          \
-        LB_LAUNCH(ctx, (lb_dense_gemm_simt_kernel<WT, E>), grid, dim3(256), 0, p);           \
-        return 0;                                                                            \
+    switch (epi) {
+        case LB_DEPI_F32: return gemm_simt_launch<WT, LB_DEPI_F32>(ctx, p);
+        case LB_DEPI_RESID: return gemm_simt_launch<WT, LB_DEPI_RESID>(ctx, p);
+        case LB_DEPI_GELU: return gemm_simt_launch<WT, LB_DEPI_GELU>(ctx, p);
+        case LB_DEPI_GLU: return gemm_simt_launch<WT, LB_DEPI_GLU>(ctx, p);
+        case LB_DEPI_SILU: return gemm_simt_launch<WT, LB_DEPI_SILU>(ctx, p);
+        case LB_DEPI_IMG: return gemm_simt_launch<WT, LB_DEPI_IMG>(ctx, p);
+        case LB_DEPI_HEADS: return gemm_simt_launch<WT, LB_DEPI_HEADS>(ctx, p);
     }
-    LB_CASE(LB_DEPI_F32)
-    LB_CASE(LB_DEPI_RESID)
-    LB_CASE(LB_DEPI_GELU)
-    LB_CASE(LB_DEPI_GLU)
-    LB_CASE(LB_DEPI_SILU)
-    LB_CASE(LB_DEPI_IMG)
-    LB_CASE(LB_DEPI_HEADS)
-#undef LB_CASE
     return lb_fail(ctx, LOOM_B200_ERR_UNSUPPORTED, "dense_gemm: epilogue %d is not built", epi);
 }
 

@@ -1,0 +1,47 @@
+"""The token-block products of a stack where their K slices are shared out: few tiles (a CTA gets a run of slices that may end inside a
+tile, or a cluster splits a tile), ragged rows, columns and tokens, and every epilogue (gate, gelu, residual, image, per-head blocks).
+
+Logits of a whole prompt against the plain oracles; tolerances as in test_gpu_donodra.py and test_gpu_stack.py.
+"""
+import numpy as np
+import pytest
+
+import donodra_oracle as do
+import donodrakit as dk
+import loom_b200
+import stack_oracle as so
+import stackkit as kit
+from loom_b200 import cabi, models
+
+pytestmark = pytest.mark.gpu
+F32, BF16 = cabi.DTYPE_F32, cabi.DTYPE_BF16
+
+
+@pytest.fixture(scope="module")
+def ctx():
+    c = loom_b200.Context(0)
+    yield c
+    c.close()
+
+
+@pytest.mark.parametrize("dtype,tensor_cores", [(F32, 1), (BF16, 1), (BF16, 0)], ids=["f32", "bf16", "bf16-plain"])
+@pytest.mark.parametrize("width,ff,tokens", [(700, 1500, 130), (1100, 2610, 33), (520, 1030, 300), (264, 4100, 9)])
+def test_prompts_over_few_tiles(ctx, dtype, tensor_cores, width, ff, tokens):
+    ctx.set_option("dense_tc", tensor_cores)
+    try:
+        for cfg, weights, oracle, tol in (
+                (dk.config(width, 150, [dk.mlstm(2, 40, 136, 9.0, ff), dk.attention(4, 2, 48, 40, 512, 90.0, 0.15, None)]), dk.random_weights, do.forward, 0.02),
+                (kit.config(width, 150, [kit.latent(3, 48, 56, 72, 0.14, kit.dense(ff)), kit.gla(2, 40, 136, 8.0, None)]), kit.random_weights, so.forward, 0.06)):
+            w = weights(cfg, 7)
+            dec = models.build(ctx, cfg, kit.Weights(w), models.LoadOptions(dtype, 512, 1))
+            tok = np.random.default_rng(tokens).integers(0, 150, tokens).astype(np.int32)
+            want, _ = oracle(cfg, w, tok)
+            first = dec.extend(tok, range(tokens))
+            e = kit.error(first, want)
+            tol = 2e-5 if dtype == F32 else tol
+            assert np.quantile(e, 0.9) < tol and e.max() < 5 * tol
+            dec.reset()
+            assert np.array_equal(dec.extend(tok, range(tokens)), first)  # whoever arrives last adds in the same order
+            dec.close()
+    finally:
+        ctx.set_option("dense_tc", 1)
