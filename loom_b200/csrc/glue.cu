@@ -107,6 +107,42 @@ __global__ void lb_rope_kernel(const LbRopeParams p) {
     lb_trace(p.trace, 5);
 }
 
+// The same for a token block without per-head norms: one CTA per token computes the token's hd/2 angles once for all heads (a
+// float64 division, sine and cosine each; one CTA per head repeated them 25 times: 1024 tokens of 20 + 5 heads took 28.8 us, 11.5 us
+// here).  Bound by the 42 MB of float64 queries it rewrites.
+constexpr int kRopeThreads = 256;
+__global__ void __launch_bounds__(kRopeThreads) lb_rope_block_kernel(const LbRopeParams p) {
+    extern __shared__ __align__(128) uint8_t smem_raw[];
+    double2* s_rot = reinterpret_cast<double2*>(smem_raw);  // [hd/2] (cosine, sine)
+    lb_pdl_launch_dependents();
+    lb_pdl_wait();
+    const int n = blockIdx.x, half = p.hd / 2;
+    const int pos = p.seq_stride > 0 ? p.pos_ptr[n] : *p.pos_ptr + n;
+    for (int d = threadIdx.x; d < half; d += kRopeThreads) {
+        double sn, c;
+        sincos(__ddiv_rn((double)pos, p.rope_div[d]), &sn, &c);
+        s_rot[d] = make_double2(c, sn);
+    }
+    __syncthreads();
+    double* q = p.q + (size_t)n * p.heads * p.hd;
+    float* k = p.cache_k + (size_t)n * (size_t)p.seq_stride + (size_t)(pos % p.msl) * p.hd;
+    for (int i = threadIdx.x; i < (p.heads + p.kv_heads) * half; i += kRopeThreads) {
+        const int h = i / half, d = i - h * half;
+        const double c = s_rot[d].x, sn = s_rot[d].y;
+        if (h < p.heads) {
+            double* r = q + (size_t)h * p.hd + d;
+            const double v0 = r[0], v1 = r[half];
+            r[0] = __dsub_rn(__dmul_rn(v0, c), __dmul_rn(v1, sn));
+            r[half] = __dadd_rn(__dmul_rn(v0, sn), __dmul_rn(v1, c));
+        } else {
+            float* r = k + (size_t)(h - p.heads) * p.msl * p.hd + d;
+            const double v0 = (double)r[0], v1 = (double)r[half];
+            r[0] = (float)__dsub_rn(__dmul_rn(v0, c), __dmul_rn(v1, sn));
+            r[half] = (float)__dadd_rn(__dmul_rn(v0, sn), __dmul_rn(v1, c));
+        }
+    }
+}
+
 // One CTA per (head, token, split).  K and V rows of the CTA's positions are brought into shared memory by
 // one 512-byte bulk async copy (TMA engine) per row, so that every HBM access of the kernel is in flight at
 // once; a pair of threads then scores one position (half of the head dimension each) and output dimension d is
@@ -790,6 +826,12 @@ int lb_launch_rope(loom_b200_ctx* ctx, const LbRopeParams& pin) {
     LbRopeParams p = pin;
     p.trace = lb_trace_row(ctx, "rope");
     LB_REQUIRE(ctx, p.hd % 2 == 0 && p.hd / 2 <= 1024, "rope: head_dim %d", p.hd);
+    const bool normed = (p.q_norm && p.q_norm_len > 0) || (p.k_norm && p.k_norm_len > 0);
+    if (!normed && p.M >= 32) {  // fewer tokens leave SMs without one: a CTA per head then
+        LB_CUDA(ctx, launch_pdl(ctx, lb_rope_block_kernel, dim3(p.M), dim3(kRopeThreads), (size_t)(p.hd / 2) * sizeof(double2), p));
+        ctx->launches++;
+        return 0;
+    }
     LB_CUDA(ctx, launch_pdl(ctx, lb_rope_kernel, dim3(p.heads + p.kv_heads, p.M), dim3(p.hd / 2), 0, p));
     ctx->launches++;
     return 0;
