@@ -238,6 +238,16 @@ int dec_stack_step(loom_b200_decoder* dec, int lane0, int M) {
     return dec_stack_tail(dec, lane0, M, 1);
 }
 
+// the selected sequence's logits row on the host
+int dec_read_logits(loom_b200_decoder* dec, float* host) {
+    loom_b200_ctx* ctx = dec->ctx;
+    const size_t bytes = (size_t)dec->d.vocab * 4;
+    LB_CUDA(ctx, cudaMemcpyAsync(dec->h_logits, dec->logits, bytes, cudaMemcpyDeviceToHost, ctx->stream));
+    if (int rc = lb_sync_checked(ctx)) return rc;
+    memcpy(host, dec->h_logits, bytes);
+    return 0;
+}
+
 // The next M tokens (already in pf_tok) of the selected sequence through a stack.  The logits at the n_want places in `want`
 // (of this block) go to the host; the last block of a call also runs the head on its last token and the greedy tail.
 int dec_stack_block(loom_b200_decoder* dec, int M, int pos0, bool last, const int32_t* want, int n_want, float* logits_host) {
@@ -247,9 +257,12 @@ int dec_stack_block(loom_b200_decoder* dec, int M, int pos0, bool last, const in
     if (int rc = lb_stack_block(ctx, st, M, pos0, dec->lane)) return rc;
     dec->last_resid = st->pf_x;
     dec->last_resid_rows = M;
-    if (n_want > 0) LB_CUDA(ctx, cudaMemcpyAsync(st->pf_rows, want, (size_t)n_want * sizeof(int), cudaMemcpyHostToDevice, ctx->stream));
-    for (int i0 = 0; i0 < n_want; i0 += kStackHeadRows) {
-        const int n = std::min(kStackHeadRows, n_want - i0);
+    // the last token's row goes through the head once, for the caller and for the greedy tail
+    const bool want_last = last && n_want > 0 && want[n_want - 1] == M - 1;
+    const int n_before = n_want - (want_last ? 1 : 0);
+    if (n_before > 0) LB_CUDA(ctx, cudaMemcpyAsync(st->pf_rows, want, (size_t)n_before * sizeof(int), cudaMemcpyHostToDevice, ctx->stream));
+    for (int i0 = 0; i0 < n_before; i0 += kStackHeadRows) {
+        const int n = std::min(kStackHeadRows, n_before - i0);
         if (i0 > 0)
             LB_CUDA(ctx, cudaMemcpyAsync(st->pf_rows, want + i0, (size_t)n * sizeof(int), cudaMemcpyHostToDevice, ctx->stream));
         if (n <= lb_dense_gemv_max_tokens(dec->d.hidden, st->d.dtype)) {
@@ -262,7 +275,8 @@ int dec_stack_block(loom_b200_decoder* dec, int M, int pos0, bool last, const in
     }
     if (!last) return lb_launch_add_scalar(ctx, dec->pos, M);
     if (int rc = lb_stack_head(ctx, st, st->pf_x + (size_t)(M - 1) * st->ldx, nullptr, 1, dec->logits, V)) return rc;
-    return dec_stack_tail(dec, dec->lane, 1, M);
+    if (int rc = dec_stack_tail(dec, dec->lane, 1, M)) return rc;
+    return want_last ? dec_read_logits(dec, logits_host + (size_t)(n_want - 1) * V) : 0;
 }
 
 // A block of M prompt tokens (already in pf_tok) at positions pos0..pos0+M-1 through the whole stack, every
@@ -702,9 +716,7 @@ int dec_extend(loom_b200_decoder* dec, const int32_t* tokens, int n, const int32
     }
     if (want_last) {
         if (int rc = dec_gather_logits(dec, dec->logits)) return rc;
-        LB_CUDA(ctx, cudaMemcpyAsync(dec->h_logits, dec->logits, V * 4, cudaMemcpyDeviceToHost, ctx->stream));
-        if (int rc = lb_sync_checked(ctx)) return rc;
-        memcpy(logits_host + (size_t)(n_want - 1) * V, dec->h_logits, V * 4);
+        if (int rc = dec_read_logits(dec, logits_host + (size_t)(n_want - 1) * V)) return rc;
     }
     dec->kv_offset += n;
     return 0;

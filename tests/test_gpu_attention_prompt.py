@@ -1,4 +1,4 @@
-"""Float64 attention and rotation of a prompt block: query heads per KV head from one to 64 (the tile of query rows changes at 32),
+"""Float64 attention and rotation of a prompt block: query heads per KV head from one to 64,
 head dimensions, and prompts that end just before, at and after a tile of keys or of query rows.
 
 Two decoder blocks against the CPU oracle's: the second block's keys carry every row of the first one's attention.  All sums are
