@@ -10,6 +10,8 @@
 #include "layers.cuh"
 #include "stack.cuh"
 
+#include <sys/mman.h>
+
 #include <algorithm>
 #include <chrono>
 #include <cmath>
@@ -25,6 +27,8 @@ struct LbDecBlock {
     int ffn_inner_len = 0;
     bool ready = false;
 };
+
+constexpr int kReadEvents = 32;  // passes of eight sequences: 256 sequences
 
 struct loom_b200_decoder {
     loom_b200_ctx* ctx = nullptr;
@@ -73,6 +77,8 @@ struct loom_b200_decoder {
     int* cur_tok = nullptr;             // the current token of the selected lane (tok when there is one sequence)
     std::vector<int> kv_offsets;        // host mirror of every lane's position
     int* h_tok_all = nullptr;           // pinned [batch]
+    cudaEvent_t read_done[kReadEvents] = {};  // pieces of a logits row on their way to the host; passes of several sequences
+    cudaStream_t read_stream = nullptr;  // several sequences: a pass's logits cross the bus beside the next pass
 };
 
 namespace {
@@ -238,14 +244,36 @@ int dec_stack_step(loom_b200_decoder* dec, int lane0, int M) {
     return dec_stack_tail(dec, lane0, M, 1);
 }
 
+// A row of logits reaches a caller's pageable memory through pinned memory in pieces: a piece is copied on while the next crosses the
+// bus.  The caller's pages are touched before that, while the GPU is still at the step (a fresh page costs a fault, up to a
+// microsecond each).  A step of the 2560-wide Zitupel with its 513 KB row: 690 us with one copy after the step, 620 so.
+constexpr int kReadPieces = 4;
+
+// Faults the pages in by one call (their contents stay).  Touching them one by one -- a read, then a write -- faults a fresh page
+// twice, 1000 of them longer than a step of eight sequences takes.  Where the kernel does not know the request the copy faults them.
+void touch_pages(void* p, size_t bytes) {
+#ifdef MADV_POPULATE_WRITE
+    const uintptr_t from = reinterpret_cast<uintptr_t>(p) & ~(uintptr_t)4095, end = reinterpret_cast<uintptr_t>(p) + bytes;
+    (void)madvise(reinterpret_cast<void*>(from), end - from, MADV_POPULATE_WRITE);
+#endif
+}
+
 // the selected sequence's logits row on the host
 int dec_read_logits(loom_b200_decoder* dec, float* host) {
     loom_b200_ctx* ctx = dec->ctx;
     const size_t bytes = (size_t)dec->d.vocab * 4;
-    LB_CUDA(ctx, cudaMemcpyAsync(dec->h_logits, dec->logits, bytes, cudaMemcpyDeviceToHost, ctx->stream));
-    if (int rc = lb_sync_checked(ctx)) return rc;
-    memcpy(host, dec->h_logits, bytes);
-    return 0;
+    size_t from[kReadPieces + 1];
+    for (int i = 0; i <= kReadPieces; ++i) from[i] = i == kReadPieces ? bytes : bytes / kReadPieces * i / 64 * 64;
+    for (int i = 0; i < kReadPieces; ++i) {
+        LB_CUDA(ctx, cudaMemcpyAsync((char*)dec->h_logits + from[i], (const char*)dec->logits + from[i], from[i + 1] - from[i], cudaMemcpyDeviceToHost, ctx->stream));
+        LB_CUDA(ctx, cudaEventRecord(dec->read_done[i], ctx->stream));
+    }
+    touch_pages(host, bytes);
+    for (int i = 0; i < kReadPieces; ++i) {
+        LB_CUDA(ctx, cudaEventSynchronize(dec->read_done[i]));
+        memcpy((char*)host + from[i], (const char*)dec->h_logits + from[i], from[i + 1] - from[i]);
+    }
+    return lb_sync_checked(ctx);
 }
 
 // The next M tokens (already in pf_tok) of the selected sequence through a stack.  The logits at the n_want places in `want`
@@ -753,6 +781,7 @@ static int dec_finish_create(loom_b200_decoder* dec, loom_b200_decoder** out) {
     }
     if (e == cudaSuccess) e = cudaMallocHost((void**)&dec->h_tok, kChunkTokens * sizeof(int));
     if (e == cudaSuccess) e = cudaMallocHost((void**)&dec->h_logits, (size_t)d.vocab * 4);
+    for (int i = 0; i < kReadEvents && e == cudaSuccess; ++i) e = cudaEventCreateWithFlags(&dec->read_done[i], cudaEventDisableTiming);
     if (e == cudaSuccess) e = cudaStreamSynchronize(ctx->stream);
     if (e != cudaSuccess) {
         loom_b200_decoder_destroy(dec);
@@ -887,6 +916,9 @@ void loom_b200_decoder_destroy(loom_b200_decoder* dec) {
     if (dec->h_tok) cudaFreeHost(dec->h_tok);
     if (dec->h_tok_all) cudaFreeHost(dec->h_tok_all);
     if (dec->h_logits) cudaFreeHost(dec->h_logits);
+    for (cudaEvent_t ev : dec->read_done)
+        if (ev) cudaEventDestroy(ev);
+    if (dec->read_stream) cudaStreamDestroy(dec->read_stream);
     delete dec;
 }
 
@@ -1105,6 +1137,7 @@ int loom_b200_decoder_set_batch(loom_b200_decoder* dec, int batch) {
     A((void**)&dec->tok_all, B * sizeof(int));
     A((void**)&dec->out_tokens_all, B * dec->out_cap * sizeof(int));
     if (e == cudaSuccess) e = cudaMallocHost((void**)&dec->h_tok_all, B * sizeof(int));
+    if (e == cudaSuccess && B > 1 && !dec->read_stream) e = cudaStreamCreateWithFlags(&dec->read_stream, cudaStreamNonBlocking);
     if (e == cudaSuccess) e = cudaStreamSynchronize(ctx->stream);
     if (e != cudaSuccess) return lb_fail(ctx, LOOM_B200_ERR_CUDA, "decoder_set_batch: %s", cudaGetErrorString(e));
     dec->batch = batch;
@@ -1153,12 +1186,32 @@ int loom_b200_decoder_step_batch(loom_b200_decoder* dec, const int32_t* tokens, 
         for (int i = 0; i < B; ++i) dec->h_tok_all[i] = tokens[i];
         LB_CUDA(ctx, cudaMemcpyAsync(dec->tok_all, dec->h_tok_all, (size_t)B * sizeof(int), cudaMemcpyHostToDevice, ctx->stream));
     }
+    // with the whole vocabulary on this GPU a pass's rows cross to the host beside the passes after it (16 sequences: 34.9 ms for eight
+    // steps with one copy at the end, 28.4 so)
+    const bool beside = logits_host && dec->read_stream && !dec->head_sharded;
+    int passes = 0;
     for (int l0 = 0; l0 < B; l0 += kChunkTokens) {
         const int M = B - l0 < kChunkTokens ? B - l0 : kChunkTokens;
         if (int rc = dec_forward_lanes(dec, l0, M)) return rc;
+        if (beside) LB_CUDA(ctx, cudaEventRecord(dec->read_done[passes++], ctx->stream));
     }
     for (int i = 0; i < B; ++i) dec->kv_offsets[i] += 1;
     dec->kv_offset = dec->kv_offsets[dec->lane];
+    if (beside) {
+        const size_t row = (size_t)dec->d.vocab * 4;
+        cudaPointerAttributes where{};
+        if (cudaPointerGetAttributes(&where, logits_host) == cudaSuccess && where.type == cudaMemoryTypeUnregistered) touch_pages(logits_host, (size_t)B * row);
+        cudaError_t e = cudaSuccess;
+        for (int i = 0; i < passes && e == cudaSuccess; ++i) {
+            const size_t at = (size_t)i * kChunkTokens * row, len = std::min((size_t)kChunkTokens, (size_t)B - (size_t)i * kChunkTokens) * row;
+            e = cudaStreamWaitEvent(dec->read_stream, dec->read_done[i], 0);
+            if (e == cudaSuccess) e = cudaMemcpyAsync((char*)logits_host + at, (const char*)dec->logits_all + at, len, cudaMemcpyDeviceToHost, dec->read_stream);
+        }
+        const cudaError_t end = cudaStreamSynchronize(dec->read_stream);  // nothing writes the rows after the call
+        if (e == cudaSuccess) e = end;
+        if (e != cudaSuccess) return lb_fail(ctx, LOOM_B200_ERR_CUDA, "decoder_step_batch: %s", cudaGetErrorString(e));
+        return lb_sync_checked(ctx);
+    }
     if (logits_host) {
         for (int i = 0; i < B; ++i)
             if (int rc = dec_gather_logits(dec, dec->logits_all + (size_t)i * dec->d.vocab)) return rc;
