@@ -44,3 +44,44 @@ def test_steps_of_wide_and_narrow_stacks(ctx, dtype, width, ff, vocab, batch):
         want, _ = do.forward(cfg, w, tok[i])
         assert kit.error(np.stack([g[i] for g in got]), want[2:]).max() < 5 * TOL[dtype], i
     dec.close()
+
+
+def normalised(row, gain, eps, threads):
+    """A row through the norm of the prologue, operation by operation: thread i of `threads` adds the squares of columns i, i + threads, ...
+    in that order, then a warp's 32 sums meet pairwise from afar to near, then the warps' in order.  (The product and sum of a fused
+    multiply-add are exact in 64 bits of mantissa up to one rounding of the sum's last bits.)"""
+    x = np.zeros(-(-len(row) // threads) * threads, np.float32)
+    x[:len(row)] = row
+    ss = np.zeros(threads, np.float32)
+    for part in x.reshape(-1, threads):
+        ss = (part.astype(np.longdouble) ** 2 + ss).astype(np.float32)
+    ss = ss.reshape(-1, 32)
+    for o in (16, 8, 4, 2, 1):
+        ss = ss + ss[:, np.arange(32) ^ o]
+    total = np.float32(0)
+    for v in ss[:, 0]:
+        total = total + v
+    rstd = np.float32(1) / np.sqrt(total / np.float32(len(row)) + np.float32(eps))
+    return row * rstd * np.float32(1) * gain
+
+
+@pytest.mark.parametrize("width,batch", [(2560, 1), (2560, 2), (2560, 3), (1111, 1), (1111, 2), (40, 5), (6200, 1), (6200, 2)])
+def test_norm_adds_columns_in_one_order(ctx, width, batch):
+    """The last bits of a norm decide which way bf16 rounds a row, and that travels through the layers that follow: the sum's order is
+    part of the result.  The embeddings' first rows are those of the unit matrix, so that the tied head hands out the normalised row."""
+    def edit(w):
+        w["embed"][:width] = np.eye(width)
+
+    cfg = dk.config(width, width + 16, [dk.mlstm(2, 8, 24, 9.0, None)])
+    w = dk.random_weights(cfg, 8, edit=edit)
+    dec = models.build(ctx, cfg, kit.Weights(w), models.LoadOptions(F32, 16, batch))
+    tok = np.random.default_rng(3).integers(width, width + 16, batch).astype(np.int32)
+    for i in range(batch):
+        dec.select(i)
+        dec.extend(tok[i:i + 1])
+    got = dec.step_batch(tok) if batch > 1 else dec.extend(tok, [0])
+    rows = dec.last_residual(batch)
+    for g, row in zip(np.asarray(got), rows):
+        want = normalised(row[:width], np.asarray(w["final.norm"], np.float32), cfg["norm"]["eps"], 128 if batch == 2 else 256)
+        assert np.array_equal(g[:width], want)
+    dec.close()
