@@ -78,9 +78,18 @@ int lb_ensure_scratch(loom_b200_ctx* ctx, size_t bytes) {
     return 0;
 }
 
-int lb_sync_checked(loom_b200_ctx* ctx) {
+int lb_status_queue(loom_b200_ctx* ctx) {
     LB_CUDA(ctx, cudaMemcpyAsync(ctx->status_host, ctx->status_dev, sizeof(int), cudaMemcpyDeviceToHost, ctx->stream));
+    return 0;
+}
+
+int lb_sync_checked(loom_b200_ctx* ctx) {
+    if (int rc = lb_status_queue(ctx)) return rc;
     LB_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
+    return lb_status_result(ctx);
+}
+
+int lb_status_result(loom_b200_ctx* ctx) {
     const int code = *ctx->status_host;
     if (code == 0) return 0;
     *ctx->status_host = 0;

@@ -116,6 +116,10 @@ int lb_ensure_scratch(loom_b200_ctx* ctx, size_t bytes);
 // Waits for the context's stream and reads the device status word with it: a bounded device-side wait that ran out
 // (a copy that never landed, a peer that never answered) comes back as LOOM_B200_ERR_TIMEOUT, and the word is cleared.
 int lb_sync_checked(loom_b200_ctx* ctx);
+// The two halves of it, for a caller that waits for copies of its own anyway: the word's copy behind the work queued so far, and
+// what it says once that copy is known to have arrived.
+int lb_status_queue(loom_b200_ctx* ctx);
+int lb_status_result(loom_b200_ctx* ctx);
 int lb_ensure_quant_scratch(loom_b200_ctx* ctx, size_t bytes);
 
 #define LB_CUDA(ctx, expr)                                                                          \

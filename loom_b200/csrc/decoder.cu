@@ -244,36 +244,53 @@ int dec_stack_step(loom_b200_decoder* dec, int lane0, int M) {
     return dec_stack_tail(dec, lane0, M, 1);
 }
 
-// A row of logits reaches a caller's pageable memory through pinned memory in pieces: a piece is copied on while the next crosses the
-// bus.  The caller's pages are touched before that, while the GPU is still at the step (a fresh page costs a fault, up to a
-// microsecond each).  A step of the 2560-wide Zitupel with its 513 KB row: 690 us with one copy after the step, 620 so.
-constexpr int kReadPieces = 4;
+// A row of logits reaches the caller's memory through pinned memory.  A large one comes in two pieces, the first copied on while the
+// second crosses the bus, and the caller's pages are touched before that, while the GPU is still at the step (a fresh page costs a
+// fault, up to a microsecond each).  us a step of a small two-layer stack, into the same memory again / into fresh memory:
+//   row       one copy       two pieces    four
+//   16 KB     52 / 53        55 / 55       61 / 62
+//   125 KB    64 / 68        65 / 68       68 / 70
+//   250 KB    93 / 105       94 / 102      98 / 105
+//   501 KB    92 / 255       91 / 139      96 / 141   (the pages of a row in one copy are not touched)
+constexpr int kReadPieces = 2;
+constexpr size_t kReadSplit = 192 * 1024;
 
-// Faults the pages in by one call (their contents stay).  Touching them one by one -- a read, then a write -- faults a fresh page
-// twice, 1000 of them longer than a step of eight sequences takes.  Where the kernel does not know the request the copy faults them.
+// Faults the pages of a pageable buffer in by one call (their contents stay).  Touching them one by one -- a read, then a write -- faults a
+// fresh page twice, 1000 of them longer than a step of eight sequences takes.  Where the kernel does not know the request the copy faults them.
 void touch_pages(void* p, size_t bytes) {
 #ifdef MADV_POPULATE_WRITE
+    cudaPointerAttributes where{};
+    if (cudaPointerGetAttributes(&where, p) != cudaSuccess) {
+        (void)cudaGetLastError();
+        return;
+    }
+    if (where.type != cudaMemoryTypeUnregistered) return;
     const uintptr_t from = reinterpret_cast<uintptr_t>(p) & ~(uintptr_t)4095, end = reinterpret_cast<uintptr_t>(p) + bytes;
     (void)madvise(reinterpret_cast<void*>(from), end - from, MADV_POPULATE_WRITE);
 #endif
 }
 
-// the selected sequence's logits row on the host
+// The selected sequence's logits row on the host.  The status word comes first: a row that it calls invalid does not reach the
+// caller, and no copy of its own has to be waited for after the row.
 int dec_read_logits(loom_b200_decoder* dec, float* host) {
     loom_b200_ctx* ctx = dec->ctx;
     const size_t bytes = (size_t)dec->d.vocab * 4;
+    const int pieces = bytes < kReadSplit ? 1 : kReadPieces;
     size_t from[kReadPieces + 1];
-    for (int i = 0; i <= kReadPieces; ++i) from[i] = i == kReadPieces ? bytes : bytes / kReadPieces * i / 64 * 64;
-    for (int i = 0; i < kReadPieces; ++i) {
+    for (int i = 0; i <= pieces; ++i) from[i] = i == pieces ? bytes : bytes / pieces * i / 64 * 64;
+    if (int rc = lb_status_queue(ctx)) return rc;
+    for (int i = 0; i < pieces; ++i) {
         LB_CUDA(ctx, cudaMemcpyAsync((char*)dec->h_logits + from[i], (const char*)dec->logits + from[i], from[i + 1] - from[i], cudaMemcpyDeviceToHost, ctx->stream));
-        LB_CUDA(ctx, cudaEventRecord(dec->read_done[i], ctx->stream));
+        if (i + 1 < pieces) LB_CUDA(ctx, cudaEventRecord(dec->read_done[i], ctx->stream));
     }
-    touch_pages(host, bytes);
-    for (int i = 0; i < kReadPieces; ++i) {
-        LB_CUDA(ctx, cudaEventSynchronize(dec->read_done[i]));
+    if (pieces > 1) touch_pages(host, bytes);
+    for (int i = 0; i < pieces; ++i) {
+        LB_CUDA(ctx, i + 1 < pieces ? cudaEventSynchronize(dec->read_done[i]) : cudaStreamSynchronize(ctx->stream));
+        if (i == 0)
+            if (int rc = lb_status_result(ctx)) return rc;
         memcpy((char*)host + from[i], (const char*)dec->h_logits + from[i], from[i + 1] - from[i]);
     }
-    return lb_sync_checked(ctx);
+    return 0;
 }
 
 // The next M tokens (already in pf_tok) of the selected sequence through a stack.  The logits at the n_want places in `want`
@@ -1137,7 +1154,7 @@ int loom_b200_decoder_set_batch(loom_b200_decoder* dec, int batch) {
     A((void**)&dec->tok_all, B * sizeof(int));
     A((void**)&dec->out_tokens_all, B * dec->out_cap * sizeof(int));
     if (e == cudaSuccess) e = cudaMallocHost((void**)&dec->h_tok_all, B * sizeof(int));
-    if (e == cudaSuccess && B > 1 && !dec->read_stream) e = cudaStreamCreateWithFlags(&dec->read_stream, cudaStreamNonBlocking);
+    if (e == cudaSuccess && B > (size_t)kChunkTokens && !dec->read_stream) e = cudaStreamCreateWithFlags(&dec->read_stream, cudaStreamNonBlocking);
     if (e == cudaSuccess) e = cudaStreamSynchronize(ctx->stream);
     if (e != cudaSuccess) return lb_fail(ctx, LOOM_B200_ERR_CUDA, "decoder_set_batch: %s", cudaGetErrorString(e));
     dec->batch = batch;
@@ -1187,20 +1204,22 @@ int loom_b200_decoder_step_batch(loom_b200_decoder* dec, const int32_t* tokens, 
         LB_CUDA(ctx, cudaMemcpyAsync(dec->tok_all, dec->h_tok_all, (size_t)B * sizeof(int), cudaMemcpyHostToDevice, ctx->stream));
     }
     // with the whole vocabulary on this GPU a pass's rows cross to the host beside the passes after it (16 sequences: 34.9 ms for eight
-    // steps with one copy at the end, 28.4 so)
-    const bool beside = logits_host && dec->read_stream && !dec->head_sharded;
+    // steps with one copy at the end, 28.4 so); one pass has nothing to cross beside (eight rows of 16 KB: 71 us a step with a copy
+    // in the step's own stream, 81 so)
+    const bool beside = logits_host && B > kChunkTokens && !dec->head_sharded;
     int passes = 0;
     for (int l0 = 0; l0 < B; l0 += kChunkTokens) {
         const int M = B - l0 < kChunkTokens ? B - l0 : kChunkTokens;
         if (int rc = dec_forward_lanes(dec, l0, M)) return rc;
+        if (beside && l0 + M == B)
+            if (int rc = lb_status_queue(ctx)) return rc;  // (before the last pass's event: the rows' stream waits for both)
         if (beside) LB_CUDA(ctx, cudaEventRecord(dec->read_done[passes++], ctx->stream));
     }
     for (int i = 0; i < B; ++i) dec->kv_offsets[i] += 1;
     dec->kv_offset = dec->kv_offsets[dec->lane];
     if (beside) {
         const size_t row = (size_t)dec->d.vocab * 4;
-        cudaPointerAttributes where{};
-        if (cudaPointerGetAttributes(&where, logits_host) == cudaSuccess && where.type == cudaMemoryTypeUnregistered) touch_pages(logits_host, (size_t)B * row);
+        touch_pages(logits_host, (size_t)B * row);
         cudaError_t e = cudaSuccess;
         for (int i = 0; i < passes && e == cudaSuccess; ++i) {
             const size_t at = (size_t)i * kChunkTokens * row, len = std::min((size_t)kChunkTokens, (size_t)B - (size_t)i * kChunkTokens) * row;
@@ -1210,13 +1229,16 @@ int loom_b200_decoder_step_batch(loom_b200_decoder* dec, const int32_t* tokens, 
         const cudaError_t end = cudaStreamSynchronize(dec->read_stream);  // nothing writes the rows after the call
         if (e == cudaSuccess) e = end;
         if (e != cudaSuccess) return lb_fail(ctx, LOOM_B200_ERR_CUDA, "decoder_step_batch: %s", cudaGetErrorString(e));
-        return lb_sync_checked(ctx);
+        return lb_status_result(ctx);
     }
     if (logits_host) {
         for (int i = 0; i < B; ++i)
             if (int rc = dec_gather_logits(dec, dec->logits_all + (size_t)i * dec->d.vocab)) return rc;
+        if (int rc = lb_status_queue(ctx)) return rc;
+        touch_pages(logits_host, (size_t)B * dec->d.vocab * 4);
         LB_CUDA(ctx, cudaMemcpyAsync(logits_host, dec->logits_all, (size_t)B * dec->d.vocab * 4, cudaMemcpyDeviceToHost, ctx->stream));
-        if (int rc = lb_sync_checked(ctx)) return rc;
+        LB_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
+        return lb_status_result(ctx);
     }
     return 0;
 }
