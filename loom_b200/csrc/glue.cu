@@ -107,26 +107,33 @@ __global__ void lb_rope_kernel(const LbRopeParams p) {
     lb_trace(p.trace, 5);
 }
 
-// The same for a token block without per-head norms: one CTA per token computes the token's hd/2 angles once for all heads (a
-// float64 division, sine and cosine each; one CTA per head repeated them 25 times: 1024 tokens of 20 + 5 heads took 28.8 us, 11.5 us
-// here).  Bound by the 42 MB of float64 queries it rewrites.
+// The same for a token block without per-head norms: a CTA computes its token's hd/2 angles once (a float64 division, sine and cosine
+// each; one CTA per head repeats them for every head) and rotates a share of the heads, so many of them that about five CTAs fall to
+// an SM.  Bound by the float64 queries it rewrites once the angles are shared (1024 tokens of 20 + 5 heads: 42 MB).  Cold launches, us,
+// one CTA per head / this kernel, by tokens x (heads + KV heads):
+//   64 x 40: 4.9 / 5.8    256 x 12: 5.2 / 5.5    160 x 25: 6.2 / 6.0    100 x 40: 6.2 / 5.9    384 x 12: 6.9 / 6.1
+//   200 x 25: 7.4 / 6.5   132 x 40: 7.6 / 6.5    512 x 25: 15.3 / 8.8   1024 x 25: 28.8 / 14.3   1024 x 40: 44.6 / 18.9
+// and with five heads or fewer to share an angle 1024 x 5: 7.5 / 8.1, 1024 x 2: 4.6 / 6.0.
 constexpr int kRopeThreads = 256;
 __global__ void __launch_bounds__(kRopeThreads) lb_rope_block_kernel(const LbRopeParams p) {
     extern __shared__ __align__(128) uint8_t smem_raw[];
     double2* s_rot = reinterpret_cast<double2*>(smem_raw);  // [hd/2] (cosine, sine)
     lb_pdl_launch_dependents();
     lb_pdl_wait();
-    const int n = blockIdx.x, half = p.hd / 2;
-    const int pos = p.seq_stride > 0 ? p.pos_ptr[n] : *p.pos_ptr + n;
+    lb_trace(p.trace, 2);
+    const int n = blockIdx.x, half = p.hd / 2, all = p.heads + p.kv_heads;
+    const int h0 = all * (int)blockIdx.y / (int)gridDim.y, h1 = all * ((int)blockIdx.y + 1) / (int)gridDim.y;
+    const int pos = *p.pos_ptr + n;
     for (int d = threadIdx.x; d < half; d += kRopeThreads) {
         double sn, c;
         sincos(__ddiv_rn((double)pos, p.rope_div[d]), &sn, &c);
         s_rot[d] = make_double2(c, sn);
     }
     __syncthreads();
+    lb_trace(p.trace, 3);
     double* q = p.q + (size_t)n * p.heads * p.hd;
-    float* k = p.cache_k + (size_t)n * (size_t)p.seq_stride + (size_t)(pos % p.msl) * p.hd;
-    for (int i = threadIdx.x; i < (p.heads + p.kv_heads) * half; i += kRopeThreads) {
+    float* k = p.cache_k + (size_t)(pos % p.msl) * p.hd;
+    for (int i = h0 * half + threadIdx.x; i < h1 * half; i += kRopeThreads) {
         const int h = i / half, d = i - h * half;
         const double c = s_rot[d].x, sn = s_rot[d].y;
         if (h < p.heads) {
@@ -141,6 +148,7 @@ __global__ void __launch_bounds__(kRopeThreads) lb_rope_block_kernel(const LbRop
             r[half] = (float)__dadd_rn(__dmul_rn(v0, sn), __dmul_rn(v1, c));
         }
     }
+    lb_trace(p.trace, 5);
 }
 
 // One CTA per (head, token, split).  K and V rows of the CTA's positions are brought into shared memory by
@@ -827,8 +835,11 @@ int lb_launch_rope(loom_b200_ctx* ctx, const LbRopeParams& pin) {
     p.trace = lb_trace_row(ctx, "rope");
     LB_REQUIRE(ctx, p.hd % 2 == 0 && p.hd / 2 <= 1024, "rope: head_dim %d", p.hd);
     const bool normed = (p.q_norm && p.q_norm_len > 0) || (p.k_norm && p.k_norm_len > 0);
-    if (!normed && p.M >= 32) {  // fewer tokens leave SMs without one: a CTA per head then
-        LB_CUDA(ctx, launch_pdl(ctx, lb_rope_block_kernel, dim3(p.M), dim3(kRopeThreads), (size_t)(p.hd / 2) * sizeof(double2), p));
+    const int all = p.heads + p.kv_heads;
+    if (!normed && p.seq_stride <= 0 && all >= 8 && (long long)p.M * all >= 4096) {
+        int shares = (5 * ctx->sm_count + p.M / 2) / p.M;
+        shares = shares < 1 ? 1 : shares > all ? all : shares;
+        LB_CUDA(ctx, launch_pdl(ctx, lb_rope_block_kernel, dim3(p.M, shares), dim3(kRopeThreads), (size_t)(p.hd / 2) * sizeof(double2), p));
         ctx->launches++;
         return 0;
     }
