@@ -103,23 +103,24 @@ struct GemvAcc<float> {
 };
 
 // the same for rows of (token, choice) pairs (routed experts, second product): xw points at the chunks that the lanes of this
-// warp fetched, lane (g, t) the one of token g, zeros where the token did not choose the expert
+// warp fetched, lane (g, t) the one of token g, zeros where the token did not choose the expert (bit m of `chose` is not set).
+// Multiply-adds leave those tokens out: an infinite weight times such a zero would reach a token that has nothing to do with it.
 template <typename WT>
-__device__ __forceinline__ void step_pairs(GemvAcc<WT>& acc, const uint4& w0, const uint4& w1, const uint4* xw, int M, int lane);
+__device__ __forceinline__ void step_pairs(GemvAcc<WT>& acc, const uint4& w0, const uint4& w1, const uint4* xw, unsigned chose, int lane);
 template <>
-__device__ __forceinline__ void step_pairs<__nv_bfloat16>(GemvAcc<__nv_bfloat16>& acc, const uint4& w0, const uint4& w1, const uint4* xw, int M, int lane) {
+__device__ __forceinline__ void step_pairs<__nv_bfloat16>(GemvAcc<__nv_bfloat16>& acc, const uint4& w0, const uint4& w1, const uint4* xw, unsigned chose, int lane) {
     const uint4 x = xw[lane];
     mma_bf16(acc.d, w0.x, w1.x, w0.y, w1.y, x.x, x.y);
     mma_bf16(acc.d, w0.z, w1.z, w0.w, w1.w, x.z, x.w);
 }
 template <>
-__device__ __forceinline__ void step_pairs<float>(GemvAcc<float>& acc, const uint4& w0, const uint4& w1, const uint4* xw, int M, int lane) {
+__device__ __forceinline__ void step_pairs<float>(GemvAcc<float>& acc, const uint4& w0, const uint4& w1, const uint4* xw, unsigned chose, int lane) {
     float p[4], q[4], x[4];
     lb_unpack_chunk<float>(w0, p);
     lb_unpack_chunk<float>(w1, q);
 #pragma unroll
     for (int m = 0; m < 8; ++m) {
-        if (m >= M) break;
+        if (!(chose >> m & 1)) continue;
         lb_unpack_chunk<float>(xw[m * 4 + (lane & 3)], x);
 #pragma unroll
         for (int i = 0; i < 4; ++i) {
@@ -558,6 +559,8 @@ __global__ void __launch_bounds__(kGemvThreads, 2) lb_dense_gemv_kernel(const Lb
         if (kDual) acc2.zero();
         if (strip < strips) {
             const int total = nact * p.slices;
+            int at_end = 0, at = -1;  // PAIRS: end of the present expert's slices, its place in the list
+            unsigned chose = 0;
             const uint8_t *d1 = strip_ptr(w1, strip) + lane_off, *d2 = kDual ? strip_ptr(w2, strip) + lane_off : nullptr;
             for (int s = kw; s < total; s += KW) {
                 uint4 w[8];
@@ -575,8 +578,13 @@ __global__ void __launch_bounds__(kGemvThreads, 2) lb_dense_gemv_kernel(const Lb
                     }
                 }
                 if (PRO == LB_DPRO_PAIRS) {
-                    step_pairs<WT>(acc, w[0], w[2], rs + 4 * kGemvThreads, p.M, lane);
-                    step_pairs<WT>(acc, w[1], w[3], rs + 5 * kGemvThreads, p.M, lane);
+                    if (s >= at_end) {  // (KW <= slices: the next expert, never one further)
+                        at_end += p.slices;
+                        ++at;
+                        chose = __ballot_sync(0xffffffffu, lane < kMaxLanesPerPass && s_route[kMaxLanesPerPass * kMaxTop + at * kMaxLanesPerPass + (lane & 7)] >= 0);
+                    }
+                    step_pairs<WT>(acc, w[0], w[2], rs + 4 * kGemvThreads, chose, lane);
+                    step_pairs<WT>(acc, w[1], w[3], rs + 5 * kGemvThreads, chose, lane);
                 } else {
                     const uint4* x0 = xs + (size_t)(s * 8 + t) * Mp;
                     acc.step(w[0], w[2], x0, Mp, M, g);

@@ -85,3 +85,31 @@ def test_norm_adds_columns_in_one_order(ctx, width, batch):
         want = normalised(row[:width], np.asarray(w["final.norm"], np.float32), cfg["norm"]["eps"], 128 if batch == 2 else 256)
         assert np.array_equal(g[:width], want)
     dec.close()
+
+
+@pytest.mark.parametrize("dtype,batch,ff", [(F32, 1, 40), (F32, 5, 40), (F32, 8, 200), (BF16, 1, 40)])
+def test_infinite_weights_of_an_expert_stay_with_its_tokens(ctx, dtype, batch, ff):
+    """One routed layer whose expert e has infinite weights in its second product: exactly the tokens that chose e lose their logits, and
+    those of the others keep every bit.  (In bf16 matrix instructions multiply the tokens of a pass that did not choose with zeros.)"""
+    E, top = 5, 2
+    cfg = kit.config(72, 90, [kit.gla(2, 16, 24, 8.0, kit.moe(ff, E, top))])
+    w = kit.random_weights(cfg, 4)
+    tok = np.random.default_rng(6).integers(0, 90, (2, batch)).astype(np.int32)
+
+    def logits(weights):
+        dec = models.build(ctx, cfg, kit.Weights(weights), models.LoadOptions(dtype, 16, batch))
+        for i in range(batch):
+            dec.select(i)
+            dec.extend(tok[0, i:i + 1])
+        got = np.array(dec.step_batch(tok[1]) if batch > 1 else dec.extend(tok[1], [0]))
+        dec.close()
+        return got
+
+    clean, chosen = logits(w), np.zeros(batch, int)
+    for e in range(E):
+        name = "l0.mlp.e%d.down" % e
+        got = logits({**w, name: np.full_like(w[name], np.inf)})
+        lost = ~np.isfinite(got).all(axis=1)
+        assert np.array_equal(got[~lost], clean[~lost])
+        chosen += lost
+    assert np.array_equal(chosen, np.full(batch, top))
