@@ -143,8 +143,9 @@ __global__ void __launch_bounds__(kAcThreads, 1) lb_attention_cluster_kernel(con
         } else if (warp == 1) {
             fetch(1, 0);
         } else if (warp == 2 && p.next_k) {  // the next block's rows of the same positions, into L2
-            l2_prefetch(p.next_k + ((size_t)kvh * p.msl + k0) * hd, (uint32_t)cnt * hd * 4);
-            l2_prefetch(p.next_v + ((size_t)kvh * p.msl + k0) * hd, (uint32_t)cnt * hd * 4);
+            const uint32_t bytes = (uint32_t)(cnt < p.next_rows ? cnt : p.next_rows) * hd * 4;
+            l2_prefetch(p.next_k + ((size_t)kvh * p.msl + k0) * hd, bytes);
+            l2_prefetch(p.next_v + ((size_t)kvh * p.msl + k0) * hd, bytes);
         }
     }
     // queries of the group, rotated (RoPE): thread idx owns the pair (d, d + hd/2) of head g
@@ -354,6 +355,10 @@ __global__ void __launch_bounds__(kAcThreads, 1) lb_attention_cluster_kernel(con
 }
 
 constexpr size_t kAcSmem = 200 * 1024;
+// Bytes of the next block's rings that are asked into L2, over all clusters: what arrives before that block's projections do.  Asking
+// for whole rings costs more the longer they are (us a block, 8 KV heads, none / 4 MB / 32 MB / all: context 4000 73.2, 72.9, 74.6, 74.7;
+// 8000 95.9, 95.8, 97.5, 97.3; 32000 232.5, 232.7, 233.6, 233.4; five KV heads, context 8000: 59.6, 59.3, 60.5, 60.7).
+constexpr size_t kAcAhead = 4 << 20;
 constexpr int kAcChunk = 128;  // positions of a chunk when a slice does not fit at once
 
 template <int G>
@@ -378,6 +383,8 @@ int launch_cluster(loom_b200_ctx* ctx, LbAttnParams p, int S, bool probe_only, i
         smem = cluster_smem<G>(p, S, kAcChunk, &tile_bytes);
     }
     p.tile = tile_bytes;
+    p.next_rows = (int)(kAcAhead / ((size_t)p.kv_heads * S * p.hd * 2 * sizeof(float)));
+    if (p.next_rows == 0) p.next_k = nullptr;
     const bool lean = !probe_only && !p.trace && p.M == 1 && p.seq_stride <= 0;
     auto kern = lean ? (one ? lb_attention_cluster_kernel<G, true, true> : lb_attention_cluster_kernel<G, true, false>)
                      : (one ? lb_attention_cluster_kernel<G, false, true> : lb_attention_cluster_kernel<G, false, false>);
