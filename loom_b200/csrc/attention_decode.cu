@@ -100,7 +100,8 @@ __global__ void __launch_bounds__(kAcThreads, 1) lb_attention_cluster_kernel(con
     __shared__ double s_m[G], s_l[G], s_alpha[G];  // this CTA's running maximum and sum per head, factor of what came before the chunk
     __shared__ double s_gw[kAcMaxS * G];     // combine: weight of every (slice, head)
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-    const int hd = p.hd, half = hd >> 1, kvh = blockIdx.y;
+    const int hd = p.hd, half = hd >> 1, kvh = blockIdx.y;  // (group of G query heads)
+    const int ring = kvh >> p.kv_shift;                     // its KV head
     const int n = LEAN ? 0 : blockIdx.z;  // token of the pass; with seq_stride > 0 every token is a sequence of its own
     const size_t seq_off = LEAN ? 0 : (size_t)n * (size_t)p.seq_stride;
     const uint32_t rank = cluster_ctarank(), S = cluster_nctarank();
@@ -130,8 +131,8 @@ __global__ void __launch_bounds__(kAcThreads, 1) lb_attention_cluster_kernel(con
     int k1 = k0 + per;
     if (k1 > total) k1 = total;
     const int cnt = k1 > k0 ? k1 - k0 : 0;
-    const float* kbase = p.cache_k + seq_off + (size_t)kvh * p.msl * hd;
-    const float* vbase = p.cache_v + seq_off + (size_t)kvh * p.msl * hd;
+    const float* kbase = p.cache_k + seq_off + (size_t)ring * p.msl * hd;
+    const float* vbase = p.cache_v + seq_off + (size_t)ring * p.msl * hd;
     auto fetch = [&](int which, int c0) {  // the K (0) or V (1) rows of the chunk that starts at c0; one thread
         const uint32_t bytes = (uint32_t)(cnt - c0 < cmax ? cnt - c0 : cmax) * hd * 4;
         lb_mbar_expect_tx(&bars[which], bytes);
@@ -142,10 +143,10 @@ __global__ void __launch_bounds__(kAcThreads, 1) lb_attention_cluster_kernel(con
             fetch(0, 0);
         } else if (warp == 1) {
             fetch(1, 0);
-        } else if (warp == 2 && p.next_k) {  // the next block's rows of the same positions, into L2
+        } else if (warp == 2 && p.next_k && ring << p.kv_shift == kvh) {  // the next block's rows of the same positions, into L2
             const uint32_t bytes = (uint32_t)(cnt < p.next_rows ? cnt : p.next_rows) * hd * 4;
-            l2_prefetch(p.next_k + ((size_t)kvh * p.msl + k0) * hd, bytes);
-            l2_prefetch(p.next_v + ((size_t)kvh * p.msl + k0) * hd, bytes);
+            l2_prefetch(p.next_k + ((size_t)ring * p.msl + k0) * hd, bytes);
+            l2_prefetch(p.next_v + ((size_t)ring * p.msl + k0) * hd, bytes);
         }
     }
     // queries of the group, rotated (RoPE): thread idx owns the pair (d, d + hd/2) of head g
@@ -184,14 +185,14 @@ __global__ void __launch_bounds__(kAcThreads, 1) lb_attention_cluster_kernel(con
         if (last >= k0 + c0 && last < k0 + c0 + rows && tid < half) {
             // the newest position belongs to this chunk: its ring row is not written yet; rotate the row the QKV projection
             // left in k_new into the tile and into the ring (threads 0..hd/2-1 hold the sine and cosine of their pair)
-            const float* knew = p.k_new + (size_t)n * p.kv_heads * hd + (size_t)kvh * hd;
+            const float* knew = p.k_new + (size_t)n * p.kv_heads * hd + (size_t)ring * hd;
             const double v0 = (double)knew[tid], v1 = (double)knew[tid + half];
             const float r0 = (float)__dsub_rn(__dmul_rn(v0, rc), __dmul_rn(v1, rsn));
             const float r1 = (float)__dadd_rn(__dmul_rn(v0, rsn), __dmul_rn(v1, rc));
             float* trow = kt + (size_t)(last - k0 - c0) * hd;
             trow[tid] = r0;
             trow[tid + half] = r1;
-            float* grow = p.cache_k_w + seq_off + ((size_t)kvh * p.msl + (size_t)(last % p.msl)) * hd;
+            float* grow = p.cache_k_w + seq_off + ((size_t)ring * p.msl + (size_t)(last % p.msl)) * hd;
             grow[tid] = r0;
             grow[tid + half] = r1;
         }
@@ -386,8 +387,9 @@ int launch_cluster(loom_b200_ctx* ctx, LbAttnParams p, int S, bool probe_only, i
     p.next_rows = (int)(kAcAhead / ((size_t)p.kv_heads * S * p.hd * 2 * sizeof(float)));
     if (p.next_rows == 0) p.next_k = nullptr;
     const bool lean = !probe_only && !p.trace && p.M == 1 && p.seq_stride <= 0;
-    auto kern = lean ? (one ? lb_attention_cluster_kernel<G, true, true> : lb_attention_cluster_kernel<G, true, false>)
-                     : (one ? lb_attention_cluster_kernel<G, false, true> : lb_attention_cluster_kernel<G, false, false>);
+    void (*kern)(LbAttnParams) = lean ? lb_attention_cluster_kernel<G, true, true> : lb_attention_cluster_kernel<G, false, true>;
+    if constexpr (G < 8)
+        if (!one) kern = lean ? lb_attention_cluster_kernel<G, true, false> : lb_attention_cluster_kernel<G, false, false>;
     // one bit per instantiation, per context (= per device)
     const unsigned bit = 1u << ((G == 1 ? 0 : G == 2 ? 1 : G == 4 ? 2 : 3) + (lean ? 4 : 0) + (one ? 0 : 16));
     if (!(ctx->func_attr_mask3 & bit)) {
@@ -396,7 +398,7 @@ int launch_cluster(loom_b200_ctx* ctx, LbAttnParams p, int S, bool probe_only, i
         ctx->func_attr_mask3 |= bit;
     }
     cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3(S, p.kv_heads, p.M);
+    cfg.gridDim = dim3(S, p.kv_heads << p.kv_shift, p.M);
     cfg.blockDim = dim3(kAcThreads);
     cfg.dynamicSmemBytes = smem;
     cfg.stream = ctx->stream;
@@ -425,12 +427,24 @@ int launch_cluster(loom_b200_ctx* ctx, LbAttnParams p, int S, bool probe_only, i
     return 0;
 }
 
-int dispatch_cluster(loom_b200_ctx* ctx, const LbAttnParams& p, int S, bool probe_only, int* active) {
+// `active`: how many KV heads' clusters the device holds at once
+int dispatch_cluster(loom_b200_ctx* ctx, LbAttnParams p, int S, bool probe_only, int* active) {
     switch (p.heads / p.kv_heads) {
         case 1: return launch_cluster<1>(ctx, p, S, probe_only, active);
         case 2: return launch_cluster<2>(ctx, p, S, probe_only, active);
         case 4: return launch_cluster<4>(ctx, p, S, probe_only, active);
-        case 8: return launch_cluster<8>(ctx, p, S, probe_only, active);
+        case 8: {
+            int tile_bytes = 0;
+            if (cluster_smem<8>(p, S, (p.msl + S - 1) / S, &tile_bytes) <= kAcSmem) return launch_cluster<8>(ctx, p, S, probe_only, active);
+            // Eight heads' sums over several chunks do not fit the registers (404 bytes of spills): two clusters of four heads each
+            // over the same KV head instead, which also fill more SMs.  Steps of one sequence, us a block with a ring of 4096, split
+            // kernel / eight heads with spills / two times four: two KV heads 36.5, 41.0, 36.4 at context 300, 50.5, 64.2, 44.1 at 3500;
+            // eight KV heads 61.7, 62.1, 57.0 and 125.7, 118.0, 92.4.
+            p.kv_shift = 1;
+            const int rc = launch_cluster<4>(ctx, p, S, probe_only, active);
+            if (probe_only) *active /= 2;
+            return rc;
+        }
         default: return LOOM_B200_ERR_UNSUPPORTED;
     }
 }

@@ -44,6 +44,7 @@ struct LbAttnParams {
     // cluster kernel only: the K and V rings of the decoder block that runs next (same layout), prefetched into L2; or null
     const float* next_k;
     const float* next_v;
+    int kv_shift;          // cluster kernel: 1 << kv_shift groups of query heads share a KV head (set by the launcher)
     int next_rows;         // positions of a slice that are prefetched at most (set by the launcher)
     unsigned long long* trace;
     int* status;           // device status word for bounded waits

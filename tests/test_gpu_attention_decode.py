@@ -51,7 +51,7 @@ def run(heads, kvh, hd, msl, offsets, seed):
         ctx.close()
 
 
-@pytest.mark.parametrize("heads,kvh,hd", [(2, 2, 128), (4, 2, 128), (4, 1, 128), (8, 1, 128), (8, 2, 48)])
+@pytest.mark.parametrize("heads,kvh,hd", [(2, 2, 128), (4, 2, 128), (4, 1, 128), (8, 1, 128), (8, 2, 48), (16, 2, 64)])
 @pytest.mark.parametrize("msl,context", [(9000, 1), (9000, 2046), (9000, 2047), (9000, 2048), (9000, 4111), (3000, 2999)])
 def test_one_sequence(heads, kvh, hd, msl, context):
     run(heads, kvh, hd, msl, [context], context)
@@ -62,6 +62,8 @@ def test_one_sequence(heads, kvh, hd, msl, context):
     (8, 8, 128, 3000, [1, 254, 255, 256, 300, 2, 700, 511]),  # pairs of CTAs
     (32, 8, 64, 6000, [126, 127, 128, 1, 2500, 3, 4, 5]),
     (8, 1, 128, 9000, [4095] * 2),
+    (64, 8, 80, 5000, [1, 2047, 300, 4000, 5, 130, 64, 2]),  # eight heads as two times four, 16 pairs of clusters
+    (16, 2, 80, 12000, [3000, 1, 9001]),
     (16, 16, 64, 4000, [127, 128, 129, 1, 400, 2, 3, 256, 5, 600, 1]),  # single CTAs, then a pass of three
 ])
 def test_several_sequences(heads, kvh, hd, msl, offsets):
