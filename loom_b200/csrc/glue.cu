@@ -850,6 +850,17 @@ int lb_launch_rope(loom_b200_ctx* ctx, const LbRopeParams& pin) {
 
 size_t lb_attn_part_elems(int M, int heads, int hd, int splits) { return (size_t)M * heads * splits * (hd + 2); }
 
+// tile: short tiles let more CTAs share an SM
+static int split_tile(const LbAttnParams& p) {
+    const int t = ((p.max_chunk + 1) / 2 + 7) / 8 * 8;  // half of the longest chunk: two tiles at most when the ring is full
+    return t > kAttnTile ? kAttnTile : t < 8 ? 8 : t;
+}
+static size_t split_smem(const LbAttnParams& p) {
+    const int G = p.hd >= kAttnThreads ? 1 : kAttnThreads / p.hd;
+    return (size_t)(p.hd + (size_t)G * p.hd + p.max_chunk) * sizeof(double) + 2 * (size_t)split_tile(p) * p.hd * sizeof(float);
+}
+bool lb_attention_splits_fit(const LbAttnParams& p) { return p.hd % 8 != 0 || split_smem(p) <= 200 * 1024; }
+
 int lb_launch_attention(loom_b200_ctx* ctx, const LbAttnParams& pin) {
     LbAttnParams p = pin;
     p.trace = lb_trace_row(ctx, "attention");
@@ -871,12 +882,8 @@ int lb_launch_attention(loom_b200_ctx* ctx, const LbAttnParams& pin) {
     LB_REQUIRE(ctx, p.heads % p.kv_heads == 0, "attention: %d heads over %d kv heads", p.heads, p.kv_heads);
     LB_REQUIRE(ctx, p.hd <= kAttnThreads, "attention: head_dim %d above %d is not supported", p.hd, kAttnThreads);
     LB_REQUIRE(ctx, p.splits >= 1 && p.splits <= 64, "attention: %d splits", p.splits);
-    const int G = p.hd >= kAttnThreads ? 1 : kAttnThreads / p.hd;
-    // tile: short tiles let more CTAs share an SM
-    p.tile = ((p.max_chunk + 1) / 2 + 7) / 8 * 8;  // half of the longest chunk: two tiles at most when the ring is full
-    if (p.tile > kAttnTile) p.tile = kAttnTile;
-    if (p.tile < 8) p.tile = 8;
-    size_t smem = (size_t)(p.hd + (size_t)G * p.hd + p.max_chunk) * sizeof(double) + 2 * (size_t)p.tile * p.hd * sizeof(float);
+    p.tile = split_tile(p);
+    const size_t smem = split_smem(p);
     if (smem > 200 * 1024) return lb_fail(ctx, LOOM_B200_ERR_UNSUPPORTED, "attention: %d positions per CTA need %zu B of shared memory", p.max_chunk, smem);
     if (smem > 48 * 1024 && !(ctx->func_attr_mask & (1u << 30))) {
         LB_CUDA(ctx, cudaFuncSetAttribute(lb_attention_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024));

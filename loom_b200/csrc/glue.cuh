@@ -50,6 +50,8 @@ struct LbAttnParams {
     int* status;           // device status word for bounded waits
 };
 int lb_launch_attention(loom_b200_ctx* ctx, const LbAttnParams& p);
+// whether a CTA of it has room for the scores of max_chunk positions
+bool lb_attention_splits_fit(const LbAttnParams& p);
 // One-token steps with RoPE folded in, of one sequence (sequences = 0) or of a pass of several: the cluster kernel
 // (attention_decode.cu).  lb_attention_cluster_size returns the cluster size to use (CTAs per sequence and KV head), or 0 when
 // the shape or the device does not allow it; the launch takes that size.

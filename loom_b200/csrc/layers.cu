@@ -224,6 +224,11 @@ int lb_mha_attn_dev(loom_b200_mha* m, const LbMhaStepArgs& a) {
             return lb_launch_attention_cluster(ctx, t, cluster);
         }
     }
+    // several sequences without the cluster kernel (its option or the folded rotation off): as many splits as the ring's length asks for
+    while (a.lanes_pos && !lb_attention_splits_fit(t) && t.splits < m->splits) {
+        t.splits = t.splits * 2 > m->splits ? m->splits : t.splits * 2;
+        t.max_chunk = (m->msl + t.splits - 1) / t.splits;
+    }
     return lb_launch_attention(ctx, t);
 }
 

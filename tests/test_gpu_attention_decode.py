@@ -16,10 +16,12 @@ pytestmark = pytest.mark.gpu
 THREADS = min(16, orc.host_threads())
 
 
-def run(heads, kvh, hd, msl, offsets, seed):
+def run(heads, kvh, hd, msl, offsets, seed, **options):
     """One step of len(offsets) sequences, sequence i behind offsets[i] restored positions."""
     rng = np.random.default_rng(seed)
     ctx = loom_b200.Context(0)
+    for name, value in options.items():
+        ctx.set_option(name, value)
     H, inter, V, B = heads * hd, 256, 64, len(offsets)
     shapes = ((H, H), (kvh * hd, H), (kvh * hd, H), (H, H), (inter, H), (inter, H), (H, inter))
     packed = [orc.pack_f32((rng.standard_normal(r * c) * 0.02).astype(np.float32), r, c) for r, c in shapes]
@@ -68,3 +70,10 @@ def test_one_sequence(heads, kvh, hd, msl, context):
 ])
 def test_several_sequences(heads, kvh, hd, msl, offsets):
     run(heads, kvh, hd, msl, offsets, len(offsets))
+
+
+@pytest.mark.parametrize("options", [dict(attn_cluster=0), dict(fold_rope=0), dict(attn_cluster=0, decode_splits=1)], ids=["cluster off", "rotation apart", "one split"])
+@pytest.mark.parametrize("heads,kvh,hd,msl", [(4, 1, 128, 61000), (8, 1, 128, 130000), (16, 16, 64, 105000)])
+def test_several_sequences_without_the_cluster_kernel(options, heads, kvh, hd, msl):
+    """Rings of which a quarter is more than a CTA's scores have room for (59,900 positions at head dimension 128)."""
+    run(heads, kvh, hd, msl, [20000, 1, 640], heads, **options)
