@@ -1,5 +1,5 @@
-"""The token-block products of a stack where their K slices are shared out: few tiles (a CTA gets a run of slices that may end inside a
-tile, or a cluster splits a tile), ragged rows, columns and tokens, and every epilogue (gate, gelu, residual, image, per-head blocks).
+"""The token-block products of a stack over few tiles (with plain multiply-adds the CTAs of a cluster share a tile's K slices), ragged rows,
+columns and tokens, and every epilogue (gate, gelu, residual, image, per-head blocks).
 
 Logits of a whole prompt against the plain oracles; tolerances as in test_gpu_donodra.py and test_gpu_stack.py.
 """
@@ -41,7 +41,7 @@ def test_prompts_over_few_tiles(ctx, dtype, tensor_cores, width, ff, tokens):
             tol = 2e-5 if dtype == F32 else tol
             assert np.quantile(e, 0.9) < tol and e.max() < 5 * tol
             dec.reset()
-            assert np.array_equal(dec.extend(tok, range(tokens)), first)  # whoever arrives last adds in the same order
+            assert np.array_equal(dec.extend(tok, range(tokens)), first)  # the parts of a tile meet in the order of K
             dec.close()
     finally:
         ctx.set_option("dense_tc", 1)

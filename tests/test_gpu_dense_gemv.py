@@ -1,8 +1,8 @@
 """The one-token products of a stack where their weight ring can go wrong: several strips of rows per CTA, fewer K slices than warps,
-rows that leave room for one slot of the ring or for none, and the input rows' edges (columns beyond the registers of a thread,
-rows that are no multiple of 16 bytes).
+rows that leave room for one slot of the ring or for none, and the input rows' edges (columns beyond the registers of a thread, for
+every prologue, rows that are no multiple of 16 bytes).
 
-Every sequence of a batch is held to the plain oracle; tolerances as in test_gpu_donodra.py.
+Every sequence of a batch is held to the plain oracle; tolerances as in test_gpu_donodra.py and test_gpu_stack.py.
 """
 import numpy as np
 import pytest
@@ -10,6 +10,7 @@ import pytest
 import donodra_oracle as do
 import donodrakit as dk
 import loom_b200
+import stack_oracle as so
 import stackkit as kit
 from loom_b200 import cabi, models
 
@@ -113,3 +114,23 @@ def test_infinite_weights_of_an_expert_stay_with_its_tokens(ctx, dtype, batch, f
         assert np.array_equal(got[~lost], clean[~lost])
         chosen += lost
     assert np.array_equal(chosen, np.full(batch, top))
+
+
+@pytest.mark.parametrize("dtype,width,heads,vdim,taps,batch", [
+    (F32, 2100, 17, 128, 4, 1), (F32, 1100, 9, 128, 3, 2), (F32, 2100, 11, 200, 2, 3),  # registers hold 2048 columns of a row, 1024 with two
+    (F32, 1101, 3, 700, 5, 2), (BF16, 4200, 17, 256, 4, 1), (BF16, 2120, 17, 128, 7, 2), (BF16, 4200, 9, 472, 4, 3)])  # 4096 and 2048
+def test_convolved_and_gated_rows_beyond_the_registers(ctx, dtype, width, heads, vdim, taps, batch):
+    """A convolution over the input rows and head norms with gates in front of the output product, both longer than what a thread keeps."""
+    cfg = kit.config(width, 70, [kit.gla(heads, 16, vdim, 8.0, kit.dense(40)), kit.gla(1, 16, 24, 8.0, None)], taps=taps)
+    w = kit.random_weights(cfg, 9)
+    dec = models.build(ctx, cfg, kit.Weights(w), models.LoadOptions(dtype, 16, batch))
+    tok = np.random.default_rng(4).integers(0, 70, (batch, 8)).astype(np.int32)
+    for i in range(batch):
+        dec.select(i)
+        dec.extend(tok[i, :1])
+    got = [np.array(dec.step_batch(tok[:, j]) if batch > 1 else dec.extend(tok[:, j], [0])) for j in range(1, 8)]
+    for i in range(batch):
+        want, _ = so.forward(cfg, w, tok[i])
+        e = kit.error(np.stack([g[i] for g in got]), want[1:])
+        assert np.quantile(e, 0.9) < {F32: 2e-5, BF16: 0.06}[dtype] and e.max() < 5 * {F32: 2e-5, BF16: 0.06}[dtype], i
+    dec.close()
