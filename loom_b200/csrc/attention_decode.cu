@@ -10,6 +10,7 @@
 //     one contiguous block) and serves all query heads of the GQA group from them: every K/V element is converted
 //     to float64 once and used by every head of the group.  A slice that does not fit goes through in chunks with a running
 //     softmax: the next K rows travel behind softmax and weighted V, the next V rows behind the next scores.
+//     (Eight query heads per KV head over several chunks: two clusters of four heads each.)
 //   * S: one sequence takes the largest cluster of which the device holds one per KV head; a pass of several takes the
 //     largest of which it holds one per (sequence, KV head), down to single CTAs (eight sequences x eight KV heads: pairs).
 //   * Bound: float64 issue and the float32 -> float64 conversions (16 lanes a clock) behind one another's latencies.  Measured:
@@ -32,11 +33,6 @@ constexpr int kAcWarps = kAcThreads / 32;
 constexpr int kAcMaxG = 8;   // query heads per KV head
 constexpr int kAcMaxS = 16;  // CTAs per cluster
 
-__device__ __forceinline__ uint32_t cluster_ctarank() {
-    uint32_t r;
-    asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(r));
-    return r;
-}
 __device__ __forceinline__ uint32_t cluster_nctarank() {
     uint32_t r;
     asm volatile("mov.u32 %0, %%cluster_nctarank;" : "=r"(r));
@@ -44,15 +40,10 @@ __device__ __forceinline__ uint32_t cluster_nctarank() {
 }
 // address of the same shared-memory location in CTA `rank` of this cluster
 __device__ __forceinline__ uint32_t map_to_rank(const void* smem_ptr, uint32_t rank) {
-    uint32_t a = lb_smem_u32(smem_ptr), r;
-    asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(a), "r"(rank));
-    return r;
+    return lb_cluster_addr(lb_smem_u32(smem_ptr), rank);
 }
 __device__ __forceinline__ void st_cluster_f64(uint32_t addr, double v) {
     asm volatile("st.shared::cluster.f64 [%0], %1;" ::"r"(addr), "d"(v) : "memory");
-}
-__device__ __forceinline__ void cluster_sync_all() {
-    asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
 }
 __device__ __forceinline__ void l2_prefetch(const void* gptr, uint32_t bytes) {
     asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;" ::"l"(gptr), "r"(bytes) : "memory");
@@ -104,7 +95,7 @@ __global__ void __launch_bounds__(kAcThreads, 1) lb_attention_cluster_kernel(con
     const int ring = kvh >> p.kv_shift;                     // its KV head
     const int n = LEAN ? 0 : blockIdx.z;  // token of the pass; with seq_stride > 0 every token is a sequence of its own
     const size_t seq_off = LEAN ? 0 : (size_t)n * (size_t)p.seq_stride;
-    const uint32_t rank = cluster_ctarank(), S = cluster_nctarank();
+    const uint32_t rank = lb_cluster_rank(), S = cluster_nctarank();
     const int cmax = p.max_chunk;  // positions one CTA holds at a time
     const int dps = hd / (int)S;   // output dimensions every CTA combines
     float* kt = reinterpret_cast<float*>(smem_raw);            // [cmax, hd]
@@ -327,7 +318,7 @@ __global__ void __launch_bounds__(kAcThreads, 1) lb_attention_cluster_kernel(con
         st_cluster_f64(map_to_rank(slot, owner), cnt > 0 ? s_m[g] : -1e300);
         st_cluster_f64(map_to_rank(slot + 1, owner), cnt > 0 ? s_l[g] : 0.0);
     }
-    cluster_sync_all();
+    lb_cluster_sync();
 
     // ---- combine the S slices for this CTA's dps dimensions of every head ----
     for (int idx = tid; idx < (int)S * G; idx += kAcThreads) {

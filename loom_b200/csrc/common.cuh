@@ -70,7 +70,7 @@ struct loom_b200_ctx {
     void* argmax_scratch = nullptr;  // per-CTA partial maxima of the greedy argmax
     void* head_scratch = nullptr;    // per-CTA partial maxima and arrival counter of the LM head's greedy tail
     unsigned func_attr_mask = 0;  // kernels whose shared-memory limit was raised on this device
-    unsigned func_attr_mask2 = 0; // the same for the streaming head
+    unsigned func_attr_mask2 = 0; // the same: the head (bits 8-10), attention of odd head dimensions (16), the int8 GEMM (20-27)
     unsigned func_attr_mask3 = 0; // the same for the cluster attention instantiations
     int opt_head_stream = 1;      // the LM head streams its rows through shared memory with bulk copies (0 = warp-per-row loads)
     int opt_attn_cluster = 1;     // one-token decoder steps run the attention as a thread-block cluster per KV head (0: off, 1: the largest cluster that fits, 2..16: at most that many CTAs)
@@ -268,6 +268,25 @@ __device__ __forceinline__ void lb_trace(unsigned long long* row, int k) {
 // ---- sm_100a plumbing: mbarrier, bulk async copy (TMA engine), programmatic dependent launch ------
 
 __device__ __forceinline__ uint32_t lb_smem_u32(const void* p) { return (uint32_t)__cvta_generic_to_shared(p); }
+
+// thread-block clusters: this CTA's place, the address of a shared-memory location in another CTA, a barrier of all
+__device__ __forceinline__ uint32_t lb_cluster_rank() {
+    uint32_t r;
+    asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(r));
+    return r;
+}
+__device__ __forceinline__ uint32_t lb_cluster_addr(uint32_t smem_addr, uint32_t rank) {
+    uint32_t r;
+    asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(smem_addr), "r"(rank));
+    return r;
+}
+__device__ __forceinline__ void lb_cluster_sync() {
+    asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
+}
+// float64 matrix instruction: eight rows x four columns times four columns x eight columns
+__device__ __forceinline__ void lb_dmma_884(double (&c)[2], double a, double b) {
+    asm volatile("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0, %1}, {%2}, {%3}, {%0, %1};" : "+d"(c[0]), "+d"(c[1]) : "d"(a), "d"(b));
+}
 
 __device__ __forceinline__ void lb_mbar_init(uint64_t* bar, uint32_t count) {
     asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(lb_smem_u32(bar)), "r"(count));

@@ -133,7 +133,7 @@ __device__ __forceinline__ void step_pairs<float>(GemvAcc<float>& acc, const uin
 // ---- the weight ring: every warp copies the chunks it will multiply itself (16 bytes a lane and copy, so no barrier of the
 // block is needed between the copies and their use), `depth` K slices ahead.  One batch in registers and one in flight (32 KB an
 // SM) left the routed products at half of HBM's rate: a step of eight sequences over 32 experts of 4096 x 1792 (four layers) took
-// 1.53 ms, 1.27 ms with the ring (100 KB an SM); a one-sequence step with gated feed-forwards of 6912 572 and 533 us.  Products
+// 1.53 ms, 1.27 ms with the ring (96 KB a CTA, two CTAs an SM); a one-sequence step with gated feed-forwards of 6912 572 and 533 us.  Products
 // whose 16-row strips are fewer than the CTAs that fit are bound by the chain of their input rows, not by this. ----
 constexpr int kRingUnit = kGemvThreads * 16;  // bytes of one 16-byte chunk per thread
 constexpr int kRingMax = 8;
@@ -723,15 +723,9 @@ int gemv_dispatch(loom_b200_ctx* ctx, int pro, int epi, const LbDenseGemv& p) {
 
 constexpr int kSimtTile = 64, kSimtThreads = 128, kSimtStages = 3, kSimtHalf = kSimtTile * 128, kSimtLd = kSimtTile + 4;
 
-__device__ __forceinline__ uint32_t simt_rank() {
-    uint32_t r;
-    asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(r));
-    return r;
-}
 __device__ __forceinline__ float4 simt_peer(uint32_t addr, uint32_t rank) {
-    uint32_t a;
+    const uint32_t a = lb_cluster_addr(addr, rank);
     float4 v;
-    asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(a) : "r"(addr), "r"(rank));
     asm volatile("ld.shared::cluster.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "r"(a) : "memory");
     return v;
 }
@@ -760,7 +754,7 @@ __global__ void __launch_bounds__(kSimtThreads, EPI == LB_DEPI_GLU || EPI == LB_
     constexpr int kParts = kDual ? 3 : 2;
     extern __shared__ __align__(16) uint8_t smem[];
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-    const uint32_t rank = S > 1 ? simt_rank() : 0;
+    const uint32_t rank = S > 1 ? lb_cluster_rank() : 0;
     const int row0 = (int)(blockIdx.x / S) * kSimtTile, tok0 = blockIdx.y * kSimtTile;
     lb_pdl_launch_dependents();
     lb_pdl_wait();
@@ -850,7 +844,7 @@ __global__ void __launch_bounds__(kSimtThreads, EPI == LB_DEPI_GLU || EPI == LB_
             }
         }
     if (S > 1)
-        asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
+        lb_cluster_sync();
     else
         __syncthreads();
     const int per = 512 / S;  // (token, eight rows) pairs of a CTA
@@ -907,7 +901,7 @@ __global__ void __launch_bounds__(kSimtThreads, EPI == LB_DEPI_GLU || EPI == LB_
         }
     }
     if (S > 1)  // a neighbour may still read this CTA's sums
-        asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
+        lb_cluster_sync();
 }
 
 template <typename WT, int EPI>

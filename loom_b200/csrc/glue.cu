@@ -608,10 +608,6 @@ __global__ void lb_set_scalar_kernel(int* p, int value) {
 // dimensions of half w%2.  Row strides are chosen so that a fragment load touches every bank once.
 constexpr int kPfRows = 64, kPfKeys = 64, kPfThreads = 256;
 
-__device__ __forceinline__ void dmma_884(double (&c)[2], double a, double b) {
-    asm volatile("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0,%1}, {%2}, {%3}, {%0,%1};" : "+d"(c[0]), "+d"(c[1]) : "d"(a), "d"(b));
-}
-
 __global__ void __launch_bounds__(kPfThreads, 1) lb_attention_prefill_kernel(const LbAttnParams p) {
     extern __shared__ __align__(128) uint8_t smem_raw[];
     __shared__ __align__(8) uint64_t bar;
@@ -714,8 +710,8 @@ __global__ void __launch_bounds__(kPfThreads, 1) lb_attention_prefill_kernel(con
                 for (int j = 0; j < 4; ++j) b[j] = kb[(size_t)(8 * j) * kstride + d];
 #pragma unroll
                 for (int j = 0; j < 4; ++j) {
-                    dmma_884(c[0][j], a0, b[j]);
-                    dmma_884(c[1][j], a1, b[j]);
+                    lb_dmma_884(c[0][j], a0, b[j]);
+                    lb_dmma_884(c[1][j], a1, b[j]);
                 }
             }
 #pragma unroll
@@ -785,8 +781,8 @@ __global__ void __launch_bounds__(kPfThreads, 1) lb_attention_prefill_kernel(con
                 for (int j = 0; j < 8; ++j) {
                     if (j < nfr) {
                         const double b = vb[(size_t)k * vstride + 8 * j];
-                        dmma_884(o[0][j], a0, b);
-                        dmma_884(o[1][j], a1, b);
+                        lb_dmma_884(o[0][j], a0, b);
+                        lb_dmma_884(o[1][j], a1, b);
                     }
                 }
             }

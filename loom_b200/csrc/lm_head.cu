@@ -227,14 +227,11 @@ __global__ void __launch_bounds__(NW * 32, 1) lb_lm_head_stream_kernel(const LbL
 // converted to float64 once per 32 rows; lane (g, t) takes 16 bytes of row g, columns 4t.. of a 16-column step, for the table
 // (global memory, straight into registers, two steps ahead) and for the hidden rows (shared memory, float32: they are float32
 // values by definition) alike, so which column an MMA calls its k-th is the same for both and needs no shuffle.  Four warps share
-// a strip of 32 rows by columns and add up in shared memory: 867 rows of a CTA's share are 27 strips for four groups.
+// a strip of 32 rows by columns and add up in shared memory: 867 rows of a CTA's share are 28 strips for four groups.
 // Bound: float64 issue (8 x 4096 columns, 128256 rows: 0.24 ms of MMAs, and the conversions to float64 share their pipe, 0.15 ms);
 // HBM alone would be 0.29 ms.  Measured 0.40 ms for eight rows where four passes of two rows on plain FMAs took 1.88 ms.
 constexpr int kHmWarps = 16, kHmSplit = 4, kHmGroups = kHmWarps / kHmSplit, kHmTiles = 4, kHmRows = 8 * kHmTiles;
 
-__device__ __forceinline__ void dmma_884(double (&c)[2], double a, double b) {
-    asm volatile("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0, %1}, {%2}, {%3}, {%0, %1};" : "+d"(c[0]), "+d"(c[1]) : "d"(a), "d"(b));
-}
 __device__ __forceinline__ float4 ldg_table(const float* p, uint64_t policy) {
     float4 v;
     asm volatile("ld.global.nc.L1::no_allocate.L2::cache_hint.v4.f32 {%0,%1,%2,%3}, [%4], %5;" : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "l"(p), "l"(policy));
@@ -319,13 +316,13 @@ __global__ void __launch_bounds__(kHmWarps * 32, 1) lb_lm_head_rows_kernel(const
                 if (g < nb && col < H) h = *reinterpret_cast<const float4*>(sh + (size_t)g * ld + col);
                 const double h0 = (double)h.x, h1 = (double)h.y, h2 = (double)h.z, h3 = (double)h.w;
 #pragma unroll
-                for (int i = 0; i < kHmTiles; ++i) dmma_884(c[i], (double)w[i].x, h0);
+                for (int i = 0; i < kHmTiles; ++i) lb_dmma_884(c[i], (double)w[i].x, h0);
 #pragma unroll
-                for (int i = 0; i < kHmTiles; ++i) dmma_884(c[i], (double)w[i].y, h1);
+                for (int i = 0; i < kHmTiles; ++i) lb_dmma_884(c[i], (double)w[i].y, h1);
 #pragma unroll
-                for (int i = 0; i < kHmTiles; ++i) dmma_884(c[i], (double)w[i].z, h2);
+                for (int i = 0; i < kHmTiles; ++i) lb_dmma_884(c[i], (double)w[i].z, h2);
 #pragma unroll
-                for (int i = 0; i < kHmTiles; ++i) dmma_884(c[i], (double)w[i].w, h3);
+                for (int i = 0; i < kHmTiles; ++i) lb_dmma_884(c[i], (double)w[i].w, h3);
             }
         }
         if (next < r1)  // the next strip's first steps travel while the sums meet
