@@ -159,7 +159,11 @@ __device__ __forceinline__ void ring_wait(int depth) {
 }
 
 // KW warps share a strip of 16 rows by K slices, 8/KW strips run side by side in a CTA.
-template <typename WT, int PRO, int EPI>
+// RING: weights through the ring; else (the input rows leave room for less than two slots) straight into registers, as far ahead as
+// those allow.  Requests on four layers with second products of 24576 columns, short prompts and 24 steps: four bf16 sequences 11.9 ms
+// (12.3 before there was a ring, 12.5 with a ring of one slot), two float32 ones 15.7 ms (17.0 with one slot).  A kernel of its own:
+// as a branch it cost the ring's registers, 31.7 -> 30.4 ms for 48 steps of the 2560-wide Zitupel behind 100 tokens without it.
+template <typename WT, int PRO, int EPI, bool RING>
 __global__ void __launch_bounds__(kGemvThreads, 2) lb_dense_gemv_kernel(const LbDenseGemv p, int Mp_launch, int KW, bool vec, int ring_off, int depth) {
     extern __shared__ __align__(16) uint8_t smem[];
     constexpr int C = LbElem<WT>::kChunk;
@@ -234,7 +238,7 @@ __global__ void __launch_bounds__(kGemvThreads, 2) lb_dense_gemv_kernel(const Lb
     };
     // the weights do not depend on earlier launches: the ring is filled before the dependency wait
     constexpr bool kEarly = PRO != LB_DPRO_MOE && PRO != LB_DPRO_PAIRS && !kStage;
-    if (kEarly)
+    if (kEarly && RING)
         for (int i = 0; i < depth; ++i) fetch();
     // nor do the vectors of the prologue, which a layer's weights have pushed out of the L2 cache since the last token
     if (kEarly || kStage) {
@@ -321,7 +325,8 @@ __global__ void __launch_bounds__(kGemvThreads, 2) lb_dense_gemv_kernel(const Lb
                 }
             s_n = n;
         }
-        for (int i = 0; i < depth; ++i) fetch();
+        if (RING)
+            for (int i = 0; i < depth; ++i) fetch();
         __syncthreads();
         M = s_n;
         Mp = 1;
@@ -562,20 +567,35 @@ __global__ void __launch_bounds__(kGemvThreads, 2) lb_dense_gemv_kernel(const Lb
             int at_end = 0, at = -1;  // PAIRS: end of the present expert's slices, its place in the list
             unsigned chose = 0;
             const uint8_t *d1 = strip_ptr(w1, strip) + lane_off, *d2 = kDual ? strip_ptr(w2, strip) + lane_off : nullptr;
+            constexpr int kParts = kDual ? 8 : 4, kDirect = kDual ? 1 : 2;
+            uint4 ahead[kDirect][kParts];
+            auto direct = [&](uint4 (&d)[kParts], int s) {
+                if (s >= total) return;
+#pragma unroll
+                for (int u = 0; u < 4; ++u) {
+                    d[u] = ldg_stream(d1 + (size_t)s * kImgBlock + u * 512);
+                    if (kDual) d[4 + u] = ldg_stream(d2 + (size_t)s * kImgBlock + u * 512);
+                }
+            };
+            if (!RING)
+#pragma unroll
+                for (int i = 0; i < kDirect; ++i) direct(ahead[i], kw + i * KW);
             for (int s = kw; s < total; s += KW) {
                 uint4 w[8];
                 const uint4* rs = reinterpret_cast<const uint4*>(ring + (size_t)slot * kUnits * kRingUnit);
-                if (PRO == LB_DPRO_PAIRS || depth > 0) {
+                if (RING) {
                     ring_wait(depth);
                     __syncwarp();  // a lane reads what other lanes fetched
 #pragma unroll
                     for (int u = 0; u < (kDual ? 8 : 4); ++u) w[u] = rs[u * kGemvThreads + at_read];
-                } else {  // the input rows leave no room for a ring
+                } else {
 #pragma unroll
-                    for (int u = 0; u < 4; ++u) {
-                        w[u] = ldg_stream(d1 + (size_t)s * kImgBlock + u * 512);
-                        if (kDual) w[4 + u] = ldg_stream(d2 + (size_t)s * kImgBlock + u * 512);
-                    }
+                    for (int u = 0; u < kParts; ++u) w[u] = ahead[0][u];
+#pragma unroll
+                    for (int i = 0; i + 1 < kDirect; ++i)
+#pragma unroll
+                        for (int u = 0; u < kParts; ++u) ahead[i][u] = ahead[i + 1][u];
+                    direct(ahead[kDirect - 1], s + kDirect * KW);
                 }
                 if (PRO == LB_DPRO_PAIRS) {
                     if (s >= at_end) {  // (KW <= slices: the next expert, never one further)
@@ -594,7 +614,7 @@ __global__ void __launch_bounds__(kGemvThreads, 2) lb_dense_gemv_kernel(const Lb
                         acc2.step(w[5], w[7], x0 + 4 * Mp, Mp, M, g);
                     }
                 }
-                if (PRO == LB_DPRO_PAIRS || depth > 0) {
+                if (RING) {
                     slot = slot + 1 == depth ? 0 : slot + 1;
                     __syncwarp();  // every lane has read the slot that is filled again
                     fetch();
@@ -660,9 +680,16 @@ int gemv_launch(loom_b200_ctx* ctx, const LbDenseGemv& pin) {
         const int room = ring_off + 2 * kSlot <= kGemvSmemHalf ? kGemvSmemHalf : (int)kGemvSmemX + 16 * 1024;
         depth = room > ring_off ? (room - ring_off) / kSlot : 0;
         if (depth > kRingMax) depth = kRingMax;
+        if (depth < 2) depth = 0;
         smem = (size_t)ring_off + (size_t)depth * kSlot;
     }
-    if (smem > 36 * 1024) LB_BIG_SMEM(ctx, (lb_dense_gemv_kernel<WT, PRO, EPI>), kGemvSmemX + 16 * 1024);
+    constexpr bool kStage = EPI == LB_DEPI_STAGE, kNoRing = !kPairs && !kStage;  // (routed pairs always have their slots, staging multiplies nothing)
+    const bool direct = kNoRing && depth == 0;
+    if (direct) {
+        LB_BIG_SMEM(ctx, (lb_dense_gemv_kernel<WT, PRO, EPI, !kNoRing>), kGemvSmemX + 16 * 1024);
+    } else if (smem > 36 * 1024) {
+        LB_BIG_SMEM(ctx, (lb_dense_gemv_kernel<WT, PRO, EPI, true>), kGemvSmemX + 16 * 1024);
+    }
     int gx = lb_ceil_div(strips, SP), gy = 1, share = cap;
     if (EPI == LB_DEPI_STAGE) {
         gx = share = p.M;
@@ -672,7 +699,11 @@ int gemv_launch(loom_b200_ctx* ctx, const LbDenseGemv& pin) {
         if (share < 1) share = 1;
     }
     if (gx > share) gx = lb_ceil_div(gx, lb_ceil_div(gx, share));  // equal numbers of strips per CTA
-    LB_LAUNCH(ctx, (lb_dense_gemv_kernel<WT, PRO, EPI>), dim3(gx, gy), dim3(kGemvThreads), smem, p, Mp, KW, vec, ring_off, depth);
+    if (direct) {
+        LB_LAUNCH(ctx, (lb_dense_gemv_kernel<WT, PRO, EPI, !kNoRing>), dim3(gx, gy), dim3(kGemvThreads), smem, p, Mp, KW, vec, ring_off, depth);
+        return 0;
+    }
+    LB_LAUNCH(ctx, (lb_dense_gemv_kernel<WT, PRO, EPI, true>), dim3(gx, gy), dim3(kGemvThreads), smem, p, Mp, KW, vec, ring_off, depth);
     return 0;
 }
 

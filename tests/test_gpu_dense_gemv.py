@@ -29,6 +29,7 @@ def ctx():
 @pytest.mark.parametrize("dtype,width,ff,vocab,batch", [
     (BF16, 64, 5000, 9500, 1), (F32, 32, 2500, 9500, 2), (BF16, 200, 4800, 70, 3), (F32, 77, 4801, 70, 1),
     (BF16, 25536, 24, 70, 4),  # 204,288 B of input rows: one slot of the single ring, none of the double one
+    (BF16, 64, 12500, 70, 8), (F32, 32, 12400, 70, 4), (BF16, 40, 24600, 70, 3),  # the same for the second product's rows
     (BF16, 17000, 40, 70, 1), (F32, 12768, 24, 70, 4), (F32, 8500, 40, 70, 1)])
 def test_steps_of_wide_and_narrow_stacks(ctx, dtype, width, ff, vocab, batch):
     cfg = dk.config(width, vocab, [dk.mlstm(2, 8, 24, 9.0, ff), dk.attention(2, 1, 16, 16, 32, 9.0, 0.3, None)])
