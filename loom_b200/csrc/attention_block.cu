@@ -68,12 +68,12 @@ __global__ void __launch_bounds__(kAtThreads, 2) lb_attn_block_kernel(const LbAt
         }
     };
     auto scores = [&](int j) {
-        for (int k = 0; k < p.dchunks / 2; ++k)
-            lb_mma_f16(tmem, lb_smem_desc(a_q + k * 256, 128, sbo_d), lb_smem_desc(a_k + (j & 1) * kbytes + k * 256, 128, sbo_d), id_s, k > 0 ? 1u : 0u);
+        const uint64_t q = lb_smem_desc(a_q, 128, sbo_d), key = lb_smem_desc(a_k + (j & 1) * kbytes, 128, sbo_d);
+        for (int k = 0; k < p.dchunks / 2; ++k) lb_mma_f16(tmem, q + k * 16, key + k * 16, id_s, k > 0 ? 1u : 0u);
         lb_mma_commit(&bar_s);
     };
     bool failed = false;
-    if (tid == 0) {
+    if (warp == 0 && lb_elect()) {
         lb_mbar_expect_tx(&bar_q, qbytes);
         lb_bulk_g2s(sq, p.q + ((size_t)qb * p.heads + h) * qbytes, qbytes, &bar_q);
         load(0);
@@ -155,13 +155,15 @@ __global__ void __launch_bounds__(kAtThreads, 2) lb_attn_block_kernel(const LbAt
         asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
         lb_tc_fence_before();
         lb_mbar_arrive(&bar_p);
-        if (tid == 0) {  // every row's weights are in shared memory, S_j and O_(j-1) have left tensor memory
+        __syncwarp();
+        if (warp == 0 && lb_elect()) {  // every row's weights are in shared memory, S_j and O_(j-1) have left tensor memory
             if (!lb_mbar_wait_bounded(&bar_p, (uint32_t)(j & 1), kTcWaitLimit) || !lb_mbar_wait_bounded(&bar_v[j & 1], (uint32_t)((j >> 1) & 1), kTcWaitLimit)) {
                 failed = true;
             } else {
                 lb_tc_fence_after();
-                for (int k = 0; k < kAtKeys / 16; ++k)
-                    lb_mma_f16(tmem + kAtKeys, lb_smem_desc(a_p + k * 256, 128, 1024), lb_smem_desc(a_v + (j & 1) * kVStage + k * 256, 128, 1024), id_o, k > 0 ? 1u : 0u);
+                const uint64_t w = lb_smem_desc(a_p, 128, 1024), val = lb_smem_desc(a_v + (j & 1) * kVStage, 128, 1024);
+#pragma unroll
+                for (int k = 0; k < kAtKeys / 16; ++k) lb_mma_f16(tmem + kAtKeys, w + k * 16, val + k * 16, id_o, k > 0 ? 1u : 0u);
                 lb_mma_commit(&bar_o);
                 if (j + 1 < ntiles) {
                     if (lb_mbar_wait_bounded(&bar_k[(j + 1) & 1], (uint32_t)(((j + 1) >> 1) & 1), kTcWaitLimit))
@@ -177,7 +179,7 @@ __global__ void __launch_bounds__(kAtThreads, 2) lb_attn_block_kernel(const LbAt
             failed = true;
             break;
         }
-        if (tid == 0 && j + 2 < ntiles) load(j + 2);  // S_j and O_j are done: their stage is free
+        if (warp == 0 && j + 2 < ntiles && lb_elect()) load(j + 2);  // S_j and O_j are done: their stage is free
         __syncwarp();
         lb_tc_fence_after();
         constexpr int VS = VC % 64 == 0 ? 64 : VC % 32 == 0 ? 32 : 16;  // columns per wait

@@ -63,71 +63,70 @@ __global__ void __launch_bounds__(kThreads, 1) lb_gemm_bf16_kernel(const LbDense
     const int my_tiles = (int)blockIdx.x < ntiles ? (ntiles - (int)blockIdx.x + (int)gridDim.x - 1) / (int)gridDim.x : 0;
 
     if (warp == kLoadWarp) {
-        bool failed = false;
-        uint32_t it = 0;
-        for (int i = 0; i < my_tiles && !failed; ++i) {
-            const int t = (int)blockIdx.x + i * (int)gridDim.x;
-            const int rt = t % row_tiles, tb = t / row_tiles;
-            const uint8_t* xb = p.x + (size_t)tb * p.slices * kImgBlock;
-            const size_t goff = p.block_group ? (size_t)p.block_group[tb] * p.group_bytes : 0;
-            const uint8_t* wb[2];
-            int nw = NB;
-            if (kDual) {
-                wb[0] = p.w + goff + (size_t)rt * p.slices * kImgBlock;
-                wb[1] = p.w2 + goff + (size_t)rt * p.slices * kImgBlock;
-            } else {
-                wb[0] = p.w + goff + (size_t)(rt * NB) * p.slices * kImgBlock;
-                wb[1] = wb[0] + (size_t)p.slices * kImgBlock;
-                if (NB == 2 && rt * NB + 1 >= nrb) nw = 1;  // the second half of the last tile has no rows: its columns are never read
-            }
-            for (int ks = 0; ks < p.slices; ++ks, ++it) {
-                const int s = (int)(it % C::kStages);
-                if (it >= (uint32_t)C::kStages && !lb_mbar_wait_bounded(&empty_bar[s], (it / C::kStages - 1) & 1, kTcWaitLimit)) {
-                    failed = true;
-                    break;
+        if (lb_elect()) {
+            bool failed = false;
+            uint32_t it = 0;
+            for (int i = 0; i < my_tiles && !failed; ++i) {
+                const int t = (int)blockIdx.x + i * (int)gridDim.x;
+                const int rt = t % row_tiles, tb = t / row_tiles;
+                const uint8_t* xb = p.x + (size_t)tb * p.slices * kImgBlock;
+                const size_t goff = p.block_group ? (size_t)p.block_group[tb] * p.group_bytes : 0;
+                const uint8_t* wb[2];
+                int nw = NB;
+                if (kDual) {
+                    wb[0] = p.w + goff + (size_t)rt * p.slices * kImgBlock;
+                    wb[1] = p.w2 + goff + (size_t)rt * p.slices * kImgBlock;
+                } else {
+                    wb[0] = p.w + goff + (size_t)(rt * NB) * p.slices * kImgBlock;
+                    wb[1] = wb[0] + (size_t)p.slices * kImgBlock;
+                    if (NB == 2 && rt * NB + 1 >= nrb) nw = 1;  // the second half of the last tile has no rows: its columns are never read
                 }
-                if (lane == 0) {
+                for (int ks = 0; ks < p.slices; ++ks, ++it) {
+                    const int s = (int)(it % C::kStages);
+                    if (it >= (uint32_t)C::kStages && !lb_mbar_wait_bounded(&empty_bar[s], (it / C::kStages - 1) & 1, kTcWaitLimit)) {
+                        failed = true;
+                        break;
+                    }
                     uint8_t* st = smem + (size_t)s * C::kStageBytes;
                     lb_mbar_expect_tx(&load_bar[s], (uint32_t)(kImgBlock * (1 + nw)));
                     lb_bulk_g2s(st, xb + (size_t)ks * kImgBlock, kImgBlock, &load_bar[s]);
                     lb_bulk_g2s(st + kImgBlock, wb[0] + (size_t)ks * kImgBlock, kImgBlock, &load_bar[s]);
                     if (nw == 2) lb_bulk_g2s(st + 2 * kImgBlock, wb[1] + (size_t)ks * kImgBlock, kImgBlock, &load_bar[s]);
                 }
-                __syncwarp();
             }
+            if (failed) atomicExch(&s_failed, 1);
         }
-        if (failed && lane == 0) atomicExch(&s_failed, 1);
+        __syncwarp();
     } else if (warp == kMmaWarp) {
-        constexpr uint32_t idesc = lb_idesc_bf16(128, 128 * NB, false);
-        bool failed = false;
-        uint32_t it = 0;
-        for (int i = 0; i < my_tiles && !failed; ++i) {
-            const int buf = i & 1;
-            if (i >= 2 && !lb_mbar_wait_bounded(&acc_empty[buf], (uint32_t)(((i >> 1) - 1) & 1), kTcWaitLimit)) {
-                failed = true;
-                break;
-            }
-            lb_tc_fence_after();
-            const uint32_t d = tmem_base + (uint32_t)(buf * C::kCols);
-            for (int ks = 0; ks < p.slices; ++ks, ++it) {
-                const int s = (int)(it % C::kStages);
-                if (!lb_mbar_wait_bounded(&load_bar[s], (it / C::kStages) & 1, kTcWaitLimit)) {
+        if (lb_elect()) {
+            constexpr uint32_t idesc = lb_idesc_bf16(128, 128 * NB, false);
+            bool failed = false;
+            uint32_t it = 0;
+            for (int i = 0; i < my_tiles && !failed; ++i) {
+                const int buf = i & 1;
+                if (i >= 2 && !lb_mbar_wait_bounded(&acc_empty[buf], (uint32_t)(((i >> 1) - 1) & 1), kTcWaitLimit)) {
                     failed = true;
                     break;
                 }
                 lb_tc_fence_after();
-                if (lane == 0) {
-                    const uint32_t a = lb_smem_u32(smem + (size_t)s * C::kStageBytes), b = a + kImgBlock;
+                const uint32_t d = tmem_base + (uint32_t)(buf * C::kCols);
+                for (int ks = 0; ks < p.slices; ++ks, ++it) {
+                    const int s = (int)(it % C::kStages);
+                    if (!lb_mbar_wait_bounded(&load_bar[s], (it / C::kStages) & 1, kTcWaitLimit)) {
+                        failed = true;
+                        break;
+                    }
+                    lb_tc_fence_after();
+                    const uint64_t a = lb_smem_desc(lb_smem_u32(smem + (size_t)s * C::kStageBytes), 128, 1024), b = a + (kImgBlock >> 4);
 #pragma unroll
-                    for (int k = 0; k < 4; ++k) lb_mma_f16(d, lb_smem_desc(a + k * 256, 128, 1024), lb_smem_desc(b + k * 256, 128, 1024), idesc, (ks > 0 || k > 0) ? 1u : 0u);
+                    for (int k = 0; k < 4; ++k) lb_mma_f16(d, a + k * 16, b + k * 16, idesc, (ks > 0 || k > 0) ? 1u : 0u);
                     lb_mma_commit(&empty_bar[s]);
                 }
-                __syncwarp();
+                if (!failed) lb_mma_commit(&acc_full[buf]);
             }
-            if (!failed && lane == 0) lb_mma_commit(&acc_full[buf]);
-            __syncwarp();
+            if (failed) atomicExch(&s_failed, 1);
         }
-        if (failed && lane == 0) atomicExch(&s_failed, 1);
+        __syncwarp();
         lb_tc_fence_before();
     } else {
         // a warp reads the 32 TMEM lanes (= tokens) of its quarter; the two warps of a quarter split the columns

@@ -35,6 +35,9 @@ constexpr int kSliceK = 128;       // K columns (= bytes) per pipeline stage
 constexpr int kExpandThreads = 256;  // eight warps: one 16-row strip each; also the epilogue warps
 constexpr int kMmaWarp = kExpandThreads / 32, kLoadWarp = kMmaWarp + 1;
 constexpr int kGemmThreads = kExpandThreads + 64;
+constexpr int kStreamEpi = 512;      // epilogue threads of the persistent kernel
+constexpr int kStreamMmaWarp = kStreamEpi / 32, kStreamLoadWarp = kStreamMmaWarp + 1;
+constexpr int kStreamThreads = kStreamEpi + 64;
 constexpr int kSliceBytesA = kRowsPerCta * kSliceK;  // 16 KB
 constexpr int kMaxStages = 6;
 constexpr uint32_t kWaitLimit = 20000000u;
@@ -101,68 +104,91 @@ __device__ __forceinline__ bool wait_bounded(uint64_t* bar, uint32_t parity) {
     return false;
 }
 
-// Float epilogue of sixteen tokens (columns c0 .. c0+15 of the CTA's tile) of weight row r: raw[j] = sum(code * x).
-// int32 -> float64 by the exponent trick (2^52 + 2^31 + a as a bit pattern, minus the constant: exact, and a full-rate
-// addition where the conversion instruction runs at quarter rate).
-__device__ __forceinline__ double gemm_i2d(int a) {
-    return __dadd_rn(__hiloint2double(0x43300000, (int)((unsigned)a ^ 0x80000000u)), -4503601774854144.0);
+// What a token's epilogue needs: the output scale, and what turns raw sums of code * x into float64 sums of w * x
+// (gemm_i2d), so that one 16-byte load brings both.
+struct __align__(16) StreamScale {
+    double os, zero;
+};
+// int32 -> float64 by the exponent trick: 2^52 + 2^31 + a as a bit pattern, minus 2^52 + 2^31 + xsum.  Exact, and a full-rate
+// addition where the conversion instruction runs at quarter rate; the correction by xsum costs nothing.
+__device__ __forceinline__ double gemm_zero(int xsum) { return -__dadd_rn(4503601774854144.0, (double)xsum); }
+__device__ __forceinline__ double gemm_i2d(int a, double zero) {
+    return __dadd_rn(__hiloint2double(0x43300000, (int)((unsigned)a ^ 0x80000000u)), zero);
 }
 
-__device__ __forceinline__ void gemm_emit16(const GemmParams& p, int r, bool row_ok, bool failed, int tok0, int c0, const int* raw,
-                                    const double* s_os, const int* s_xsum, double bias, bool has_bias) {
-    int acc[16];
-    double y[16];
-    float f[16];
+// sixteen consecutive columns of this thread's TMEM lane
+__device__ __forceinline__ void gemm_tmem_ld16(uint32_t addr, uint32_t (&v)[16]) {
+    asm volatile("tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15}, [%16];"
+                 : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]), "=r"(v[4]), "=r"(v[5]), "=r"(v[6]), "=r"(v[7]), "=r"(v[8]),
+                   "=r"(v[9]), "=r"(v[10]), "=r"(v[11]), "=r"(v[12]), "=r"(v[13]), "=r"(v[14]), "=r"(v[15])
+                 : "r"(addr)
+                 : "memory");
+}
+
+// Float epilogue of eight tokens from `tok` on (sc: theirs) of weight row r: v[j] = sum(code * x).
+__device__ __forceinline__ void gemm_emit8(const GemmParams& p, int r, bool row_ok, int tok, const uint32_t* v, const StreamScale* sc, double bias, bool has_bias) {
+    if (!row_ok) return;
+    const int ntok = p.tokens - tok;  // columns of this step that are real tokens
+    size_t o0 = (size_t)tok * p.rows + r, ostride = (size_t)p.rows;
+    if (p.kv_hd > 0) {
+        o0 = ((size_t)(r / p.kv_hd) * p.kv_msl + p.kv_pos0 + tok) * p.kv_hd + r % p.kv_hd;
+        ostride = (size_t)p.kv_hd;
+    }
+    float rs[8];
+    if (p.residual) {  // asked for in front of the arithmetic
+        const float* at = p.residual + o0;
 #pragma unroll
-    for (int j = 0; j < 16; ++j) {
-        acc[j] = raw[j] - s_xsum[c0 + j];
-        const double t = __dmul_rn(gemm_i2d(acc[j]), s_os[c0 + j]);
+        for (int j = 0; j < 8; ++j, at += ostride) rs[j] = j < ntok ? *at : 0.f;
+    }
+    double y[8];
+    float f[8];
+#pragma unroll
+    for (int j = 0; j < 8; ++j) {
+        const StreamScale s = sc[j];
+        const double t = __dmul_rn(gemm_i2d((int)v[j], s.zero), s.os);
         y[j] = has_bias ? __dadd_rn(t, bias) : t;
-        f[j] = (float)y[j];
     }
-    if (row_ok && !failed) {
-        const int ntok = p.tokens - (tok0 + c0);  // columns of this step that are real tokens
-        size_t o0 = (size_t)(tok0 + c0) * p.rows + r, ostride = (size_t)p.rows;
-        if (p.kv_hd > 0) {
-            o0 = ((size_t)(r / p.kv_hd) * p.kv_msl + p.kv_pos0 + tok0 + c0) * p.kv_hd + r % p.kv_hd;
-            ostride = (size_t)p.kv_hd;
-        }
-        if (p.acc_out) {
+    if (p.acc_out) {
+        int32_t* at = p.acc_out + o0;
 #pragma unroll
-            for (int j = 0; j < 16; ++j)
-                if (j < ntok) p.acc_out[o0 + j * ostride] = acc[j];
-        }
-        if (p.out_f64) {
+        for (int j = 0; j < 8; ++j, at += ostride)
+            if (j < ntok) *at = (int)gemm_i2d((int)v[j], sc[j].zero);
+    }
+    if (p.out_f64) {
+        double* at = p.out_f64 + o0;
 #pragma unroll
-            for (int j = 0; j < 16; ++j)
-                if (j < ntok) p.out_f64[o0 + j * ostride] = y[j];
-        }
-        if (p.out) {
-            if (p.pre_out) {
+        for (int j = 0; j < 8; ++j, at += ostride)
+            if (j < ntok) *at = y[j];
+    }
+    if (!p.out) return;
 #pragma unroll
-                for (int j = 0; j < 16; ++j)
-                    if (j < ntok) p.pre_out[o0 + j * ostride] = f[j];
-            }
-            if (p.act != LOOM_B200_ACT_LINEAR) {
+    for (int j = 0; j < 8; ++j) f[j] = (float)y[j];
+    if (p.pre_out) {
+        float* at = p.pre_out + o0;
 #pragma unroll
-                for (int j = 0; j < 16; ++j) {
-                    if (p.act == LOOM_B200_ACT_RELU) f[j] = f[j] < 0.f ? 0.f : f[j];
-                    else if (p.act == LOOM_B200_ACT_RELU2) f[j] = f[j] < 0.f ? 0.f : __fmul_rn(f[j], f[j]);
-                    else f[j] = lb_activate(f[j], p.act);
-                }
-            }
-            if (p.residual) {
-                float rs[16];
+        for (int j = 0; j < 8; ++j, at += ostride)
+            if (j < ntok) *at = f[j];
+    }
+    if (p.act != LOOM_B200_ACT_LINEAR) {
 #pragma unroll
-                for (int j = 0; j < 16; ++j) rs[j] = j < ntok ? p.residual[o0 + j * ostride] : 0.f;
-#pragma unroll
-                for (int j = 0; j < 16; ++j) f[j] = __fadd_rn(f[j], rs[j]);
-            }
-#pragma unroll
-            for (int j = 0; j < 16; ++j)
-                if (j < ntok) p.out[o0 + j * ostride] = f[j];
+        for (int j = 0; j < 8; ++j) {
+            if (p.act == LOOM_B200_ACT_RELU) f[j] = f[j] < 0.f ? 0.f : f[j];
+            else if (p.act == LOOM_B200_ACT_RELU2) f[j] = f[j] < 0.f ? 0.f : __fmul_rn(f[j], f[j]);
+            else f[j] = lb_activate(f[j], p.act);
         }
     }
+    if (p.residual) {
+#pragma unroll
+        for (int j = 0; j < 8; ++j) f[j] = __fadd_rn(f[j], rs[j]);
+    }
+    float* at = p.out + o0;
+#pragma unroll
+    for (int j = 0; j < 8; ++j, at += ostride)
+        if (j < ntok) *at = f[j];
+}
+__device__ __forceinline__ void gemm_emit16(const GemmParams& p, int r, bool row_ok, int tok, const uint32_t* v, const StreamScale* sc, double bias, bool has_bias) {
+#pragma unroll
+    for (int h = 0; h < 16; h += 8) gemm_emit8(p, r, row_ok, tok + h, v + h, sc + h, bias, has_bias);
 }
 
 // stages that fit beside 1 KB of alignment slack
@@ -183,8 +209,7 @@ __global__ void __launch_bounds__(kGemmThreads, 1) lb_gemm_ternary_i8_kernel(con
     extern __shared__ __align__(1024) uint8_t smem[];
     __shared__ __align__(8) uint64_t load_bar[kMaxStages], a_bar[kMaxStages], empty_bar[kMaxStages], done_bar;
     __shared__ uint32_t tmem_base_s;
-    __shared__ double s_os[NTOK];
-    __shared__ int s_xsum[NTOK];
+    __shared__ StreamScale s_scale[NTOK];
     __shared__ int s_failed;
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const int row0 = blockIdx.x * kRowsPerCta, tok0 = blockIdx.y * NTOK;
@@ -227,7 +252,7 @@ __global__ void __launch_bounds__(kGemmThreads, 1) lb_gemm_ternary_i8_kernel(con
             const int s = ks % kStages;
             if (ks >= kStages && !failed && !wait_bounded(&empty_bar[s], (uint32_t)((ks / kStages - 1) & 1))) failed = true;
             if (failed) break;
-            if (lane == 0) {
+            if (lb_elect()) {
                 lb_mbar_expect_tx(&load_bar[s], (uint32_t)(Cfg::kSliceBytesB + (MODE != GEMM_EXPAND ? Cfg::kStageBytesA : 0)));
                 lb_bulk_g2s(b_ring + (size_t)s * Cfg::kSliceBytesB, qbase + (size_t)ks * 32768, (uint32_t)Cfg::kSliceBytesB, &load_bar[s]);
                 if (MODE != GEMM_EXPAND) {  // the weights of this (row block, k-slice): 16 KB per matrix, already in the tensor core's layout
@@ -243,8 +268,8 @@ __global__ void __launch_bounds__(kGemmThreads, 1) lb_gemm_ternary_i8_kernel(con
         // ---------------- expansion warps ----------------
         for (int i = tid; i < NTOK; i += kExpandThreads) {
             const int tok = tok0 + i;
-            s_os[i] = tok < p.tokens ? lb_output_scale(p.scale, p.amax[tok]) : 0.0;
-            s_xsum[i] = tok < p.tokens ? p.xsum[tok] : 0;
+            s_scale[i].os = tok < p.tokens ? lb_output_scale(p.scale, p.amax[tok]) : 0.0;
+            s_scale[i].zero = gemm_zero(tok < p.tokens ? p.xsum[tok] : 0);
         }
         asm volatile("bar.sync 1, 256;" ::: "memory");  // the per-token scales are read by other expansion warps later
         if (tr && tid == 0) tr[1] = lb_gtime();
@@ -295,24 +320,17 @@ __global__ void __launch_bounds__(kGemmThreads, 1) lb_gemm_ternary_i8_kernel(con
         // (sixteen independent int -> float64 -> float32 chains in flight: with two warps per scheduler the epilogue is
         // bound by instruction latency, not throughput), then stored under the per-output conditions.
         const bool has_bias = row_ok && p.bias != nullptr;
-        auto emit = [&](int c0, const int* raw) { gemm_emit16(p, r, row_ok, failed, tok0, c0, raw, s_os, s_xsum, bias, has_bias); };
+        auto emit = [&](int c0, const uint32_t* raw) { gemm_emit16(p, r, row_ok && !failed, tok0 + c0, raw, s_scale + c0, bias, has_bias); };
         const bool split = gridDim.z > 1;
 #pragma unroll 1
         for (int c0 = chalf * (NTOK / 2); c0 < (chalf + 1) * (NTOK / 2); c0 += 16) {
             uint32_t v[16];
             const uint32_t taddr = tmem_base + ((uint32_t)(quarter * 32) << 16) + (uint32_t)c0;
-            asm volatile("tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15}, [%16];"
-                         : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]), "=r"(v[4]), "=r"(v[5]), "=r"(v[6]), "=r"(v[7]), "=r"(v[8]),
-                           "=r"(v[9]), "=r"(v[10]), "=r"(v[11]), "=r"(v[12]), "=r"(v[13]), "=r"(v[14]), "=r"(v[15])
-                         : "r"(taddr)
-                         : "memory");
+            gemm_tmem_ld16(taddr, v);
             asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
             if (tr && tid == 0 && c0 == 0) tr[5] = lb_gtime();
             if (!split) {
-                int raw[16];
-#pragma unroll
-                for (int j = 0; j < 16; ++j) raw[j] = (int)v[j];
-                emit(c0, raw);
+                emit(c0, v);
             } else if (row_ok && !failed) {  // split-K: add this CTA's part to the tile's sums (integer addition: any order, same bits)
                 const int ntok = p.tokens - (tok0 + c0);
                 int32_t* dst = p.part_acc + (size_t)(tok0 + c0) * p.rows + r;
@@ -333,14 +351,14 @@ __global__ void __launch_bounds__(kGemmThreads, 1) lb_gemm_ternary_i8_kernel(con
                 __threadfence();
 #pragma unroll 1
                 for (int c0 = chalf * (NTOK / 2); c0 < (chalf + 1) * (NTOK / 2); c0 += 16) {
-                    int raw[16];
+                    uint32_t raw[16];
                     const int ntok = p.tokens - (tok0 + c0);
                     int32_t* src = p.part_acc + (size_t)(tok0 + c0) * p.rows + r;
 #pragma unroll
                     for (int j = 0; j < 16; ++j) {
                         raw[j] = 0;
                         if (row_ok && j < ntok) {
-                            raw[j] = __ldcg(src + (size_t)j * p.rows);
+                            raw[j] = (uint32_t)__ldcg(src + (size_t)j * p.rows);
                             src[(size_t)j * p.rows] = 0;
                         }
                     }
@@ -362,7 +380,7 @@ __global__ void __launch_bounds__(kGemmThreads, 1) lb_gemm_ternary_i8_kernel(con
             if (!failed && !wait_bounded(&load_bar[s], (uint32_t)((ks / kStages) & 1))) failed = true;  // the activations (and the cached codes)
             asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
             if (tr && lane == 0) tr[(1 + ks) * 8 + 4] = lb_gtime();
-            if (lane == 0 && !failed) {
+            if (!failed && lb_elect()) {
                 const uint32_t a_addr = lb_smem_u32(a_ring + (size_t)s * Cfg::kStageBytesA);
                 const uint32_t b_addr = lb_smem_u32(b_ring + (size_t)s * Cfg::kSliceBytesB);
 #pragma unroll
@@ -373,7 +391,7 @@ __global__ void __launch_bounds__(kGemmThreads, 1) lb_gemm_ternary_i8_kernel(con
             }
             __syncwarp();
         }
-        if (lane == 0) {
+        if (lb_elect()) {
             if (failed) atomicExch(&s_failed, 1);
             mma_commit(&done_bar);
         }
@@ -392,9 +410,14 @@ __global__ void __launch_bounds__(kGemmThreads, 1) lb_gemm_ternary_i8_kernel(con
 // ------------------------------------------------------------------------------------------------------------------
 // Persistent variant over pre-expanded codes.  One CTA per SM walks output tiles (row tile fastest, so the CTAs that run
 // together share a token tile's activations in L2); the shared-memory ring runs on across tile boundaries, and tensor
-// memory holds TWO accumulator buffers, so the eight epilogue warps drain tile i (tcgen05.ld, float64 rescale, stores)
+// memory holds TWO accumulator buffers, so the epilogue warps drain tile i (tcgen05.ld, float64 rescale, stores)
 // while the MMA warp already accumulates tile i+1.  In the one-shot kernel above the epilogue of a 128 x 256 tile costs
 // about as long as its twenty k-slices of MMAs, and two co-resident CTAs ran in lockstep instead of overlapping.
+// What bounds it (operands replaced by 16-byte copies change nothing): the epilogue, whose float64 instructions take 2.4 times
+// as long while the tensor core is at work (18,500 clocks for a 128 x 256 tile against 7,700 behind the last MMA, twenty slices of MMAs
+// 11,000), and how fast one thread can issue (lb_elect).  Sixteen epilogue warps instead of eight, statistics fetched a tile ahead,
+// a token's scale and correction in one 16-byte load, copies and MMAs from elected threads: 2048 x 6912 x 2560 43 -> 36 us,
+// 512 x 2560 x 6912 25 -> 17.5, 2999 x 14336 x 4096 164 -> 147; gate and up of 1024 x 6912 x 2560 67 -> 53.
 // DUAL: a gate / up pair that shares the activations -- both code blocks ride in one stage, two accumulators per buffer
 // (gate at column 0, up at column NTOK), and the epilogue writes float32(gateProduct(yg + bg, yu + bu)) only
 // (poly/swiglu.go:299-310): the two int32 accumulator planes never travel through memory.
@@ -411,14 +434,14 @@ struct StreamCfg {
 };
 
 template <int NTOK, bool DUAL>
-__global__ void __launch_bounds__(kGemmThreads, 1) lb_gemm_stream_kernel(const GemmParams p, int row_tiles, int ntiles) {
+__global__ void __launch_bounds__(kStreamThreads, 1) lb_gemm_stream_kernel(const GemmParams p, int row_tiles, int ntiles) {
     using Cfg = StreamCfg<NTOK, DUAL>;
     constexpr int kStages = Cfg::kStages;
     extern __shared__ __align__(1024) uint8_t smem[];
     __shared__ __align__(8) uint64_t load_bar[kMaxStages], empty_bar[kMaxStages], acc_full[2], acc_empty[2];
     __shared__ uint32_t tmem_base_s;
-    __shared__ double s_os[NTOK], s_os_up[DUAL ? NTOK : 1];
-    __shared__ int s_xsum[NTOK];
+    __shared__ StreamScale s_scale[2][NTOK];
+    __shared__ double s_os_up[2][DUAL ? NTOK : 1];
     __shared__ int s_failed;
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     uint8_t* a_ring = smem;
@@ -433,12 +456,12 @@ __global__ void __launch_bounds__(kGemmThreads, 1) lb_gemm_stream_kernel(const G
         }
         for (int b = 0; b < 2; ++b) {
             lb_mbar_init(&acc_full[b], 1);
-            lb_mbar_init(&acc_empty[b], kExpandThreads / 32);  // one arrival per epilogue warp
+            lb_mbar_init(&acc_empty[b], kStreamEpi / 32);  // one arrival per epilogue warp
         }
         lb_fence_mbar_init();
         s_failed = 0;
     }
-    if (warp == kMmaWarp) {
+    if (warp == kStreamMmaWarp) {
         asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(lb_smem_u32(&tmem_base_s)), "r"(2 * Cfg::kAccCols) : "memory");
         asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
     }
@@ -448,18 +471,18 @@ __global__ void __launch_bounds__(kGemmThreads, 1) lb_gemm_stream_kernel(const G
     const uint32_t tmem_base = tmem_base_s;
     lb_pdl_launch_dependents();
 
-    if (warp == kLoadWarp) {
+    if (warp == kStreamLoadWarp) {
         // ---------------- loads: per stage the activations of the tile's tokens and the code block(s) of its rows ----------------
-        bool failed = false;
-        uint32_t it = 0;
-        // The weights do not depend on the quantizer that runs before this kernel: the code blocks of the first stages
-        // are requested before the dependency wait, their activations after it (one barrier counts the bytes of both).
-        int pre = 0;
-        if (my_tiles > 0) {
-            const int rt0 = (int)blockIdx.x % row_tiles;
-            const size_t blk00 = (size_t)rt0 * ktot * kSliceBytesA;
-            pre = ktot < kStages ? ktot : kStages;
-            if (lane == 0) {
+        if (lb_elect()) {
+            bool failed = false;
+            uint32_t it = 0;
+            // The weights do not depend on the quantizer that runs before this kernel: the code blocks of the first stages
+            // are requested before the dependency wait, their activations after it (one barrier counts the bytes of both).
+            int pre = 0;
+            if (my_tiles > 0) {
+                const int rt0 = (int)blockIdx.x % row_tiles;
+                const size_t blk00 = (size_t)rt0 * ktot * kSliceBytesA;
+                pre = ktot < kStages ? ktot : kStages;
                 for (int ks = 0; ks < pre; ++ks) {
                     lb_mbar_expect_tx(&load_bar[ks], (uint32_t)Cfg::kStageBytes);
                     lb_bulk_g2s(a_ring + (size_t)ks * Cfg::kBytesA, p.codes8 + blk00 + (size_t)ks * kSliceBytesA, (uint32_t)kSliceBytesA, &load_bar[ks]);
@@ -468,20 +491,18 @@ __global__ void __launch_bounds__(kGemmThreads, 1) lb_gemm_stream_kernel(const G
                                     (uint32_t)kSliceBytesA, &load_bar[ks]);
                 }
             }
-        }
-        lb_pdl_wait();
-        for (int i = 0; i < my_tiles && !failed; ++i) {
-            const int t = (int)blockIdx.x + i * (int)gridDim.x;
-            const int rt = t % row_tiles, tok0 = (t / row_tiles) * NTOK;
-            const int8_t* qbase = p.q + (size_t)(tok0 >> 8) * ktot * 32768 + (size_t)((tok0 & 255) >> 3) * 1024;
-            const size_t blk0 = (size_t)rt * ktot * kSliceBytesA;
-            for (int ks = 0; ks < ktot; ++ks, ++it) {
-                const int s = (int)(it % kStages);
-                if (it >= (uint32_t)kStages && !wait_bounded(&empty_bar[s], (it / kStages - 1) & 1)) {
-                    failed = true;
-                    break;
-                }
-                if (lane == 0) {
+            lb_pdl_wait();
+            for (int i = 0; i < my_tiles && !failed; ++i) {
+                const int t = (int)blockIdx.x + i * (int)gridDim.x;
+                const int rt = t % row_tiles, tok0 = (t / row_tiles) * NTOK;
+                const int8_t* qbase = p.q + (size_t)(tok0 >> 8) * ktot * 32768 + (size_t)((tok0 & 255) >> 3) * 1024;
+                const size_t blk0 = (size_t)rt * ktot * kSliceBytesA;
+                for (int ks = 0; ks < ktot; ++ks, ++it) {
+                    const int s = (int)(it % kStages);
+                    if (it >= (uint32_t)kStages && !wait_bounded(&empty_bar[s], (it / kStages - 1) & 1)) {
+                        failed = true;
+                        break;
+                    }
                     const bool a_done = i == 0 && ks < pre;  // requested before the dependency wait
                     if (!a_done) lb_mbar_expect_tx(&load_bar[s], (uint32_t)Cfg::kStageBytes);
                     lb_bulk_g2s(b_ring + (size_t)s * Cfg::kBytesB, qbase + (size_t)ks * 32768, (uint32_t)Cfg::kBytesB, &load_bar[s]);
@@ -492,69 +513,77 @@ __global__ void __launch_bounds__(kGemmThreads, 1) lb_gemm_stream_kernel(const G
                                         (uint32_t)kSliceBytesA, &load_bar[s]);
                     }
                 }
-                __syncwarp();
             }
+            if (failed) atomicExch(&s_failed, 1);
         }
-        if (failed && lane == 0) atomicExch(&s_failed, 1);
-    } else if (warp == kMmaWarp) {
+        __syncwarp();
+    } else if (warp == kStreamMmaWarp) {
         // ---------------- MMA issuer ----------------
-        const uint32_t idesc = (2u << 4) | (0u << 7) | (1u << 10) | ((uint32_t)(NTOK >> 3) << 17) | ((uint32_t)(kRowsPerCta >> 4) << 24);
-        bool failed = false;
-        uint32_t it = 0;
-        for (int i = 0; i < my_tiles && !failed; ++i) {
-            const int buf = i & 1;
-            // the epilogue must have drained this buffer's previous tile
-            if (i >= 2 && !wait_bounded(&acc_empty[buf], (uint32_t)(((i >> 1) - 1) & 1))) {
-                failed = true;
-                break;
-            }
-            asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-            const uint32_t d = tmem_base + (uint32_t)(buf * Cfg::kAccCols);
-            for (int ks = 0; ks < ktot; ++ks, ++it) {
-                const int s = (int)(it % kStages);
-                if (!wait_bounded(&load_bar[s], (it / kStages) & 1)) {
+        if (lb_elect()) {
+            const uint32_t idesc = (2u << 4) | (0u << 7) | (1u << 10) | ((uint32_t)(NTOK >> 3) << 17) | ((uint32_t)(kRowsPerCta >> 4) << 24);
+            bool failed = false;
+            uint32_t it = 0;
+            for (int i = 0; i < my_tiles && !failed; ++i) {
+                const int buf = i & 1;
+                // the epilogue must have drained this buffer's previous tile
+                if (i >= 2 && !wait_bounded(&acc_empty[buf], (uint32_t)(((i >> 1) - 1) & 1))) {
                     failed = true;
                     break;
                 }
                 asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-                if (lane == 0) {
-                    const uint32_t a_addr = lb_smem_u32(a_ring + (size_t)s * Cfg::kBytesA);
-                    const uint32_t b_addr = lb_smem_u32(b_ring + (size_t)s * Cfg::kBytesB);
+                const uint32_t d = tmem_base + (uint32_t)(buf * Cfg::kAccCols);
+                for (int ks = 0; ks < ktot; ++ks, ++it) {
+                    const int s = (int)(it % kStages);
+                    if (!wait_bounded(&load_bar[s], (it / kStages) & 1)) {
+                        failed = true;
+                        break;
+                    }
+                    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+                    const uint64_t a_desc = smem_desc(lb_smem_u32(a_ring + (size_t)s * Cfg::kBytesA));
+                    const uint64_t b_desc = smem_desc(lb_smem_u32(b_ring + (size_t)s * Cfg::kBytesB));
 #pragma unroll
-                    for (int k = 0; k < kSliceK / 32; ++k)
-                        mma_i8(d, smem_desc(a_addr + k * 256), smem_desc(b_addr + k * 256), idesc, (ks > 0 || k > 0) ? 1u : 0u);
+                    for (int k = 0; k < kSliceK / 32; ++k)  // (256 bytes further in K, in units of 16)
+                        mma_i8(d, a_desc + k * 16, b_desc + k * 16, idesc, (ks > 0 || k > 0) ? 1u : 0u);
                     if (DUAL) {
 #pragma unroll
                         for (int k = 0; k < kSliceK / 32; ++k)
-                            mma_i8(d + (uint32_t)NTOK, smem_desc(a_addr + kSliceBytesA + k * 256), smem_desc(b_addr + k * 256), idesc,
-                                   (ks > 0 || k > 0) ? 1u : 0u);
+                            mma_i8(d + (uint32_t)NTOK, a_desc + (kSliceBytesA >> 4) + k * 16, b_desc + k * 16, idesc, (ks > 0 || k > 0) ? 1u : 0u);
                     }
                     mma_commit(&empty_bar[s]);
                 }
-                __syncwarp();
+                if (!failed) mma_commit(&acc_full[buf]);  // arrives when every MMA of the tile is done
             }
-            if (!failed && lane == 0) mma_commit(&acc_full[buf]);  // arrives when every MMA of the tile is done
-            __syncwarp();
+            if (failed) atomicExch(&s_failed, 1);
         }
-        if (failed && lane == 0) atomicExch(&s_failed, 1);
+        __syncwarp();
         asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
     } else {
         // ---------------- epilogue warps: tile i while the MMA warp is on tile i + 1 ----------------
-        // a warp may only touch the 32 TMEM lanes of its quarter (warp % 4); the two warps of a quarter split the columns
-        const int quarter = warp & 3, chalf = warp >> 2;
+        // a warp may only touch the 32 TMEM lanes of its quarter (warp % 4); the warps of a quarter split the columns
+        constexpr int kShare = NTOK / (kStreamEpi / 128);  // columns of a warp
+        const int quarter = warp & 3, first = (warp >> 2) * kShare;
         bool failed = false;  // after a wait ran out the warp keeps walking the tiles (its named-barrier count must match) without touching TMEM or memory
         lb_pdl_wait();  // the per-token scales, the residual rows and the output buffer belong to earlier launches until here
+        // a token's statistics are fetched a tile ahead and become scales behind the tile in front: one barrier per tile
+        float amax = 0.f;
+        int xsum = 0;
+        auto fetch_stats = [&](int i) {
+            const int tok = ((int)blockIdx.x + i * (int)gridDim.x) / row_tiles * NTOK + tid;
+            const bool ok = tid < NTOK && i < my_tiles && tok < p.tokens;
+            amax = ok ? p.amax[tok] : 0.f;
+            xsum = ok ? p.xsum[tok] : 0;
+        };
+        fetch_stats(0);
         for (int i = 0; i < my_tiles; ++i) {
             const int t = (int)blockIdx.x + i * (int)gridDim.x;
             const int rt = t % row_tiles, tok0 = (t / row_tiles) * NTOK, buf = i & 1;
-            asm volatile("bar.sync 1, 256;" ::: "memory");  // the previous tile's scales are no longer read
-            for (int c = tid; c < NTOK; c += kExpandThreads) {
-                const int tok = tok0 + c;
-                s_os[c] = tok < p.tokens ? lb_output_scale(p.scale, p.amax[tok]) : 0.0;
-                if (DUAL) s_os_up[c] = tok < p.tokens ? lb_output_scale(p.scale_up, p.amax[tok]) : 0.0;
-                s_xsum[c] = tok < p.tokens ? p.xsum[tok] : 0;
+            if (tid < NTOK) {  // (columns of absent tokens are computed and not stored)
+                s_scale[buf][tid].os = lb_output_scale(p.scale, amax);
+                s_scale[buf][tid].zero = gemm_zero(xsum);
+                if (DUAL) s_os_up[buf][tid] = lb_output_scale(p.scale_up, amax);
             }
-            asm volatile("bar.sync 1, 256;" ::: "memory");
+            asm volatile("bar.sync 1, %0;" ::"n"(kStreamEpi) : "memory");  // (everyone is also done with the scales of two tiles ago)
+            fetch_stats(i + 1);
             if (!failed && !wait_bounded(&acc_full[buf], (uint32_t)((i >> 1) & 1))) {
                 failed = true;
                 atomicExch(&s_failed, 1);
@@ -562,50 +591,34 @@ __global__ void __launch_bounds__(kGemmThreads, 1) lb_gemm_stream_kernel(const G
             asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
             const int r = rt * kRowsPerCta + quarter * 32 + lane;
             const bool row_ok = r < p.rows;
-            const bool has_bias = row_ok && p.bias != nullptr;
-            const double bias = has_bias ? (double)p.bias[r] : 0.0;
+            const bool has_bias = row_ok && p.bias != nullptr, has_bias_up = DUAL && row_ok && p.bias_up != nullptr;
+            const double bias = has_bias ? (double)p.bias[r] : 0.0, bias_up = has_bias_up ? (double)p.bias_up[r] : 0.0;
             const uint32_t tacc = tmem_base + (uint32_t)(buf * Cfg::kAccCols) + ((uint32_t)(quarter * 32) << 16);
             if (!failed) {
 #pragma unroll 1
-                for (int c0 = chalf * (NTOK / 2); c0 < (chalf + 1) * (NTOK / 2); c0 += 16) {
+                for (int c0 = first; c0 < first + kShare; c0 += 16) {
                     uint32_t v[16];
-                    asm volatile("tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15}, [%16];"
-                                 : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]), "=r"(v[4]), "=r"(v[5]), "=r"(v[6]), "=r"(v[7]), "=r"(v[8]),
-                                   "=r"(v[9]), "=r"(v[10]), "=r"(v[11]), "=r"(v[12]), "=r"(v[13]), "=r"(v[14]), "=r"(v[15])
-                                 : "r"(tacc + (uint32_t)c0)
-                                 : "memory");
+                    gemm_tmem_ld16(tacc + (uint32_t)c0, v);
                     if (!DUAL) {
                         asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
-                        int raw[16];
-#pragma unroll
-                        for (int j = 0; j < 16; ++j) raw[j] = (int)v[j];
-                        gemm_emit16(p, r, row_ok, false, tok0, c0, raw, s_os, s_xsum, bias, has_bias);
+                        gemm_emit16(p, r, row_ok, tok0 + c0, v, s_scale[buf] + c0, bias, has_bias);
                     } else {
                         uint32_t u[16];
-                        asm volatile("tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15}, [%16];"
-                                     : "=r"(u[0]), "=r"(u[1]), "=r"(u[2]), "=r"(u[3]), "=r"(u[4]), "=r"(u[5]), "=r"(u[6]), "=r"(u[7]), "=r"(u[8]),
-                                       "=r"(u[9]), "=r"(u[10]), "=r"(u[11]), "=r"(u[12]), "=r"(u[13]), "=r"(u[14]), "=r"(u[15])
-                                     : "r"(tacc + (uint32_t)(NTOK + c0))
-                                     : "memory");
+                        gemm_tmem_ld16(tacc + (uint32_t)(NTOK + c0), u);
                         asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
-                        const bool has_bias_up = row_ok && p.bias_up != nullptr;
-                        const double bias_up = has_bias_up ? (double)p.bias_up[r] : 0.0;
-                        float f[16];
-#pragma unroll
-                        for (int j = 0; j < 16; ++j) {
-                            const int xs = s_xsum[c0 + j];
-                            double yg = __dmul_rn(gemm_i2d((int)v[j] - xs), s_os[c0 + j]);
-                            double yu = __dmul_rn(gemm_i2d((int)u[j] - xs), s_os_up[c0 + j]);
-                            if (has_bias) yg = __dadd_rn(yg, bias);
-                            if (has_bias_up) yu = __dadd_rn(yu, bias_up);
-                            f[j] = (float)lb_gate_product(yg, yu, p.act);
-                        }
                         if (row_ok) {
                             const int ntok = p.tokens - (tok0 + c0);
-                            const size_t o0 = (size_t)(tok0 + c0) * p.rows + r;
+                            float* o = p.out + (size_t)(tok0 + c0) * p.rows + r;
 #pragma unroll
-                            for (int j = 0; j < 16; ++j)
-                                if (j < ntok) p.out[o0 + (size_t)j * p.rows] = f[j];
+                            for (int j = 0; j < 16; ++j, o += p.rows) {
+                                const StreamScale sc = s_scale[buf][c0 + j];
+                                double yg = __dmul_rn(gemm_i2d((int)v[j], sc.zero), sc.os);
+                                double yu = __dmul_rn(gemm_i2d((int)u[j], sc.zero), s_os_up[buf][c0 + j]);
+                                if (has_bias) yg = __dadd_rn(yg, bias);
+                                if (has_bias_up) yu = __dadd_rn(yu, bias_up);
+                                const float f = (float)lb_gate_product(yg, yu, p.act);
+                                if (j < ntok) *o = f;
+                            }
                         }
                     }
                 }
@@ -617,7 +630,7 @@ __global__ void __launch_bounds__(kGemmThreads, 1) lb_gemm_stream_kernel(const G
         }
     }
     __syncthreads();
-    if (warp == kMmaWarp) {
+    if (warp == kStreamMmaWarp) {
         asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
         asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem_base), "r"(2 * Cfg::kAccCols) : "memory");
     }
@@ -1081,7 +1094,7 @@ static int gemm_launch_stream(loom_b200_ctx* ctx, const GemmParams& p, unsigned 
     const int grid = ntiles < ctx->sm_count ? ntiles : ctx->sm_count;
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(grid);
-    cfg.blockDim = dim3(kGemmThreads);
+    cfg.blockDim = dim3(kStreamThreads);
     cfg.dynamicSmemBytes = Cfg::kSmem;
     cfg.stream = ctx->stream;
     cudaLaunchAttribute attr[1];
