@@ -371,20 +371,19 @@ int dec_prefill_block(loom_b200_decoder* dec, int M, int pos0, bool head) {
         if (int rc = lb_gemm_quantize(ctx, qa)) return rc;
         LbGemmOut o = {};
         o.act = LOOM_B200_ACT_LINEAR;
-        o.bias = m.bq;
-        o.out_f64 = dec->pf_q;
-        if (int rc = lb_gemm_run(ctx, m.wq, M, o)) return rc;
-        o = LbGemmOut{};
-        o.act = LOOM_B200_ACT_LINEAR;
-        o.bias = m.bk;
-        o.out = m.cache_k;  // head-major ring: token t of the block goes to position pos0 + t of every KV head (a prompt never wraps)
-        o.kv_hd = m.head_dim;
-        o.kv_msl = m.msl;
-        o.kv_pos0 = pos0;
-        if (int rc = lb_gemm_run(ctx, m.wk, M, o)) return rc;
-        o.bias = m.bv;
-        o.out = m.cache_v;
-        if (int rc = lb_gemm_run(ctx, m.wv, M, o)) return rc;
+        LbGemmOut qkv[3] = {o, o, o};
+        qkv[0].bias = m.bq;
+        qkv[0].out_f64 = dec->pf_q;
+        qkv[1].bias = m.bk;
+        qkv[1].out = m.cache_k;  // head-major ring: token t of the block goes to position pos0 + t of every KV head (a prompt never wraps)
+        qkv[1].kv_hd = m.head_dim;
+        qkv[1].kv_msl = m.msl;
+        qkv[1].kv_pos0 = pos0;
+        qkv[2] = qkv[1];
+        qkv[2].bias = m.bv;
+        qkv[2].out = m.cache_v;
+        const loom_b200_weight* wqkv[3] = {m.wq, m.wk, m.wv};
+        if (int rc = lb_gemm_run_group(ctx, wqkv, 3, M, qkv)) return rc;
 
         LbRopeParams r = {};
         r.q = dec->pf_q;

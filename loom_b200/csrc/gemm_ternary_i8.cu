@@ -36,8 +36,8 @@ constexpr int kExpandThreads = 256;  // eight warps: one 16-row strip each; also
 constexpr int kMmaWarp = kExpandThreads / 32, kLoadWarp = kMmaWarp + 1;
 constexpr int kGemmThreads = kExpandThreads + 64;
 constexpr int kStreamEpi = 512;      // epilogue threads of the persistent kernel
-constexpr int kStreamMmaWarp = kStreamEpi / 32, kStreamLoadWarp = kStreamMmaWarp + 1;
-constexpr int kStreamThreads = kStreamEpi + 64;
+constexpr int kStreamMmaWarp = kStreamEpi / 32, kStreamCodesWarp = kStreamMmaWarp + 1, kStreamRowsWarp = kStreamMmaWarp + 2;
+constexpr int kStreamThreads = kStreamEpi + 96;
 constexpr int kSliceBytesA = kRowsPerCta * kSliceK;  // 16 KB
 constexpr int kMaxStages = 6;
 constexpr uint32_t kWaitLimit = 20000000u;
@@ -109,6 +109,33 @@ __device__ __forceinline__ bool wait_bounded(uint64_t* bar, uint32_t parity) {
 struct __align__(16) StreamScale {
     double os, zero;
 };
+// The same for the epilogue without float64: os = h + m + (less than 2^-48 of it), and what turns a raw sum into the bits of
+// 1.5 * 2^23 + sum of w * x.  m is a NaN where h is no ordinary number.
+struct __align__(16) StreamScale32 {
+    float h, m;
+    int zero, unused;
+};
+constexpr int kF32MaxK = 32640;  // columns up to which |sum of w * x| stays below 2^22
+__device__ __forceinline__ StreamScale32 gemm_scale32(double os, int xsum) {
+    StreamScale32 s;
+    s.h = (float)os;
+    const bool ordinary = s.h > 0x1p-60f && s.h < 0x1p60f;
+    s.m = ordinary ? (float)__dsub_rn(os, (double)s.h) : __int_as_float(0x7fffffff);
+    s.zero = 0x4B400000 - xsum;
+    s.unused = 0;
+    return s;
+}
+// float32(float64(a) * os) for a = sum of w * x, bit for bit, in float arithmetic: the product's rounding error and the second part of
+// os give a correction good to 2^-46 of the product, and the sum with it is the answer if moving it by 2^-45 either way rounds to the
+// same float.  Where it does not (one output in a million), or h is no ordinary number, `open` is set and the caller repeats it in float64.
+__device__ __forceinline__ float gemm_scaled32(int raw, const StreamScale32& s, bool& open) {
+    const float a = __int_as_float(raw + s.zero) - 12582912.f;
+    const float prod = __fmul_rn(a, s.h);
+    const float corr = fmaf(a, s.m, fmaf(a, s.h, -prod));
+    const float lo = __fadd_rn(prod, fmaf(fabsf(prod), -0x1p-45f, corr)), hi = __fadd_rn(prod, fmaf(fabsf(prod), 0x1p-45f, corr));
+    open = open || !(lo == hi);
+    return lo;
+}
 // int32 -> float64 by the exponent trick: 2^52 + 2^31 + a as a bit pattern, minus 2^52 + 2^31 + xsum.  Exact, and a full-rate
 // addition where the conversion instruction runs at quarter rate; the correction by xsum costs nothing.
 __device__ __forceinline__ double gemm_zero(int xsum) { return -__dadd_rn(4503601774854144.0, (double)xsum); }
@@ -116,7 +143,13 @@ __device__ __forceinline__ double gemm_i2d(int a, double zero) {
     return __dadd_rn(__hiloint2double(0x43300000, (int)((unsigned)a ^ 0x80000000u)), zero);
 }
 
-// sixteen consecutive columns of this thread's TMEM lane
+// eight / sixteen consecutive columns of this thread's TMEM lane
+__device__ __forceinline__ void gemm_tmem_ld8(uint32_t addr, uint32_t (&v)[8]) {
+    asm volatile("tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];"
+                 : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]), "=r"(v[4]), "=r"(v[5]), "=r"(v[6]), "=r"(v[7])
+                 : "r"(addr)
+                 : "memory");
+}
 __device__ __forceinline__ void gemm_tmem_ld16(uint32_t addr, uint32_t (&v)[16]) {
     asm volatile("tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15}, [%16];"
                  : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]), "=r"(v[4]), "=r"(v[5]), "=r"(v[6]), "=r"(v[7]), "=r"(v[8]),
@@ -125,8 +158,11 @@ __device__ __forceinline__ void gemm_tmem_ld16(uint32_t addr, uint32_t (&v)[16])
                  : "memory");
 }
 
-// Float epilogue of eight tokens from `tok` on (sc: theirs) of weight row r: v[j] = sum(code * x).
-__device__ __forceinline__ void gemm_emit8(const GemmParams& p, int r, bool row_ok, int tok, const uint32_t* v, const StreamScale* sc, double bias, bool has_bias) {
+// Float epilogue of eight tokens from `tok` on (sc, sc32: theirs) of weight row r: v[j] = sum(code * x).  F32: without a bias, raw sums
+// and float64 outputs, in float arithmetic (float64 instructions are slow beside the tensor core's work).
+template <bool F32>
+__device__ __forceinline__ void gemm_emit8(const GemmParams& p, int r, bool row_ok, int tok, const uint32_t* v, const StreamScale* sc, const StreamScale32* sc32, double bias,
+                                           bool has_bias) {
     if (!row_ok) return;
     const int ntok = p.tokens - tok;  // columns of this step that are real tokens
     size_t o0 = (size_t)tok * p.rows + r, ostride = (size_t)p.rows;
@@ -140,29 +176,38 @@ __device__ __forceinline__ void gemm_emit8(const GemmParams& p, int r, bool row_
 #pragma unroll
         for (int j = 0; j < 8; ++j, at += ostride) rs[j] = j < ntok ? *at : 0.f;
     }
-    double y[8];
     float f[8];
+    if (F32) {
+        bool open = false;
 #pragma unroll
-    for (int j = 0; j < 8; ++j) {
-        const StreamScale s = sc[j];
-        const double t = __dmul_rn(gemm_i2d((int)v[j], s.zero), s.os);
-        y[j] = has_bias ? __dadd_rn(t, bias) : t;
-    }
-    if (p.acc_out) {
-        int32_t* at = p.acc_out + o0;
+        for (int j = 0; j < 8; ++j) f[j] = gemm_scaled32((int)v[j], sc32[j], open);
+        if (open) {
 #pragma unroll
-        for (int j = 0; j < 8; ++j, at += ostride)
-            if (j < ntok) *at = (int)gemm_i2d((int)v[j], sc[j].zero);
-    }
-    if (p.out_f64) {
-        double* at = p.out_f64 + o0;
+            for (int j = 0; j < 8; ++j) f[j] = (float)__dmul_rn(gemm_i2d((int)v[j], sc[j].zero), sc[j].os);
+        }
+    } else {
+        double y[8];
 #pragma unroll
-        for (int j = 0; j < 8; ++j, at += ostride)
-            if (j < ntok) *at = y[j];
+        for (int j = 0; j < 8; ++j) {
+            const StreamScale s = sc[j];
+            const double t = __dmul_rn(gemm_i2d((int)v[j], s.zero), s.os);
+            y[j] = has_bias ? __dadd_rn(t, bias) : t;
+            f[j] = (float)y[j];
+        }
+        if (p.acc_out) {
+            int32_t* at = p.acc_out + o0;
+#pragma unroll
+            for (int j = 0; j < 8; ++j, at += ostride)
+                if (j < ntok) *at = (int)gemm_i2d((int)v[j], sc[j].zero);
+        }
+        if (p.out_f64) {
+            double* at = p.out_f64 + o0;
+#pragma unroll
+            for (int j = 0; j < 8; ++j, at += ostride)
+                if (j < ntok) *at = y[j];
+        }
     }
     if (!p.out) return;
-#pragma unroll
-    for (int j = 0; j < 8; ++j) f[j] = (float)y[j];
     if (p.pre_out) {
         float* at = p.pre_out + o0;
 #pragma unroll
@@ -186,11 +231,6 @@ __device__ __forceinline__ void gemm_emit8(const GemmParams& p, int r, bool row_
     for (int j = 0; j < 8; ++j, at += ostride)
         if (j < ntok) *at = f[j];
 }
-__device__ __forceinline__ void gemm_emit16(const GemmParams& p, int r, bool row_ok, int tok, const uint32_t* v, const StreamScale* sc, double bias, bool has_bias) {
-#pragma unroll
-    for (int h = 0; h < 16; h += 8) gemm_emit8(p, r, row_ok, tok + h, v + h, sc + h, bias, has_bias);
-}
-
 // stages that fit beside 1 KB of alignment slack
 template <int NTOK, int MODE>
 struct GemmCfg {
@@ -320,7 +360,10 @@ __global__ void __launch_bounds__(kGemmThreads, 1) lb_gemm_ternary_i8_kernel(con
         // (sixteen independent int -> float64 -> float32 chains in flight: with two warps per scheduler the epilogue is
         // bound by instruction latency, not throughput), then stored under the per-output conditions.
         const bool has_bias = row_ok && p.bias != nullptr;
-        auto emit = [&](int c0, const uint32_t* raw) { gemm_emit16(p, r, row_ok && !failed, tok0 + c0, raw, s_scale + c0, bias, has_bias); };
+        auto emit = [&](int c0, const uint32_t* raw) {
+#pragma unroll
+            for (int h = 0; h < 16; h += 8) gemm_emit8<false>(p, r, row_ok && !failed, tok0 + c0 + h, raw + h, s_scale + c0 + h, nullptr, bias, has_bias);
+        };
         const bool split = gridDim.z > 1;
 #pragma unroll 1
         for (int c0 = chalf * (NTOK / 2); c0 < (chalf + 1) * (NTOK / 2); c0 += 16) {
@@ -418,40 +461,62 @@ __global__ void __launch_bounds__(kGemmThreads, 1) lb_gemm_ternary_i8_kernel(con
 // 11,000), and how fast one thread can issue (lb_elect).  Sixteen epilogue warps instead of eight, statistics fetched a tile ahead,
 // a token's scale and correction in one 16-byte load, copies and MMAs from elected threads: 2048 x 6912 x 2560 43 -> 36 us,
 // 512 x 2560 x 6912 25 -> 17.5, 2999 x 14336 x 4096 164 -> 147; gate and up of 1024 x 6912 x 2560 67 -> 53.
+// A launch takes up to three products of the same activations (Q, K and V), whose row tiles follow one another.  Tiles are `ntok`
+// tokens wide, a multiple of 16 (gemm_stream_tokens has the rule), and of a group of token tiles the token runs fastest, so that the
+// CTAs at work together read few rows and few tokens: 2999 x 14336 x 4096 147 -> 142 us against rows first, 2048 x 2560 x 6912 52 -> 48.6.
 // DUAL: a gate / up pair that shares the activations -- both code blocks ride in one stage, two accumulators per buffer
-// (gate at column 0, up at column NTOK), and the epilogue writes float32(gateProduct(yg + bg, yu + bu)) only
+// (gate at column 0, up at column 128), and the epilogue writes float32(gateProduct(yg + bg, yu + bu)) only
 // (poly/swiglu.go:299-310): the two int32 accumulator planes never travel through memory.
-template <int NTOK, bool DUAL>
+constexpr int kStreamGroup = 12;  // token tiles of a group
+constexpr int kStreamMaxSegs = 3;
+struct StreamJob {
+    GemmParams seg[kStreamMaxSegs];
+    int first[kStreamMaxSegs];  // first row tile of a product (beyond the last one: row_tiles)
+    int row_tiles, tok_tiles, ntok, padded;  // padded: tokens of the activation image
+};
+template <bool DUAL>
 struct StreamCfg {
     static constexpr int kMats = DUAL ? 2 : 1;
-    static constexpr int kBytesB = NTOK * kSliceK;
     static constexpr int kBytesA = kSliceBytesA * kMats;
-    static constexpr int kStageBytes = kBytesA + kBytesB;
-    static constexpr int kStages = (200 * 1024) / kStageBytes > kMaxStages ? kMaxStages : (200 * 1024) / kStageBytes;
-    static constexpr int kAccCols = NTOK * kMats;  // TMEM columns of one accumulator buffer
-    static constexpr size_t kSmem = (size_t)kStages * kStageBytes + 1024;
-    static_assert(2 * kAccCols <= 512, "two accumulator buffers must fit the 512 TMEM columns");
+    static constexpr int kMaxTok = DUAL ? 128 : 256;
+    static constexpr int kRing = 200 * 1024;
+    static constexpr size_t kSmem = (size_t)kRing + 1024;
+    static __host__ __device__ int stages(int ntok) {
+        const int n = kRing / (kBytesA + ntok * kSliceK);
+        return n > kMaxStages ? kMaxStages : n;
+    }
 };
 
-template <int NTOK, bool DUAL>
-__global__ void __launch_bounds__(kStreamThreads, 1) lb_gemm_stream_kernel(const GemmParams p, int row_tiles, int ntiles) {
-    using Cfg = StreamCfg<NTOK, DUAL>;
-    constexpr int kStages = Cfg::kStages;
+template <bool DUAL, bool F32>
+__global__ void __launch_bounds__(kStreamThreads, 1) lb_gemm_stream_kernel(const __grid_constant__ StreamJob job) {
+    using Cfg = StreamCfg<DUAL>;
     extern __shared__ __align__(1024) uint8_t smem[];
     __shared__ __align__(8) uint64_t load_bar[kMaxStages], empty_bar[kMaxStages], acc_full[2], acc_empty[2];
     __shared__ uint32_t tmem_base_s;
-    __shared__ StreamScale s_scale[2][NTOK];
-    __shared__ double s_os_up[2][DUAL ? NTOK : 1];
+    __shared__ StreamScale s_scale[2][Cfg::kMaxTok];
+    __shared__ StreamScale32 s_scale32[2][F32 ? Cfg::kMaxTok : 1];
+    __shared__ double s_os_up[2][DUAL ? Cfg::kMaxTok : 1];
     __shared__ int s_failed;
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    const int ntok = job.ntok, stages = Cfg::stages(ntok), bytes_b = ntok * kSliceK;
     uint8_t* a_ring = smem;
-    uint8_t* b_ring = smem + kStages * Cfg::kBytesA;
-    const int ktot = p.kblocks;
+    uint8_t* b_ring = smem + stages * Cfg::kBytesA;
+    const int ktot = job.seg[0].kblocks, ntiles = job.row_tiles * job.tok_tiles;
     const int my_tiles = (int)blockIdx.x < ntiles ? (ntiles - (int)blockIdx.x + (int)gridDim.x - 1) / (int)gridDim.x : 0;
+    struct Tile {
+        int seg, row, tok0;  // product, row tile inside it, first token
+    };
+    auto tile_at = [&](int i) {
+        const int t = (int)blockIdx.x + i * (int)gridDim.x;
+        const int g0 = t / (kStreamGroup * job.row_tiles) * kStreamGroup, left = job.tok_tiles - g0, gn = left < kStreamGroup ? left : kStreamGroup;
+        const int in = t - g0 * job.row_tiles, rt = in / gn;
+        const int seg = DUAL || rt < job.first[1] ? 0 : rt < job.first[2] ? 1 : 2;
+        return Tile{seg, rt - job.first[seg], (g0 + in - rt * gn) * ntok};
+    };
 
     if (tid == 0) {
-        for (int s = 0; s < kStages; ++s) {
-            lb_mbar_init(&load_bar[s], 1);
+        for (int s = 0; s < stages; ++s) {
+            lb_mbar_init(&load_bar[s], 2);
             lb_mbar_init(&empty_bar[s], 1);
         }
         for (int b = 0; b < 2; ++b) {
@@ -462,7 +527,7 @@ __global__ void __launch_bounds__(kStreamThreads, 1) lb_gemm_stream_kernel(const
         s_failed = 0;
     }
     if (warp == kStreamMmaWarp) {
-        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(lb_smem_u32(&tmem_base_s)), "r"(2 * Cfg::kAccCols) : "memory");
+        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(lb_smem_u32(&tmem_base_s)), "r"(512) : "memory");
         asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
     }
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
@@ -471,46 +536,50 @@ __global__ void __launch_bounds__(kStreamThreads, 1) lb_gemm_stream_kernel(const
     const uint32_t tmem_base = tmem_base_s;
     lb_pdl_launch_dependents();
 
-    if (warp == kStreamLoadWarp) {
-        // ---------------- loads: per stage the activations of the tile's tokens and the code block(s) of its rows ----------------
+    if (warp == kStreamCodesWarp || warp == kStreamRowsWarp) {
+        // ---------------- loads: a thread for the code block(s) of the tile's rows, one for the activations of its tokens ----------------
+        // (one thread for both issues a slice's copies in about the time the tensor core takes for a slice of 128 tokens)
         if (lb_elect()) {
+            const bool rows = warp == kStreamRowsWarp;
+            // The codes do not depend on the quantizer that runs before this kernel, only the activations do.
+            if (rows) lb_pdl_wait();
             bool failed = false;
-            uint32_t it = 0;
-            // The weights do not depend on the quantizer that runs before this kernel: the code blocks of the first stages
-            // are requested before the dependency wait, their activations after it (one barrier counts the bytes of both).
-            int pre = 0;
-            if (my_tiles > 0) {
-                const int rt0 = (int)blockIdx.x % row_tiles;
-                const size_t blk00 = (size_t)rt0 * ktot * kSliceBytesA;
-                pre = ktot < kStages ? ktot : kStages;
-                for (int ks = 0; ks < pre; ++ks) {
-                    lb_mbar_expect_tx(&load_bar[ks], (uint32_t)Cfg::kStageBytes);
-                    lb_bulk_g2s(a_ring + (size_t)ks * Cfg::kBytesA, p.codes8 + blk00 + (size_t)ks * kSliceBytesA, (uint32_t)kSliceBytesA, &load_bar[ks]);
-                    if (DUAL)
-                        lb_bulk_g2s(a_ring + (size_t)ks * Cfg::kBytesA + kSliceBytesA, p.codes8_up + blk00 + (size_t)ks * kSliceBytesA,
-                                    (uint32_t)kSliceBytesA, &load_bar[ks]);
-                }
-            }
-            lb_pdl_wait();
+            int s = 0;
+            uint32_t parity = 1;  // (the first round's waits are over at once)
             for (int i = 0; i < my_tiles && !failed; ++i) {
-                const int t = (int)blockIdx.x + i * (int)gridDim.x;
-                const int rt = t % row_tiles, tok0 = (t / row_tiles) * NTOK;
-                const int8_t* qbase = p.q + (size_t)(tok0 >> 8) * ktot * 32768 + (size_t)((tok0 & 255) >> 3) * 1024;
-                const size_t blk0 = (size_t)rt * ktot * kSliceBytesA;
-                for (int ks = 0; ks < ktot; ++ks, ++it) {
-                    const int s = (int)(it % kStages);
-                    if (it >= (uint32_t)kStages && !wait_bounded(&empty_bar[s], (it / kStages - 1) & 1)) {
+                const Tile t = tile_at(i);
+                const GemmParams& p = job.seg[t.seg];
+                // a tile's tokens lie in one block of 256 or in two; the image ends with the block of the last token
+                const int n = job.padded - t.tok0 < ntok ? job.padded - t.tok0 : ntok, n0 = 256 - (t.tok0 & 255) < n ? 256 - (t.tok0 & 255) : n;
+                const uint8_t* code = p.codes8 + (size_t)t.row * ktot * kSliceBytesA;
+                const uint8_t* code_up = DUAL ? p.codes8_up + (size_t)t.row * ktot * kSliceBytesA : nullptr;
+                const int8_t* q0 = p.q + (size_t)(t.tok0 >> 8) * ktot * 32768 + (size_t)((t.tok0 & 255) >> 3) * 1024;
+                const int8_t* q1 = p.q + (size_t)((t.tok0 >> 8) + 1) * ktot * 32768;
+                for (int ks = 0; ks < ktot; ++ks) {
+                    if (!wait_bounded(&empty_bar[s], parity)) {
                         failed = true;
                         break;
                     }
-                    const bool a_done = i == 0 && ks < pre;  // requested before the dependency wait
-                    if (!a_done) lb_mbar_expect_tx(&load_bar[s], (uint32_t)Cfg::kStageBytes);
-                    lb_bulk_g2s(b_ring + (size_t)s * Cfg::kBytesB, qbase + (size_t)ks * 32768, (uint32_t)Cfg::kBytesB, &load_bar[s]);
-                    if (!a_done) {
-                        lb_bulk_g2s(a_ring + (size_t)s * Cfg::kBytesA, p.codes8 + blk0 + (size_t)ks * kSliceBytesA, (uint32_t)kSliceBytesA, &load_bar[s]);
-                        if (DUAL)
-                            lb_bulk_g2s(a_ring + (size_t)s * Cfg::kBytesA + kSliceBytesA, p.codes8_up + blk0 + (size_t)ks * kSliceBytesA,
-                                        (uint32_t)kSliceBytesA, &load_bar[s]);
+                    if (rows) {
+                        uint8_t* dst = b_ring + s * bytes_b;
+                        lb_mbar_expect_tx(&load_bar[s], (uint32_t)(n * kSliceK));
+                        lb_bulk_g2s(dst, q0, (uint32_t)(n0 * kSliceK), &load_bar[s]);
+                        if (n > n0) lb_bulk_g2s(dst + n0 * kSliceK, q1, (uint32_t)((n - n0) * kSliceK), &load_bar[s]);
+                        q0 += 32768;
+                        q1 += 32768;
+                    } else {
+                        uint8_t* dst = a_ring + s * Cfg::kBytesA;
+                        lb_mbar_expect_tx(&load_bar[s], (uint32_t)Cfg::kBytesA);
+                        lb_bulk_g2s(dst, code, (uint32_t)kSliceBytesA, &load_bar[s]);
+                        code += kSliceBytesA;
+                        if (DUAL) {
+                            lb_bulk_g2s(dst + kSliceBytesA, code_up, (uint32_t)kSliceBytesA, &load_bar[s]);
+                            code_up += kSliceBytesA;
+                        }
+                    }
+                    if (++s == stages) {
+                        s = 0;
+                        parity ^= 1;
                     }
                 }
             }
@@ -520,9 +589,10 @@ __global__ void __launch_bounds__(kStreamThreads, 1) lb_gemm_stream_kernel(const
     } else if (warp == kStreamMmaWarp) {
         // ---------------- MMA issuer ----------------
         if (lb_elect()) {
-            const uint32_t idesc = (2u << 4) | (0u << 7) | (1u << 10) | ((uint32_t)(NTOK >> 3) << 17) | ((uint32_t)(kRowsPerCta >> 4) << 24);
+            const uint32_t idesc = (2u << 4) | (0u << 7) | (1u << 10) | ((uint32_t)(ntok >> 3) << 17) | ((uint32_t)(kRowsPerCta >> 4) << 24);
             bool failed = false;
-            uint32_t it = 0;
+            int s = 0;
+            uint32_t parity = 0;
             for (int i = 0; i < my_tiles && !failed; ++i) {
                 const int buf = i & 1;
                 // the epilogue must have drained this buffer's previous tile
@@ -531,25 +601,28 @@ __global__ void __launch_bounds__(kStreamThreads, 1) lb_gemm_stream_kernel(const
                     break;
                 }
                 asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-                const uint32_t d = tmem_base + (uint32_t)(buf * Cfg::kAccCols);
-                for (int ks = 0; ks < ktot; ++ks, ++it) {
-                    const int s = (int)(it % kStages);
-                    if (!wait_bounded(&load_bar[s], (it / kStages) & 1)) {
+                const uint32_t d = tmem_base + (uint32_t)(buf * 256);
+                for (int ks = 0; ks < ktot; ++ks) {
+                    if (!wait_bounded(&load_bar[s], parity)) {
                         failed = true;
                         break;
                     }
                     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
                     const uint64_t a_desc = smem_desc(lb_smem_u32(a_ring + (size_t)s * Cfg::kBytesA));
-                    const uint64_t b_desc = smem_desc(lb_smem_u32(b_ring + (size_t)s * Cfg::kBytesB));
+                    const uint64_t b_desc = smem_desc(lb_smem_u32(b_ring + (size_t)s * bytes_b));
 #pragma unroll
                     for (int k = 0; k < kSliceK / 32; ++k)  // (256 bytes further in K, in units of 16)
                         mma_i8(d, a_desc + k * 16, b_desc + k * 16, idesc, (ks > 0 || k > 0) ? 1u : 0u);
                     if (DUAL) {
 #pragma unroll
                         for (int k = 0; k < kSliceK / 32; ++k)
-                            mma_i8(d + (uint32_t)NTOK, a_desc + (kSliceBytesA >> 4) + k * 16, b_desc + k * 16, idesc, (ks > 0 || k > 0) ? 1u : 0u);
+                            mma_i8(d + 128, a_desc + (kSliceBytesA >> 4) + k * 16, b_desc + k * 16, idesc, (ks > 0 || k > 0) ? 1u : 0u);
                     }
                     mma_commit(&empty_bar[s]);
+                    if (++s == stages) {
+                        s = 0;
+                        parity ^= 1;
+                    }
                 }
                 if (!failed) mma_commit(&acc_full[buf]);  // arrives when every MMA of the tile is done
             }
@@ -559,66 +632,66 @@ __global__ void __launch_bounds__(kStreamThreads, 1) lb_gemm_stream_kernel(const
         asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
     } else {
         // ---------------- epilogue warps: tile i while the MMA warp is on tile i + 1 ----------------
-        // a warp may only touch the 32 TMEM lanes of its quarter (warp % 4); the warps of a quarter split the columns
-        constexpr int kShare = NTOK / (kStreamEpi / 128);  // columns of a warp
-        const int quarter = warp & 3, first = (warp >> 2) * kShare;
+        // a warp may only touch the 32 TMEM lanes of its quarter (warp % 4); the warps of a quarter take turns at eight columns
+        const int quarter = warp & 3;
         bool failed = false;  // after a wait ran out the warp keeps walking the tiles (its named-barrier count must match) without touching TMEM or memory
         lb_pdl_wait();  // the per-token scales, the residual rows and the output buffer belong to earlier launches until here
         // a token's statistics are fetched a tile ahead and become scales behind the tile in front: one barrier per tile
         float amax = 0.f;
         int xsum = 0;
-        auto fetch_stats = [&](int i) {
-            const int tok = ((int)blockIdx.x + i * (int)gridDim.x) / row_tiles * NTOK + tid;
-            const bool ok = tid < NTOK && i < my_tiles && tok < p.tokens;
-            amax = ok ? p.amax[tok] : 0.f;
-            xsum = ok ? p.xsum[tok] : 0;
+        Tile next = my_tiles > 0 ? tile_at(0) : Tile{0, 0, 0};
+        auto fetch_stats = [&](bool any) {
+            const int tok = next.tok0 + tid;
+            const bool ok = any && tid < ntok && tok < job.seg[0].tokens;
+            amax = ok ? job.seg[0].amax[tok] : 0.f;
+            xsum = ok ? job.seg[0].xsum[tok] : 0;
         };
-        fetch_stats(0);
+        fetch_stats(my_tiles > 0);
         for (int i = 0; i < my_tiles; ++i) {
-            const int t = (int)blockIdx.x + i * (int)gridDim.x;
-            const int rt = t % row_tiles, tok0 = (t / row_tiles) * NTOK, buf = i & 1;
-            if (tid < NTOK) {  // (columns of absent tokens are computed and not stored)
-                s_scale[buf][tid].os = lb_output_scale(p.scale, amax);
+            const Tile t = next;
+            const GemmParams& p = job.seg[t.seg];
+            const int buf = i & 1;
+            if (tid < ntok) {  // (columns of absent tokens are computed and not stored)
+                const double os = lb_output_scale(p.scale, amax);
+                s_scale[buf][tid].os = os;
                 s_scale[buf][tid].zero = gemm_zero(xsum);
                 if (DUAL) s_os_up[buf][tid] = lb_output_scale(p.scale_up, amax);
+                if (F32) s_scale32[buf][tid] = gemm_scale32(os, xsum);
             }
             asm volatile("bar.sync 1, %0;" ::"n"(kStreamEpi) : "memory");  // (everyone is also done with the scales of two tiles ago)
-            fetch_stats(i + 1);
+            if (i + 1 < my_tiles) next = tile_at(i + 1);
+            fetch_stats(i + 1 < my_tiles);
             if (!failed && !wait_bounded(&acc_full[buf], (uint32_t)((i >> 1) & 1))) {
                 failed = true;
                 atomicExch(&s_failed, 1);
             }
             asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-            const int r = rt * kRowsPerCta + quarter * 32 + lane;
+            const int r = t.row * kRowsPerCta + quarter * 32 + lane;
             const bool row_ok = r < p.rows;
             const bool has_bias = row_ok && p.bias != nullptr, has_bias_up = DUAL && row_ok && p.bias_up != nullptr;
             const double bias = has_bias ? (double)p.bias[r] : 0.0, bias_up = has_bias_up ? (double)p.bias_up[r] : 0.0;
-            const uint32_t tacc = tmem_base + (uint32_t)(buf * Cfg::kAccCols) + ((uint32_t)(quarter * 32) << 16);
+            const uint32_t tacc = tmem_base + (uint32_t)(buf * 256) + ((uint32_t)(quarter * 32) << 16);
             if (!failed) {
 #pragma unroll 1
-                for (int c0 = first; c0 < first + kShare; c0 += 16) {
-                    uint32_t v[16];
-                    gemm_tmem_ld16(tacc + (uint32_t)c0, v);
+                for (int c0 = (warp >> 2) * 8; c0 < ntok; c0 += 8 * (kStreamEpi / 128)) {
+                    uint32_t v[8], u[8];
+                    gemm_tmem_ld8(tacc + (uint32_t)c0, v);
+                    if (DUAL) gemm_tmem_ld8(tacc + (uint32_t)(128 + c0), u);
+                    asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
                     if (!DUAL) {
-                        asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
-                        gemm_emit16(p, r, row_ok, tok0 + c0, v, s_scale[buf] + c0, bias, has_bias);
-                    } else {
-                        uint32_t u[16];
-                        gemm_tmem_ld16(tacc + (uint32_t)(NTOK + c0), u);
-                        asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
-                        if (row_ok) {
-                            const int ntok = p.tokens - (tok0 + c0);
-                            float* o = p.out + (size_t)(tok0 + c0) * p.rows + r;
+                        gemm_emit8<F32>(p, r, row_ok, t.tok0 + c0, v, s_scale[buf] + c0, s_scale32[F32 ? buf : 0] + c0, bias, has_bias);
+                    } else if (row_ok) {
+                        const int left = p.tokens - (t.tok0 + c0);
+                        float* o = p.out + (size_t)(t.tok0 + c0) * p.rows + r;
 #pragma unroll
-                            for (int j = 0; j < 16; ++j, o += p.rows) {
-                                const StreamScale sc = s_scale[buf][c0 + j];
-                                double yg = __dmul_rn(gemm_i2d((int)v[j], sc.zero), sc.os);
-                                double yu = __dmul_rn(gemm_i2d((int)u[j], sc.zero), s_os_up[buf][c0 + j]);
-                                if (has_bias) yg = __dadd_rn(yg, bias);
-                                if (has_bias_up) yu = __dadd_rn(yu, bias_up);
-                                const float f = (float)lb_gate_product(yg, yu, p.act);
-                                if (j < ntok) *o = f;
-                            }
+                        for (int j = 0; j < 8; ++j, o += p.rows) {
+                            const StreamScale sc = s_scale[buf][c0 + j];
+                            double yg = __dmul_rn(gemm_i2d((int)v[j], sc.zero), sc.os);
+                            double yu = __dmul_rn(gemm_i2d((int)u[j], sc.zero), s_os_up[buf][c0 + j]);
+                            if (has_bias) yg = __dadd_rn(yg, bias);
+                            if (has_bias_up) yu = __dadd_rn(yu, bias_up);
+                            const float f = (float)lb_gate_product(yg, yu, p.act);
+                            if (j < left) *o = f;
                         }
                     }
                 }
@@ -632,9 +705,9 @@ __global__ void __launch_bounds__(kStreamThreads, 1) lb_gemm_stream_kernel(const
     __syncthreads();
     if (warp == kStreamMmaWarp) {
         asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-        asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem_base), "r"(2 * Cfg::kAccCols) : "memory");
+        asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem_base), "r"(512) : "memory");
     }
-    if (tid == 0 && s_failed) atomicExch(p.status, 3);
+    if (tid == 0 && s_failed) atomicExch(job.seg[0].status, 3);
 }
 
 // Measures what the tensor pipe can do on this shape of instruction: one CTA per SM, operands resident in shared memory
@@ -1081,19 +1154,50 @@ static int gemm_launch(loom_b200_ctx* ctx, const GemmParams& p, dim3 grid, unsig
     return 0;
 }
 
-// the persistent kernel: one CTA per SM (or per tile, if there are fewer tiles)
-template <int NTOK, bool DUAL>
-static int gemm_launch_stream(loom_b200_ctx* ctx, const GemmParams& p, unsigned attr_bit) {
-    using Cfg = StreamCfg<NTOK, DUAL>;
+// Tokens per tile of the persistent kernel: the widest, or what is five percent better in the time until the busiest CTA is done plus the
+// time all SMs together are kept from other streams' work.  Measured: a k-slice takes 0.25 us with up to 128 tokens and 0.39 with 256; an
+// epilogue beside MMAs 2 us and 0.036 us a token (a gate / up pair: twice the slice, 0.11 us a token), the last one 0.02.  Wide tiles
+// leave a last wave of few of them: 2048 tokens of 20 row tiles, K = 6912, take 42 us as 160 tiles of 256 and 32 us as 260 of 160;
+// 700 x 4096 x 4096 29 us with 256 tokens and 24 with 176.  Narrow ones load the codes more often: three streams that each multiply 512
+// tokens by both 2B projections take 30 us a pass with 256, 33 with 128, 36 with 112 and 80.
+static int gemm_stream_tokens(const loom_b200_ctx* ctx, int row_tiles, int tokens, int kblocks, bool dual) {
+    const int most = dual ? 128 : 256;
+    if (ctx->opt_gemm_tile) return ctx->opt_gemm_tile < most ? ctx->opt_gemm_tile : most;
+    int best = most;
+    double best_us = 1e30;
+    for (int n = most; n >= 48; n -= 16) {
+        const int tiles = row_tiles * ((tokens + n - 1) / n), waves = (tiles + ctx->sm_count - 1) / ctx->sm_count;
+        const double slices = kblocks * (dual ? 2 : 1) * (n <= 128 ? 0.25 : 0.25 + (n - 128) * (0.14 / 128));
+        const double beside = 2.0 + n * (dual ? 0.11 : 0.036), tile = slices > beside ? slices : beside;
+        const double us = slices + (waves - 1) * tile + n * (dual ? 0.06 : 0.02) + tile * tiles / ctx->sm_count;
+        if (us < 0.95 * best_us) {
+            best_us = us;
+            best = n;
+        }
+    }
+    return best;
+}
+
+// the persistent kernel over the products of job.seg[0 .. nseg): one CTA per SM (or per tile, if there are fewer tiles)
+template <bool DUAL, bool F32>
+static int gemm_launch_stream(loom_b200_ctx* ctx, StreamJob& job, int nseg, unsigned attr_bit) {
+    using Cfg = StreamCfg<DUAL>;
     if (!(ctx->func_attr_mask2 & attr_bit)) {
-        LB_CUDA(ctx, cudaFuncSetAttribute(lb_gemm_stream_kernel<NTOK, DUAL>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)Cfg::kSmem));
+        LB_CUDA(ctx, cudaFuncSetAttribute(lb_gemm_stream_kernel<DUAL, F32>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)Cfg::kSmem));
         ctx->func_attr_mask2 |= attr_bit;
     }
-    const int row_tiles = (p.rows + kRowsPerCta - 1) / kRowsPerCta;
-    const int ntiles = row_tiles * ((p.tokens + NTOK - 1) / NTOK);
-    const int grid = ntiles < ctx->sm_count ? ntiles : ctx->sm_count;
+    job.row_tiles = 0;
+    for (int i = 0; i < kStreamMaxSegs; ++i) {
+        job.first[i] = job.row_tiles;
+        if (i < nseg) job.row_tiles += (job.seg[i].rows + kRowsPerCta - 1) / kRowsPerCta;
+    }
+    const int tokens = job.seg[0].tokens;
+    job.ntok = gemm_stream_tokens(ctx, job.row_tiles, tokens, job.seg[0].kblocks, DUAL);
+    job.tok_tiles = (tokens + job.ntok - 1) / job.ntok;
+    job.padded = padded_tokens(tokens);
+    const int ntiles = job.row_tiles * job.tok_tiles;
     cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3(grid);
+    cfg.gridDim = dim3(ntiles < ctx->sm_count ? ntiles : ctx->sm_count);
     cfg.blockDim = dim3(kStreamThreads);
     cfg.dynamicSmemBytes = Cfg::kSmem;
     cfg.stream = ctx->stream;
@@ -1104,18 +1208,25 @@ static int gemm_launch_stream(loom_b200_ctx* ctx, const GemmParams& p, unsigned 
     // (a launch that follows the build of its code cache starts only when that build is complete and visible)
     cfg.numAttrs = ctx->opt_pdl && !ctx->gemm_codes_fresh ? 1 : 0;
     ctx->gemm_codes_fresh = false;
-    LB_CUDA(ctx, cudaLaunchKernelEx(&cfg, lb_gemm_stream_kernel<NTOK, DUAL>, p, row_tiles, ntiles));
+    LB_CUDA(ctx, cudaLaunchKernelEx(&cfg, lb_gemm_stream_kernel<DUAL, F32>, job));
     ctx->launches++;
     return 0;
 }
 
-int lb_gemm_run(loom_b200_ctx* ctx, const loom_b200_weight* w, int tokens, const LbGemmOut& o) {
+static int gemm_launch_plain(loom_b200_ctx* ctx, StreamJob& job, int nseg) {
+    bool f32 = true;
+    for (int i = 0; i < nseg; ++i) f32 = f32 && !job.seg[i].bias && !job.seg[i].acc_out && !job.seg[i].out_f64 && job.seg[i].Kp <= kF32MaxK;
+    return f32 ? gemm_launch_stream<false, true>(ctx, job, nseg, 1u << 27) : gemm_launch_stream<false, false>(ctx, job, nseg, 1u << 26);
+}
+
+// what a product of the activations quantized last needs; 0 or an error
+static int gemm_params(loom_b200_ctx* ctx, const loom_b200_weight* w, int tokens, const LbGemmOut& o, GemmParams& p) {
     LB_REQUIRE(ctx, w && tokens > 0 && (o.out || o.out_f64 || o.acc_out), "gemm_run: bad arguments");
     LB_REQUIRE(ctx, w->device == ctx->device, "ternary_gemm: weight lives on device %d, context on %d", w->device, ctx->device);
     const int Kp = w->kblocks * kTileCols;
     LB_REQUIRE(ctx, (size_t)padded_tokens(tokens) * Kp <= ctx->gemm_scratch_bytes, "gemm_run: no quantized activations for %d tokens of %d columns", tokens, w->cols);
     GemmScratch g = gemm_scratch_at(ctx->gemm_scratch, tokens, Kp);
-    GemmParams p = {};
+    p = GemmParams{};
     p.tiles = w->tiles;
     p.rows = w->rows;
     p.strips = w->strips;
@@ -1137,6 +1248,28 @@ int lb_gemm_run(loom_b200_ctx* ctx, const loom_b200_weight* w, int tokens, const
     p.kv_msl = o.kv_msl;
     p.kv_pos0 = o.kv_pos0;
     p.status = ctx->status_dev;
+    return 0;
+}
+
+// Several products of the same activations: one launch over pre-expanded codes, else one after the other.  Q, K and V of 1024 tokens
+// x 2560 + 640 + 640 rows were three launches of 80, 40 and 40 tiles.
+int lb_gemm_run_group(loom_b200_ctx* ctx, const loom_b200_weight* const* w, int n, int tokens, const LbGemmOut* o) {
+    bool one = ctx->opt_gemm_stream && !ctx->trace_dev && n <= kStreamMaxSegs;
+    StreamJob job = {};
+    for (int i = 0; i < n && one; ++i) {
+        if (int rc = gemm_params(ctx, w[i], tokens, o[i], job.seg[i])) return rc;
+        one = w[i]->kblocks == w[0]->kblocks && gemm_ensure_codes(ctx, w[i]);
+        job.seg[i].codes8 = w[i]->codes8;
+    }
+    if (one) return gemm_launch_plain(ctx, job, n);
+    for (int i = 0; i < n; ++i)
+        if (int rc = lb_gemm_run(ctx, w[i], tokens, o[i])) return rc;
+    return 0;
+}
+
+int lb_gemm_run(loom_b200_ctx* ctx, const loom_b200_weight* w, int tokens, const LbGemmOut& o) {
+    GemmParams p;
+    if (int rc = gemm_params(ctx, w, tokens, o, p)) return rc;
     // phase trace: one row for the kernel and one per k-slice, kept contiguous (skipped if the ring of rows would wrap)
     p.trace = nullptr;
     if (ctx->trace_dev && (ctx->trace_seq % kTraceSlots) + w->kblocks + 2 < kTraceSlots) {
@@ -1163,9 +1296,11 @@ int lb_gemm_run(loom_b200_ctx* ctx, const loom_b200_weight* w, int tokens, const
         if (splits > w->kblocks / 4) splits = w->kblocks / 4;
         if (splits > 8) splits = 8;
         if (splits < 1) splits = 1;
-        // measured: a k-slice costs a CTA about 0.5 us, the atomic hand-over of a split about 0.15 us per token of the tile + 2 us
+        // measured: a k-slice costs a CTA of this kernel about 0.5 us, of the persistent one 0.25; the atomic hand-over of a split costs
+        // 0.15 to 0.35 us per token of the tile + 2 us (2560 x 6912: 64 tokens 28 us in seven splits, 13 us in the persistent kernel)
         const int tile_tokens = tokens < (wide ? 256 : 128) ? tokens : (wide ? 256 : 128);
-        if (splits > 1 && 0.5 * w->kblocks * (1.0 - 1.0 / splits) <= 0.15 * tile_tokens + 2.0) splits = 1;
+        const bool stream = cached && !p.trace && ctx->opt_gemm_stream;
+        if (splits > 1 && (stream ? 0.25 : 0.5) * w->kblocks - 0.5 * w->kblocks / splits <= (stream ? 0.35 : 0.15) * tile_tokens + 2.0) splits = 1;
     }
     if (splits > 1) {
         if (int rc = lb_ensure_fixup(ctx, (size_t)tokens * w->rows, (size_t)tiles)) return rc;
@@ -1173,12 +1308,9 @@ int lb_gemm_run(loom_b200_ctx* ctx, const loom_b200_weight* w, int tokens, const
         p.part_cnt = ctx->fix_cnt;
     }
     if (cached && splits == 1 && !p.trace && ctx->opt_gemm_stream) {
-        // persistent kernel: a tile's time follows the bytes its stages load (32 KB per slice for 128 tokens, 48 KB for
-        // 256), the launch's time the tiles of the busiest CTA
-        bool wide_s = tokens > 128 && 48 * ((ct256 + sms - 1) / sms) <= 32 * ((ct128 + sms - 1) / sms);
-        if (ctx->opt_gemm_tile == 128) wide_s = false;
-        if (ctx->opt_gemm_tile == 256) wide_s = true;
-        return wide_s ? gemm_launch_stream<256, false>(ctx, p, 1u << 26) : gemm_launch_stream<128, false>(ctx, p, 1u << 27);
+        StreamJob job = {};
+        job.seg[0] = p;
+        return gemm_launch_plain(ctx, job, 1);
     }
     if (wide) {
         dim3 grid(row_tiles, (tokens + 255) / 256, splits);
@@ -1196,30 +1328,19 @@ int lb_gemm_run_swiglu(loom_b200_ctx* ctx, const loom_b200_weight* gate, const l
     LB_REQUIRE(ctx, gate && up && tokens > 0 && prod, "gemm_run_swiglu: bad arguments");
     LB_REQUIRE(ctx, gate->rows == up->rows && gate->cols == up->cols, "gemm_run_swiglu: gate %dx%d and up %dx%d differ", gate->rows, gate->cols, up->rows, up->cols);
     if (!ctx->opt_gemm_stream || !gemm_ensure_codes(ctx, gate) || !gemm_ensure_codes(ctx, up)) return LOOM_B200_ERR_UNSUPPORTED;
-    const int Kp = gate->kblocks * kTileCols;
-    LB_REQUIRE(ctx, (size_t)padded_tokens(tokens) * Kp <= ctx->gemm_scratch_bytes, "gemm_run_swiglu: no quantized activations for %d tokens of %d columns", tokens, gate->cols);
-    GemmScratch g = gemm_scratch_at(ctx->gemm_scratch, tokens, Kp);
-    GemmParams p = {};
-    p.tiles = gate->tiles;
+    LbGemmOut o = {};
+    o.bias = bias_g;
+    o.act = act;
+    o.out = prod;
+    StreamJob job = {};
+    GemmParams& p = job.seg[0];
+    if (int rc = gemm_params(ctx, gate, tokens, o, p)) return rc;
     p.codes8 = gate->codes8;
     p.codes8_up = up->codes8;
-    p.rows = gate->rows;
-    p.strips = gate->strips;
-    p.kblocks = gate->kblocks;
-    p.scale = gate->scale;
     p.scale_up = up->scale;
-    p.q = g.q;
-    p.amax = g.amax;
-    p.xsum = g.xsum;
-    p.tokens = tokens;
-    p.Kp = Kp;
-    p.bias = bias_g;
     p.bias_up = bias_u;
-    p.act = act;
-    p.out = prod;
-    p.status = ctx->status_dev;
-    // 128 tokens per tile: two accumulators of 128 columns in each of the two TMEM buffers
-    return gemm_launch_stream<128, true>(ctx, p, 1u << 25);
+    // at most 128 tokens per tile: two accumulators of 128 columns in each of the two TMEM buffers
+    return gemm_launch_stream<true, false>(ctx, job, 1, 1u << 25);
 }
 
 int lb_gemm_gate_product(loom_b200_ctx* ctx, const int32_t* acc_g, const int32_t* acc_u, int tokens, int inter, int K, float scale_g,

@@ -139,6 +139,8 @@ struct LbGemmOut {
 };
 int lb_gemm_quantize(loom_b200_ctx* ctx, const LbGemmQuant& a);
 int lb_gemm_run(loom_b200_ctx* ctx, const loom_b200_weight* w, int tokens, const LbGemmOut& o);
+// several products of the rows quantized last (matrices of one width), in one launch where that can be
+int lb_gemm_run_group(loom_b200_ctx* ctx, const loom_b200_weight* const* w, int n, int tokens, const LbGemmOut* o);
 // gate and up projections fused with the gate product (needs the pre-expanded codes; LOOM_B200_ERR_UNSUPPORTED otherwise)
 int lb_gemm_run_swiglu(loom_b200_ctx* ctx, const loom_b200_weight* gate, const loom_b200_weight* up, int tokens, const float* bias_g,
                        const float* bias_u, int act, float* prod);
