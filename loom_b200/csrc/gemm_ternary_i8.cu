@@ -26,6 +26,7 @@
 //     rescale, bias, activation and residual exactly like the GEMV epilogue.
 // Every mbarrier wait is bounded; on expiry the kernel raises the context's status word, frees its tensor memory
 // and returns.
+#include "dense.cuh"
 #include "layers.cuh"
 
 namespace {
@@ -840,6 +841,26 @@ __global__ void __launch_bounds__(256) lb_quantize_gemm_kernel(const LbGemmQuant
     }
 }
 
+// Sixteen values against the scale s = 127 / absmax, bit for bit what lb_quant_i8 makes of them, in float arithmetic: h = s rounded, a value
+// times h is off by less than 2^-16 (127 times two roundings) and the sum with one half by 2^-18 more, so its floor is the answer unless
+// it lies within 2^-15 of an integer (one value in 16,000, and what is no number).  False: some value does; nothing is decided.
+__device__ __forceinline__ bool gemm_quant16_f32(const float* v, float h, uint32_t (&wds)[4]) {
+    bool sure = true;
+    uint32_t q[16];
+#pragma unroll
+    for (int k = 0; k < 16; ++k) {
+        const float t = __fadd_rn(__fmul_rn(fabsf(v[k]), h), 0.5f);
+        const float u = __fadd_rz(t, 8388608.f);  // floor(t) in the low bits
+        sure = sure && fabsf(__fadd_rn(__fsub_rn(t, __fsub_rn(u, 8388608.f)), -0.5f)) < 0.5f - 0x1p-15f;
+        const uint32_t neg = (uint32_t)(__float_as_int(v[k]) >> 31);
+        q[k] = (__float_as_uint(u) ^ neg) - neg;  // (only the low byte counts)
+    }
+#pragma unroll
+    for (int j = 0; j < 4; ++j)  // byte 4j + b of the chunk holds column 4b + j
+        wds[j] = __byte_perm(__byte_perm(q[j], q[4 + j], 0x0040), __byte_perm(q[8 + j], q[12 + j], 0x0040), 0x5410);
+    return sure;
+}
+
 // The same quantizer with the token's row held in registers: thread t owns the 16-column chunks t, t + T, ... (CPT of them),
 // loads each with four 16-byte loads (all in flight together), and never stages the row in shared memory; one block
 // reduction for the norm's sum of squares, one for the absmax.  The arithmetic per element is that of the kernel above;
@@ -945,13 +966,15 @@ __global__ void __launch_bounds__(256) lb_quantize_gemm_regs_kernel(const LbGemm
     for (int c = 0; c < CPT; ++c) {
         const int ch = tid + c * T;
         if (ch < nchunks) {
-            uint32_t wds[4] = {0u, 0u, 0u, 0u};
+            uint32_t wds[4];
+            if (f64 || a.given_amax || !gemm_quant16_f32(reinterpret_cast<const float*>(v[c]), (float)s, wds)) {
+                wds[0] = wds[1] = wds[2] = wds[3] = 0u;
 #pragma unroll
-            for (int k = 0; k < 16; ++k) {  // k = 4b + j -> destination byte 4j + b
-                const int qv = lb_quant_i8((double)v[c][k], s);
-                sum += qv;
-                wds[k & 3] |= (uint32_t)(qv & 0xff) << (8 * (k >> 2));
+                for (int k = 0; k < 16; ++k)  // k = 4b + j -> destination byte 4j + b
+                    wds[k & 3] |= (uint32_t)(lb_quant_i8((double)v[c][k], s) & 0xff) << (8 * (k >> 2));
             }
+#pragma unroll
+            for (int j = 0; j < 4; ++j) sum = __dp4a((int)wds[j], 0x01010101, sum);
             *chunk_ptr(ch) = make_uint4(wds[0], wds[1], wds[2], wds[3]);
         }
     }
@@ -964,6 +987,168 @@ __global__ void __launch_bounds__(256) lb_quantize_gemm_regs_kernel(const LbGemm
         amax_out[blockIdx.x] = m;
         xsum_out[blockIdx.x] = tot;
     }
+}
+
+// The same for blocks of many tokens: a CTA takes every gridDim.x-th token, a thread owns one 16-column chunk of all of them (the norm's
+// weights stay in its registers), and the rows of the next tokens travel into shared memory while it works on this one.  A CTA
+// per token keeps two of them an SM waiting for memory.  Bound now: issue (half of the slots) and two barriers a token; with a norm the
+// conversions, a quarter-rate instruction.  With the float quantizer and largest values and sums met by integer reductions instead of
+// loops over the warps: 2999 x 14336 float32 63 -> 47 us (4.5 TB/s), 2999 x 4096 21 -> 15, 1024 x 6912 with a norm 25 -> 19, 1024 x 2560 with
+// a norm 13 -> 8.5, float64 rows 13 -> 7.8.
+template <int PRO, int MAXT>
+__global__ void __launch_bounds__(MAXT, MAXT == 256 ? 3 : MAXT == 512 ? 2 : 1) lb_quantize_gemm_rows_kernel(const LbGemmQuant a, int Kp, int padded, int depth, int8_t* __restrict__ q,
+                                                                     float* __restrict__ amax_out, int* __restrict__ xsum_out) {
+    constexpr bool f64 = PRO == LB_PRO_INNERNORM64, kNorm = PRO >= LB_PRO_BLOCKNORM;
+    using VT = typename std::conditional<f64, double, float>::type;
+    using V16 = typename std::conditional<f64, double2, float4>::type;
+    constexpr int kPer = 16 / (int)sizeof(VT), kVecs = 16 / kPer;  // values of 16 bytes, such pieces of a chunk
+    constexpr int kMaxDepth = 4;
+    extern __shared__ __align__(128) uint8_t qsm[];
+    __shared__ __align__(8) uint64_t full[kMaxDepth];
+    __shared__ double s_ss[MAXT / 32];
+    __shared__ unsigned s_m[3];  // bits of the largest value of this token, the next and the one after
+    __shared__ int s_sum[2];
+    const int K = a.K, tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, nwarps = blockDim.x >> 5, G = gridDim.x;
+    const uint32_t row_bytes = (uint32_t)K * (uint32_t)sizeof(VT), slot_bytes = (uint32_t)Kp * (uint32_t)sizeof(VT);
+    const int nchunks = Kp >> 4, base = tid << 4, ncol = K - base < 0 ? 0 : K - base < 16 ? K - base : 16;  // columns of this thread's chunk
+    if (tid == 0) {
+        for (int i = 0; i < depth; ++i) lb_mbar_init(&full[i], 1);
+        lb_fence_mbar_init();
+        s_m[0] = s_m[1] = s_m[2] = 0u;
+        s_sum[0] = s_sum[1] = 0;
+    }
+    __syncthreads();
+    lb_pdl_launch_dependents();
+    lb_pdl_wait();
+    auto fetch = [&](int t, int slot) {
+        lb_mbar_expect_tx(&full[slot], row_bytes);
+        lb_bulk_g2s(qsm + (size_t)slot * slot_bytes, static_cast<const uint8_t*>(a.x) + (size_t)t * row_bytes, row_bytes, &full[slot]);
+    };
+    if (tid == 0)
+        for (int i = 0; i < depth && (int)blockIdx.x + i * G < a.tokens; ++i) fetch((int)blockIdx.x + i * G, i);
+    float w[kNorm ? 16 : 1];
+    if (kNorm)
+#pragma unroll
+        for (int k = 0; k < 16; ++k) w[kNorm ? k : 0] = 1.f;
+    // A lane starts its chunk at another 16-byte piece than its neighbours (bank conflicts): pieces, and with them the weights and the
+    // bytes of the result, are rotated by `rot` of the four columns groups.
+    const int rot = f64 ? lane & 3 : (lane >> 1) & 3;
+    if (kNorm && a.norm_w) {
+#pragma unroll
+        for (int k = 0; k < 16; ++k) {
+            const int col = base + ((k + 4 * rot) & 15);
+            if (col < a.norm_w_len && col < K) w[kNorm ? k : 0] = __ldg(a.norm_w + col);
+        }
+    }
+    int slot = 0, nth = 0, at = 0;
+    uint32_t parity = 0;
+    bool failed = false;
+    int prev = -1;
+    float prev_m = 0.f;
+    auto finish = [&]() {  // the previous token's sum, behind a barrier
+        if (tid == 0 && prev >= 0) {
+            amax_out[prev] = prev_m;
+            xsum_out[prev] = s_sum[(nth - 1) & 1];
+            s_sum[(nth - 1) & 1] = 0;
+        }
+    };
+    for (int t = blockIdx.x; t < padded; t += G) {
+        int8_t* qrow = q + (size_t)(t >> 8) * (Kp >> 7) * 32768 + (size_t)((t & 255) >> 3) * 1024 + (t & 7) * 16;
+        uint4* dst = reinterpret_cast<uint4*>(qrow + (size_t)(tid >> 3) * 32768 + (tid & 7) * 128);
+        if (t >= a.tokens) {  // padding token: zeros
+            if (tid < nchunks) *dst = make_uint4(0u, 0u, 0u, 0u);
+            continue;
+        }
+        if (!failed && !lb_mbar_wait_bounded(&full[slot], parity)) failed = true;
+        VT v[16];
+        {
+            const VT* row = reinterpret_cast<const VT*>(qsm + (size_t)slot * slot_bytes) + base;
+            if (ncol == 16) {
+#pragma unroll
+                for (int i = 0; i < kVecs; ++i) {
+                    const V16 d = *reinterpret_cast<const V16*>(row + ((i * kPer + 4 * rot) & 15));
+#pragma unroll
+                    for (int e = 0; e < kPer; ++e) v[i * kPer + e] = reinterpret_cast<const VT*>(&d)[e];
+                }
+            } else {
+#pragma unroll
+                for (int k = 0; k < 16; ++k) {
+                    const int c = (k + 4 * rot) & 15;
+                    v[k] = c < ncol ? row[c] : (VT)0;
+                }
+            }
+        }
+        float m = 0.f;
+        if (kNorm) {
+            double part[4] = {0.0, 0.0, 0.0, 0.0};
+#pragma unroll
+            for (int k = 0; k < 16; ++k) part[k & 3] = __dadd_rn(part[k & 3], __dmul_rn((double)v[k], (double)v[k]));  // columns past K hold zero
+            double ss = __dadd_rn(__dadd_rn(part[0], part[1]), __dadd_rn(part[2], part[3]));
+            ss = lb_warp_sum(ss);
+            if (lane == 0) s_ss[warp] = ss;
+            __syncthreads();
+            ss = 0.0;
+            for (int i = 0; i < nwarps; ++i) ss += s_ss[i];
+            const double root = sqrt(__dadd_rn(__ddiv_rn(ss, (double)K), a.eps));
+            const double rr = __ddiv_rn(1.0, root);
+#pragma unroll
+            for (int k = 0; k < 16; ++k) {
+                if (ncol == 16 || ((k + 4 * rot) & 15) < ncol) {
+                    const double wk = (double)w[kNorm ? k : 0];
+                    if (f64) {
+                        v[k] = (VT)lb_pro_value<PRO>((double)v[k], root, rr, wk);
+                    } else {  // (rounded to float once: every conversion is a quarter-rate instruction)
+                        v[k] = (VT)__dmul_rn(PRO == LB_PRO_BLOCKNORM ? lb_div_by((double)v[k], root, rr) : __dmul_rn((double)v[k], rr), wk);
+                    }
+                    m = fmaxf(m, fabsf((float)v[k]));
+                }
+            }
+        } else {
+#pragma unroll
+            for (int k = 0; k < 16; ++k) m = fmaxf(m, fabsf((float)v[k]));
+        }
+        // (not negative, so the order of the bits is the order of the numbers)
+        const unsigned wm = __reduce_max_sync(0xffffffffu, __float_as_uint(m));
+        if (lane == 0) atomicMax(&s_m[at], wm);
+        __syncthreads();  // every thread has its values of this row
+        finish();
+        if (tid == 0) {
+            s_m[at == 0 ? 2 : at - 1] = 0u;  // the token before last's, read by everyone before this barrier
+            if (t + depth * G < a.tokens && !failed) {
+                asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+                fetch(t + depth * G, slot);
+            }
+        }
+        m = __uint_as_float(s_m[at]);
+        at = at == 2 ? 0 : at + 1;
+        if (m < 1e-5f) m = 1e-5f;
+        uint32_t wds[4];
+        if (f64 || !gemm_quant16_f32(reinterpret_cast<const float*>(v), __fdiv_rn(127.f, m), wds)) {
+            const double s = __ddiv_rn(127.0, (double)m);
+            wds[0] = wds[1] = wds[2] = wds[3] = 0u;
+#pragma unroll
+            for (int k = 0; k < 16; ++k) wds[k & 3] |= (uint32_t)(lb_quant_i8((double)v[k], s) & 0xff) << (8 * (k >> 2));
+        }
+        int sum = 0;
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+            sum = __dp4a((int)wds[j], 0x01010101, sum);
+            wds[j] = __funnelshift_l(wds[j], wds[j], 8 * rot);
+        }
+        if (tid < nchunks) *dst = make_uint4(wds[0], wds[1], wds[2], wds[3]);
+        sum = __reduce_add_sync(0xffffffffu, sum);
+        if (lane == 0) atomicAdd(&s_sum[nth & 1], sum);
+        prev = t;
+        prev_m = m;
+        ++nth;
+        if (++slot == depth) {
+            slot = 0;
+            parity ^= 1;
+        }
+    }
+    __syncthreads();
+    finish();
+    if (failed) atomicExch(a.status, 1);
 }
 
 // gate product of a token block from the raw accumulators of the gate and up GEMMs (swigluGateProduct in float64,
@@ -1039,8 +1224,48 @@ int lb_gemm_quantize(loom_b200_ctx* ctx, const LbGemmQuant& a) {
         ctx->gemm_scratch_bytes = need + need / 4;
     }
     GemmScratch g = gemm_scratch_at(ctx->gemm_scratch, a.tokens, Kp);
-    // rows of up to 256 * CPT chunks of 16 columns stay in registers (float rows: CPT up to 8, float64 rows: up to 4)
     const int nchunks = Kp >> 4;
+    // Blocks of several tokens per SM whose rows bulk copies can fetch: rows behind one another in shared memory.  A slot is a row; as
+    // many CTAs per SM as registers and two slots each leave room for.
+    const bool f64 = a.pro == LB_PRO_INNERNORM64;
+    const size_t slot = (size_t)Kp * (f64 ? 8 : 4);
+    if (ctx->opt_quant_regs && !a.given_ss && !a.given_amax && !a.norm_out && !a.norm_count && a.tokens >= 2 * ctx->sm_count && nchunks <= (f64 ? 512 : 1024) &&
+        a.K % (f64 ? 2 : 4) == 0 && ((uintptr_t)a.x & 15) == 0 && 2 * slot <= 216 * 1024) {
+        const int T = (nchunks + 31) / 32 * 32;
+        int per = 65536 / (T * (T <= 256 ? 80 : 64));  // (registers of a thread)
+        if (per > 8) per = 8;
+        while (per > 1 && (size_t)per * (2 * slot + 2048) > 220 * 1024) --per;
+        if (per < 1) per = 1;
+        int depth = (int)((220 * 1024 / per - 2048) / slot);
+        if (depth > 4) depth = 4;
+        LbGemmQuant aq = a;
+        aq.status = ctx->status_dev;
+        const int grid = pt < per * ctx->sm_count ? pt : per * ctx->sm_count;
+#define LB_QROWS(PRO, MAXT)                                                                                                           \
+    do {                                                                                                                              \
+        LB_BIG_SMEM(ctx, (lb_quantize_gemm_rows_kernel<PRO, MAXT>), 220 * 1024);                                                      \
+        LB_LAUNCH(ctx, (lb_quantize_gemm_rows_kernel<PRO, MAXT>), dim3(grid), dim3(T), depth * slot, aq, Kp, pt, depth, g.q, g.amax, g.xsum); \
+        return 0;                                                                                                                     \
+    } while (0)
+#define LB_QROWS_T(PRO)                        \
+    do {                                       \
+        if (T > 512) LB_QROWS(PRO, 1024);      \
+        if (T > 256) LB_QROWS(PRO, 512);       \
+        LB_QROWS(PRO, 256);                    \
+    } while (0)
+        switch (a.pro) {
+            case LB_PRO_F32: LB_QROWS_T(LB_PRO_F32);
+            case LB_PRO_BLOCKNORM: LB_QROWS_T(LB_PRO_BLOCKNORM);
+            case LB_PRO_INNERNORM: LB_QROWS_T(LB_PRO_INNERNORM);
+            case LB_PRO_INNERNORM64:
+                if (T > 256) LB_QROWS(LB_PRO_INNERNORM64, 512);
+                LB_QROWS(LB_PRO_INNERNORM64, 256);
+            default: return lb_fail(ctx, LOOM_B200_ERR_INVALID, "gemm_quantize: prologue %d", a.pro);
+        }
+#undef LB_QROWS_T
+#undef LB_QROWS
+    }
+    // rows of up to 256 * CPT chunks of 16 columns stay in registers (float rows: CPT up to 8, float64 rows: up to 4)
     const int cpt_need = (nchunks + 255) / 256;
     const int cpt = cpt_need <= 1 ? 1 : cpt_need <= 2 ? 2 : cpt_need <= 4 ? 4 : 8;
     const bool regs_ok = cpt_need <= (a.pro == LB_PRO_INNERNORM64 ? 4 : 8);

@@ -125,6 +125,7 @@ struct LbGemmQuant {
     const double* given_ss;   // [tokens] sum of squares over the whole row, or null
     const float* given_amax;  // [tokens] absmax of the normalised whole row, or null
     int norm_count;           // elements the mean runs over (0 = K)
+    int* status;              // set by lb_gemm_quantize
 };
 struct LbGemmOut {
     const float* bias;      // [rows] or null

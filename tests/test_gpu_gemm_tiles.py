@@ -93,3 +93,42 @@ def test_widest_rows(ctx, cols):
     x[1::2] *= -1
     x[4:] = rng.standard_normal((tokens - 4, cols))
     check(ctx, words, 0.0123, x, rows, cols)
+
+
+# rows of blocks of many tokens are quantized behind bulk copies, a thread per sixteen columns: 256, 512 and 1024 threads, ragged last
+# chunks, rows that bulk copies cannot take (columns not a multiple of four) or that are too wide
+@pytest.mark.parametrize("cols,tokens", [(4, 296), (20, 297), (102, 300), (252, 513), (4096, 296), (4100, 300), (8192, 297), (8196, 301), (16384, 296), (16388, 299)])
+def test_quantized_rows_of_many_tokens(ctx, cols, tokens):
+    rng = np.random.default_rng(cols)
+    x = rng.standard_normal((tokens, cols)).astype(np.float32)
+    x[5] = 0
+    x[7, 0] = 1e30
+    # values whose codes lie half way between two integers, from either side
+    x[9:40] = ((rng.integers(-127, 127, (31, cols)) + 0.5) / 127).astype(np.float32)
+    x[9:40, 0] = 1
+    check(ctx, *matrix(rng, 64, cols), x, 64, cols)
+
+
+@pytest.mark.parametrize("heads,hd,inter", [(4, 16, 320), (3, 16, 4400), (2, 24, 8400), (20, 16, 17000)])
+def test_normed_rows_of_many_tokens(heads, hd, inter):
+    # prompts of more than two tokens an SM: block norm, inner norm of float64 and of float32 rows; logits as in test_gpu_attention_prompt.py
+    rng = np.random.default_rng(inter)
+    c = loom_b200.Context(0)
+    H, V, L, msl = heads * hd, 64, 2, 512
+    shapes = ((H, H), (hd, H), (hd, H), (H, H), (inter, H), (inter, H), (H, inter))
+    gdec = cabi.Decoder(c, L, H, heads, 1, hd, inter, V, 1e-5, 500000.0, cabi.ACT_SILU, msl)
+    odec = orc.Decoder(L, H, heads, 1, hd, inter, V, 1e-5, 500000.0, orc.ACT_SILU, msl)
+    try:
+        for b in range(L):
+            packed = [orc.pack_f32((rng.standard_normal(r * k) * 0.02).astype(np.float32), r, k) for r, k in shapes]
+            gdec.set_block(b, [c.upload_ternary(p[0], r, k, p[1]) for p, (r, k) in zip(packed, shapes)])
+            odec.set_block_packed(b, [p[0] for p in packed], [p[1] for p in packed])
+        emb = (rng.standard_normal((V, H)) * 0.02).astype(np.float32)
+        gdec.set_embeddings(c.to_device(emb))
+        odec.set_embeddings(emb)
+        tok = rng.integers(0, V, 301).astype(np.int32)
+        got, want = gdec.forward(tok), odec.forward(tok, threads=min(16, orc.host_threads()))
+        assert np.max(np.abs(got - want)) <= 1e-6 * max(1.0, float(np.max(np.abs(want))))
+    finally:
+        gdec.close()
+        c.close()
