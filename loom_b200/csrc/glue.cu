@@ -596,7 +596,7 @@ __global__ void lb_set_scalar_kernel(int* p, int value) {
     if (threadIdx.x == 0) *p = value;
 }
 
-// Causal attention of a block of prompt tokens.  One CTA per (KV head, tile of query tokens): the 64 query rows of
+// Causal attention of a block of prompt tokens, for head dimensions that attention_prompt.cu does not take.  One CTA per (KV head, tile of query tokens): the 64 query rows of
 // a CTA are the heads of one GQA group times 64/group consecutive tokens, so every K and V tile that is brought
 // into shared memory (64 positions, one 512-byte bulk copy per row) serves all of them.  Scores, the running
 // softmax (maximum, sum, rescaling of the partial output when the maximum moves) and the weighted V sum are float64
@@ -902,6 +902,7 @@ int lb_launch_attention_prefill(loom_b200_ctx* ctx, const LbAttnParams& pin) {
     p.status = ctx->status_dev;
     LB_REQUIRE(ctx, lb_attention_prefill_supported(p), "attention (prompt block): %d heads over %d kv heads of %d dimensions", p.heads,
                p.kv_heads, p.hd);
+    if (lb_attention_prompt_takes(p)) return lb_launch_attention_prompt(ctx, p);
     const int TQ = kPfRows / (p.heads / p.kv_heads);
     const size_t smem = (size_t)kPfRows * (p.hd + 4) * sizeof(double) + (size_t)kPfKeys * (p.hd + 8) * sizeof(double) +
                         (size_t)kPfRows * (kPfKeys + 4) * sizeof(double) + (size_t)kPfKeys * p.hd * sizeof(float);
