@@ -15,6 +15,7 @@
 #include <algorithm>
 #include <chrono>
 #include <cmath>
+#include <functional>
 #include <vector>
 
 struct loom_b200_graph;  // defined in abi.cu
@@ -28,7 +29,7 @@ struct LbDecBlock {
     bool ready = false;
 };
 
-constexpr int kReadEvents = 32;  // passes of eight sequences: 256 sequences
+constexpr int kReadEvents = 32;  // parts of the logits on their way to the host
 
 struct loom_b200_decoder {
     loom_b200_ctx* ctx = nullptr;
@@ -586,15 +587,18 @@ int dec_forward_chunk(loom_b200_decoder* dec, int M, int splits, bool head, int 
     return lb_launch_add_scalar(ctx, dec->pos, M);
 }
 
-// One token for each of the sequences lane0 .. lane0+M-1 (M <= 8), every sequence at its own position of its own KV
+// One token for each of the sequences lane0 .. lane0+M-1 (M <= lb_pass_tokens), every sequence at its own position of its own KV
 // rings: the projections carry the M tokens in one pass over the weights (the same GEMV launches as an M-token chunk of
 // one sequence), RoPE and attention run per (sequence, head), and the head serves several hidden rows per pass over the
-// table.  Its tail publishes every sequence's next token and advances its position.
-int dec_forward_lanes(loom_b200_decoder* dec, int lane0, int M) {
+// table.  Its tail publishes every sequence's next token and advances its position.  rows_done: called when the logits of some more
+// sequences have been queued.
+int dec_forward_lanes(loom_b200_decoder* dec, int lane0, int M, const std::function<int(int)>& rows_done = nullptr) {
     loom_b200_ctx* ctx = dec->ctx;
     if (dec->stack) {
         for (int m0 = 0, per = lb_stack_max_lanes(dec->stack); m0 < M; m0 += per)
             if (int rc = dec_stack_step(dec, lane0 + m0, std::min(per, M - m0))) return rc;
+            else if (rows_done)
+                if (int rc2 = rows_done(std::min(per, M - m0))) return rc2;
         return 0;
     }
     const loom_b200_decoder_dims& d = dec->d;
@@ -660,8 +664,16 @@ int dec_forward_lanes(loom_b200_decoder* dec, int lane0, int M) {
         h.pos = dec->pos_all + lane0 + r0;
         h.pos_delta = 1;
         if (int rc = lb_launch_lm_head(ctx, h)) return rc;
+        if (rows_done)
+            if (int rc = rows_done(h.nb)) return rc;
     }
     return 0;
+}
+
+// sequences of one dec_forward_lanes: what the widest input row of the projections allows
+int dec_pass_lanes(const loom_b200_decoder* dec) {
+    if (dec->stack) return kChunkTokens;
+    return lb_pass_tokens(dec->ctx, dec->inter_l > dec->d.hidden ? dec->inter_l : dec->d.hidden);
 }
 
 int dec_check_ready(loom_b200_decoder* dec) {
@@ -748,7 +760,7 @@ int dec_extend(loom_b200_decoder* dec, const int32_t* tokens, int n, const int32
     } else {
         // tokens per pass: what the widest input row (hidden, or this rank's slice of the intermediate) leaves room for
         const int widest = dec->inter_l > dec->d.hidden ? dec->inter_l : dec->d.hidden;
-        const int chunk = lb_gemv_max_tokens(widest) < kChunkTokens ? lb_gemv_max_tokens(widest) : kChunkTokens;
+        const int chunk = lb_pass_tokens(ctx, widest);
         for (int s0 = 0; s0 < n; s0 += chunk) {
             const int M = n - s0 < chunk ? n - s0 : chunk;
             LB_CUDA(ctx, cudaStreamSynchronize(ctx->stream));  // h_tok is reused
@@ -780,11 +792,11 @@ static int dec_finish_create(loom_b200_decoder* dec, loom_b200_decoder** out) {
         if (e == cudaSuccess) e = cudaMalloc(p, bytes);
         if (e == cudaSuccess) e = cudaMemsetAsync(*p, 0, bytes, ctx->stream);
     };
-    A((void**)&dec->x, (size_t)kChunkTokens * d.hidden * 4);
-    if (!dec->stack) A((void**)&dec->prod, (size_t)kChunkTokens * dec->inter_l * 4);
+    A((void**)&dec->x, (size_t)kPassTokens * d.hidden * 4);
+    if (!dec->stack) A((void**)&dec->prod, (size_t)kPassTokens * dec->inter_l * 4);
     A((void**)&dec->logits_all, (size_t)d.vocab * 4);
     A((void**)&dec->hidden, (size_t)d.hidden * 4);
-    A((void**)&dec->tok, kChunkTokens * sizeof(int));
+    A((void**)&dec->tok, kPassTokens * sizeof(int));
     A((void**)&dec->pos_all, sizeof(int));
     A((void**)&dec->step_all, sizeof(int));
     A((void**)&dec->tok_all, sizeof(int));
@@ -795,7 +807,7 @@ static int dec_finish_create(loom_b200_decoder* dec, loom_b200_decoder** out) {
         A((void**)&dec->tp_stats, 2 * kChunkTokens * sizeof(double));
         A((void**)&dec->tp_acc, (size_t)kChunkTokens * d.hidden * sizeof(int32_t));
     }
-    if (e == cudaSuccess) e = cudaMallocHost((void**)&dec->h_tok, kChunkTokens * sizeof(int));
+    if (e == cudaSuccess) e = cudaMallocHost((void**)&dec->h_tok, kPassTokens * sizeof(int));
     if (e == cudaSuccess) e = cudaMallocHost((void**)&dec->h_logits, (size_t)d.vocab * 4);
     for (int i = 0; i < kReadEvents && e == cudaSuccess; ++i) e = cudaEventCreateWithFlags(&dec->read_done[i], cudaEventDisableTiming);
     if (e == cudaSuccess) e = cudaStreamSynchronize(ctx->stream);
@@ -1202,26 +1214,31 @@ int loom_b200_decoder_step_batch(loom_b200_decoder* dec, const int32_t* tokens, 
         for (int i = 0; i < B; ++i) dec->h_tok_all[i] = tokens[i];
         LB_CUDA(ctx, cudaMemcpyAsync(dec->tok_all, dec->h_tok_all, (size_t)B * sizeof(int), cudaMemcpyHostToDevice, ctx->stream));
     }
-    // with the whole vocabulary on this GPU a pass's rows cross to the host beside the passes after it (16 sequences: 34.9 ms for eight
-    // steps with one copy at the end, 28.4 so); one pass has nothing to cross beside (eight rows of 16 KB: 71 us a step with a copy
-    // in the step's own stream, 81 so)
+    // with the whole vocabulary on this GPU the rows that a pass over the head has made cross to the host beside the passes after it (16
+    // sequences: 34.9 ms for eight steps with one copy at the end, 28.4 so); one pass has nothing to cross beside (eight rows of 16 KB:
+    // 71 us a step with a copy in the step's own stream, 81 so)
     const bool beside = logits_host && B > kChunkTokens && !dec->head_sharded;
-    int passes = 0;
-    for (int l0 = 0; l0 < B; l0 += kChunkTokens) {
-        const int M = B - l0 < kChunkTokens ? B - l0 : kChunkTokens;
-        if (int rc = dec_forward_lanes(dec, l0, M)) return rc;
-        if (beside && l0 + M == B)
-            if (int rc = lb_status_queue(ctx)) return rc;  // (before the last pass's event: the rows' stream waits for both)
-        if (beside) LB_CUDA(ctx, cudaEventRecord(dec->read_done[passes++], ctx->stream));
-    }
+    int parts = 0, done = 0, ends[kReadEvents];
+    const auto rows_done = [&](int rows) -> int {
+        done += rows;
+        if (done == B)
+            if (int rc = lb_status_queue(ctx)) return rc;  // (before the last event: the rows' stream waits for both)
+        if (parts == kReadEvents) --parts;  // (out of events: the last one takes the rest)
+        LB_CUDA(ctx, cudaEventRecord(dec->read_done[parts], ctx->stream));
+        ends[parts++] = done;
+        return 0;
+    };
+    const int per = dec_pass_lanes(dec);
+    for (int l0 = 0; l0 < B; l0 += per)
+        if (int rc = beside ? dec_forward_lanes(dec, l0, std::min(per, B - l0), rows_done) : dec_forward_lanes(dec, l0, std::min(per, B - l0))) return rc;
     for (int i = 0; i < B; ++i) dec->kv_offsets[i] += 1;
     dec->kv_offset = dec->kv_offsets[dec->lane];
     if (beside) {
         const size_t row = (size_t)dec->d.vocab * 4;
         touch_pages(logits_host, (size_t)B * row);
         cudaError_t e = cudaSuccess;
-        for (int i = 0; i < passes && e == cudaSuccess; ++i) {
-            const size_t at = (size_t)i * kChunkTokens * row, len = std::min((size_t)kChunkTokens, (size_t)B - (size_t)i * kChunkTokens) * row;
+        for (int i = 0; i < parts && e == cudaSuccess; ++i) {
+            const size_t at = i ? (size_t)ends[i - 1] * row : 0, len = (size_t)ends[i] * row - at;
             e = cudaStreamWaitEvent(dec->read_stream, dec->read_done[i], 0);
             if (e == cudaSuccess) e = cudaMemcpyAsync((char*)logits_host + at, (const char*)dec->logits_all + at, len, cudaMemcpyDeviceToHost, dec->read_stream);
         }
@@ -1250,11 +1267,10 @@ int loom_b200_decoder_continue_batch(loom_b200_decoder* dec, int steps) {
     if (int rc = lb_set_device(ctx)) return rc;
     if (int rc = dec_batch_ready(dec, steps, "decoder_continue_batch")) return rc;
     const int B = dec->batch;
+    const int per = dec_pass_lanes(dec);
     for (int s = 0; s < steps; ++s)
-        for (int l0 = 0; l0 < B; l0 += kChunkTokens) {
-            const int M = B - l0 < kChunkTokens ? B - l0 : kChunkTokens;
-            if (int rc = dec_forward_lanes(dec, l0, M)) return rc;
-        }
+        for (int l0 = 0; l0 < B; l0 += per)
+            if (int rc = dec_forward_lanes(dec, l0, std::min(per, B - l0))) return rc;
     for (int i = 0; i < B; ++i) dec->kv_offsets[i] += steps;
     dec->kv_offset = dec->kv_offsets[dec->lane];
     return 0;

@@ -366,7 +366,7 @@ __device__ __forceinline__ void stage_activations(const LbGemvParams& p, const S
 // Activations other than linear/ReLU/ReLU2 pull in transcendental code: keep it out of the straight-line path.
 __device__ __noinline__ float activate_slow(float v, int act) { return lb_activate(v, act); }
 
-__device__ __forceinline__ size_t out_index(const LbGemvParams& p, const Smem& sm, const LbGemvSeg& sg, int n, int r) {
+__device__ __forceinline__ size_t out_index(const LbGemvParams& p, int pos0, const LbGemvSeg& sg, int n, int r) {
     if (sg.out_ring > 0) {
         size_t base = 0;
         int pos;
@@ -374,7 +374,7 @@ __device__ __forceinline__ size_t out_index(const LbGemvParams& p, const Smem& s
             pos = p.pos_ptr[n] % sg.out_ring;
             base = (size_t)n * (size_t)sg.seq_stride;
         } else {
-            pos = (sm.pos0 + n) % sg.out_ring;
+            pos = (pos0 + n) % sg.out_ring;
         }
         if (sg.ring_hd > 0) return base + ((size_t)(r / sg.ring_hd) * sg.out_ring + pos) * sg.ring_hd + r % sg.ring_hd;  // head-major KV ring
         return base + (size_t)pos * sg.rows + r;
@@ -382,21 +382,20 @@ __device__ __forceinline__ size_t out_index(const LbGemvParams& p, const Smem& s
     return (size_t)n * sg.rows + r;
 }
 
-// Epilogue of one finished row (or gate/up row pair).  vals = [group][M][16] complete sums of sum(code*x).
-template <int EPI, bool LEAN = false>
-__device__ __forceinline__ void finish_row(const LbGemvParams& p, const Smem& sm, int group_first_vstrip, int e, int n,
-                                           int i, const int* vals) {
-    const int M = p.M;
+// Epilogue of one finished row (or gate/up row pair): a0 (and a1, the up row's) = sum(code*x) of token n.  os: [segment][os_ld] output
+// scales, xsum: sum(x) of the token.
+template <int EPI>
+__device__ __forceinline__ void finish_value(const LbGemvParams& p, const double* os, int os_ld, int xsum, int pos0, int group_first_vstrip, int e, int n, int i, int a0, int a1) {
     if (EPI == LB_EPI_SWIGLU) {
         if (e != 0) return;  // pairs are finished from the gate side
         const int r = (group_first_vstrip >> 1) * kTileRows + i;
         const LbGemvSeg& sg = p.seg[0];
         const LbGemvSeg& su = p.seg[1];
         if (r >= sg.rows) return;
-        const int ag = vals[(0 * M + n) * 16 + i] - sm.xsum[n];
-        const int au = vals[(1 * M + n) * 16 + i] - sm.xsum[n];
-        double yg = __dmul_rn((double)ag, sm.os[0 * kMaxM + n]);
-        double yu = __dmul_rn((double)au, sm.os[1 * kMaxM + n]);
+        const int ag = a0 - xsum;
+        const int au = a1 - xsum;
+        double yg = __dmul_rn((double)ag, os[n]);
+        double yu = __dmul_rn((double)au, os[os_ld + n]);
         if (sg.bias) yg = __dadd_rn(yg, (double)sg.bias[r]);
         if (su.bias) yu = __dadd_rn(yu, (double)su.bias[r]);
         ((float*)sg.out)[(size_t)n * sg.rows + r] = (float)lb_gate_product(yg, yu, p.act);
@@ -411,16 +410,16 @@ __device__ __forceinline__ void finish_row(const LbGemvParams& p, const Smem& sm
     const LbGemvSeg& sg = p.seg[s];
     const int r = (v - sg.vstrip0) * kTileRows + i;
     if (r >= sg.rows) return;
-    const int acc = vals[(e * M + n) * 16 + i] - sm.xsum[n];
+    const int acc = a0 - xsum;
     if (EPI == LB_EPI_GENERIC) {
         const size_t o = (size_t)n * sg.rows + r;
         if (sg.acc_out) sg.acc_out[o] = acc;
         if (sg.kind == LB_OUT_ACC || !sg.out) return;
     }
-    double y = __dmul_rn((double)acc, sm.os[s * kMaxM + n]);
+    double y = __dmul_rn((double)acc, os[s * os_ld + n]);
     if (sg.bias) y = __dadd_rn(y, (double)sg.bias[r]);
     if (EPI == LB_EPI_QKV) {
-        const size_t o = out_index(p, sm, sg, n, r);
+        const size_t o = out_index(p, pos0, sg, n, r);
         if (s == 0) ((double*)sg.out)[o] = y;
         else ((float*)sg.out)[o] = (float)y;
         return;
@@ -445,6 +444,13 @@ __device__ __forceinline__ void finish_row(const LbGemvParams& p, const Smem& sm
     else if (p.act != LOOM_B200_ACT_LINEAR) f = activate_slow(f, p.act);
     if (p.residual && s == 0) f = __fadd_rn(f, p.residual[o]);
     ((float*)sg.out)[o] = f;
+}
+
+// the same on complete sums vals = [group][M][16] in shared memory
+template <int EPI, bool LEAN = false>
+__device__ __forceinline__ void finish_row(const LbGemvParams& p, const Smem& sm, int group_first_vstrip, int e, int n, int i, const int* vals) {
+    if (EPI == LB_EPI_SWIGLU && e != 0) return;
+    finish_value<EPI>(p, sm.os, kMaxM, sm.xsum[n], sm.pos0, group_first_vstrip, e, n, i, vals[(e * p.M + n) * 16 + i], EPI == LB_EPI_SWIGLU ? vals[(p.M + n) * 16 + i] : 0);
 }
 
 }  // namespace

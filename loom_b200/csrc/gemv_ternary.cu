@@ -465,7 +465,7 @@ int lb_gemv_max_tokens(int K) {
 
 int lb_gemv_finalize_params(loom_b200_ctx* ctx, LbGemvParams& p) {
     LB_REQUIRE(ctx, p.nseg >= 1 && p.nseg <= 3, "gemv: %d segments", p.nseg);
-    LB_REQUIRE(ctx, p.M >= 1 && p.M <= kMaxM, "gemv: %d tokens per pass (max %d)", p.M, kMaxM);
+    LB_REQUIRE(ctx, p.M >= 1 && p.M <= kPassTokens, "gemv: %d tokens per pass (max %d)", p.M, kPassTokens);
     LB_REQUIRE(ctx, p.K > 0, "gemv: K=%d", p.K);
     p.kblocks = (p.K + kTileCols - 1) / kTileCols;
     int v = 0;
@@ -563,6 +563,8 @@ static void gemv_plan(const loom_b200_ctx* ctx, LbGemvParams& p, int cps, int* g
 }
 
 int lb_launch_gemv(loom_b200_ctx* ctx, const LbGemvParams& pin) {
+    if (lb_gemv_tokens_takes(ctx, pin)) return lb_launch_gemv_tokens(ctx, pin);
+    LB_REQUIRE(ctx, pin.M <= kMaxM, "gemv: %d tokens per pass (max %d)", pin.M, kMaxM);
     LbGemvParams p = pin;
     // Wide inputs, or three and more tokens: normalise and quantize once in a launch of its own (one CTA per token), then
     // stream the weights against the int8 rows.  The fused prologue is repeated by every CTA and costs it 4-6 us per token:
@@ -690,7 +692,7 @@ extern "C" int loom_b200_ternary_linear(loom_b200_ctx* ctx, const loom_b200_weig
     LB_REQUIRE(ctx, out || acc_out, "ternary_linear: no output buffer");
     LB_REQUIRE(ctx, w->device == ctx->device, "ternary_linear: weight lives on device %d, context on %d", w->device, ctx->device);
     if (int rc = lb_set_device(ctx)) return rc;
-    const int pass = lb_gemv_max_tokens(w->cols);  // tokens one pass carries: 8, fewer for very wide inputs
+    const int pass = lb_pass_tokens(ctx, w->cols);
     for (int b0 = 0; b0 < batch; b0 += pass) {
         LbGemvParams p = {};
         p.nseg = 1;

@@ -49,6 +49,8 @@ struct LbGemvSeg {
 // Tokens one pass can carry for K input columns: the int8 activations of all tokens sit in shared memory beside a
 // weight ring of at least two stages.  8 for every K up to ~19,000; 5 for K = 28,672.
 int lb_gemv_max_tokens(int K);
+// Passes of 3 to kPassTokens tokens over inputs of at most kGtMaxColumns columns have a kernel of their own (gemv_tokens.cu).
+constexpr int kPassTokens = 24, kGtMaxColumns = 32768;
 
 struct LbGemvParams {
     LbGemvSeg seg[3];
@@ -117,4 +119,8 @@ __device__ __forceinline__ double lb_pro_value(double x, double root, double rr,
 // instead of inside every CTA of the GEMV.
 constexpr int kSplitQuantK = 8192;
 constexpr int kSplitQuantTokens = 3;  // ... and so are passes of at least this many tokens
+bool lb_gemv_tokens_takes(const loom_b200_ctx* ctx, const LbGemvParams& p);
+int lb_launch_gemv_tokens(loom_b200_ctx* ctx, const LbGemvParams& p);
+// tokens a caller should put into one pass over inputs of K columns
+int lb_pass_tokens(const loom_b200_ctx* ctx, int K);
 int lb_launch_norm_quantize(loom_b200_ctx* ctx, const LbGemvParams& p, int8_t* q, float* amax);

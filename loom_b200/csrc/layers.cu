@@ -78,12 +78,12 @@ int lb_mha_alloc(loom_b200_ctx* ctx, loom_b200_mha* m, int max_splits, int lanes
     LB_CUDA(ctx, cudaMemsetAsync(m->cache_v_base, 0, cache, ctx->stream));
     m->cache_k = m->cache_k_base;
     m->cache_v = m->cache_v_base;
-    LB_CUDA(ctx, cudaMalloc(&m->q, (size_t)kChunkTokens * m->q_dim * sizeof(double)));
-    LB_CUDA(ctx, cudaMalloc(&m->attn, (size_t)kChunkTokens * m->q_dim * sizeof(double)));
+    LB_CUDA(ctx, cudaMalloc(&m->q, (size_t)kPassTokens * m->q_dim * sizeof(double)));
+    LB_CUDA(ctx, cudaMalloc(&m->attn, (size_t)kPassTokens * m->q_dim * sizeof(double)));
     LB_CUDA(ctx, cudaMalloc(&m->part, lb_attn_part_elems(kChunkTokens, m->heads, m->head_dim, max_splits) * sizeof(double)));
-    LB_CUDA(ctx, cudaMalloc(&m->cnt, (size_t)kChunkTokens * m->heads * sizeof(unsigned int)));
-    LB_CUDA(ctx, cudaMemsetAsync(m->cnt, 0, (size_t)kChunkTokens * m->heads * sizeof(unsigned int), ctx->stream));
-    LB_CUDA(ctx, cudaMalloc(&m->k_new, (size_t)kChunkTokens * m->kv_dim * sizeof(float)));
+    LB_CUDA(ctx, cudaMalloc(&m->cnt, (size_t)kPassTokens * m->heads * sizeof(unsigned int)));
+    LB_CUDA(ctx, cudaMemsetAsync(m->cnt, 0, (size_t)kPassTokens * m->heads * sizeof(unsigned int), ctx->stream));
+    LB_CUDA(ctx, cudaMalloc(&m->k_new, (size_t)kPassTokens * m->kv_dim * sizeof(float)));
     LB_CUDA(ctx, cudaMalloc(&m->pos_dev, sizeof(int)));
     LB_CUDA(ctx, cudaMemsetAsync(m->pos_dev, 0, sizeof(int), ctx->stream));
     // pow(theta, 2d/hd) in double on the host: the same libm call the CPU path makes once per use
@@ -127,7 +127,7 @@ static bool mha_folds_rope(loom_b200_mha* m, const LbMhaStepArgs& a) {
     // one token of one sequence: RoPE goes into the attention kernel; one token of each of several sequences: only the
     // cluster kernel knows that layout, otherwise RoPE runs as a launch of its own
     if (!a.fold_rope || m->q_norm || m->k_norm || !m->ctx->opt_fold_rope || m->head_dim % 8 != 0) return false;
-    return a.lanes_pos ? mha_cluster_size(m, a.M) > 0 : a.M == 1;
+    return a.lanes_pos ? mha_cluster_size(m, a.M < kChunkTokens ? a.M : kChunkTokens) > 0 : a.M == 1;
 }
 
 int lb_mha_qkv_dev(loom_b200_mha* m, const LbMhaStepArgs& a) {
@@ -167,11 +167,11 @@ int lb_mha_qkv_dev(loom_b200_mha* m, const LbMhaStepArgs& a) {
     return lb_launch_gemv(ctx, p);
 }
 
-int lb_mha_attn_dev(loom_b200_mha* m, const LbMhaStepArgs& a) {
+// tokens n0 .. n0 + a.M - 1 of the pass (a: theirs)
+static int mha_attn_part(loom_b200_mha* m, const LbMhaStepArgs& a, int n0, bool fold_rope) {
     loom_b200_ctx* ctx = m->ctx;
-    const bool fold_rope = mha_folds_rope(m, a);
     LbRopeParams r = {};
-    r.q = m->q;
+    r.q = m->q + (size_t)n0 * m->q_dim;
     r.cache_k = m->cache_k;
     r.pos_ptr = m->pos_dev;
     r.rope_div = m->rope_div;
@@ -194,11 +194,11 @@ int lb_mha_attn_dev(loom_b200_mha* m, const LbMhaStepArgs& a) {
         if (int rc = lb_launch_rope(ctx, r)) return rc;
 
     LbAttnParams t = {};
-    t.q = m->q;
+    t.q = m->q + (size_t)n0 * m->q_dim;
     t.cache_k = m->cache_k;
     t.cache_v = m->cache_v;
     t.pos_ptr = m->pos_dev;
-    t.out = m->attn;
+    t.out = m->attn + (size_t)n0 * m->q_dim;
     t.part = m->part;
     t.cnt = m->cnt;
     t.M = a.M;
@@ -216,7 +216,7 @@ int lb_mha_attn_dev(loom_b200_mha* m, const LbMhaStepArgs& a) {
     }
     if (fold_rope) {
         t.rope_div = m->rope_div;
-        t.k_new = m->k_new;
+        t.k_new = m->k_new + (size_t)n0 * m->kv_dim;
         t.cache_k_w = a.lanes_pos ? m->cache_k_base + (size_t)a.lane0 * m->ring_elems : m->cache_k;
         if (const int cluster = mha_cluster_size(m, a.lanes_pos ? a.M : 0)) {
             t.next_k = a.lanes_pos ? nullptr : m->next_k;  // (the prefetch follows one sequence's rings)
@@ -230,6 +230,19 @@ int lb_mha_attn_dev(loom_b200_mha* m, const LbMhaStepArgs& a) {
         t.max_chunk = (m->msl + t.splits - 1) / t.splits;
     }
     return lb_launch_attention(ctx, t);
+}
+
+int lb_mha_attn_dev(loom_b200_mha* m, const LbMhaStepArgs& a) {
+    const bool fold_rope = mha_folds_rope(m, a);
+    if (!a.lanes_pos) return mha_attn_part(m, a, 0, fold_rope);
+    for (int n0 = 0; n0 < a.M; n0 += kChunkTokens) {  // (the scratch of split positions holds so many sequences)
+        LbMhaStepArgs s = a;
+        s.M = a.M - n0 < kChunkTokens ? a.M - n0 : kChunkTokens;
+        s.lanes_pos += n0;
+        s.lane0 += n0;
+        if (int rc = mha_attn_part(m, s, n0, fold_rope)) return rc;
+    }
+    return 0;
 }
 
 int lb_mha_o_dev(loom_b200_mha* m, const LbMhaStepArgs& a) {
@@ -313,7 +326,7 @@ int loom_b200_dense_forward(loom_b200_ctx* ctx, const loom_b200_weight* w, int a
     float* pre = ar.take<float>((size_t)batch * N);
     float* post = ar.take<float>((size_t)batch * N);
     LB_CUDA(ctx, cudaMemcpyAsync(x, in_host, (size_t)batch * K * 4, cudaMemcpyHostToDevice, ctx->stream));
-    const int chunk = lb_gemv_max_tokens(K) < kChunkTokens ? lb_gemv_max_tokens(K) : kChunkTokens;
+    const int chunk = lb_pass_tokens(ctx, K);
     // a block of tokens is a dense contraction: tensor cores (tcgen05) from kGemmMinTokens on, the GEMV below it
     if (batch >= kGemmMinTokens) {
         if (int rc = lb_ternary_gemm(ctx, w, batch, x, nullptr, nullptr, activation, post, pre, nullptr, nullptr)) return rc;
@@ -372,7 +385,7 @@ int loom_b200_swiglu_forward(loom_b200_ctx* ctx, const loom_b200_weight* gate, c
     LB_CUDA(ctx, h2d(bu, bias_up, I));
     LB_CUDA(ctx, h2d(bd, bias_down, H));
     LB_CUDA(ctx, h2d(iw, inner_norm_w, inner_norm_len));
-    const int sw_chunk = lb_gemv_max_tokens(I > H ? I : H) < kChunkTokens ? lb_gemv_max_tokens(I > H ? I : H) : kChunkTokens;
+    const int sw_chunk = lb_pass_tokens(ctx, I > H ? I : H);
     for (int s0 = 0; s0 < seq; s0 += sw_chunk) {
         LbSwigluArgs a = {};
         a.gate = gate;
@@ -499,7 +512,7 @@ int loom_b200_mha_forward(loom_b200_mha* m, const float* in_host, int batch, int
     LB_CUDA(ctx, cudaMemcpyAsync(m->pos_dev, &m->kv_offset, sizeof(int), cudaMemcpyHostToDevice, ctx->stream));
     LB_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
     const int widest = m->q_dim > D ? m->q_dim : D;
-    const int mh_chunk = lb_gemv_max_tokens(widest) < kChunkTokens ? lb_gemv_max_tokens(widest) : kChunkTokens;
+    const int mh_chunk = lb_pass_tokens(ctx, widest);
     for (int s0 = 0; s0 < total; s0 += mh_chunk) {
         LbMhaStepArgs a = {};
         a.pro_mode = LB_PRO_F32;

@@ -4,9 +4,9 @@
 #include "gemv_ternary.cuh"
 #include "glue.cuh"
 
-constexpr int kChunkTokens = 8;  // tokens one GEMV pass carries in its N dimension
+constexpr int kChunkTokens = 8;  // sequences whose attention is one launch; tokens of a pass under a tensor-parallel group
 
-// SwiGLUForwardPackedTernaryCPU on device buffers for M <= 8 tokens.
+// SwiGLUForwardPackedTernaryCPU on device buffers for M <= lb_pass_tokens tokens.
 struct LbSwigluArgs {
     const loom_b200_weight *gate, *up, *down;
     const float *bias_gate, *bias_up, *bias_down;  // device or null
@@ -55,7 +55,7 @@ struct loom_b200_mha {
     int splits = 1, max_total = 0;
     float* k_new = nullptr;                        // [kv_dim] the newest K row before RoPE (one-token steps with RoPE folded into attention)
     // CTAs per (sequence, KV head) of the cluster attention (0 = not usable, -1 = not decided yet): [0] a step of one sequence,
-    // [M] a pass of M sequences
+    // [M] a launch for M sequences
     int attn_cluster[kChunkTokens + 1] = {-1, -1, -1, -1, -1, -1, -1, -1, -1};
     const float *next_k = nullptr, *next_v = nullptr;  // KV rings of the decoder block that follows (L2 prefetch), or null
     // tensor parallelism: > 0 when this object holds heads/world heads (wq/wk/wv row slices, wo a column slice);
@@ -81,7 +81,7 @@ struct LbMhaStepArgs {
     const int* lanes_pos = nullptr;
     int lane0 = 0;
 };
-// One chunk (M <= 8 tokens at positions *pos_dev ...): QKV -> q/k norm + RoPE -> attention -> inner norm -> O.
+// One chunk (M <= lb_pass_tokens tokens at positions *pos_dev ...): QKV -> q/k norm + RoPE -> attention -> inner norm -> O.
 // Does not advance pos_dev.
 int lb_mha_step_dev(loom_b200_mha* m, const LbMhaStepArgs& a);
 // its three parts: the QKV projection, q/k norm + RoPE + attention, inner norm + output projection
