@@ -47,24 +47,31 @@ __global__ void __launch_bounds__(256) lb_embed_image_kernel(const uint8_t* __re
     }
 }
 
-constexpr int kNormTokens = 8;  // tokens of a CTA
 constexpr int kMaxTaps = 16;
 
 __device__ __forceinline__ float row_rstd(const float* row, int width, float eps, int lane) {  // a warp per row
     float ss = 0.f;
-    for (int k = lane; k < width; k += 32) ss = fmaf(row[k], row[k], ss);
+    constexpr int U = 16;  // asked for at once: the row is a chain of memory latencies otherwise
+    for (int k0 = lane; k0 < width; k0 += 32 * U) {
+        float v[U];
+#pragma unroll
+        for (int i = 0; i < U; ++i) v[i] = k0 + 32 * i < width ? row[k0 + 32 * i] : 0.f;
+#pragma unroll
+        for (int i = 0; i < U; ++i) ss = fmaf(v[i], v[i], ss);
+    }
     ss = lb_warp_sumf(ss);
     return __fdiv_rn(1.f, sqrtf(__fadd_rn(__fdiv_rn(ss, (float)width), eps)));
 }
 
-template <typename WT>
+// PER: tokens of a CTA
+template <typename WT, int PER>
 __global__ void __launch_bounds__(256) lb_norm_conv_kernel(const LbNormBlock p, bool vec) {
     constexpr int C = LbElem<WT>::kChunk;
-    __shared__ float s_r[kNormTokens + kMaxTaps];
+    __shared__ float s_r[PER + kMaxTaps];
     lb_pdl_launch_dependents();
     lb_pdl_wait();
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int t0 = blockIdx.x * kNormTokens, t1 = min(p.T, t0 + kNormTokens);
+    const int t0 = blockIdx.x * PER, t1 = min(p.T, t0 + PER);
     const int back = p.taps - 1;
     const float gain = *p.gain;
     for (int i = warp; i < t1 - t0 + back; i += 8) {
@@ -171,7 +178,14 @@ __global__ void __launch_bounds__(256) lb_conv_commit_kernel(const LbNormBlock p
     if (t < 0) return;
     const float* row = p.x + (size_t)t * p.ldx;
     float ss = 0.f;
-    for (int k = threadIdx.x; k < p.width; k += blockDim.x) ss = fmaf(row[k], row[k], ss);
+    constexpr int U = 8;
+    for (int k0 = threadIdx.x; k0 < p.width; k0 += 256 * U) {
+        float v[U];
+#pragma unroll
+        for (int i = 0; i < U; ++i) v[i] = k0 + 256 * i < p.width ? row[k0 + 256 * i] : 0.f;
+#pragma unroll
+        for (int i = 0; i < U; ++i) ss = fmaf(v[i], v[i], ss);
+    }
     ss = lb_block_sumf(ss, red);
     const float r = __fdiv_rn(1.f, sqrtf(__fadd_rn(__fdiv_rn(ss, (float)p.width), p.eps))) * *p.gain;
     float* out = p.ring + (size_t)((p.pos0 + t) % p.taps) * p.ring_ld;
@@ -533,8 +547,15 @@ int lb_norm_block(loom_b200_ctx* ctx, int dtype, const LbNormBlock& p) {
                  lb_vec_rows(p.x, p.ldx) && (!p.gain_w || lb_vec_rows(p.gain_w, 4)) && (!p.rows || lb_vec_rows(p.rows, p.ldx)));
         return 0;
     }
-    LB_TYPED(dtype, lb_norm_conv_kernel<float>, lb_norm_conv_kernel<__nv_bfloat16>, dim3(lb_ceil_div(p.T, kNormTokens)), dim3(256), 0, p,
-             lb_vec_rows(p.x, p.ldx) && lb_vec_rows(p.conv_w, p.ring_ld) && lb_vec_rows(p.ring, p.ring_ld));
+    // a CTA also norms the rows in front of its own, so fewer tokens to one only where SMs would be idle: 61 tokens of 4096 columns 63 us
+    // in eight CTAs with a row's loads one after the other, 12 so; 2048 tokens of 2560 28 us with eight a CTA, 24 with four, 26 with two
+    const bool vec = lb_vec_rows(p.x, p.ldx) && lb_vec_rows(p.conv_w, p.ring_ld) && lb_vec_rows(p.ring, p.ring_ld);
+    if (p.T >= 4 * ctx->sm_count)
+        LB_TYPED(dtype, (lb_norm_conv_kernel<float, 4>), (lb_norm_conv_kernel<__nv_bfloat16, 4>), dim3(lb_ceil_div(p.T, 4)), dim3(256), 0, p, vec);
+    else if (p.T >= 2 * ctx->sm_count)
+        LB_TYPED(dtype, (lb_norm_conv_kernel<float, 2>), (lb_norm_conv_kernel<__nv_bfloat16, 2>), dim3(lb_ceil_div(p.T, 2)), dim3(256), 0, p, vec);
+    else
+        LB_TYPED(dtype, (lb_norm_conv_kernel<float, 1>), (lb_norm_conv_kernel<__nv_bfloat16, 1>), dim3(p.T), dim3(256), 0, p, vec);
     return 0;
 }
 
