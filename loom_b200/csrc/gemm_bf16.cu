@@ -3,11 +3,13 @@
 //   D[128 tokens, N rows] (float, TMEM) += X[128 tokens, 64] (bf16, shared) * W[N rows, 64]^T (bf16, shared)
 //
 // The same machine as the persistent int8 GEMM (gemm_ternary_i8.cu): both operands are stored in HBM as the shared-memory
-// image the tensor core reads (dense.cuh), a load warp brings one K slice of 64 columns per pipeline stage with two or three
-// bulk copies, one elected thread issues four K = 16 MMAs per slice, tensor memory holds two accumulator buffers and eight
+// image the tensor core reads (dense.cuh), two threads bring one K slice of 64 columns per pipeline stage with bulk
+// copies, one issues four K = 16 MMAs per slice, tensor memory holds two accumulator buffers and eight
 // epilogue warps drain tile i while tile i + 1 accumulates.  Tokens are the M side, so a thread of the epilogue owns a
 // token and eight consecutive output columns of it are one 16-byte chunk of the next product's input image.
-// N is 256 (two row blocks, or a gate and an up block side by side) or 128.  Routed experts: the token blocks of the image
+// N, a tile's columns, is any multiple of 16 up to 256 (gate and up side by side: up to 128 of each): plan() takes what makes the
+// busiest CTA finish first.  Few tiles are split over K by the CTAs of a cluster, whose sums meet in distributed shared memory in the
+// order of K.  Routed experts: the token blocks of the image
 // are grouped by expert and a table names each block's expert; the number of blocks in use is read on the device.
 // Every mbarrier wait is bounded; on expiry the kernel raises the context's status word, frees its tensor memory and returns.
 #include "dense.cuh"
@@ -16,32 +18,87 @@
 namespace {
 
 constexpr int kEpiThreads = 256;
-constexpr int kMmaWarp = kEpiThreads / 32, kLoadWarp = kMmaWarp + 1;
-constexpr int kThreads = kEpiThreads + 64;
+constexpr int kMmaWarp = kEpiThreads / 32, kRowsWarp = kMmaWarp + 1, kWeightsWarp = kMmaWarp + 2;
+constexpr int kThreads = kEpiThreads + 96;
+constexpr int kRing = 200 * 1024, kMaxStages = 8;
+constexpr size_t kSmem = kRing + 1024;
 
-template <int NB>
-struct Cfg {
-    static constexpr int kStageBytes = kImgBlock * (1 + NB);
-    static constexpr int kStages = (200 * 1024) / kStageBytes > 6 ? 6 : (200 * 1024) / kStageBytes;
-    static constexpr int kCols = 128 * NB;  // TMEM columns of one accumulator buffer
-    static constexpr size_t kSmem = (size_t)kStages * kStageBytes + 1024;
+struct Plan {
+    int n, split, row_tiles;  // columns of a tile (of each matrix), CTAs that share a tile, tiles over the rows of W
 };
+__host__ __device__ __forceinline__ int stage_bytes(int cols) { return kImgBlock + cols * 128; }  // cols: of both matrices
 
-// NB = 128-row blocks of W side by side in one tile (GLU: block 0 of the gate, block 1 of the up matrix)
-template <int NB, int EPI>
-__global__ void __launch_bounds__(kThreads, 1) lb_gemm_bf16_kernel(const LbDenseGemm p, int row_tiles) {
-    using C = Cfg<NB>;
+__device__ __forceinline__ void st_peer4(uint32_t addr, const float* f) {
+    asm volatile("st.shared::cluster.v4.f32 [%0], {%1, %2, %3, %4};" ::"r"(addr), "f"(f[0]), "f"(f[1]), "f"(f[2]), "f"(f[3]) : "memory");
+}
+
+// RESID: sixteen columns of a token's residual row from column r on
+__device__ __forceinline__ void load_residual(const LbDenseGemm& p, int tok, int r, float4 (&x)[4]) {
+    const float4* o = reinterpret_cast<const float4*>(p.out + (size_t)tok * p.ldo + r);
+    if (r < p.ldo) {
+        x[0] = o[0];
+        x[1] = o[1];
+    }
+    if (r + 8 < p.ldo) {
+        x[2] = o[2];
+        x[3] = o[3];
+    }
+}
+
+// eight consecutive columns of a token from column r on: v8 of the first matrix, u8 of the second; RESID: res, the residual's
+template <int EPI>
+__device__ __forceinline__ void emit8(const LbDenseGemm& p, int tok, int r, const float* v8, const float* u8, const float4* res) {
+    if (EPI == LB_DEPI_F32 || EPI == LB_DEPI_RESID) {
+        if (r >= p.ldo) return;
+        float4* o = reinterpret_cast<float4*>(p.out + (size_t)tok * p.ldo + r);
+        if (EPI == LB_DEPI_F32) {
+            o[0] = make_float4(v8[0], v8[1], v8[2], v8[3]);
+            o[1] = make_float4(v8[4], v8[5], v8[6], v8[7]);
+        } else {
+            float4 x = res[0], y = res[1];
+            x.x = fmaf(p.mult, v8[0], p.res_mult * x.x);
+            x.y = fmaf(p.mult, v8[1], p.res_mult * x.y);
+            x.z = fmaf(p.mult, v8[2], p.res_mult * x.z);
+            x.w = fmaf(p.mult, v8[3], p.res_mult * x.w);
+            y.x = fmaf(p.mult, v8[4], p.res_mult * y.x);
+            y.y = fmaf(p.mult, v8[5], p.res_mult * y.y);
+            y.z = fmaf(p.mult, v8[6], p.res_mult * y.z);
+            y.w = fmaf(p.mult, v8[7], p.res_mult * y.w);
+            o[0] = x;
+            o[1] = y;
+        }
+        return;
+    }
+    if (EPI == LB_DEPI_HEADS ? r >= p.rows : r / 64 >= p.img_slices) return;
+    float f[8];
+#pragma unroll
+    for (int j = 0; j < 8; ++j) {
+        f[j] = v8[j];
+        if (EPI == LB_DEPI_GELU) f[j] = lb_gelu_erff(v8[j]);
+        if (EPI == LB_DEPI_GLU) f[j] = lb_clamped_glu(v8[j], u8[j], p.limit);
+        if (EPI == LB_DEPI_SILU) f[j] = lb_siluf(v8[j]) * u8[j];
+    }
+    if (EPI == LB_DEPI_HEADS)
+        *reinterpret_cast<uint4*>(p.img + lb_heads_chunk(tok, r, p.heads, p.head_dim, p.head_chunks)) = lb_pack_chunk<__nv_bfloat16>(f);
+    else
+        lb_img_store8<__nv_bfloat16>(p.img, tok, r, p.img_slices, f);
+}
+
+template <int EPI>
+__global__ void __launch_bounds__(kThreads, 1) lb_gemm_bf16_kernel(const LbDenseGemm p, const Plan plan) {
     constexpr bool kDual = EPI == LB_DEPI_GLU || EPI == LB_DEPI_SILU;
     extern __shared__ __align__(1024) uint8_t smem[];
-    __shared__ __align__(8) uint64_t load_bar[C::kStages], empty_bar[C::kStages], acc_full[2], acc_empty[2];
+    __shared__ __align__(8) uint64_t load_bar[kMaxStages], empty_bar[kMaxStages], acc_full[2], acc_empty[2];
     __shared__ uint32_t tmem_base_s;
     __shared__ int s_failed;
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-    const int nrb = lb_ceil_div(p.rows, kImgRows);  // 128-row blocks of W
+    const int n = plan.n, cols = kDual ? 2 * n : n, row_tiles = plan.row_tiles, S = plan.split;
+    const int stage = stage_bytes(cols), stages = kRing / stage < kMaxStages ? kRing / stage : kMaxStages;
+    const int padded_rows = lb_round_up(p.rows, kImgRows);
 
     if (tid == 0) {
-        for (int s = 0; s < C::kStages; ++s) {
-            lb_mbar_init(&load_bar[s], 1);
+        for (int s = 0; s < stages; ++s) {
+            lb_mbar_init(&load_bar[s], 2);
             lb_mbar_init(&empty_bar[s], 1);
         }
         for (int b = 0; b < 2; ++b) {
@@ -51,7 +108,7 @@ __global__ void __launch_bounds__(kThreads, 1) lb_gemm_bf16_kernel(const LbDense
         lb_fence_mbar_init();
         s_failed = 0;
     }
-    if (warp == kMmaWarp) lb_tmem_alloc(&tmem_base_s, 2 * C::kCols);
+    if (warp == kMmaWarp) lb_tmem_alloc(&tmem_base_s, 512);
     lb_tc_fence_before();
     __syncthreads();
     lb_tc_fence_after();
@@ -60,38 +117,46 @@ __global__ void __launch_bounds__(kThreads, 1) lb_gemm_bf16_kernel(const LbDense
     lb_pdl_wait();
     const int nblocks = p.nblocks ? *p.nblocks : lb_ceil_div(p.tokens, kImgRows);
     const int ntiles = nblocks * row_tiles;
-    const int my_tiles = (int)blockIdx.x < ntiles ? (ntiles - (int)blockIdx.x + (int)gridDim.x - 1) / (int)gridDim.x : 0;
+    // S > 1: the cluster's tile, this CTA's slices of it; else every gridDim.x-th tile
+    const int rank = S > 1 ? (int)lb_cluster_rank() : 0, first_tile = (int)blockIdx.x / S, tile_step = (int)gridDim.x / S;
+    const int my_tiles = first_tile < ntiles ? (S > 1 ? 1 : (ntiles - first_tile + tile_step - 1) / tile_step) : 0;
+    const int ks0 = p.slices * rank / S, ks1 = p.slices * (rank + 1) / S;
 
-    if (warp == kLoadWarp) {
+    if (warp == kRowsWarp || warp == kWeightsWarp) {
         if (lb_elect()) {
             bool failed = false;
-            uint32_t it = 0;
+            int s = 0;
+            uint32_t parity = 1;  // (the first round's waits are over at once)
             for (int i = 0; i < my_tiles && !failed; ++i) {
-                const int t = (int)blockIdx.x + i * (int)gridDim.x;
-                const int rt = t % row_tiles, tb = t / row_tiles;
-                const uint8_t* xb = p.x + (size_t)tb * p.slices * kImgBlock;
+                const int t = first_tile + i * tile_step, rt = t % row_tiles, tb = t / row_tiles;
+                const uint8_t* xb = p.x + ((size_t)tb * p.slices + ks0) * kImgBlock;
+                // the tile's rows of W: pieces of up to three blocks of 128
                 const size_t goff = p.block_group ? (size_t)p.block_group[tb] * p.group_bytes : 0;
-                const uint8_t* wb[2];
-                int nw = NB;
-                if (kDual) {
-                    wb[0] = p.w + goff + (size_t)rt * p.slices * kImgBlock;
-                    wb[1] = p.w2 + goff + (size_t)rt * p.slices * kImgBlock;
-                } else {
-                    wb[0] = p.w + goff + (size_t)(rt * NB) * p.slices * kImgBlock;
-                    wb[1] = wb[0] + (size_t)p.slices * kImgBlock;
-                    if (NB == 2 && rt * NB + 1 >= nrb) nw = 1;  // the second half of the last tile has no rows: its columns are never read
-                }
-                for (int ks = 0; ks < p.slices; ++ks, ++it) {
-                    const int s = (int)(it % C::kStages);
-                    if (it >= (uint32_t)C::kStages && !lb_mbar_wait_bounded(&empty_bar[s], (it / C::kStages - 1) & 1, kTcWaitLimit)) {
+                const int r0 = rt * n, rows = padded_rows - r0 < n ? padded_rows - r0 : n;
+                for (int ks = ks0; ks < ks1; ++ks) {
+                    if (!lb_mbar_wait_bounded(&empty_bar[s], parity, kTcWaitLimit)) {
                         failed = true;
                         break;
                     }
-                    uint8_t* st = smem + (size_t)s * C::kStageBytes;
-                    lb_mbar_expect_tx(&load_bar[s], (uint32_t)(kImgBlock * (1 + nw)));
-                    lb_bulk_g2s(st, xb + (size_t)ks * kImgBlock, kImgBlock, &load_bar[s]);
-                    lb_bulk_g2s(st + kImgBlock, wb[0] + (size_t)ks * kImgBlock, kImgBlock, &load_bar[s]);
-                    if (nw == 2) lb_bulk_g2s(st + 2 * kImgBlock, wb[1] + (size_t)ks * kImgBlock, kImgBlock, &load_bar[s]);
+                    uint8_t* st = smem + (size_t)s * stage;
+                    if (warp == kRowsWarp) {
+                        lb_mbar_expect_tx(&load_bar[s], kImgBlock);
+                        lb_bulk_g2s(st, xb, kImgBlock, &load_bar[s]);
+                        xb += kImgBlock;
+                    } else {
+                        lb_mbar_expect_tx(&load_bar[s], (uint32_t)rows * 128 * (kDual ? 2 : 1));
+                        for (int r = r0; r < r0 + rows;) {
+                            const int m = (r & ~127) + 128 - r < r0 + rows - r ? (r & ~127) + 128 - r : r0 + rows - r;
+                            const size_t at = goff + ((size_t)(r >> 7) * p.slices + ks) * kImgBlock + (size_t)(r & 127) * 128;
+                            lb_bulk_g2s(st + kImgBlock + (r - r0) * 128, p.w + at, (uint32_t)m * 128, &load_bar[s]);
+                            if (kDual) lb_bulk_g2s(st + kImgBlock + (n + r - r0) * 128, p.w2 + at, (uint32_t)m * 128, &load_bar[s]);
+                            r += m;
+                        }
+                    }
+                    if (++s == stages) {
+                        s = 0;
+                        parity ^= 1;
+                    }
                 }
             }
             if (failed) atomicExch(&s_failed, 1);
@@ -99,9 +164,10 @@ __global__ void __launch_bounds__(kThreads, 1) lb_gemm_bf16_kernel(const LbDense
         __syncwarp();
     } else if (warp == kMmaWarp) {
         if (lb_elect()) {
-            constexpr uint32_t idesc = lb_idesc_bf16(128, 128 * NB, false);
+            const uint32_t idesc = lb_idesc_bf16(128, cols, false);
             bool failed = false;
-            uint32_t it = 0;
+            int s = 0;
+            uint32_t parity = 0;
             for (int i = 0; i < my_tiles && !failed; ++i) {
                 const int buf = i & 1;
                 if (i >= 2 && !lb_mbar_wait_bounded(&acc_empty[buf], (uint32_t)(((i >> 1) - 1) & 1), kTcWaitLimit)) {
@@ -109,18 +175,21 @@ __global__ void __launch_bounds__(kThreads, 1) lb_gemm_bf16_kernel(const LbDense
                     break;
                 }
                 lb_tc_fence_after();
-                const uint32_t d = tmem_base + (uint32_t)(buf * C::kCols);
-                for (int ks = 0; ks < p.slices; ++ks, ++it) {
-                    const int s = (int)(it % C::kStages);
-                    if (!lb_mbar_wait_bounded(&load_bar[s], (it / C::kStages) & 1, kTcWaitLimit)) {
+                const uint32_t d = tmem_base + (uint32_t)(buf * 256);
+                for (int ks = ks0; ks < ks1; ++ks) {
+                    if (!lb_mbar_wait_bounded(&load_bar[s], parity, kTcWaitLimit)) {
                         failed = true;
                         break;
                     }
                     lb_tc_fence_after();
-                    const uint64_t a = lb_smem_desc(lb_smem_u32(smem + (size_t)s * C::kStageBytes), 128, 1024), b = a + (kImgBlock >> 4);
+                    const uint64_t a = lb_smem_desc(lb_smem_u32(smem + (size_t)s * stage), 128, 1024), b = a + (kImgBlock >> 4);
 #pragma unroll
-                    for (int k = 0; k < 4; ++k) lb_mma_f16(d, a + k * 16, b + k * 16, idesc, (ks > 0 || k > 0) ? 1u : 0u);
+                    for (int k = 0; k < 4; ++k) lb_mma_f16(d, a + k * 16, b + k * 16, idesc, (ks > ks0 || k > 0) ? 1u : 0u);
                     lb_mma_commit(&empty_bar[s]);
+                    if (++s == stages) {
+                        s = 0;
+                        parity ^= 1;
+                    }
                 }
                 if (!failed) lb_mma_commit(&acc_full[buf]);
             }
@@ -128,115 +197,176 @@ __global__ void __launch_bounds__(kThreads, 1) lb_gemm_bf16_kernel(const LbDense
         }
         __syncwarp();
         lb_tc_fence_before();
-    } else {
-        // a warp reads the 32 TMEM lanes (= tokens) of its quarter; the two warps of a quarter split the columns
-        const int quarter = warp & 3, half = warp >> 2;
-        constexpr int kOut = kDual ? 128 : 128 * NB;  // output columns of a tile
-        bool failed = false;
+    }
+    // a warp reads the 32 TMEM lanes (= tokens) of its quarter; the two warps of a quarter take turns at sixteen columns
+    const int quarter = warp & 3, half = warp >> 2;
+    bool failed = false;
+    if (warp < kMmaWarp) {
         for (int i = 0; i < my_tiles && !failed; ++i) {
-            const int t = (int)blockIdx.x + i * (int)gridDim.x;
-            const int rt = t % row_tiles, tb = t / row_tiles, buf = i & 1;
+            const int t = first_tile + i * tile_step, rt = t % row_tiles, tb = t / row_tiles, buf = i & 1;
+            const int tok = tb * kImgRows + quarter * 32 + lane;
+            const bool tok_ok = p.nblocks || tok < p.tokens;
+            // RESID: the residual's columns are asked for sixteen ahead, the first ones and the rest's way into L2 while the sums are made (a
+            // read behind every accumulator: 2048 x 2560 x 6912 in tiles of 144 took 97 us, 78 so)
+            float4 next[4] = {};
+            if (EPI == LB_DEPI_RESID && S == 1 && tok_ok) {
+                load_residual(p, tok, rt * n + half * 16, next);
+                for (int c = half * 32; c < n; c += 64)
+                    if (rt * n + c < p.ldo) asm volatile("prefetch.global.L2 [%0];" ::"l"(p.out + (size_t)tok * p.ldo + rt * n + c));
+            }
             if (!lb_mbar_wait_bounded(&acc_full[buf], (uint32_t)((i >> 1) & 1), kTcWaitLimit)) {
                 failed = true;
                 if (lane == 0) atomicExch(&s_failed, 1);
                 break;
             }
             lb_tc_fence_after();
-            const int tok = tb * kImgRows + quarter * 32 + lane;
-            const bool tok_ok = p.nblocks || tok < p.tokens;
-            const uint32_t tacc = tmem_base + (uint32_t)(buf * C::kCols) + ((uint32_t)(quarter * 32) << 16);
+            if (S > 1) break;  // the sums of the other CTAs first
+            const uint32_t tacc = tmem_base + (uint32_t)(buf * 256) + ((uint32_t)(quarter * 32) << 16);
 #pragma unroll 1
-            for (int c0 = half * (kOut / 2); c0 < (half + 1) * (kOut / 2); c0 += 16) {
+            for (int c0 = half * 16; c0 < n; c0 += 32) {
                 float v[16], u[16];
-                lb_tmem_ld16(tacc + (uint32_t)c0, v);
-                if (kDual) lb_tmem_ld16(tacc + (uint32_t)(128 + c0), u);
-                lb_tmem_wait_ld();
+                float4 res[4];
+                if (EPI == LB_DEPI_RESID) {
 #pragma unroll
-                for (int hh = 0; hh < 2; ++hh) {
-                    const int r = rt * kOut + c0 + 8 * hh;
-                    const float *v8 = v + 8 * hh, *u8 = u + 8 * hh;
-                    if (!tok_ok) continue;
-                    if (EPI == LB_DEPI_F32 || EPI == LB_DEPI_RESID) {
-                        if (r >= p.ldo) continue;
-                        float4* o = reinterpret_cast<float4*>(p.out + (size_t)tok * p.ldo + r);
-                        if (EPI == LB_DEPI_F32) {
-                            o[0] = make_float4(v8[0], v8[1], v8[2], v8[3]);
-                            o[1] = make_float4(v8[4], v8[5], v8[6], v8[7]);
-                        } else {
-                            float4 x = o[0], y = o[1];
-                            x.x = fmaf(p.mult, v8[0], p.res_mult * x.x);
-                            x.y = fmaf(p.mult, v8[1], p.res_mult * x.y);
-                            x.z = fmaf(p.mult, v8[2], p.res_mult * x.z);
-                            x.w = fmaf(p.mult, v8[3], p.res_mult * x.w);
-                            y.x = fmaf(p.mult, v8[4], p.res_mult * y.x);
-                            y.y = fmaf(p.mult, v8[5], p.res_mult * y.y);
-                            y.z = fmaf(p.mult, v8[6], p.res_mult * y.z);
-                            y.w = fmaf(p.mult, v8[7], p.res_mult * y.w);
-                            o[0] = x;
-                            o[1] = y;
-                        }
-                    } else {
-                        if (EPI == LB_DEPI_HEADS ? r >= p.rows : r / 64 >= p.img_slices) continue;
-                        float f[8];
-#pragma unroll
-                        for (int j = 0; j < 8; ++j) {
-                            f[j] = v8[j];
-                            if (EPI == LB_DEPI_GELU) f[j] = lb_gelu_erff(v8[j]);
-                            if (EPI == LB_DEPI_GLU) f[j] = lb_clamped_glu(v8[j], u8[j], p.limit);
-                            if (EPI == LB_DEPI_SILU) f[j] = lb_siluf(v8[j]) * u8[j];
-                        }
-                        if (EPI == LB_DEPI_HEADS)
-                            *reinterpret_cast<uint4*>(p.img + lb_heads_chunk(tok, r, p.heads, p.head_dim, p.head_chunks)) = lb_pack_chunk<__nv_bfloat16>(f);
-                        else
-                            lb_img_store8<__nv_bfloat16>(p.img, tok, r, p.img_slices, f);
-                    }
+                    for (int e = 0; e < 4; ++e) res[e] = next[e];
+                    if (tok_ok && c0 + 32 < n) load_residual(p, tok, rt * n + c0 + 32, next);
                 }
+                lb_tmem_ld16(tacc + (uint32_t)c0, v);
+                if (kDual) lb_tmem_ld16(tacc + (uint32_t)(n + c0), u);
+                lb_tmem_wait_ld();
+                if (tok_ok)
+#pragma unroll
+                    for (int h = 0; h < 16; h += 8) emit8<EPI>(p, tok, rt * n + c0 + h, v + h, u + h, res + h / 4);
             }
             lb_tc_fence_before();
             __syncwarp();
             if (lane == 0) lb_mbar_arrive(&acc_empty[buf]);
         }
     }
+    if (S > 1) {
+        // Sixteen columns belong to CTA (column / 16) % S: the others write their sums of them into its pipeline buffers, once all of the
+        // cluster's MMAs are done, [source][group of the owner][token][16 + 4 floats]
+        __syncwarp();
+        lb_cluster_sync();
+        constexpr int kLd = 20, kMats = kDual ? 2 : 1;
+        const int groups = n / 16, slots = lb_ceil_div(groups, S);  // 16-column groups of a matrix; of an owner
+        const int lane_row = quarter * 32 + lane;
+        const uint32_t base = lb_smem_u32(smem), tacc = tmem_base + ((uint32_t)(quarter * 32) << 16);
+        const bool work = warp < kMmaWarp && my_tiles > 0;
+        if (work)
+            for (int c = half; c < groups; c += 2) {
+                const int owner = c % S;
+                if (owner == rank) continue;
+#pragma unroll
+                for (int m = 0; m < kMats; ++m) {
+                    float v[16];
+                    lb_tmem_ld16(tacc + (uint32_t)(m * n + c * 16), v);
+                    lb_tmem_wait_ld();
+                    const uint32_t to = lb_cluster_addr(base + (uint32_t)((((rank * slots + c / S) * kMats + m) * 128 + lane_row) * kLd * 4), (uint32_t)owner);
+#pragma unroll
+                    for (int e = 0; e < 16; e += 4) st_peer4(to + e * 4, v + e);
+                }
+            }
+        __syncwarp();
+        lb_cluster_sync();
+        if (work) {
+            const int rt = first_tile % row_tiles, tb = first_tile / row_tiles, tok = tb * kImgRows + lane_row;
+            const bool tok_ok = p.nblocks || tok < p.tokens;
+            for (int c = rank + S * half; c < groups; c += 2 * S) {
+                float own[kMats][16], sum[kMats][16];
+                float4 res[4] = {};
+                if (EPI == LB_DEPI_RESID && tok_ok) load_residual(p, tok, rt * n + c * 16, res);
+#pragma unroll
+                for (int m = 0; m < kMats; ++m) {
+                    lb_tmem_ld16(tacc + (uint32_t)(m * n + c * 16), own[m]);
+#pragma unroll
+                    for (int e = 0; e < 16; ++e) sum[m][e] = 0.f;
+                }
+                lb_tmem_wait_ld();
+                for (int q = 0; q < S; ++q) {
+#pragma unroll
+                    for (int m = 0; m < kMats; ++m) {
+                        const float* from = reinterpret_cast<const float*>(smem) + (size_t)(((q * slots + c / S) * kMats + m) * 128 + lane_row) * kLd;
+#pragma unroll
+                        for (int e = 0; e < 16; ++e) sum[m][e] += q == rank ? own[m][e] : from[e];
+                    }
+                }
+                if (tok_ok && !s_failed)
+#pragma unroll
+                    for (int h = 0; h < 16; h += 8) emit8<EPI>(p, tok, rt * n + c * 16 + h, sum[0] + h, sum[kMats - 1] + h, res + h / 4);
+            }
+        }
+        lb_tc_fence_before();
+    }
     __syncthreads();
     if (warp == kMmaWarp) {
         lb_tc_fence_after();
-        lb_tmem_dealloc(tmem_base, 2 * C::kCols);
+        lb_tmem_dealloc(tmem_base, 512);
     }
     if (tid == 0 && s_failed) atomicExch(p.status, 3);
 }
 
-template <int NB, int EPI>
-int launch(loom_b200_ctx* ctx, const LbDenseGemm& p) {
-    using C = Cfg<NB>;
-    const int per = EPI == LB_DEPI_GLU || EPI == LB_DEPI_SILU ? 1 : NB;
-    const int row_tiles = lb_ceil_div(lb_ceil_div(p.rows, kImgRows), per);
-    const int blocks = p.nblocks ? p.max_blocks : lb_ceil_div(p.tokens, kImgRows);
-    const int ntiles = row_tiles * blocks;
-    LB_BIG_SMEM(ctx, (lb_gemm_bf16_kernel<NB, EPI>), C::kSmem);
-    LB_LAUNCH(ctx, (lb_gemm_bf16_kernel<NB, EPI>), dim3(ntiles < ctx->sm_count ? ntiles : ctx->sm_count), dim3(kThreads), C::kSmem, p, row_tiles);
-    return 0;
+// Columns of a tile and CTAs that share one.  Measured with every SM at work: a slice takes 0.32 us with up to 128 columns (both
+// matrices together), 0.355 with 144, 0.40 with 192 and 0.46 with 256; meeting in a cluster 3 us, an epilogue behind the last MMA 0.015 us
+// a column.  Wide tiles leave a last wave of few of them: 2048 x 2560 x 6912 takes 96 us as 160 tiles of 256, 83 as 224 of 192 and 78
+// as 288 of 144 (100 before residual rows were asked for ahead); 2048 x 7696 x 2560 78 us with 256, 75 with 224, 84 with 144.  100
+// tokens x 2560 x 6912 are 20 tiles: 43 us, 25 shared by four CTAs each.
+Plan plan(const loom_b200_ctx* ctx, const LbDenseGemm& p, bool dual) {
+    const int blocks = p.nblocks ? p.max_blocks : lb_ceil_div(p.tokens, kImgRows), most = dual ? 128 : 256, rows = lb_round_up(p.rows, kImgRows);  // (the padding's zeros too)
+    Plan best = {};
+    double best_us = 1e30;
+    for (int n = most < rows ? most : rows; n >= 48; n -= 16) {
+        const int tiles = lb_ceil_div(rows, n) * blocks, cols = dual ? 2 * n : n;
+        const double slice = cols <= 106 ? 0.32 : 0.22 + cols * 0.00094;
+        for (int S = 1; S <= 8; S *= 2) {
+            // clusters of whole SMs: what the groups of SMs hold of them
+            if (S > 1 && (tiles * S > ctx->sm_count - 5 * S || p.slices < 4 * S)) break;
+            const int waves = S > 1 ? 1 : lb_ceil_div(tiles, ctx->sm_count);
+            const double us = waves * lb_ceil_div(p.slices, S) * slice + (S > 1 ? 3.0 : 0.0) + cols * 0.015 / S;
+            if (us < 0.98 * best_us) {
+                best_us = us;
+                best = {n, S, lb_ceil_div(rows, n)};
+            }
+        }
+    }
+    return best;
 }
 
 template <int EPI>
-int launch_plain(loom_b200_ctx* ctx, const LbDenseGemm& p) {
-    // a tile's time follows the bytes of its stages (48 KB for two row blocks, 32 KB for one), the launch's the busiest CTA
-    const int nrb = lb_ceil_div(p.rows, kImgRows), blocks = p.nblocks ? p.max_blocks : lb_ceil_div(p.tokens, kImgRows), sms = ctx->sm_count;
-    const int t1 = nrb * blocks, t2 = lb_ceil_div(nrb, 2) * blocks;
-    const bool wide = nrb > 1 && 3 * lb_ceil_div(t2, sms) <= 2 * lb_ceil_div(t1, sms);
-    return wide ? launch<2, EPI>(ctx, p) : launch<1, EPI>(ctx, p);
+int launch(loom_b200_ctx* ctx, const LbDenseGemm& p) {
+    constexpr bool kDual = EPI == LB_DEPI_GLU || EPI == LB_DEPI_SILU;
+    const Plan pl = plan(ctx, p, kDual);
+    const int blocks = p.nblocks ? p.max_blocks : lb_ceil_div(p.tokens, kImgRows), tiles = pl.row_tiles * blocks;
+    LB_BIG_SMEM(ctx, lb_gemm_bf16_kernel<EPI>, kSmem);
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(pl.split > 1 ? tiles * pl.split : tiles < ctx->sm_count ? tiles : ctx->sm_count);
+    cfg.blockDim = dim3(kThreads);
+    cfg.dynamicSmemBytes = kSmem;
+    cfg.stream = ctx->stream;
+    cudaLaunchAttribute attr[2];
+    attr[0].id = cudaLaunchAttributeClusterDimension;
+    attr[0].val.clusterDim.x = (unsigned)pl.split;
+    attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
+    attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[1].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = ctx->opt_pdl ? 2 : 1;
+    LB_CUDA(ctx, cudaLaunchKernelEx(&cfg, lb_gemm_bf16_kernel<EPI>, p, pl));
+    ctx->launches++;
+    return 0;
 }
 
 }  // namespace
 
 int lb_gemm_bf16_run(loom_b200_ctx* ctx, int epi, const LbDenseGemm& p) {
     switch (epi) {
-        case LB_DEPI_F32: return launch_plain<LB_DEPI_F32>(ctx, p);
-        case LB_DEPI_RESID: return launch_plain<LB_DEPI_RESID>(ctx, p);
-        case LB_DEPI_GELU: return launch_plain<LB_DEPI_GELU>(ctx, p);
-        case LB_DEPI_IMG: return launch_plain<LB_DEPI_IMG>(ctx, p);
-        case LB_DEPI_HEADS: return launch_plain<LB_DEPI_HEADS>(ctx, p);
-        case LB_DEPI_GLU: return launch<2, LB_DEPI_GLU>(ctx, p);
-        case LB_DEPI_SILU: return launch<2, LB_DEPI_SILU>(ctx, p);
+        case LB_DEPI_F32: return launch<LB_DEPI_F32>(ctx, p);
+        case LB_DEPI_RESID: return launch<LB_DEPI_RESID>(ctx, p);
+        case LB_DEPI_GELU: return launch<LB_DEPI_GELU>(ctx, p);
+        case LB_DEPI_IMG: return launch<LB_DEPI_IMG>(ctx, p);
+        case LB_DEPI_HEADS: return launch<LB_DEPI_HEADS>(ctx, p);
+        case LB_DEPI_GLU: return launch<LB_DEPI_GLU>(ctx, p);
+        case LB_DEPI_SILU: return launch<LB_DEPI_SILU>(ctx, p);
     }
     return lb_fail(ctx, LOOM_B200_ERR_UNSUPPORTED, "gemm_bf16: epilogue %d is not built", epi);
 }
