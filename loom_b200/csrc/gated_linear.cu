@@ -252,38 +252,67 @@ __global__ void __launch_bounds__(kPrepThreads, 2) lb_gla_prep_kernel(const LbGl
     }
 }
 
-// 64 x 64 output tiles of products of float matrices: 128 threads, 8 x 4 each
-constexpr int kTile = 64, kTileLd = 68, kTileK = 32, kTileThreads = 128;
+// 64 x 64 output tiles of products of float matrices: 128 threads, 8 x 4 each, on packed multiply-adds of two rows at a time; the next 32
+// of K are on their way to registers while these are multiplied.  Bound: shared-memory reads and multiply-adds about alike.  One slice
+// after the other between two barriers, with the first factor's rows read 16 bytes a line: 32 chunks x 10 heads, 128 x 256: outputs 83
+// us, states 48; so 52 and 37.
+constexpr int kTile = 64, kTileLd = 68, kTileK = 32, kTileThreads = 128, kTileLoads = kTileK * kTile / 4 / kTileThreads;
 
-__device__ __forceinline__ void tile_fma(const float (*sa)[kTileLd], const float (*sb)[kTileLd], int ty, int tx, float (*acc)[4]) {
+__device__ __forceinline__ void tile_fma(const float (*sa)[kTileLd], const float (*sb)[kTileLd], int ty, int tx, uint64_t (*acc)[4]) {
 #pragma unroll 8
     for (int k = 0; k < kTileK; ++k) {
-        const float4 a = *reinterpret_cast<const float4*>(&sa[k][ty * 8]), a2 = *reinterpret_cast<const float4*>(&sa[k][ty * 8 + 4]);
+        const ulonglong2 a = *reinterpret_cast<const ulonglong2*>(&sa[k][ty * 8]), a2 = *reinterpret_cast<const ulonglong2*>(&sa[k][ty * 8 + 4]);
         const float4 b = *reinterpret_cast<const float4*>(&sb[k][tx * 4]);
-        const float av[8] = {a.x, a.y, a.z, a.w, a2.x, a2.y, a2.z, a2.w}, bv[4] = {b.x, b.y, b.z, b.w};
+        const uint64_t av[4] = {a.x, a.y, a2.x, a2.y}, bv[4] = {lb_pack2(b.x, b.x), lb_pack2(b.y, b.y), lb_pack2(b.z, b.z), lb_pack2(b.w, b.w)};
 #pragma unroll
-        for (int i = 0; i < 8; ++i)
+        for (int i = 0; i < 4; ++i)
 #pragma unroll
-            for (int j = 0; j < 4; ++j) acc[i][j] = fmaf(av[i], bv[j], acc[i][j]);
+            for (int j = 0; j < 4; ++j) acc[i][j] = lb_fma2(av[i], bv[j], acc[i][j]);
     }
 }
-// rows k0 .. of a row-major matrix (nk of them exist), columns c0 .. (nc exist)
-__device__ __forceinline__ void tile_rows(float (*s)[kTileLd], const float* m, size_t ld, int nk, int c0, int nc, bool vec) {
-    for (int i = threadIdx.x; i < kTileK * kTile / 4; i += kTileThreads) {
-        const int k = i >> 4, c = (i & 15) * 4;
-        float f[4] = {0.f, 0.f, 0.f, 0.f};
-        if (k < nk) lb_load_cols<4>(m + (size_t)k * ld, c0 + c, nc, vec, f);
-        *reinterpret_cast<float4*>(&s[k][c]) = make_float4(f[0], f[1], f[2], f[3]);
+// row i of a thread's eight
+__device__ __forceinline__ void tile_row(const uint64_t (*acc)[4], int i, float* f) {
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+        float lo, hi;
+        lb_unpack2(acc[i >> 1][j], lo, hi);
+        f[j] = i & 1 ? hi : lo;
     }
 }
-// the same transposed: s[k][row] = m[row][k0 + k]
-__device__ __forceinline__ void tile_cols(float (*s)[kTileLd], const float* m, size_t ld, int nr, int k0, int nk, bool vec) {
-    for (int i = threadIdx.x; i < kTile * kTileK / 4; i += kTileThreads) {
-        const int r = i & 63, k = (i >> 6) * 4;
-        float f[4] = {0.f, 0.f, 0.f, 0.f};
-        if (r < nr) lb_load_cols<4>(m + (size_t)r * ld, k0 + k, nk, vec, f);
+// rows k0 .. of a row-major matrix (nk of them exist), columns c0 .. (nc exist): to registers, and from there to s[k][column]
+__device__ __forceinline__ void tile_rows_load(float (*f)[4], const float* m, size_t ld, int nk, int c0, int nc, bool vec) {
 #pragma unroll
-        for (int e = 0; e < 4; ++e) s[k + e][r] = f[e];
+    for (int q = 0; q < kTileLoads; ++q) {
+        const int i = threadIdx.x + q * kTileThreads, k = i >> 4, c = (i & 15) * 4;
+        f[q][0] = f[q][1] = f[q][2] = f[q][3] = 0.f;
+        if (k < nk) lb_load_cols<4>(m + (size_t)k * ld, c0 + c, nc, vec, f[q]);
+    }
+}
+__device__ __forceinline__ void tile_rows_store(float (*s)[kTileLd], const float (*f)[4]) {
+#pragma unroll
+    for (int q = 0; q < kTileLoads; ++q) {
+        const int i = threadIdx.x + q * kTileThreads;
+        *reinterpret_cast<float4*>(&s[i >> 4][(i & 15) * 4]) = make_float4(f[q][0], f[q][1], f[q][2], f[q][3]);
+    }
+}
+// the same transposed, s[k][row] = m[row][k0 + k]: eight lanes read 128 bytes of a row and start at another of their four columns each, so
+// that a store touches every bank once
+__device__ __forceinline__ void tile_cols_load(float (*f)[4], const float* m, size_t ld, int nr, int k0, int nk, bool vec) {
+#pragma unroll
+    for (int q = 0; q < kTileLoads; ++q) {
+        const int i = threadIdx.x + q * kTileThreads, r = i >> 3, k = (i & 7) * 4;
+        f[q][0] = f[q][1] = f[q][2] = f[q][3] = 0.f;
+        if (r < nr) lb_load_cols<4>(m + (size_t)r * ld, k0 + k, nk, vec, f[q]);
+    }
+}
+__device__ __forceinline__ void tile_cols_store(float (*s)[kTileLd], const float (*f)[4]) {
+#pragma unroll
+    for (int q = 0; q < kTileLoads; ++q) {
+        const int i = threadIdx.x + q * kTileThreads, r = i >> 3, k = (i & 7) * 4, rot = (i >> 1) & 3;
+        const float a0 = rot & 1 ? f[q][1] : f[q][0], a1 = rot & 1 ? f[q][2] : f[q][1], a2 = rot & 1 ? f[q][3] : f[q][2], a3 = rot & 1 ? f[q][0] : f[q][3];
+        const float g[4] = {rot & 2 ? a2 : a0, rot & 2 ? a3 : a1, rot & 2 ? a0 : a2, rot & 2 ? a1 : a3};
+#pragma unroll
+        for (int e = 0; e < 4; ++e) s[k + ((e + rot) & 3)][r] = g[e];
     }
 }
 
@@ -294,12 +323,19 @@ __global__ void __launch_bounds__(kTileThreads) lb_chunk_state_kernel(const LbCh
     lb_pdl_wait();
     const int d0 = (blockIdx.x % dtiles) * kTile, v0 = (blockIdx.x / dtiles) * kTile, h = blockIdx.y, ch = blockIdx.z, tid = threadIdx.x;
     const int HD = b.heads * b.dim, t0 = ch * b.C, n = min(b.C, T - t0), ty = tid >> 4, tx = tid & 15;
-    float acc[8][4] = {};
+    uint64_t acc[4][4] = {};
+    float fa[kTileLoads][4], fb[kTileLoads][4];
+    auto load = [&](int s0) {
+        tile_rows_load(fa, b.kd + (size_t)(t0 + s0) * HD + h * b.dim, HD, n - s0, d0, b.dim, vec);
+        tile_rows_load(fb, b.v + (size_t)(t0 + s0) * b.ldv + h * b.vdim, b.ldv, n - s0, v0, b.vdim, vec);
+    };
+    load(0);
     for (int s0 = 0; s0 < n; s0 += kTileK) {
         __syncthreads();
-        tile_rows(sa, b.kd + (size_t)(t0 + s0) * HD + h * b.dim, HD, n - s0, d0, b.dim, vec);
-        tile_rows(sb, b.v + (size_t)(t0 + s0) * b.ldv + h * b.vdim, b.ldv, n - s0, v0, b.vdim, vec);
+        tile_rows_store(sa, fa);
+        tile_rows_store(sb, fb);
         __syncthreads();
+        if (s0 + kTileK < n) load(s0 + kTileK);
         tile_fma(sa, sb, ty, tx, acc);
     }
     float* out = b.states + ((size_t)ch * b.heads + h) * b.dim * b.vdim;
@@ -307,12 +343,14 @@ __global__ void __launch_bounds__(kTileThreads) lb_chunk_state_kernel(const LbCh
     for (int i = 0; i < 8; ++i) {
         const int d = d0 + ty * 8 + i, v = v0 + tx * 4;
         if (d >= b.dim) continue;
+        float f[4];
+        tile_row(acc, i, f);
         if (vec && v + 4 <= b.vdim)
-            *reinterpret_cast<float4*>(out + (size_t)d * b.vdim + v) = make_float4(acc[i][0], acc[i][1], acc[i][2], acc[i][3]);
+            *reinterpret_cast<float4*>(out + (size_t)d * b.vdim + v) = make_float4(f[0], f[1], f[2], f[3]);
         else
 #pragma unroll
             for (int j = 0; j < 4; ++j)
-                if (v + j < b.vdim) out[(size_t)d * b.vdim + v + j] = acc[i][j];
+                if (v + j < b.vdim) out[(size_t)d * b.vdim + v + j] = f[j];
     }
 }
 
@@ -351,19 +389,26 @@ __global__ void __launch_bounds__(kTileThreads) lb_chunk_out_kernel(const LbChun
     const int HD = b.heads * b.dim, t0 = ch * C, n = min(C, T - t0), ty = tid >> 4, tx = tid & 15;
     const float* S = b.states + ((size_t)ch * b.heads + h) * b.dim * b.vdim;
     const float* A = b.weights + ((size_t)ch * b.heads + h) * C * C;
-    float acc[8][4] = {};
-    for (int k0 = 0; k0 < b.dim; k0 += kTileK) {
+    uint64_t acc[4][4] = {};
+    float fa[kTileLoads][4], fb[kTileLoads][4];
+    const int first = lb_ceil_div(b.dim, kTileK), all = first + lb_ceil_div(n, kTileK);  // K slices of the state, then of the chunk's tokens
+    auto load = [&](int x) {
+        const int k0 = (x < first ? x : x - first) * kTileK;
+        if (x < first) {
+            tile_cols_load(fa, b.qd + (size_t)t0 * HD + h * b.dim, HD, n, k0, b.dim, vec);
+            tile_rows_load(fb, S + (size_t)k0 * b.vdim, b.vdim, b.dim - k0, v0, b.vdim, vec);
+        } else {
+            tile_cols_load(fa, A, C, n, k0, n, true);
+            tile_rows_load(fb, b.v + (size_t)(t0 + k0) * b.ldv + h * b.vdim, b.ldv, n - k0, v0, b.vdim, vec);
+        }
+    };
+    load(0);
+    for (int x = 0; x < all; ++x) {
         __syncthreads();
-        tile_cols(sa, b.qd + (size_t)t0 * HD + h * b.dim, HD, n, k0, b.dim, vec);
-        tile_rows(sb, S + (size_t)k0 * b.vdim, b.vdim, b.dim - k0, v0, b.vdim, vec);
+        tile_cols_store(sa, fa);
+        tile_rows_store(sb, fb);
         __syncthreads();
-        tile_fma(sa, sb, ty, tx, acc);
-    }
-    for (int s0 = 0; s0 < n; s0 += kTileK) {
-        __syncthreads();
-        tile_cols(sa, A, C, n, s0, n, true);
-        tile_rows(sb, b.v + (size_t)(t0 + s0) * b.ldv + h * b.vdim, b.ldv, n - s0, v0, b.vdim, vec);
-        __syncthreads();
+        if (x + 1 < all) load(x + 1);
         tile_fma(sa, sb, ty, tx, acc);
     }
 #pragma unroll
@@ -371,12 +416,14 @@ __global__ void __launch_bounds__(kTileThreads) lb_chunk_out_kernel(const LbChun
         const int t = ty * 8 + i, v = v0 + tx * 4;
         if (t >= n) continue;
         float* out = b.o + (size_t)(t0 + t) * b.ldo + h * b.vdim + v;
+        float f[4];
+        tile_row(acc, i, f);
         if (vec && v + 4 <= b.vdim)
-            *reinterpret_cast<float4*>(out) = make_float4(acc[i][0], acc[i][1], acc[i][2], acc[i][3]);
+            *reinterpret_cast<float4*>(out) = make_float4(f[0], f[1], f[2], f[3]);
         else
 #pragma unroll
             for (int j = 0; j < 4; ++j)
-                if (v + j < b.vdim) out[j] = acc[i][j];
+                if (v + j < b.vdim) out[j] = f[j];
     }
 }
 
