@@ -1,6 +1,7 @@
 // abi.cu -- context, device buffers and packed-weight management behind the C ABI.
 #include "common.cuh"
 
+#include <sys/mman.h>
 #include <cstdlib>
 #include <mutex>
 #include <vector>
@@ -76,6 +77,21 @@ int lb_ensure_scratch(loom_b200_ctx* ctx, size_t bytes) {
     LB_CUDA(ctx, cudaMalloc(&ctx->scratch, n));
     ctx->scratch_bytes = n;
     return 0;
+}
+
+// Faults the pages of a pageable buffer in by one call (their contents stay).  Touching them one by one -- a read, then a write -- faults a
+// fresh page twice, 1000 of them longer than a step of eight sequences takes.  Where the kernel does not know the request the copy faults them.
+void lb_touch_pages(void* p, size_t bytes) {
+#ifdef MADV_POPULATE_WRITE
+    cudaPointerAttributes where{};
+    if (cudaPointerGetAttributes(&where, p) != cudaSuccess) {
+        (void)cudaGetLastError();
+        return;
+    }
+    if (where.type != cudaMemoryTypeUnregistered) return;
+    const uintptr_t from = reinterpret_cast<uintptr_t>(p) & ~(uintptr_t)4095, end = reinterpret_cast<uintptr_t>(p) + bytes;
+    (void)madvise(reinterpret_cast<void*>(from), end - from, MADV_POPULATE_WRITE);
+#endif
 }
 
 int lb_status_queue(loom_b200_ctx* ctx) {
@@ -422,6 +438,9 @@ void loom_b200_ctx_destroy(loom_b200_ctx* ctx) {
     if (ctx->scratch) cudaFree(ctx->scratch);
     if (ctx->status_dev) cudaFree(ctx->status_dev);
     if (ctx->status_host) cudaFreeHost(ctx->status_host);
+    if (ctx->stage_host) cudaFreeHost(ctx->stage_host);
+    for (cudaEvent_t e : ctx->stage_done)
+        if (e) cudaEventDestroy(e);
     if (ctx->trace_dev) cudaFree(ctx->trace_dev);
     if (ctx->argmax_scratch) cudaFree(ctx->argmax_scratch);
     if (ctx->head_scratch) cudaFree(ctx->head_scratch);

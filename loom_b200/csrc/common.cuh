@@ -43,6 +43,8 @@ struct loom_b200_weight {
     size_t tile_bytes() const { return (size_t)strips * kblocks * kTileBytes; }
 };
 
+constexpr int kStageSlots = 8;
+
 struct loom_b200_ctx {
     int device = 0;
     cudaStream_t stream = nullptr;
@@ -61,6 +63,8 @@ struct loom_b200_ctx {
     // device status word written by kernels with bounded waits (0 = ok)
     int* status_dev = nullptr;
     int* status_host = nullptr;    // pinned mirror, refreshed by lb_sync_checked
+    char* stage_host = nullptr;      // pinned slots that a layer call's host rows cross through (layers.cu)
+    cudaEvent_t stage_done[kStageSlots] = {};
     void* quant_scratch = nullptr;   // int8 row and absmax of the stand-alone GEMV prologue (wide inputs)
     size_t quant_scratch_bytes = 0;
     void* stage_scratch = nullptr;   // input rows of the float GEMV for several sequences
@@ -120,6 +124,8 @@ int lb_sync_checked(loom_b200_ctx* ctx);
 // what it says once that copy is known to have arrived.
 int lb_status_queue(loom_b200_ctx* ctx);
 int lb_status_result(loom_b200_ctx* ctx);
+// Faults the pages of a pageable buffer in by one call (their contents stay); nothing for memory that CUDA knows.
+void lb_touch_pages(void* p, size_t bytes);
 int lb_ensure_quant_scratch(loom_b200_ctx* ctx, size_t bytes);
 
 #define LB_CUDA(ctx, expr)                                                                          \

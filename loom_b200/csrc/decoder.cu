@@ -256,21 +256,6 @@ int dec_stack_step(loom_b200_decoder* dec, int lane0, int M) {
 constexpr int kReadPieces = 2;
 constexpr size_t kReadSplit = 192 * 1024;
 
-// Faults the pages of a pageable buffer in by one call (their contents stay).  Touching them one by one -- a read, then a write -- faults a
-// fresh page twice, 1000 of them longer than a step of eight sequences takes.  Where the kernel does not know the request the copy faults them.
-void touch_pages(void* p, size_t bytes) {
-#ifdef MADV_POPULATE_WRITE
-    cudaPointerAttributes where{};
-    if (cudaPointerGetAttributes(&where, p) != cudaSuccess) {
-        (void)cudaGetLastError();
-        return;
-    }
-    if (where.type != cudaMemoryTypeUnregistered) return;
-    const uintptr_t from = reinterpret_cast<uintptr_t>(p) & ~(uintptr_t)4095, end = reinterpret_cast<uintptr_t>(p) + bytes;
-    (void)madvise(reinterpret_cast<void*>(from), end - from, MADV_POPULATE_WRITE);
-#endif
-}
-
 // The selected sequence's logits row on the host.  The status word comes first: a row that it calls invalid does not reach the
 // caller, and no copy of its own has to be waited for after the row.
 int dec_read_logits(loom_b200_decoder* dec, float* host) {
@@ -284,7 +269,7 @@ int dec_read_logits(loom_b200_decoder* dec, float* host) {
         LB_CUDA(ctx, cudaMemcpyAsync((char*)dec->h_logits + from[i], (const char*)dec->logits + from[i], from[i + 1] - from[i], cudaMemcpyDeviceToHost, ctx->stream));
         if (i + 1 < pieces) LB_CUDA(ctx, cudaEventRecord(dec->read_done[i], ctx->stream));
     }
-    if (pieces > 1) touch_pages(host, bytes);
+    if (pieces > 1) lb_touch_pages(host, bytes);
     for (int i = 0; i < pieces; ++i) {
         LB_CUDA(ctx, i + 1 < pieces ? cudaEventSynchronize(dec->read_done[i]) : cudaStreamSynchronize(ctx->stream));
         if (i == 0)
@@ -1215,7 +1200,7 @@ int loom_b200_decoder_step_batch(loom_b200_decoder* dec, const int32_t* tokens, 
         LB_CUDA(ctx, cudaMemcpyAsync(dec->tok_all, dec->h_tok_all, (size_t)B * sizeof(int), cudaMemcpyHostToDevice, ctx->stream));
     }
     // with the whole vocabulary on this GPU the rows that a pass over the head has made cross to the host beside the passes after it (16
-    // sequences: 34.9 ms for eight steps with one copy at the end, 28.4 so); one pass has nothing to cross beside (eight rows of 16 KB:
+    // sequences: 34.9 ms for eight steps with one copy at the end, 28.4 so at the time); one pass has nothing to cross beside (eight rows of 16 KB:
     // 71 us a step with a copy in the step's own stream, 81 so)
     const bool beside = logits_host && B > kChunkTokens && !dec->head_sharded;
     int parts = 0, done = 0, ends[kReadEvents];
@@ -1235,7 +1220,7 @@ int loom_b200_decoder_step_batch(loom_b200_decoder* dec, const int32_t* tokens, 
     dec->kv_offset = dec->kv_offsets[dec->lane];
     if (beside) {
         const size_t row = (size_t)dec->d.vocab * 4;
-        touch_pages(logits_host, (size_t)B * row);
+        lb_touch_pages(logits_host, (size_t)B * row);
         cudaError_t e = cudaSuccess;
         for (int i = 0; i < parts && e == cudaSuccess; ++i) {
             const size_t at = i ? (size_t)ends[i - 1] * row : 0, len = (size_t)ends[i] * row - at;
@@ -1251,7 +1236,7 @@ int loom_b200_decoder_step_batch(loom_b200_decoder* dec, const int32_t* tokens, 
         for (int i = 0; i < B; ++i)
             if (int rc = dec_gather_logits(dec, dec->logits_all + (size_t)i * dec->d.vocab)) return rc;
         if (int rc = lb_status_queue(ctx)) return rc;
-        touch_pages(logits_host, (size_t)B * dec->d.vocab * 4);
+        lb_touch_pages(logits_host, (size_t)B * dec->d.vocab * 4);
         LB_CUDA(ctx, cudaMemcpyAsync(logits_host, dec->logits_all, (size_t)B * dec->d.vocab * 4, cudaMemcpyDeviceToHost, ctx->stream));
         LB_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
         return lb_status_result(ctx);

@@ -4,6 +4,7 @@
 #include "layers.cuh"
 
 #include <cmath>
+#include <cstring>
 #include <vector>
 
 int lb_ternary_gemm(loom_b200_ctx* ctx, const loom_b200_weight* w, int tokens, const float* x, const float* bias,
@@ -296,6 +297,113 @@ struct Arena {
 
 size_t align256(size_t n) { return (n + 255) & ~(size_t)255; }
 
+// The host rows of a layer call cross through pinned slots of the context: rows on their way in are copied to one slot while the slot before
+// crosses the bus, and rows on their way out are copied on while the next crosses.  The caller's fresh pages are faulted in while the GPU is
+// still at the layer.  The driver's own path for pageable memory moves 6 GB/s (636 KB out: 107 us) and starts when the layer is done.
+// Attention and feed-forward of a 2B-shaped block, 23 tokens and one more, four calls: 464 us that way, 402 so; of a call's 142 us with
+// 23 tokens the copies from the slots take 36.  A context's first call pays a millisecond for the slots; memory that CUDA knows is copied
+// as it is.
+constexpr size_t kSlotBytes = 128 * 1024;
+
+struct HostPart {
+    const float* dev;
+    float* host;
+    size_t n;  // floats
+};
+
+class HostRows {
+public:
+    explicit HostRows(loom_b200_ctx* ctx) : ctx_(ctx) {}
+    // (a call that failed leaves nothing behind that still reads or writes a slot)
+    ~HostRows() {
+        if (open_) cudaStreamSynchronize(ctx_->stream);
+    }
+    // rows to dev; `host` may be changed afterwards unless CUDA knows it
+    int send(float* dev, const float* host, size_t n) {
+        if (!dev || n == 0) return 0;
+        if (int rc = ready()) return rc;
+        if (known(host)) {
+            LB_CUDA(ctx_, cudaMemcpyAsync(dev, host, n * 4, cudaMemcpyHostToDevice, ctx_->stream));
+            return 0;
+        }
+        for (size_t at = 0; at < n * 4; at += kSlotBytes, ++sent_) {
+            const size_t len = n * 4 - at < kSlotBytes ? n * 4 - at : kSlotBytes;
+            if (sent_ >= kStageSlots) LB_CUDA(ctx_, cudaEventSynchronize(ctx_->stage_done[sent_ % kStageSlots]));
+            memcpy(slot(sent_), (const char*)host + at, len);
+            LB_CUDA(ctx_, cudaMemcpyAsync((char*)dev + at, slot(sent_), len, cudaMemcpyHostToDevice, ctx_->stream));
+            LB_CUDA(ctx_, cudaEventRecord(ctx_->stage_done[sent_ % kStageSlots], ctx_->stream));
+        }
+        return 0;
+    }
+    // both results (host side null: not asked for), behind the work queued so far; returns when they are there
+    int fetch(const HostPart (&parts)[2]) {
+        if (int rc = ready()) return rc;
+        size_t pieces[2] = {};
+        bool direct = false;
+        for (int i = 0; i < 2; ++i) {
+            const HostPart& p = parts[i];
+            if (p.host && !known(p.host))
+                pieces[i] = (p.n * 4 + kSlotBytes - 1) / kSlotBytes;
+            else if (p.host) {
+                direct = true;
+                LB_CUDA(ctx_, cudaMemcpyAsync(p.host, p.dev, p.n * 4, cudaMemcpyDeviceToHost, ctx_->stream));
+            }
+        }
+        const size_t all = pieces[0] + pieces[1];
+        auto part = [&](size_t i, size_t* at, size_t* len) -> const HostPart& {
+            const HostPart& p = parts[i < pieces[0] ? 0 : 1];
+            *at = (i < pieces[0] ? i : i - pieces[0]) * kSlotBytes;
+            *len = p.n * 4 - *at < kSlotBytes ? p.n * 4 - *at : kSlotBytes;
+            return p;
+        };
+        auto ask = [&](size_t i) -> int {
+            size_t at, len;
+            const HostPart& p = part(i, &at, &len);
+            LB_CUDA(ctx_, cudaMemcpyAsync(slot(i), (const char*)p.dev + at, len, cudaMemcpyDeviceToHost, ctx_->stream));
+            LB_CUDA(ctx_, cudaEventRecord(ctx_->stage_done[i % kStageSlots], ctx_->stream));
+            return 0;
+        };
+        for (size_t i = 0; i < all && i < kStageSlots; ++i)
+            if (int rc = ask(i)) return rc;
+        for (int i = 0; i < 2; ++i)
+            if (pieces[i] > 0) lb_touch_pages(parts[i].host, parts[i].n * 4);
+        for (size_t i = 0; i < all; ++i) {
+            size_t at, len;
+            const HostPart& p = part(i, &at, &len);
+            LB_CUDA(ctx_, cudaEventSynchronize(ctx_->stage_done[i % kStageSlots]));
+            memcpy((char*)p.host + at, slot(i), len);
+            if (i + kStageSlots < all)
+                if (int rc = ask(i + kStageSlots)) return rc;
+        }
+        // (the last piece is behind all of the call's work; copies that CUDA makes by itself have no event)
+        if (all == 0 || direct) LB_CUDA(ctx_, cudaStreamSynchronize(ctx_->stream));
+        open_ = false;
+        return 0;
+    }
+
+private:
+    static bool known(const void* host) {
+        cudaPointerAttributes where{};
+        if (cudaPointerGetAttributes(&where, host) != cudaSuccess) {
+            (void)cudaGetLastError();
+            return false;
+        }
+        return where.type != cudaMemoryTypeUnregistered;
+    }
+    char* slot(size_t i) const { return ctx_->stage_host + i % kStageSlots * kSlotBytes; }
+    int ready() {
+        open_ = true;
+        if (ctx_->stage_host) return 0;
+        for (cudaEvent_t& e : ctx_->stage_done)
+            if (!e) LB_CUDA(ctx_, cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
+        LB_CUDA(ctx_, cudaMallocHost((void**)&ctx_->stage_host, kStageSlots * kSlotBytes));
+        return 0;
+    }
+    loom_b200_ctx* ctx_;
+    size_t sent_ = 0;
+    bool open_ = false;
+};
+
 int upload_opt(loom_b200_ctx* ctx, const float* host, size_t n, float** dev) {
     *dev = nullptr;
     if (!host || n == 0) return 0;
@@ -325,7 +433,8 @@ int loom_b200_dense_forward(loom_b200_ctx* ctx, const loom_b200_weight* w, int a
     float* x = ar.take<float>((size_t)batch * K);
     float* pre = ar.take<float>((size_t)batch * N);
     float* post = ar.take<float>((size_t)batch * N);
-    LB_CUDA(ctx, cudaMemcpyAsync(x, in_host, (size_t)batch * K * 4, cudaMemcpyHostToDevice, ctx->stream));
+    HostRows rows(ctx);
+    if (int rc = rows.send(x, in_host, (size_t)batch * K)) return rc;
     const int chunk = lb_pass_tokens(ctx, K);
     // a block of tokens is a dense contraction: tensor cores (tcgen05) from kGemmMinTokens on, the GEMV below it
     if (batch >= kGemmMinTokens) {
@@ -346,10 +455,8 @@ int loom_b200_dense_forward(loom_b200_ctx* ctx, const loom_b200_weight* w, int a
         if (int rc = lb_gemv_finalize_params(ctx, p)) return rc;
         if (int rc = lb_launch_gemv(ctx, p)) return rc;
     }
-    if (pre_host) LB_CUDA(ctx, cudaMemcpyAsync(pre_host, pre, (size_t)batch * N * 4, cudaMemcpyDeviceToHost, ctx->stream));
-    if (post_host) LB_CUDA(ctx, cudaMemcpyAsync(post_host, post, (size_t)batch * N * 4, cudaMemcpyDeviceToHost, ctx->stream));
-    LB_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
-    return 0;
+    const HostPart parts[2] = {{pre, pre_host, (size_t)batch * N}, {post, post_host, (size_t)batch * N}};
+    return rows.fetch(parts);
 }
 
 int loom_b200_swiglu_forward(loom_b200_ctx* ctx, const loom_b200_weight* gate, const loom_b200_weight* up,
@@ -377,14 +484,12 @@ int loom_b200_swiglu_forward(loom_b200_ctx* ctx, const loom_b200_weight* gate, c
     float* bu = bias_up ? ar.take<float>(I) : nullptr;
     float* iw = inner_norm_len > 0 ? ar.take<float>(inner_norm_len) : nullptr;
     float* bd = bias_down ? ar.take<float>(H) : nullptr;
-    auto h2d = [&](float* d, const float* h, size_t n) {
-        return d ? cudaMemcpyAsync(d, h, n * 4, cudaMemcpyHostToDevice, ctx->stream) : cudaSuccess;
-    };
-    LB_CUDA(ctx, h2d(x, in_host, (size_t)seq * H));
-    LB_CUDA(ctx, h2d(bg, bias_gate, I));
-    LB_CUDA(ctx, h2d(bu, bias_up, I));
-    LB_CUDA(ctx, h2d(bd, bias_down, H));
-    LB_CUDA(ctx, h2d(iw, inner_norm_w, inner_norm_len));
+    HostRows rows(ctx);
+    if (int rc = rows.send(x, in_host, (size_t)seq * H)) return rc;
+    if (int rc = rows.send(bg, bias_gate, I)) return rc;
+    if (int rc = rows.send(bu, bias_up, I)) return rc;
+    if (int rc = rows.send(bd, bias_down, H)) return rc;
+    if (int rc = rows.send(iw, inner_norm_w, inner_norm_len)) return rc;
     const int sw_chunk = lb_pass_tokens(ctx, I > H ? I : H);
     for (int s0 = 0; s0 < seq; s0 += sw_chunk) {
         LbSwigluArgs a = {};
@@ -406,10 +511,8 @@ int loom_b200_swiglu_forward(loom_b200_ctx* ctx, const loom_b200_weight* gate, c
         a.M = seq - s0 < sw_chunk ? seq - s0 : sw_chunk;
         if (int rc = lb_swiglu_dev(ctx, a)) return rc;
     }
-    if (pre_host) LB_CUDA(ctx, cudaMemcpyAsync(pre_host, pre, (size_t)seq * I * 4, cudaMemcpyDeviceToHost, ctx->stream));
-    if (post_host) LB_CUDA(ctx, cudaMemcpyAsync(post_host, out, (size_t)seq * H * 4, cudaMemcpyDeviceToHost, ctx->stream));
-    LB_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
-    return 0;
+    const HostPart parts[2] = {{pre, pre_host, (size_t)seq * I}, {out, post_host, (size_t)seq * H}};
+    return rows.fetch(parts);
 }
 
 int loom_b200_mha_create(loom_b200_ctx* ctx, int d_model, int num_heads, int num_kv_heads, int head_dim,
@@ -508,9 +611,9 @@ int loom_b200_mha_forward(loom_b200_mha* m, const float* in_host, int batch, int
     float* x = ar.take<float>((size_t)total * D);
     float* pre = ar.take<float>((size_t)total * D);
     float* post = ar.take<float>((size_t)total * D);
-    LB_CUDA(ctx, cudaMemcpyAsync(x, in_host, (size_t)total * D * 4, cudaMemcpyHostToDevice, ctx->stream));
-    LB_CUDA(ctx, cudaMemcpyAsync(m->pos_dev, &m->kv_offset, sizeof(int), cudaMemcpyHostToDevice, ctx->stream));
-    LB_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
+    HostRows rows(ctx);
+    if (int rc = rows.send(x, in_host, (size_t)total * D)) return rc;
+    if (int rc = lb_launch_set_scalar(ctx, m->pos_dev, m->kv_offset)) return rc;
     const int widest = m->q_dim > D ? m->q_dim : D;
     const int mh_chunk = lb_pass_tokens(ctx, widest);
     for (int s0 = 0; s0 < total; s0 += mh_chunk) {
@@ -525,10 +628,8 @@ int loom_b200_mha_forward(loom_b200_mha* m, const float* in_host, int batch, int
         if (int rc = lb_launch_add_scalar(ctx, m->pos_dev, a.M)) return rc;
     }
     m->kv_offset += total;
-    if (pre_host) LB_CUDA(ctx, cudaMemcpyAsync(pre_host, pre, (size_t)total * D * 4, cudaMemcpyDeviceToHost, ctx->stream));
-    if (post_host) LB_CUDA(ctx, cudaMemcpyAsync(post_host, post, (size_t)total * D * 4, cudaMemcpyDeviceToHost, ctx->stream));
-    LB_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
-    return 0;
+    const HostPart parts[2] = {{pre, pre_host, (size_t)total * D}, {post, post_host, (size_t)total * D}};
+    return rows.fetch(parts);
 }
 
 int loom_b200_mha_download_cache(loom_b200_mha* m, float* k_host, float* v_host) {
