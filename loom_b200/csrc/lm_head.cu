@@ -225,16 +225,19 @@ __global__ void __launch_bounds__(NW * 32, 1) lb_lm_head_stream_kernel(const LbL
 // A pass of up to eight rows is a product of the table with an [H, 8] matrix in float64: eight table rows x four columns against
 // four columns x eight hidden rows is one m8n8k4 MMA.  A warp holds 32 table rows (four MMA tiles) so that a hidden value is
 // converted to float64 once per 32 rows; lane (g, t) takes 16 bytes of row g, columns 4t.. of a 16-column step, for the table
-// (global memory, straight into registers, two steps ahead) and for the hidden rows (shared memory, float32: they are float32
+// (global memory, straight into registers, three steps ahead) and for the hidden rows (shared memory, float32: they are float32
 // values by definition) alike, so which column an MMA calls its k-th is the same for both and needs no shuffle.  Four warps share
 // a strip of 32 rows by columns and add up in shared memory: 867 rows of a CTA's share are 28 strips for four groups.
-// Bound: float64 issue (8 x 4096 columns, 128256 rows: 0.24 ms of MMAs, and the conversions to float64 share their pipe, 0.15 ms);
-// HBM alone would be 0.29 ms.  Measured 0.40 ms for eight rows where four passes of two rows on plain FMAs took 1.88 ms.
+// Bound: the table's way from HBM.  A load takes 64 bytes each of eight rows 16 KB apart, and DRAM pays for every page it opens for so
+// little; so a load asks L2 for the 256 bytes around it.  128256 rows x 4096 columns, eight hidden rows, us: without that 500 (606 with
+// the MMAs left out, 274 with the loads left out: the MMAs are 240), with it 446, three steps ahead instead of two 432; fewer rows and more
+// columns of each a step 570 to 670, explicit prefetches of 256 to 1024 bytes a row 505 to 657, CTAs that start at different columns 530.
+// HBM alone would be 300.  (Conversions to float64 run beside the MMAs.)
 constexpr int kHmWarps = 16, kHmSplit = 4, kHmGroups = kHmWarps / kHmSplit, kHmTiles = 4, kHmRows = 8 * kHmTiles;
 
 __device__ __forceinline__ float4 ldg_table(const float* p, uint64_t policy) {
     float4 v;
-    asm volatile("ld.global.nc.L1::no_allocate.L2::cache_hint.v4.f32 {%0,%1,%2,%3}, [%4], %5;" : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "l"(p), "l"(policy));
+    asm volatile("ld.global.nc.L1::no_allocate.L2::cache_hint.L2::256B.v4.f32 {%0,%1,%2,%3}, [%4], %5;" : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "l"(p), "l"(policy));
     return v;
 }
 
@@ -260,7 +263,7 @@ __global__ void __launch_bounds__(kHmWarps * 32, 1) lb_lm_head_rows_kernel(const
             w[i] = col < H ? ldg_table(p.head + (size_t)(r < r1 ? r : r1 - 1) * H + col, policy) : make_float4(0.f, 0.f, 0.f, 0.f);
         }
     };
-    constexpr int kAhead = 2;
+    constexpr int kAhead = 3;
     float4 ring[kAhead][kHmTiles];
     lb_pdl_launch_dependents();
     int row = r0 + group * kHmRows;
