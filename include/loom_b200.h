@@ -335,7 +335,7 @@ int loom_b200_decoder_continue(loom_b200_decoder* dec, int steps);
  * of one sequence (poly/mha.go:258-270, poly/mha_layout.go:62-70), so "batch 16" there means sixteen positions, not
  * sixteen sequences.  Serving several sequences at once is therefore an extension, defined by its oracle: the result
  * for every sequence is that of a decoder of its own fed the same tokens.  `batch` KV rings per block share the
- * weights; a decode step carries up to eight sequences per pass over every packed matrix (the M dimension of the
+ * weights; a decode step carries up to 24 sequences per pass over every packed matrix (eight in tensor-parallel groups; the M dimension of the
  * GEMV) and several hidden rows per pass over the LM head.  One GPU, or a tensor-parallel group with the peer
  * mailboxes attached and a vocabulary that divides by the group (the sharded head's tail then exchanges the ranks'
  * (maximum, index) pairs).

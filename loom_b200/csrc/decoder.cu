@@ -1199,9 +1199,9 @@ int loom_b200_decoder_step_batch(loom_b200_decoder* dec, const int32_t* tokens, 
         for (int i = 0; i < B; ++i) dec->h_tok_all[i] = tokens[i];
         LB_CUDA(ctx, cudaMemcpyAsync(dec->tok_all, dec->h_tok_all, (size_t)B * sizeof(int), cudaMemcpyHostToDevice, ctx->stream));
     }
-    // with the whole vocabulary on this GPU the rows that a pass over the head has made cross to the host beside the passes after it (16
-    // sequences: 34.9 ms for eight steps with one copy at the end, 28.4 so at the time); one pass has nothing to cross beside (eight rows of 16 KB:
-    // 71 us a step with a copy in the step's own stream, 81 so)
+    // with the whole vocabulary on this GPU the rows that a pass over the head has made cross to the host beside the passes after it
+    // (16 sequences, eight steps, with slower products than now: 34.9 ms with one copy at the end, 28.4 so); one pass has nothing to cross
+    // beside (eight rows of 16 KB: 71 us a step with a copy in the step's own stream, 81 so)
     const bool beside = logits_host && B > kChunkTokens && !dec->head_sharded;
     int parts = 0, done = 0, ends[kReadEvents];
     const auto rows_done = [&](int rows) -> int {

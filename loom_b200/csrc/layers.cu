@@ -321,8 +321,8 @@ public:
     // rows to dev; `host` may be changed afterwards unless CUDA knows it
     int send(float* dev, const float* host, size_t n) {
         if (!dev || n == 0) return 0;
-        if (int rc = ready()) return rc;
-        if (known(host)) {
+        open_ = true;
+        if (!slots() || known(host)) {
             LB_CUDA(ctx_, cudaMemcpyAsync(dev, host, n * 4, cudaMemcpyHostToDevice, ctx_->stream));
             return 0;
         }
@@ -337,12 +337,12 @@ public:
     }
     // both results (host side null: not asked for), behind the work queued so far; returns when they are there
     int fetch(const HostPart (&parts)[2]) {
-        if (int rc = ready()) return rc;
+        open_ = true;
         size_t pieces[2] = {};
         bool direct = false;
         for (int i = 0; i < 2; ++i) {
             const HostPart& p = parts[i];
-            if (p.host && !known(p.host))
+            if (p.host && slots() && !known(p.host))
                 pieces[i] = (p.n * 4 + kSlotBytes - 1) / kSlotBytes;
             else if (p.host) {
                 direct = true;
@@ -391,13 +391,17 @@ private:
         return where.type != cudaMemoryTypeUnregistered;
     }
     char* slot(size_t i) const { return ctx_->stage_host + i % kStageSlots * kSlotBytes; }
-    int ready() {
-        open_ = true;
-        if (ctx_->stage_host) return 0;
-        for (cudaEvent_t& e : ctx_->stage_done)
-            if (!e) LB_CUDA(ctx_, cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
-        LB_CUDA(ctx_, cudaMallocHost((void**)&ctx_->stage_host, kStageSlots * kSlotBytes));
-        return 0;
+    // false where there is no pinned memory left: rows then go as they are
+    bool slots() {
+        if (ctx_->stage_host) return true;
+        cudaError_t e = cudaSuccess;
+        for (cudaEvent_t& done : ctx_->stage_done)
+            if (!done && e == cudaSuccess) e = cudaEventCreateWithFlags(&done, cudaEventDisableTiming);
+        if (e == cudaSuccess) e = cudaMallocHost((void**)&ctx_->stage_host, kStageSlots * kSlotBytes);
+        if (e == cudaSuccess) return true;
+        (void)cudaGetLastError();
+        ctx_->stage_host = nullptr;
+        return false;
     }
     loom_b200_ctx* ctx_;
     size_t sent_ = 0;
