@@ -8,8 +8,8 @@
 // epilogue warps drain tile i while tile i + 1 accumulates.  Tokens are the M side, so a thread of the epilogue owns a
 // token and eight consecutive output columns of it are one 16-byte chunk of the next product's input image.
 // N, a tile's columns, is any multiple of 16 up to 256 (gate and up side by side: up to 128 of each): plan() takes what makes the
-// busiest CTA finish first.  Few tiles are split over K by the CTAs of a cluster, whose sums meet in distributed shared memory in the
-// order of K.  Routed experts: the token blocks of the image
+// busiest CTA finish first.  One accumulator takes all of K, so that an output's bits depend on its row of X and its row of W alone.
+// Routed experts: the token blocks of the image
 // are grouped by expert and a table names each block's expert; the number of blocks in use is read on the device.
 // Every mbarrier wait is bounded; on expiry the kernel raises the context's status word, frees its tensor memory and returns.
 #include "dense.cuh"
@@ -24,13 +24,9 @@ constexpr int kRing = 200 * 1024, kMaxStages = 8;
 constexpr size_t kSmem = kRing + 1024;
 
 struct Plan {
-    int n, split, row_tiles;  // columns of a tile (of each matrix), CTAs that share a tile, tiles over the rows of W
+    int n, row_tiles;  // columns of a tile (of each matrix), tiles over the rows of W
 };
 __host__ __device__ __forceinline__ int stage_bytes(int cols) { return kImgBlock + cols * 128; }  // cols: of both matrices
-
-__device__ __forceinline__ void st_peer4(uint32_t addr, const float* f) {
-    asm volatile("st.shared::cluster.v4.f32 [%0], {%1, %2, %3, %4};" ::"r"(addr), "f"(f[0]), "f"(f[1]), "f"(f[2]), "f"(f[3]) : "memory");
-}
 
 // RESID: sixteen columns of a token's residual row from column r on
 __device__ __forceinline__ void load_residual(const LbDenseGemm& p, int tok, int r, float4 (&x)[4]) {
@@ -92,7 +88,7 @@ __global__ void __launch_bounds__(kThreads, 1) lb_gemm_bf16_kernel(const LbDense
     __shared__ uint32_t tmem_base_s;
     __shared__ int s_failed;
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-    const int n = plan.n, cols = kDual ? 2 * n : n, row_tiles = plan.row_tiles, S = plan.split;
+    const int n = plan.n, cols = kDual ? 2 * n : n, row_tiles = plan.row_tiles;
     const int stage = stage_bytes(cols), stages = kRing / stage < kMaxStages ? kRing / stage : kMaxStages;
     const int padded_rows = lb_round_up(p.rows, kImgRows);
 
@@ -117,10 +113,8 @@ __global__ void __launch_bounds__(kThreads, 1) lb_gemm_bf16_kernel(const LbDense
     lb_pdl_wait();
     const int nblocks = p.nblocks ? *p.nblocks : lb_ceil_div(p.tokens, kImgRows);
     const int ntiles = nblocks * row_tiles;
-    // S > 1: the cluster's tile, this CTA's slices of it; else every gridDim.x-th tile
-    const int rank = S > 1 ? (int)lb_cluster_rank() : 0, first_tile = (int)blockIdx.x / S, tile_step = (int)gridDim.x / S;
-    const int my_tiles = first_tile < ntiles ? (S > 1 ? 1 : (ntiles - first_tile + tile_step - 1) / tile_step) : 0;
-    const int ks0 = p.slices * rank / S, ks1 = p.slices * (rank + 1) / S;
+    const int first_tile = (int)blockIdx.x, tile_step = (int)gridDim.x;
+    const int my_tiles = first_tile < ntiles ? (ntiles - first_tile + tile_step - 1) / tile_step : 0;
 
     if (warp == kRowsWarp || warp == kWeightsWarp) {
         if (lb_elect()) {
@@ -129,11 +123,11 @@ __global__ void __launch_bounds__(kThreads, 1) lb_gemm_bf16_kernel(const LbDense
             uint32_t parity = 1;  // (the first round's waits are over at once)
             for (int i = 0; i < my_tiles && !failed; ++i) {
                 const int t = first_tile + i * tile_step, rt = t % row_tiles, tb = t / row_tiles;
-                const uint8_t* xb = p.x + ((size_t)tb * p.slices + ks0) * kImgBlock;
+                const uint8_t* xb = p.x + (size_t)tb * p.slices * kImgBlock;
                 // the tile's rows of W: pieces of up to three blocks of 128
                 const size_t goff = p.block_group ? (size_t)p.block_group[tb] * p.group_bytes : 0;
                 const int r0 = rt * n, rows = padded_rows - r0 < n ? padded_rows - r0 : n;
-                for (int ks = ks0; ks < ks1; ++ks) {
+                for (int ks = 0; ks < p.slices; ++ks) {
                     if (!lb_mbar_wait_bounded(&empty_bar[s], parity, kTcWaitLimit)) {
                         failed = true;
                         break;
@@ -176,7 +170,7 @@ __global__ void __launch_bounds__(kThreads, 1) lb_gemm_bf16_kernel(const LbDense
                 }
                 lb_tc_fence_after();
                 const uint32_t d = tmem_base + (uint32_t)(buf * 256);
-                for (int ks = ks0; ks < ks1; ++ks) {
+                for (int ks = 0; ks < p.slices; ++ks) {
                     if (!lb_mbar_wait_bounded(&load_bar[s], parity, kTcWaitLimit)) {
                         failed = true;
                         break;
@@ -184,7 +178,7 @@ __global__ void __launch_bounds__(kThreads, 1) lb_gemm_bf16_kernel(const LbDense
                     lb_tc_fence_after();
                     const uint64_t a = lb_smem_desc(lb_smem_u32(smem + (size_t)s * stage), 128, 1024), b = a + (kImgBlock >> 4);
 #pragma unroll
-                    for (int k = 0; k < 4; ++k) lb_mma_f16(d, a + k * 16, b + k * 16, idesc, (ks > ks0 || k > 0) ? 1u : 0u);
+                    for (int k = 0; k < 4; ++k) lb_mma_f16(d, a + k * 16, b + k * 16, idesc, (ks > 0 || k > 0) ? 1u : 0u);
                     lb_mma_commit(&empty_bar[s]);
                     if (++s == stages) {
                         s = 0;
@@ -209,7 +203,7 @@ __global__ void __launch_bounds__(kThreads, 1) lb_gemm_bf16_kernel(const LbDense
             // RESID: the residual's columns are asked for sixteen ahead, the first ones and the rest's way into L2 while the sums are made (a
             // read behind every accumulator: 2048 x 2560 x 6912 in tiles of 144 took 97 us, 78 so)
             float4 next[4] = {};
-            if (EPI == LB_DEPI_RESID && S == 1 && tok_ok) {
+            if (EPI == LB_DEPI_RESID && tok_ok) {
                 load_residual(p, tok, rt * n + half * 16, next);
                 for (int c = half * 32; c < n; c += 64)
                     if (rt * n + c < p.ldo) asm volatile("prefetch.global.L2 [%0];" ::"l"(p.out + (size_t)tok * p.ldo + rt * n + c));
@@ -220,7 +214,6 @@ __global__ void __launch_bounds__(kThreads, 1) lb_gemm_bf16_kernel(const LbDense
                 break;
             }
             lb_tc_fence_after();
-            if (S > 1) break;  // the sums of the other CTAs first
             const uint32_t tacc = tmem_base + (uint32_t)(buf * 256) + ((uint32_t)(quarter * 32) << 16);
 #pragma unroll 1
             for (int c0 = half * 16; c0 < n; c0 += 32) {
@@ -243,61 +236,6 @@ __global__ void __launch_bounds__(kThreads, 1) lb_gemm_bf16_kernel(const LbDense
             if (lane == 0) lb_mbar_arrive(&acc_empty[buf]);
         }
     }
-    if (S > 1) {
-        // Sixteen columns belong to CTA (column / 16) % S: the others write their sums of them into its pipeline buffers, once all of the
-        // cluster's MMAs are done, [source][group of the owner][token][16 + 4 floats]
-        __syncwarp();
-        lb_cluster_sync();
-        constexpr int kLd = 20, kMats = kDual ? 2 : 1;
-        const int groups = n / 16, slots = lb_ceil_div(groups, S);  // 16-column groups of a matrix; of an owner
-        const int lane_row = quarter * 32 + lane;
-        const uint32_t base = lb_smem_u32(smem), tacc = tmem_base + ((uint32_t)(quarter * 32) << 16);
-        const bool work = warp < kMmaWarp && my_tiles > 0;
-        if (work)
-            for (int c = half; c < groups; c += 2) {
-                const int owner = c % S;
-                if (owner == rank) continue;
-#pragma unroll
-                for (int m = 0; m < kMats; ++m) {
-                    float v[16];
-                    lb_tmem_ld16(tacc + (uint32_t)(m * n + c * 16), v);
-                    lb_tmem_wait_ld();
-                    const uint32_t to = lb_cluster_addr(base + (uint32_t)((((rank * slots + c / S) * kMats + m) * 128 + lane_row) * kLd * 4), (uint32_t)owner);
-#pragma unroll
-                    for (int e = 0; e < 16; e += 4) st_peer4(to + e * 4, v + e);
-                }
-            }
-        __syncwarp();
-        lb_cluster_sync();
-        if (work) {
-            const int rt = first_tile % row_tiles, tb = first_tile / row_tiles, tok = tb * kImgRows + lane_row;
-            const bool tok_ok = p.nblocks || tok < p.tokens;
-            for (int c = rank + S * half; c < groups; c += 2 * S) {
-                float own[kMats][16], sum[kMats][16];
-                float4 res[4] = {};
-                if (EPI == LB_DEPI_RESID && tok_ok) load_residual(p, tok, rt * n + c * 16, res);
-#pragma unroll
-                for (int m = 0; m < kMats; ++m) {
-                    lb_tmem_ld16(tacc + (uint32_t)(m * n + c * 16), own[m]);
-#pragma unroll
-                    for (int e = 0; e < 16; ++e) sum[m][e] = 0.f;
-                }
-                lb_tmem_wait_ld();
-                for (int q = 0; q < S; ++q) {
-#pragma unroll
-                    for (int m = 0; m < kMats; ++m) {
-                        const float* from = reinterpret_cast<const float*>(smem) + (size_t)(((q * slots + c / S) * kMats + m) * 128 + lane_row) * kLd;
-#pragma unroll
-                        for (int e = 0; e < 16; ++e) sum[m][e] += q == rank ? own[m][e] : from[e];
-                    }
-                }
-                if (tok_ok && !s_failed)
-#pragma unroll
-                    for (int h = 0; h < 16; h += 8) emit8<EPI>(p, tok, rt * n + c * 16 + h, sum[0] + h, sum[kMats - 1] + h, res + h / 4);
-            }
-        }
-        lb_tc_fence_before();
-    }
     __syncthreads();
     if (warp == kMmaWarp) {
         lb_tc_fence_after();
@@ -306,11 +244,12 @@ __global__ void __launch_bounds__(kThreads, 1) lb_gemm_bf16_kernel(const LbDense
     if (tid == 0 && s_failed) atomicExch(p.status, 3);
 }
 
-// Columns of a tile and CTAs that share one.  Measured with every SM at work: a slice takes 0.32 us with up to 128 columns (both
-// matrices together), 0.355 with 144, 0.40 with 192 and 0.46 with 256; meeting in a cluster 3 us, an epilogue behind the last MMA 0.015 us
-// a column.  Wide tiles leave a last wave of few of them: 2048 x 2560 x 6912 takes 96 us as 160 tiles of 256, 83 as 224 of 192 and 78
-// as 288 of 144 (100 before residual rows were asked for ahead); 2048 x 7696 x 2560 78 us with 256, 75 with 224, 84 with 144.  100
-// tokens x 2560 x 6912 are 20 tiles: 43 us, 25 shared by four CTAs each.
+// Columns of a tile.  Measured with every SM at work: a slice takes 0.32 us with up to 128 columns (both matrices together), 0.355 with
+// 144, 0.40 with 192 and 0.46 with 256; an epilogue behind the last MMA 0.015 us a column.  Wide tiles leave a last wave of few of them:
+// 2048 x 2560 x 6912 takes 96 us as 160 tiles of 256, 83 as 224 of 192 and 78 as 288 of 144 (100 before residual rows were asked for
+// ahead); 2048 x 7696 x 2560 78 us with 256, 75 with 224, 84 with 144.
+// (Few tiles split over K by the CTAs of a cluster were quicker, 100 tokens x 2560 x 6912 25 us for 43, but sums of parts are other bits
+// than one accumulator's, and a token's result then depends on how many others are in its block.)
 Plan plan(const loom_b200_ctx* ctx, const LbDenseGemm& p, bool dual) {
     const int blocks = p.nblocks ? p.max_blocks : lb_ceil_div(p.tokens, kImgRows), most = dual ? 128 : 256, rows = lb_round_up(p.rows, kImgRows);  // (the padding's zeros too)
     Plan best = {};
@@ -318,15 +257,10 @@ Plan plan(const loom_b200_ctx* ctx, const LbDenseGemm& p, bool dual) {
     for (int n = most < rows ? most : rows; n >= 48; n -= 16) {
         const int tiles = lb_ceil_div(rows, n) * blocks, cols = dual ? 2 * n : n;
         const double slice = cols <= 106 ? 0.32 : 0.22 + cols * 0.00094;
-        for (int S = 1; S <= 8; S *= 2) {
-            // clusters of whole SMs: what the groups of SMs hold of them
-            if (S > 1 && (tiles * S > ctx->sm_count - 5 * S || p.slices < 4 * S)) break;
-            const int waves = S > 1 ? 1 : lb_ceil_div(tiles, ctx->sm_count);
-            const double us = waves * lb_ceil_div(p.slices, S) * slice + (S > 1 ? 3.0 : 0.0) + cols * 0.015 / S;
-            if (us < 0.98 * best_us) {
-                best_us = us;
-                best = {n, S, lb_ceil_div(rows, n)};
-            }
+        const double us = lb_ceil_div(tiles, ctx->sm_count) * p.slices * slice + cols * 0.015;
+        if (us < 0.98 * best_us) {
+            best_us = us;
+            best = {n, lb_ceil_div(rows, n)};
         }
     }
     return best;
@@ -338,21 +272,7 @@ int launch(loom_b200_ctx* ctx, const LbDenseGemm& p) {
     const Plan pl = plan(ctx, p, kDual);
     const int blocks = p.nblocks ? p.max_blocks : lb_ceil_div(p.tokens, kImgRows), tiles = pl.row_tiles * blocks;
     LB_BIG_SMEM(ctx, lb_gemm_bf16_kernel<EPI>, kSmem);
-    cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3(pl.split > 1 ? tiles * pl.split : tiles < ctx->sm_count ? tiles : ctx->sm_count);
-    cfg.blockDim = dim3(kThreads);
-    cfg.dynamicSmemBytes = kSmem;
-    cfg.stream = ctx->stream;
-    cudaLaunchAttribute attr[2];
-    attr[0].id = cudaLaunchAttributeClusterDimension;
-    attr[0].val.clusterDim.x = (unsigned)pl.split;
-    attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
-    attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    attr[1].val.programmaticStreamSerializationAllowed = 1;
-    cfg.attrs = attr;
-    cfg.numAttrs = ctx->opt_pdl ? 2 : 1;
-    LB_CUDA(ctx, cudaLaunchKernelEx(&cfg, lb_gemm_bf16_kernel<EPI>, p, pl));
-    ctx->launches++;
+    LB_LAUNCH(ctx, lb_gemm_bf16_kernel<EPI>, dim3(tiles < ctx->sm_count ? tiles : ctx->sm_count), dim3(kThreads), kSmem, p, pl);
     return 0;
 }
 
