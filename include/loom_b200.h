@@ -89,7 +89,8 @@ int loom_b200_selftest_wait_timeout(loom_b200_ctx* ctx, unsigned int polls);
  * ForwardTokenIDsWGPU, poly/wgpu_forward.go:99,564): the dispatches issued between begin and end are
  * recorded into a CUDA graph instead of running; graph_launch replays them with one submission.
  * Run the same dispatches once before graph_begin so that every scratch buffer already has its size;
- * allocation, upload, download and sync are refused while recording. */
+ * allocation, upload, download and sync are refused while recording.  Later calls may need larger scratch than a
+ * recorded frame: what the frame uses stays allocated until the context's last frame has been freed. */
 int loom_b200_graph_begin(loom_b200_ctx* ctx);
 int loom_b200_graph_end(loom_b200_ctx* ctx, loom_b200_graph** out);
 int loom_b200_graph_launch(loom_b200_ctx* ctx, loom_b200_graph* graph);

@@ -35,48 +35,51 @@ struct loom_b200_graph {
     cudaGraphExec_t exec = nullptr;
 };
 
+// a buffer that recorded frames may hold the address of
+static void let_go(loom_b200_ctx* ctx, void* p) {
+    if (p && ctx->frames > 0) ctx->retired.push_back(p);
+    else if (p) cudaFree(p);
+}
+static void free_retired(loom_b200_ctx* ctx) {
+    for (void* p : ctx->retired) cudaFree(p);
+    ctx->retired.clear();
+}
+
 #define LB_NO_CAPTURE(ctx, what)                                                                               \
     do {                                                                                                       \
         if ((ctx)->capturing)                                                                                  \
             return lb_fail((ctx), LOOM_B200_ERR_INVALID, "%s is not allowed between graph_begin and graph_end", what); \
     } while (0)
 
-int lb_ensure_fixup(loom_b200_ctx* ctx, size_t acc_elems, size_t cnt_elems) {
-    if ((acc_elems > ctx->fix_acc_elems || cnt_elems > ctx->fix_cnt_elems) && ctx->capturing)
-        return lb_fail(ctx, LOOM_B200_ERR_INVALID, "scratch would grow while recording a graph: run the same calls once before graph_begin");
-    if (acc_elems > ctx->fix_acc_elems) {
-        // growing happens between launches on this stream; wait for users of the old buffer first
-        LB_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
-        if (ctx->fix_acc) cudaFree(ctx->fix_acc);
-        ctx->fix_acc = nullptr;
-        size_t n = acc_elems + acc_elems / 2;
-        LB_CUDA(ctx, cudaMalloc(&ctx->fix_acc, n * sizeof(int32_t)));
-        LB_CUDA(ctx, cudaMemsetAsync(ctx->fix_acc, 0, n * sizeof(int32_t), ctx->stream));
-        ctx->fix_acc_elems = n;
-    }
-    if (cnt_elems > ctx->fix_cnt_elems) {
-        LB_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
-        if (ctx->fix_cnt) cudaFree(ctx->fix_cnt);
-        ctx->fix_cnt = nullptr;
-        size_t n = cnt_elems + cnt_elems / 2;
-        LB_CUDA(ctx, cudaMalloc(&ctx->fix_cnt, n * sizeof(unsigned int)));
-        LB_CUDA(ctx, cudaMemsetAsync(ctx->fix_cnt, 0, n * sizeof(unsigned int), ctx->stream));
-        ctx->fix_cnt_elems = n;
-    }
+int lb_grow(loom_b200_ctx* ctx, void** buf, size_t* have, size_t need, size_t ask, const char* what) {
+    if (need <= *have) return 0;
+    if (ctx->capturing) return lb_fail(ctx, LOOM_B200_ERR_INVALID, "%s would grow while recording a graph: run the same calls once before graph_begin", what);
+    LB_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
+    let_go(ctx, *buf);
+    *buf = nullptr;
+    *have = 0;
+    LB_CUDA(ctx, cudaMalloc(buf, ask));
+    *have = ask;
     return 0;
 }
 
-int lb_ensure_scratch(loom_b200_ctx* ctx, size_t bytes) {
-    if (bytes <= ctx->scratch_bytes) return 0;
-    LB_NO_CAPTURE(ctx, "growing the scratch buffer");
-    LB_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
-    if (ctx->scratch) cudaFree(ctx->scratch);
-    ctx->scratch = nullptr;
-    ctx->scratch_bytes = 0;
-    size_t n = bytes + bytes / 4 + 4096;
-    LB_CUDA(ctx, cudaMalloc(&ctx->scratch, n));
-    ctx->scratch_bytes = n;
-    return 0;
+int lb_ensure_fixup(loom_b200_ctx* ctx, size_t acc_elems, size_t cnt_elems) {
+    const auto zeroed = [&](void** buf, size_t* have, size_t elems) -> int {
+        const size_t bytes = elems * sizeof(int32_t);
+        if (bytes <= *have) return 0;
+        if (int rc = lb_grow(ctx, buf, have, bytes, bytes + bytes / 2, "scratch")) return rc;
+        LB_CUDA(ctx, cudaMemsetAsync(*buf, 0, *have, ctx->stream));
+        return 0;
+    };
+    if (int rc = zeroed((void**)&ctx->fix_acc, &ctx->fix_acc_bytes, acc_elems)) return rc;
+    return zeroed((void**)&ctx->fix_cnt, &ctx->fix_cnt_bytes, cnt_elems);
+}
+
+int lb_ensure_scratch(loom_b200_ctx* ctx, size_t bytes) { return lb_grow(ctx, &ctx->scratch, &ctx->scratch_bytes, bytes, bytes + bytes / 4 + 4096, "the scratch buffer"); }
+
+// (twice what is asked for now: later calls with more tokens or wider rows find it large enough more often)
+int lb_ensure_quant_scratch(loom_b200_ctx* ctx, size_t bytes) {
+    return lb_grow(ctx, &ctx->quant_scratch, &ctx->quant_scratch_bytes, bytes, bytes * 2 + 4096, "the quantization scratch buffer");
 }
 
 // Faults the pages of a pageable buffer in by one call (their contents stay).  Touching them one by one -- a read, then a write -- faults a
@@ -115,20 +118,6 @@ int lb_status_result(loom_b200_ctx* ctx) {
                                  "self-test: a flag that nothing sets"};
     return lb_fail(ctx, LOOM_B200_ERR_TIMEOUT, "a bounded device-side wait ran out (%d: %s); results of the calls since the last sync are invalid",
                    code, code >= 1 && code <= 6 ? what[code] : "unknown");
-}
-
-int lb_ensure_quant_scratch(loom_b200_ctx* ctx, size_t bytes) {
-    if (bytes <= ctx->quant_scratch_bytes) return 0;
-    LB_NO_CAPTURE(ctx, "growing the quantization scratch buffer");
-    LB_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
-    if (ctx->quant_scratch) cudaFree(ctx->quant_scratch);
-    ctx->quant_scratch = nullptr;
-    ctx->quant_scratch_bytes = 0;
-    // sized for a full pass of kMaxM tokens at this width, so that later calls with more tokens find it large enough
-    size_t n = bytes * 2 + 4096;
-    LB_CUDA(ctx, cudaMalloc(&ctx->quant_scratch, n));
-    ctx->quant_scratch_bytes = n;
-    return 0;
 }
 
 // ---- re-tiling kernels -------------------------------------------------------------------------
@@ -383,7 +372,7 @@ int loom_b200_ctx_set_option(loom_b200_ctx* ctx, const char* key, int value) {
             LB_CUDA(ctx, cudaMalloc(&ctx->trace_dev, (size_t)kTraceSlots * 8 * sizeof(unsigned long long)));
             LB_CUDA(ctx, cudaMemset(ctx->trace_dev, 0, (size_t)kTraceSlots * 8 * sizeof(unsigned long long)));
         } else if (!value && ctx->trace_dev) {
-            cudaFree(ctx->trace_dev);
+            let_go(ctx, ctx->trace_dev);
             ctx->trace_dev = nullptr;
         }
     } else if (!strcmp(key, "head_stream")) {
@@ -447,6 +436,7 @@ void loom_b200_ctx_destroy(loom_b200_ctx* ctx) {
     if (ctx->gemm_scratch) cudaFree(ctx->gemm_scratch);
     if (ctx->quant_scratch) cudaFree(ctx->quant_scratch);
     if (ctx->stage_scratch) cudaFree(ctx->stage_scratch);
+    free_retired(ctx);
     if (ctx->owns_stream) cudaStreamDestroy(ctx->stream);
     delete ctx;
 }
@@ -505,6 +495,7 @@ int loom_b200_graph_end(loom_b200_ctx* ctx, loom_b200_graph** out) {
         delete gr;
         return lb_fail(ctx, LOOM_B200_ERR_CUDA, "cudaGraphInstantiate: %s", cudaGetErrorString(e));
     }
+    ctx->frames++;
     *out = gr;
     return 0;
 }
@@ -527,6 +518,7 @@ void loom_b200_graph_free(loom_b200_ctx* ctx, loom_b200_graph* graph) {
     if (graph->exec) cudaGraphExecDestroy(graph->exec);
     if (graph->graph) cudaGraphDestroy(graph->graph);
     delete graph;
+    if (ctx && --ctx->frames == 0 && !ctx->capturing) free_retired(ctx);
 }
 
 const char* loom_b200_trace_label(const loom_b200_ctx* ctx, int slot) {

@@ -9,6 +9,7 @@
 #include <cstdio>
 #include <cstring>
 #include <string>
+#include <vector>
 
 #include "../../include/loom_b200.h"
 
@@ -56,7 +57,7 @@ struct loom_b200_ctx {
     // whenever no kernel is in flight (the last arriver of every group clears what it used).
     int32_t* fix_acc = nullptr;
     unsigned int* fix_cnt = nullptr;
-    size_t fix_acc_elems = 0, fix_cnt_elems = 0;
+    size_t fix_acc_bytes = 0, fix_cnt_bytes = 0;
     // small device scratch reused by the layer-level calls
     void* scratch = nullptr;
     size_t scratch_bytes = 0;
@@ -87,6 +88,8 @@ struct loom_b200_ctx {
     int trace_seq = 0;                          // next row
     const char* trace_label[kTraceSlots] = {};  // kernel that wrote each row
     bool capturing = false;        // between graph_begin and graph_end
+    int frames = 0;                // recorded frames that have not been freed
+    std::vector<void*> retired;    // buffers that were outgrown while a recorded frame may hold their address: freed with the last frame
     // tensor parallelism (tp.cu): rank and world size of this context's group; the NCCL communicator or null
     int tp_rank = 0, tp_world = 1;
     int opt_fold_rope = 1;         // one-token decoder steps rotate q and the newest K row inside the attention kernel
@@ -115,6 +118,9 @@ struct loom_b200_ctx {
 
 int lb_fail(loom_b200_ctx* ctx, int code, const char* fmt, ...);
 const char* lb_global_error();
+// Makes *buf hold `need` bytes: waits for its users, lets it go and asks for `ask` bytes.  Refused while a frame is being recorded; while
+// recorded frames exist the old buffer stays allocated, since their kernels go on using its address.
+int lb_grow(loom_b200_ctx* ctx, void** buf, size_t* have, size_t need, size_t ask, const char* what);
 int lb_ensure_fixup(loom_b200_ctx* ctx, size_t acc_elems, size_t cnt_elems);
 int lb_ensure_scratch(loom_b200_ctx* ctx, size_t bytes);
 // Waits for the context's stream and reads the device status word with it: a bounded device-side wait that ran out

@@ -713,15 +713,7 @@ int gemv_rows(loom_b200_ctx* ctx, const LbDenseGemv& pin) {
     if (pin.M < kStageTokens) return gemv_launch<WT, PRO, EPI>(ctx, pin);
     LbDenseGemv p = pin;
     const size_t bytes = (size_t)p.slices * 8 * kMaxLanesPerPass * 16;
-    if (bytes > ctx->stage_scratch_bytes) {
-        if (ctx->capturing) return lb_fail(ctx, LOOM_B200_ERR_INVALID, "the staging buffer of the GEMV would grow while recording a graph");
-        LB_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
-        if (ctx->stage_scratch) cudaFree(ctx->stage_scratch);
-        ctx->stage_scratch = nullptr;
-        ctx->stage_scratch_bytes = 0;
-        LB_CUDA(ctx, cudaMalloc(&ctx->stage_scratch, bytes));
-        ctx->stage_scratch_bytes = bytes;
-    }
+    if (int rc = lb_grow(ctx, &ctx->stage_scratch, &ctx->stage_scratch_bytes, bytes, bytes, "the staging buffer of the GEMV")) return rc;
     p.staged = static_cast<uint4*>(ctx->stage_scratch);
     if (int rc = gemv_launch<WT, PRO, LB_DEPI_STAGE>(ctx, p)) return rc;
     return gemv_launch<WT, LB_DPRO_STAGED, EPI>(ctx, p);

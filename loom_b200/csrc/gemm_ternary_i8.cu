@@ -1214,15 +1214,8 @@ int lb_gemm_quantize(loom_b200_ctx* ctx, const LbGemmQuant& a) {
     // scratch: permuted int8 activations, amax, sum per token
     const int pt = padded_tokens(a.tokens);
     size_t need = (size_t)pt * Kp + 256 + (size_t)pt * 8 + 256;
-    if (need > ctx->gemm_scratch_bytes) {  // its own buffer: layer calls keep their tensors in ctx->scratch
-        if (ctx->capturing) return lb_fail(ctx, LOOM_B200_ERR_INVALID, "ternary_gemm: scratch would grow while recording a graph");
-        LB_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
-        if (ctx->gemm_scratch) cudaFree(ctx->gemm_scratch);
-        ctx->gemm_scratch = nullptr;
-        ctx->gemm_scratch_bytes = 0;
-        LB_CUDA(ctx, cudaMalloc(&ctx->gemm_scratch, need + need / 4));
-        ctx->gemm_scratch_bytes = need + need / 4;
-    }
+    // its own buffer: layer calls keep their tensors in ctx->scratch
+    if (int rc = lb_grow(ctx, &ctx->gemm_scratch, &ctx->gemm_scratch_bytes, need, need + need / 4, "ternary_gemm: scratch")) return rc;
     GemmScratch g = gemm_scratch_at(ctx->gemm_scratch, a.tokens, Kp);
     const int nchunks = Kp >> 4;
     // Blocks of several tokens per SM whose rows bulk copies can fetch: rows behind one another in shared memory.  A slot is a row; as

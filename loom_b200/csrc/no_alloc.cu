@@ -81,12 +81,12 @@ extern "C" int loom_b200_ternary_linear_no_alloc(loom_b200_ctx* ctx, const loom_
     // launcher has nothing to grow.  The status word stays the context's own.
     int32_t* save_acc = ctx->fix_acc;
     unsigned int* save_cnt = ctx->fix_cnt;
-    size_t save_acc_n = ctx->fix_acc_elems, save_cnt_n = ctx->fix_cnt_elems;
+    size_t save_acc_n = ctx->fix_acc_bytes, save_cnt_n = ctx->fix_cnt_bytes;
     int save_part = ctx->opt_gemv_partition;
     ctx->fix_acc = acc;
     ctx->fix_cnt = cnt;
-    ctx->fix_acc_elems = kAccInts;
-    ctx->fix_cnt_elems = kCntInts;
+    ctx->fix_acc_bytes = kAccInts * sizeof(int32_t);
+    ctx->fix_cnt_bytes = kCntInts * sizeof(unsigned int);
     ctx->opt_gemv_partition = 1;  // stream-K over tiles: the variant whose partial sums go through the scratch
     int rc = 0;
     for (int b0 = 0; b0 < batch && !rc; b0 += pass) {
@@ -111,8 +111,8 @@ extern "C" int loom_b200_ternary_linear_no_alloc(loom_b200_ctx* ctx, const loom_
     }
     ctx->fix_acc = save_acc;
     ctx->fix_cnt = save_cnt;
-    ctx->fix_acc_elems = save_acc_n;
-    ctx->fix_cnt_elems = save_cnt_n;
+    ctx->fix_acc_bytes = save_acc_n;
+    ctx->fix_cnt_bytes = save_cnt_n;
     ctx->opt_gemv_partition = save_part;
     if (rc == LOOM_B200_ERR_UNSUPPORTED)  // e.g. a shared-memory limit of the launcher: say where the caller can go instead
         ctx->last_error += " (loom_b200_ternary_linear_no_alloc; loom_b200_ternary_linear takes the same shapes)";
