@@ -68,6 +68,8 @@ struct loom_b200_ctx {
     cudaEvent_t stage_done[kStageSlots] = {};
     void* quant_scratch = nullptr;   // int8 row and absmax of the stand-alone GEMV prologue (wide inputs)
     size_t quant_scratch_bytes = 0;
+    void* tp_rows = nullptr;         // this rank's int8 slices of the rows of a row-parallel product (their GEMV may use quant_scratch)
+    size_t tp_rows_bytes = 0;
     void* stage_scratch = nullptr;   // input rows of the float GEMV for several sequences
     size_t stage_scratch_bytes = 0;
     void* gemm_scratch = nullptr;    // int8 activations, amax and sums of the tensor-core GEMM path

@@ -314,8 +314,9 @@ int lb_tp_rowsharded_linear(loom_b200_ctx* ctx, const loom_b200_weight* w, bool 
     int8_t* q8 = nullptr;
     if (peer) {
         LB_REQUIRE(ctx, (Kl & 3) == 0, "tensor-parallel shard width %d must be a multiple of 4", Kl);
-        if (int rc = lb_ensure_quant_scratch(ctx, (size_t)kChunkTokens * Kl + 256)) return rc;
-        q8 = reinterpret_cast<int8_t*>(ctx->quant_scratch);
+        const size_t bytes = (size_t)kChunkTokens * Kl;
+        if (int rc = lb_grow(ctx, &ctx->tp_rows, &ctx->tp_rows_bytes, bytes, bytes * 2, "the rows of a row-parallel product")) return rc;
+        q8 = static_cast<int8_t*>(ctx->tp_rows);
         void* const* peers = (void* const*)ctx->peer_xbuf_dev;
         if (x_is_f64)
             lb_tp_stats_peer_kernel<double><<<M, kStatThreads, 0, ctx->stream>>>((const double*)x, Kl, K_global, eps, inner_w, inner_w ? inner_w_len : 0,

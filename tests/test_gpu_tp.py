@@ -1,6 +1,8 @@
 """Tensor parallelism on the GPU.  The one-GPU cases run the row-sharded path with a group of one (no exchange,
-but the supplied-statistics prologue, the raw-accumulator epilogue and the finalize kernel); the multi-GPU case
+but the supplied-statistics prologue, the raw-accumulator epilogue and the finalize kernel) and as rank 0 of a pair whose second rank is
+played by messages that lie in the mailbox beforehand; the multi-GPU case
 needs at least two GPUs and runs one process per GPU against the unsharded CPU oracle."""
+import ctypes as C
 import os
 import socket
 import subprocess
@@ -9,8 +11,10 @@ import sys
 import numpy as np
 import pytest
 
+import harness
 from loom_b200 import cabi
 from oracle import oracle as orc
+from refkit import np_unpack
 
 pytestmark = pytest.mark.gpu
 HERE = os.path.dirname(os.path.abspath(__file__))
@@ -48,6 +52,49 @@ def test_rowsharded_linear_group_of_one(rows, K, batch, with_inner):
     with pytest.raises(cabi.LoomB200Error):
         ctx.tp_rowsharded_linear(w, 1, d_x, K - 16, d_out)  # whole vector narrower than the slice
     ctx.close()
+
+
+@pytest.mark.parametrize("fused", [0, 1])
+def test_rowsharded_linear_of_rank_0_of_two(fused):
+    """Three and eight tokens through the peer exchange on one GPU: the second rank's sums lie in the mailbox before the first rank asks for
+    them.  Twice each, behind narrower and wider shards on one context; bit for bit."""
+    ctx = cabi.Context(0)
+    other = C.c_void_p()
+    ctx._check(harness.lib().t_pair_begin(ctx.h, C.byref(other)))
+    ctx.set_option("tp_fused", fused)
+    seq = 0
+    try:
+        for rows, Kl, batch in ((96, 256, 3), (96, 256, 8), (2560, 4096, 8), (130, 1040, 3), (300, 4096, 5), (96, 256, 8), (64, 640, 1)):
+            rng = np.random.default_rng(rows + Kl + batch)
+            K = 2 * Kl
+            full = (rng.standard_normal((rows, K)) * 0.05).astype(np.float32)
+            words, scale = orc.pack_f32(full.reshape(-1), rows, K)
+            codes = np_unpack(words, rows, K)
+            shard = np.ascontiguousarray(words.reshape(rows, -1)[:, :Kl // 16])
+            w = ctx.upload_ternary(shard, rows, Kl, scale)
+            inner, bias = (1 + 0.1 * rng.standard_normal(K)).astype(np.float32), (0.01 * rng.standard_normal(rows)).astype(np.float32)
+            d_in, d_b, d_out = ctx.to_device(inner[:Kl]), ctx.to_device(bias), ctx.alloc(batch * rows * 4)
+            for _ in range(2):
+                seq += 1
+                x = rng.standard_normal((batch, K)).astype(np.float32)
+                y = np.stack([orc.inner_rmsnorm_f32(r, inner, 0.0) for r in x])
+                q, amax = orc.quantize_rows_f32(y)
+                acc = q.astype(np.int32) @ codes.astype(np.int32).T
+                theirs = np.ascontiguousarray(q[:, Kl:].astype(np.int32) @ codes[:, Kl:].astype(np.int32).T)
+                ss, top = (x[:, Kl:].astype(np.float64) ** 2).sum(1), np.ascontiguousarray(np.abs(y[:, Kl:]).max(1))
+                ctx._check(harness.lib().t_pair_message(ctx.h, seq, batch, ss.ctypes.data, top.ctypes.data, theirs.ctypes.data, theirs.size))
+                d_x = ctx.to_device(np.ascontiguousarray(x[:, :Kl]))
+                ctx.tp_rowsharded_linear(w, batch, d_x, K, d_out, inner_w=d_in, inner_w_len=Kl, eps=0.0, bias=d_b)
+                got = ctx.download(d_out, (batch, rows), np.float32)
+                ctx.sync()
+                want = (acc * (np.float64(scale) * amax.astype(np.float64) / 127.0)[:, None] + bias.astype(np.float64)).astype(np.float32)
+                assert np.array_equal(got, want)
+                ctx.free(d_x)
+            for p in (d_in, d_b, d_out):
+                ctx.free(p)
+    finally:
+        harness.lib().t_pair_end(ctx.h, other)
+        ctx.close()
 
 
 def test_decoder_refuses_dimensions_that_do_not_divide():
