@@ -10,6 +10,7 @@ namespace {
 
 std::mutex g_err_mu;
 std::string g_global_error;  // errors raised without a context (ctx_create)
+std::atomic<int> g_contexts{0};
 
 }  // namespace
 
@@ -347,6 +348,7 @@ int loom_b200_ctx_create(int device, void* stream, loom_b200_ctx** out) {
     if (const char* v = getenv("LOOM_B200_GEMV_VARIANT")) ctx->opt_gemv_variant = atoi(v) == 1 ? 1 : 0;
     if (const char* v = getenv("LOOM_B200_GEMV_CTAS_PER_SM")) ctx->opt_gemv_ctas_per_sm = atoi(v) > 0 ? atoi(v) : 2;
     if (const char* v = getenv("LOOM_B200_PDL")) ctx->opt_pdl = atoi(v) != 0;
+    ++g_contexts;
     *out = ctx;
     return 0;
 }
@@ -427,9 +429,6 @@ void loom_b200_ctx_destroy(loom_b200_ctx* ctx) {
     if (ctx->scratch) cudaFree(ctx->scratch);
     if (ctx->status_dev) cudaFree(ctx->status_dev);
     if (ctx->status_host) cudaFreeHost(ctx->status_host);
-    if (ctx->stage_host) cudaFreeHost(ctx->stage_host);
-    for (cudaEvent_t e : ctx->stage_done)
-        if (e) cudaEventDestroy(e);
     if (ctx->trace_dev) cudaFree(ctx->trace_dev);
     if (ctx->argmax_scratch) cudaFree(ctx->argmax_scratch);
     if (ctx->head_scratch) cudaFree(ctx->head_scratch);
@@ -440,6 +439,7 @@ void loom_b200_ctx_destroy(loom_b200_ctx* ctx) {
     free_retired(ctx);
     if (ctx->owns_stream) cudaStreamDestroy(ctx->stream);
     delete ctx;
+    if (--g_contexts == 0) lb_free_idle_slots();
 }
 
 int loom_b200_sync(loom_b200_ctx* ctx) {

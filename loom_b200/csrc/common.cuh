@@ -44,8 +44,6 @@ struct loom_b200_weight {
     size_t tile_bytes() const { return (size_t)strips * kblocks * kTileBytes; }
 };
 
-constexpr int kStageSlots = 8;
-
 struct loom_b200_ctx {
     int device = 0;
     cudaStream_t stream = nullptr;
@@ -64,8 +62,6 @@ struct loom_b200_ctx {
     // device status word written by kernels with bounded waits (0 = ok)
     int* status_dev = nullptr;
     int* status_host = nullptr;    // pinned mirror, refreshed by lb_sync_checked
-    char* stage_host = nullptr;      // pinned slots that a layer call's host rows cross through (layers.cu)
-    cudaEvent_t stage_done[kStageSlots] = {};
     void* quant_scratch = nullptr;   // int8 row and absmax of the stand-alone GEMV prologue (wide inputs)
     size_t quant_scratch_bytes = 0;
     void* tp_rows = nullptr;         // this rank's int8 slices of the rows of a row-parallel product (their GEMV may use quant_scratch)
@@ -132,6 +128,8 @@ int lb_sync_checked(loom_b200_ctx* ctx);
 // what it says once that copy is known to have arrived.
 int lb_status_queue(loom_b200_ctx* ctx);
 int lb_status_result(loom_b200_ctx* ctx);
+// Frees the pinned slots that no layer call is using (layers.cu): the process's last context is gone.
+void lb_free_idle_slots();
 // Faults the pages of a pageable buffer in by one call (their contents stay); nothing for memory that CUDA knows.
 void lb_touch_pages(void* p, size_t bytes);
 int lb_ensure_quant_scratch(loom_b200_ctx* ctx, size_t bytes);

@@ -5,6 +5,7 @@
 
 #include <cmath>
 #include <cstring>
+#include <mutex>
 #include <vector>
 
 int lb_ternary_gemm(loom_b200_ctx* ctx, const loom_b200_weight* w, int tokens, const float* x, const float* bias,
@@ -297,13 +298,62 @@ struct Arena {
 
 size_t align256(size_t n) { return (n + 255) & ~(size_t)255; }
 
-// The host rows of a layer call cross through pinned slots of the context: rows on their way in are copied to one slot while the slot before
+// The host rows of a layer call cross through pinned slots: rows on their way in are copied to one slot while the slot before
 // crosses the bus, and rows on their way out are copied on while the next crosses.  The caller's fresh pages are faulted in while the GPU is
 // still at the layer.  The driver's own path for pageable memory moves 6 GB/s (636 KB out: 107 us) and starts when the layer is done.
 // Attention and feed-forward of a 2B-shaped block, 23 tokens and one more, four calls: 464 us that way, 402 so; of a call's 142 us with
-// 23 tokens the copies from the slots take 36.  A context's first call pays a millisecond for the slots; memory that CUDA knows is copied
-// as it is.
+// 23 tokens the copies from the slots take 36.  Memory that CUDA knows is copied as it is.
+// Pinned memory costs one to three milliseconds to get, so the slots belong to the process: a call borrows a set of them and gives it back
+// when its copies are done.  Up to kIdleSets wait for the next call; they are freed with the process's last context.
 constexpr size_t kSlotBytes = 128 * 1024;
+constexpr int kStageSlots = 8;
+constexpr size_t kIdleSets = 4;
+
+struct SlotSet {
+    int device = 0;
+    char* host = nullptr;
+    cudaEvent_t done[kStageSlots] = {};
+};
+std::mutex g_sets_mu;
+std::vector<SlotSet*> g_idle_sets;  // nothing is in flight to or from any of them
+
+void free_set(SlotSet* set) {
+    if (set->host) cudaFreeHost(set->host);
+    for (cudaEvent_t e : set->done)
+        if (e) cudaEventDestroy(e);
+    delete set;
+}
+// a set of the current device; null where there is no pinned memory left
+SlotSet* borrow_set(int device) {
+    {
+        std::lock_guard<std::mutex> lk(g_sets_mu);
+        for (size_t i = 0; i < g_idle_sets.size(); ++i) {
+            SlotSet* set = g_idle_sets[i];
+            if (set->device != device) continue;
+            g_idle_sets.erase(g_idle_sets.begin() + i);
+            return set;
+        }
+    }
+    auto* set = new SlotSet();
+    set->device = device;
+    cudaError_t e = cudaMallocHost((void**)&set->host, kStageSlots * kSlotBytes);
+    for (cudaEvent_t& done : set->done)
+        if (e == cudaSuccess) e = cudaEventCreateWithFlags(&done, cudaEventDisableTiming);
+    if (e == cudaSuccess) return set;
+    (void)cudaGetLastError();
+    free_set(set);
+    return nullptr;
+}
+void give_back(SlotSet* set) {
+    {
+        std::lock_guard<std::mutex> lk(g_sets_mu);
+        if (g_idle_sets.size() < kIdleSets) {
+            g_idle_sets.push_back(set);
+            return;
+        }
+    }
+    free_set(set);
+}
 
 struct HostPart {
     const float* dev;
@@ -317,21 +367,22 @@ public:
     // (a call that failed leaves nothing behind that still reads or writes a slot)
     ~HostRows() {
         if (open_) cudaStreamSynchronize(ctx_->stream);
+        if (set_) give_back(set_);
     }
     // rows to dev; `host` may be changed afterwards unless CUDA knows it
     int send(float* dev, const float* host, size_t n) {
         if (!dev || n == 0) return 0;
         open_ = true;
-        if (!slots() || known(host)) {
+        if (known(host) || !slots()) {
             LB_CUDA(ctx_, cudaMemcpyAsync(dev, host, n * 4, cudaMemcpyHostToDevice, ctx_->stream));
             return 0;
         }
         for (size_t at = 0; at < n * 4; at += kSlotBytes, ++sent_) {
             const size_t len = n * 4 - at < kSlotBytes ? n * 4 - at : kSlotBytes;
-            if (sent_ >= kStageSlots) LB_CUDA(ctx_, cudaEventSynchronize(ctx_->stage_done[sent_ % kStageSlots]));
+            if (sent_ >= kStageSlots) LB_CUDA(ctx_, cudaEventSynchronize(set_->done[sent_ % kStageSlots]));
             memcpy(slot(sent_), (const char*)host + at, len);
             LB_CUDA(ctx_, cudaMemcpyAsync((char*)dev + at, slot(sent_), len, cudaMemcpyHostToDevice, ctx_->stream));
-            LB_CUDA(ctx_, cudaEventRecord(ctx_->stage_done[sent_ % kStageSlots], ctx_->stream));
+            LB_CUDA(ctx_, cudaEventRecord(set_->done[sent_ % kStageSlots], ctx_->stream));
         }
         return 0;
     }
@@ -342,7 +393,7 @@ public:
         bool direct = false;
         for (int i = 0; i < 2; ++i) {
             const HostPart& p = parts[i];
-            if (p.host && slots() && !known(p.host))
+            if (p.host && !known(p.host) && slots())
                 pieces[i] = (p.n * 4 + kSlotBytes - 1) / kSlotBytes;
             else if (p.host) {
                 direct = true;
@@ -360,7 +411,7 @@ public:
             size_t at, len;
             const HostPart& p = part(i, &at, &len);
             LB_CUDA(ctx_, cudaMemcpyAsync(slot(i), (const char*)p.dev + at, len, cudaMemcpyDeviceToHost, ctx_->stream));
-            LB_CUDA(ctx_, cudaEventRecord(ctx_->stage_done[i % kStageSlots], ctx_->stream));
+            LB_CUDA(ctx_, cudaEventRecord(set_->done[i % kStageSlots], ctx_->stream));
             return 0;
         };
         for (size_t i = 0; i < all && i < kStageSlots; ++i)
@@ -370,7 +421,7 @@ public:
         for (size_t i = 0; i < all; ++i) {
             size_t at, len;
             const HostPart& p = part(i, &at, &len);
-            LB_CUDA(ctx_, cudaEventSynchronize(ctx_->stage_done[i % kStageSlots]));
+            LB_CUDA(ctx_, cudaEventSynchronize(set_->done[i % kStageSlots]));
             memcpy((char*)p.host + at, slot(i), len);
             if (i + kStageSlots < all)
                 if (int rc = ask(i + kStageSlots)) return rc;
@@ -390,22 +441,17 @@ private:
         }
         return where.type != cudaMemoryTypeUnregistered;
     }
-    char* slot(size_t i) const { return ctx_->stage_host + i % kStageSlots * kSlotBytes; }
+    char* slot(size_t i) const { return set_->host + i % kStageSlots * kSlotBytes; }
     // false where there is no pinned memory left: rows then go as they are
     bool slots() {
-        if (ctx_->stage_host) return true;
-        cudaError_t e = cudaSuccess;
-        for (cudaEvent_t& done : ctx_->stage_done)
-            if (!done && e == cudaSuccess) e = cudaEventCreateWithFlags(&done, cudaEventDisableTiming);
-        if (e == cudaSuccess) e = cudaMallocHost((void**)&ctx_->stage_host, kStageSlots * kSlotBytes);
-        if (e == cudaSuccess) return true;
-        (void)cudaGetLastError();
-        ctx_->stage_host = nullptr;
-        return false;
+        if (!set_ && !none_) set_ = borrow_set(ctx_->device);
+        none_ = !set_;
+        return set_ != nullptr;
     }
     loom_b200_ctx* ctx_;
+    SlotSet* set_ = nullptr;
     size_t sent_ = 0;
-    bool open_ = false;
+    bool open_ = false, none_ = false;
 };
 
 int upload_opt(loom_b200_ctx* ctx, const float* host, size_t n, float** dev) {
@@ -418,6 +464,15 @@ int upload_opt(loom_b200_ctx* ctx, const float* host, size_t n, float** dev) {
 }
 
 }  // namespace
+
+void lb_free_idle_slots() {
+    std::vector<SlotSet*> sets;
+    {
+        std::lock_guard<std::mutex> lk(g_sets_mu);
+        sets.swap(g_idle_sets);
+    }
+    for (SlotSet* set : sets) free_set(set);
+}
 
 extern "C" {
 

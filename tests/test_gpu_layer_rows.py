@@ -1,5 +1,7 @@
 """Host rows of the layer calls.  They cross in slots of 128 KB, eight in flight: the sizes are a slot's edges and more than the eight, in
 and out.  Pinned memory of the caller is copied as it is.  The sums are whole numbers with one rescale: the oracle's bits."""
+import threading
+
 import numpy as np
 import pytest
 import torch
@@ -38,3 +40,33 @@ def test_rows_cross_whole(ctx, batch, K, N):
                 assert (pre.numpy().view(np.uint32) == epre.view(np.uint32)).all()
             if want_post:
                 assert (post.numpy().view(np.uint32) == epost.view(np.uint32)).all()
+
+
+def test_threads_and_contexts_share_the_slots():
+    wrong, meet = [], threading.Barrier(7)
+
+    def work(i):
+        try:
+            rng = np.random.default_rng(i)
+            m = orc.Matrix.from_f32((rng.standard_normal(640 * 900) * 0.02).astype(np.float32), 640, 900)
+            x = rng.standard_normal((30, 900)).astype(np.float32)
+            _, want = orc.dense_forward(m, cabi.ACT_RELU2, x)
+            meet.wait(60)
+            for _ in range(4):
+                c = loom_b200.Context(0)
+                w = c.upload_ternary(m.words, 640, 900, m.scale)
+                for n in (30, 1, 7):
+                    _, post = cabi.dense_forward(c, w, cabi.ACT_RELU2, x[:n])
+                    if not np.array_equal(post.view(np.uint32), want[:n].view(np.uint32)):
+                        wrong.append((i, n))
+                w.free()
+                c.close()
+        except Exception as e:  # noqa: BLE001 (reported by the caller)
+            wrong.append((i, e))
+
+    threads = [threading.Thread(target=work, args=(i,)) for i in range(7)]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    assert not wrong
