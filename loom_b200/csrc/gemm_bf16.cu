@@ -208,8 +208,8 @@ __global__ void __launch_bounds__(kThreads, 1) lb_gemm_bf16_kernel(const LbDense
                 for (int c = half * 32; c < n; c += 64)
                     if (rt * n + c < p.ldo) asm volatile("prefetch.global.L2 [%0];" ::"l"(p.out + (size_t)tok * p.ldo + rt * n + c));
             }
-            if (!lb_mbar_wait_bounded(&acc_full[buf], (uint32_t)((i >> 1) & 1), kTcWaitLimit)) {
-                failed = true;
+            failed = __any_sync(0xffffffffu, !lb_mbar_wait_bounded(&acc_full[buf], (uint32_t)((i >> 1) & 1), kTcWaitLimit));
+            if (failed) {
                 if (lane == 0) atomicExch(&s_failed, 1);
                 break;
             }

@@ -291,7 +291,8 @@ __global__ void __launch_bounds__(kGemmThreads, 1) lb_gemm_ternary_i8_kernel(con
         const int8_t* qbase = p.q + ((size_t)(tok0 >> 8) * ktot + kbase) * 32768 + (size_t)((tok0 & 255) >> 3) * 1024;
         for (int ks = 0; ks < nslices; ++ks) {
             const int s = ks % kStages;
-            if (ks >= kStages && !failed && !wait_bounded(&empty_bar[s], (uint32_t)((ks / kStages - 1) & 1))) failed = true;
+            // (every lane polls by itself and elect wants all of them: the warp gives up together)
+            failed = __any_sync(0xffffffffu, ks >= kStages && !wait_bounded(&empty_bar[s], (uint32_t)((ks / kStages - 1) & 1)));
             if (failed) break;
             if (lb_elect()) {
                 lb_mbar_expect_tx(&load_bar[s], (uint32_t)(Cfg::kSliceBytesB + (MODE != GEMM_EXPAND ? Cfg::kStageBytesA : 0)));
@@ -422,6 +423,7 @@ __global__ void __launch_bounds__(kGemmThreads, 1) lb_gemm_ternary_i8_kernel(con
             const int s = ks % kStages;
             if (MODE == GEMM_EXPAND && !failed && !wait_bounded(&a_bar[s], (uint32_t)((ks / kStages) & 1))) failed = true;
             if (!failed && !wait_bounded(&load_bar[s], (uint32_t)((ks / kStages) & 1))) failed = true;  // the activations (and the cached codes)
+            failed = __any_sync(0xffffffffu, failed);
             asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
             if (tr && lane == 0) tr[(1 + ks) * 8 + 4] = lb_gtime();
             if (!failed && lb_elect()) {
@@ -662,10 +664,8 @@ __global__ void __launch_bounds__(kStreamThreads, 1) lb_gemm_stream_kernel(const
             asm volatile("bar.sync 1, %0;" ::"n"(kStreamEpi) : "memory");  // (everyone is also done with the scales of two tiles ago)
             if (i + 1 < my_tiles) next = tile_at(i + 1);
             fetch_stats(i + 1 < my_tiles);
-            if (!failed && !wait_bounded(&acc_full[buf], (uint32_t)((i >> 1) & 1))) {
-                failed = true;
-                atomicExch(&s_failed, 1);
-            }
+            failed = __any_sync(0xffffffffu, failed || !wait_bounded(&acc_full[buf], (uint32_t)((i >> 1) & 1)));
+            if (failed && lane == 0) atomicExch(&s_failed, 1);
             asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
             const int r = t.row * kRowsPerCta + quarter * 32 + lane;
             const bool row_ok = r < p.rows;
