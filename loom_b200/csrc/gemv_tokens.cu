@@ -316,26 +316,32 @@ __global__ void __launch_bounds__(kThreads, 2) lb_gemv_tokens_kernel(const __gri
     if (C > 1) lb_cluster_sync();  // nobody leaves while its sums are read
 }
 
+// Clusters of C CTAs to launch at most, two CTAs to an SM (or one): what the SMs' groups hold of whole clusters, and a few SMs
+// fewer for clusters of several, since one that finds no place at once is a second wave: 16384 x 14336, three tokens, 64 clusters of four
+// 18.8 us, the 71 that the occupancy query reports 25.4.
+int most_clusters(const loom_b200_ctx* ctx, int C, int per_sm) {
+    const int left[2][4] = {{0, 4, 16, 28}, {0, 4, 20, 20}};
+    return per_sm * (ctx->sm_count - left[per_sm - 1][C == 1 ? 0 : C == 2 ? 1 : C == 4 ? 2 : 3]) / C;
+}
+
 template <int EPI>
 int launch(loom_b200_ctx* ctx, LbGemvParams& p, const uint8_t* img, const int* xsum) {
     const int NT = (p.M + 7) / 8, Mp = 8 * NT, groups = p.total_tiles / p.kblocks / p.group;
-    // As many CTAs to a cluster as keep the rows' share small and the device busy.  Clusters of eight: four per group of SMs.
+    // as many CTAs to a cluster as keep the rows' share small and the device busy
     int C = 1;
     while (C < 8 && p.kblocks >= 4 * C && (((p.kblocks + C - 1) / C) * Mp * 128 > kGtRowsBytes || groups * C < ctx->sm_count)) C *= 2;
     const int rows_bytes = ((p.kblocks + C - 1) / C) * Mp * 128;
     auto smem_of = [&](int clusters, int stages) {
         return (size_t)kWarps * stages * kStageBytes + rows_bytes + (size_t)((groups + clusters - 1) / clusters) * p.group * p.M * 64;
     };
-    const int most[4] = {2 * ctx->sm_count, ctx->sm_count - 4, 64, 32};
-    int clusters = most[C == 1 ? 0 : C == 2 ? 1 : C == 4 ? 2 : 3];
-    if (clusters > groups) clusters = groups;
+    // two CTAs to an SM, or one with the whole of its shared memory: where no SM gets a second one, or two do not fit
+    const int one = most_clusters(ctx, C, 1), two = most_clusters(ctx, C, 2);
+    int clusters = groups < two ? groups : two;
+    const bool alone = groups <= one || smem_of(clusters, 1) > kGtSmemHalf;
+    if (alone) clusters = groups < one ? groups : one;
+    const size_t most = alone ? 2 * kGtSmemHalf : kGtSmemHalf;
     p.stages = kStages;
-    while (p.stages > 1 && smem_of(clusters, p.stages) > kGtSmemHalf) --p.stages;
-    if (smem_of(clusters, p.stages) > kGtSmemHalf && clusters > (ctx->sm_count - 4) / C) {  // one CTA an SM
-        clusters = (ctx->sm_count - 4) / C;
-        p.stages = kStages;
-        while (p.stages > 1 && smem_of(clusters, p.stages) > 2 * kGtSmemHalf) --p.stages;
-    }
+    while (p.stages > 1 && smem_of(clusters, p.stages) > most) --p.stages;
     while (smem_of(clusters, p.stages) > 2 * kGtSmemHalf && clusters < groups) clusters = clusters * 2 < groups ? clusters * 2 : groups;  // (many rows: several waves)
     const size_t smem = smem_of(clusters, p.stages);
     if (smem > 2 * kGtSmemHalf) return lb_fail(ctx, LOOM_B200_ERR_UNSUPPORTED, "gemv: %d tokens of %d columns need %zu B of shared memory", p.M, p.K, smem);
