@@ -387,6 +387,10 @@ int prepare(loom_b200_ctx* ctx, const LbGemvParams& p, int Mp, uint8_t* img, flo
 // statistics and no exchange (tensor-parallel shards)
 bool lb_gemv_tokens_takes(const loom_b200_ctx* ctx, const LbGemvParams& p) {
     if (p.M < kSplitQuantTokens || p.M > kGtMaxTokens || p.K > kGtMaxColumns || p.given_ss || p.given_amax || p.norm_count > 0 || p.epi == LB_EPI_TPSUM) return false;
+    // int8 rows of one block of columns and few rows: the launch in front costs more than every CTA's own fragments (3 x 256 x 128 4.4 us in
+    // one launch, 6.8 in two; 5 x 1024 x 128 5.9 and 6.8, 6 x 16 x 128 6.4 and 6.6; 5 x 256 x 64, read byte by byte, 7.7 and 6.6; 3 x 4096 x 128
+    // 7.4 and 6.8, 3 x 256 x 256 7.1 and 6.7)
+    if (p.pro == LB_PRO_Q8 && p.kblocks == 1 && p.M <= (p.K == kTileCols ? 5 : 4) && p.total_tiles <= 64) return false;
     // the options that ask for something of the one-token kernel, and a recording that the scratch would have to grow for
     return p.M > kMaxM || (!ctx->opt_gemv_partition && !ctx->trace_dev && !(ctx->capturing && gt_scratch(p.kblocks) > ctx->quant_scratch_bytes));
 }

@@ -1,5 +1,5 @@
 """Ternary products of 3 to 24 tokens per pass: one to three MMA columns of tokens, one to eight CTAs to a cluster, ragged last strips and
-columns, more rows than one wave of CTAs holds, rows too wide for the pass.  Sums, outputs and codes are compared bit for bit."""
+columns, more rows than one wave of CTAs holds, rows too wide for the pass, products so small that the one-token kernel keeps them.  Sums, outputs and codes are compared bit for bit."""
 import numpy as np
 import pytest
 
@@ -19,11 +19,11 @@ def ctx():
 
 
 # (cols: 1 to 256 blocks of 128 columns)
-SHAPES = [(16, 128), (40, 100), (33, 1000), (2560, 6912), (6912, 2560), (300, 14336), (5, 32768), (70, 32769), (140000, 64), (130, 511)]
+SHAPES = [(16, 128), (40, 100), (1024, 128), (1025, 128), (33, 1000), (2560, 6912), (6912, 2560), (300, 14336), (5, 32768), (70, 32769), (140000, 64), (130, 511)]
 
 
 @pytest.mark.parametrize("rows,cols", SHAPES)
-@pytest.mark.parametrize("tokens", [3, 8, 9, 16, 23, 24, 25])
+@pytest.mark.parametrize("tokens", [3, 5, 6, 8, 9, 16, 23, 24, 25, 29])
 def test_linear(ctx, rows, cols, tokens):
     rng = np.random.default_rng(rows + cols + tokens)
     words = orc.pack_f32((rng.standard_normal(rows * cols) * 0.02).astype(np.float32), rows, cols)[0]
