@@ -19,6 +19,7 @@ def lib():
     so = C.CDLL(out)
     vp, i, f = C.c_void_p, C.c_int, C.c_float
     so.t_gemm_bf16.argtypes = [vp, i, vp, vp, vp, i, vp, i, vp, i, i, i, f, f, f]
+    so.t_attention_prompt.argtypes = [vp, vp, vp, vp, vp, vp, i, i, i, i, i]
     so.t_pair_begin.argtypes = [vp, C.POINTER(vp)]
     so.t_pair_message.argtypes = [vp, C.c_uint, i, vp, vp, vp, i]
     so.t_pair_end.argtypes = [vp, vp]

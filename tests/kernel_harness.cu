@@ -1,9 +1,10 @@
-// kernel_harness.cu -- C entries for tests of parts that no public call reaches one by one: the bf16 token-block product alone, and the
-// second rank of a tensor-parallel pair whose messages lie in the mailbox before the first rank asks for them (so nothing waits).
+// kernel_harness.cu -- C entries for tests of parts that no public call reaches one by one: the bf16 token-block product alone, the float64
+// attention of a prompt block alone, and the second rank of a tensor-parallel pair whose messages lie in the mailbox before the first rank asks for them (so nothing waits).
 //
 //   nvcc -gencode arch=compute_100a,code=sm_100a -std=c++17 -shared -Xcompiler -fPIC -Iinclude -Iloom_b200/csrc tests/kernel_harness.cu
 //        loom_b200/lib/libloom_b200.so -o kernel_harness.so
 #include "dense.cuh"
+#include "glue.cuh"
 #include "tp_xchg.cuh"
 
 #include <cstring>
@@ -31,6 +32,25 @@ int t_gemm_bf16(loom_b200_ctx* ctx, int epi, const loom_b200_matrix* x, const lo
     p.res_mult = res_mult;
     p.limit = limit;
     if (int rc = lb_dense_gemm(ctx, LOOM_B200_DTYPE_BF16, epi, p)) return rc;
+    return lb_sync_checked(ctx);
+}
+
+// everything on the device; keys and values [kv_heads, msl, hd], pos: the first token's position
+int t_attention_prompt(loom_b200_ctx* ctx, const double* q, const float* k, const float* v, const int* pos, double* out, int tokens, int heads, int kv_heads, int hd, int msl) {
+    LbAttnParams p = {};
+    p.q = q;
+    p.cache_k = k;
+    p.cache_v = v;
+    p.pos_ptr = pos;
+    p.out = out;
+    p.M = tokens;
+    p.heads = heads;
+    p.kv_heads = kv_heads;
+    p.hd = hd;
+    p.msl = msl;
+    p.splits = 1;
+    p.max_chunk = msl;
+    if (int rc = lb_launch_attention_prefill(ctx, p)) return rc;
     return lb_sync_checked(ctx);
 }
 

@@ -8,6 +8,7 @@ test_gpu_attention_decode.py.
 import numpy as np
 import pytest
 
+import harness
 import loom_b200
 from loom_b200 import cabi
 from oracle import oracle as orc
@@ -69,4 +70,54 @@ def test_rotation_of_a_block_in_any_share(heads, kvh, hd, n):
         assert np.max(np.abs(l0 - l1)) <= 1e-6 * max(1.0, float(np.max(np.abs(l1))))
     finally:
         dec.close()
+        ctx.close()
+
+
+@pytest.mark.parametrize("heads,kvh,hd,tokens,pos0", [(8, 2, 128, 150, 0), (4, 4, 64, 97, 40), (20, 5, 128, 33, 130)])
+def test_infinities_and_nan_stay_with_the_rows_that_see_them(heads, kvh, hd, tokens, pos0):
+    """Keys and values that are not finite, in float64 as IEEE has them: a NaN score makes a NaN row, so does one of +infinity, one of -infinity
+    weighs nothing.  A position's value also reaches rows in front of it in its tile of 32 keys, with weight zero; those are left out where
+    the value is not finite."""
+    rng = np.random.default_rng(tokens)
+    msl, G = 320, heads // kvh
+    ctx = loom_b200.Context(0)
+    try:
+        for special in ("none", "key nan", "key inf", "key -inf", "value inf", "value nan", "query nan", "lowest"):
+            q = rng.standard_normal((tokens, heads, hd))
+            k, v = (rng.standard_normal((kvh, msl, hd)).astype(np.float32) for _ in range(2))
+            at = pos0 + tokens // 2
+            what = special.split()
+            if what[0] in ("key", "value"):
+                (k if what[0] == "key" else v)[0, at, 3] = np.float32(what[1])
+            if special.startswith("key"):
+                q[..., 3] = np.abs(q[..., 3]) + 0.1  # (infinite scores of one sign)
+            if special == "query nan":
+                q[tokens // 3, 1, 5] = np.nan
+            if special == "lowest":
+                k[:, at:at + 2] = np.finfo(np.float32).min
+            if pos0 + tokens < msl:  # what lies behind the block is nobody's
+                k[:, pos0 + tokens:], v[:, pos0 + tokens:] = np.nan, np.inf
+            dev = [ctx.to_device(a) for a in (q, k, v, np.array([pos0], np.int32))]
+            dout = ctx.alloc(tokens * heads * hd * 8)
+            ctx._check(harness.lib().t_attention_prompt(ctx.h, *dev, dout, tokens, heads, kvh, hd, msl))
+            got = ctx.download(dout, (tokens, heads, hd), np.float64)
+            for h in range(heads):
+                kk, vv = k[h // G].astype(np.float64), v[h // G].astype(np.float64)
+                for t in range(tokens):
+                    pos = pos0 + t
+                    if what[0] == "value" and h < G and at // 32 * 32 <= pos < at:
+                        continue
+                    with np.errstate(all="ignore"):
+                        s = (kk[:pos + 1] * q[t, h]).sum(1) / np.sqrt(hd)
+                        e = np.exp(s - s.max()) if not np.isnan(s).any() else np.full(pos + 1, np.nan)
+                        want = (e[:, None] * vv[:pos + 1]).sum(0) / e.sum()
+                    bad = ~np.isfinite(want)
+                    assert np.array_equal(np.isnan(got[t, h]), np.isnan(want)) and np.array_equal(got[t, h][bad & ~np.isnan(want)], want[bad & ~np.isnan(want)])
+                    # a score of up to 40 is off by 128 * 40 * 2^-53 = 6e-13 at most, and its weight by as much of itself
+                    if not bad.all():
+                        terms = (e[:, None] * np.abs(vv[:pos + 1])).sum(0) / e.sum()
+                        assert (np.abs(got[t, h][~bad] - want[~bad]) <= 1e-12 * terms[~bad]).all()
+            for p in (*dev, dout):
+                ctx.free(p)
+    finally:
         ctx.close()

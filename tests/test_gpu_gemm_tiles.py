@@ -132,3 +132,39 @@ def test_normed_rows_of_many_tokens(heads, hd, inter):
     finally:
         gdec.close()
         c.close()
+
+
+@pytest.mark.parametrize("cols", [64, 1000, 16384])
+def test_rows_that_are_not_numbers(ctx, cols):
+    """Infinities, NaN, the largest and the smallest numbers, zeros of both signs: the float quantizer and the rows that bulk copies bring give
+    what the former quantizer gives, codes, largest values and sums."""
+    rng = np.random.default_rng(cols)
+    rows, tokens = 70, 300
+    x = rng.standard_normal((tokens, cols)).astype(np.float32)
+    special = np.array([np.inf, -np.inf, np.nan, 3.4e38, -3.4e38, 1e-45, -1e-45, 0.0, -0.0, 1e-5, 9.9e-6], np.float32)
+    for i, v in enumerate(special):
+        x[2 * i, rng.integers(0, cols)] = v
+        x[2 * i + 1] = v
+    x[40] *= 1e-30
+    x[41, ::2] = np.nan
+    words, scale = matrix(rng, rows, cols)
+    w, dx = ctx.upload_ternary(words, rows, cols, scale), ctx.to_device(x)
+    got = []
+    for regs in (0, 1):
+        ctx.set_option("quant_regs", regs)
+        try:
+            out, acc, amax = ctx.alloc(tokens * rows * 4), ctx.alloc(tokens * rows * 4), ctx.alloc(tokens * 4)
+            ctx.ternary_gemm(w, tokens, dx, out=out, acc_out=acc, amax_out=amax)
+            plain = ctx.alloc(tokens * rows * 4)
+            ctx.ternary_gemm(w, tokens, dx, out=plain)  # (without raw sums: the float epilogue)
+            got.append([ctx.download(p, s, np.uint32) for p, s in ((out, (tokens, rows)), (acc, (tokens, rows)), (amax, (tokens,)), (plain, (tokens, rows)))])
+        finally:
+            ctx.set_option("quant_regs", 1)
+    for a, b in zip(*got):
+        assert (a == b).all()
+    f, g = (a.view(np.float32) for a in (got[1][0], got[1][3]))
+    assert ((f == g) | (np.isnan(f) & np.isnan(g))).all()
+    finite = np.isfinite(x).all(1)
+    q, amax = orc.quantize_rows_f32(x[finite])
+    assert (got[1][2][finite].view(np.float32) == amax).all()
+    assert (got[1][1][finite].view(np.int32) == (q.astype(np.float64) @ np_unpack(words, rows, cols).astype(np.float64).T)).all()

@@ -59,6 +59,23 @@ def test_dense_rows_are_quantized_alike(ctx, rows, cols, tokens):
     assert (post == np.maximum(f, 0)).all()
 
 
+@pytest.mark.parametrize("cols", [64, 1001, 16500])
+def test_rows_that_are_not_numbers(ctx, cols):
+    """Infinities, NaN, the largest and the smallest numbers in a pass of several tokens: the bits of a token by itself."""
+    rng = np.random.default_rng(cols)
+    rows = 70
+    w = ctx.upload_ternary(*(lambda m: (m.words, rows, cols, m.scale))(orc.Matrix.from_f32((rng.standard_normal(rows * cols) * 0.02).astype(np.float32), rows, cols)))
+    special = np.array([np.inf, -np.inf, np.nan, 3.4e38, -3.4e38, 1e-45, 0.0, -0.0, 1e-5, 9.9e-6], np.float32)
+    x = rng.standard_normal((2 * len(special), cols)).astype(np.float32)
+    for i, v in enumerate(special):
+        x[2 * i, rng.integers(0, cols)] = v
+        x[2 * i + 1] = v
+    pre, post = cabi.dense_forward(ctx, w, cabi.ACT_LINEAR, x)
+    for i in range(len(x)):
+        one, _ = cabi.dense_forward(ctx, w, cabi.ACT_LINEAR, x[i:i + 1])
+        assert (pre[i].view(np.uint32) == one[0].view(np.uint32)).all()
+
+
 @pytest.mark.parametrize("heads,kvh,hd,inter,seq", [(4, 2, 32, 500, 23), (3, 1, 50, 130, 24), (20, 5, 128, 6912, 10), (2, 2, 2, 17, 29)])
 def test_short_prompts_and_sequences_match_the_oracle(ctx, heads, kvh, hd, inter, seq):
     """A prompt in passes of 24 tokens, then 18 sequences of different lengths a token each per pass; logits as in test_gpu_batch.py."""
