@@ -87,6 +87,13 @@ def test_rowsharded_linear_of_rank_0_of_two(fused):
                 ctx.tp_rowsharded_linear(w, batch, d_x, K, d_out, inner_w=d_in, inner_w_len=Kl, eps=0.0, bias=d_b)
                 got = ctx.download(d_out, (batch, rows), np.float32)
                 ctx.sync()
+                # (a pass of more tokens than a group's passes carry)
+                q20, a20 = orc.quantize_rows_f32(rng.standard_normal((20, Kl)).astype(np.float32))
+                d20 = [ctx.to_device(q20), ctx.to_device(a20), ctx.alloc(20 * rows * 4)]
+                ctx.ternary_linear(w, 20, d20[0], d20[1], None, acc_out=d20[2])
+                assert np.array_equal(ctx.download(d20[2], (20, rows), np.int32), q20.astype(np.int32) @ codes[:, :Kl].astype(np.int32).T)
+                for p in d20:
+                    ctx.free(p)
                 want = (acc * (np.float64(scale) * amax.astype(np.float64) / 127.0)[:, None] + bias.astype(np.float64)).astype(np.float32)
                 assert np.array_equal(got, want)
                 ctx.free(d_x)
