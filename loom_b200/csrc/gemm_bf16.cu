@@ -244,19 +244,20 @@ __global__ void __launch_bounds__(kThreads, 1) lb_gemm_bf16_kernel(const LbDense
     if (tid == 0 && s_failed) atomicExch(p.status, 3);
 }
 
-// Columns of a tile.  Measured with every SM at work: a slice takes 0.32 us with up to 128 columns (both matrices together), 0.355 with
-// 144, 0.40 with 192 and 0.46 with 256; an epilogue behind the last MMA 0.015 us a column.  Wide tiles leave a last wave of few of them:
-// 2048 x 2560 x 6912 takes 96 us as 160 tiles of 256, 83 as 224 of 192 and 78 as 288 of 144 (100 before residual rows were asked for
-// ahead); 2048 x 7696 x 2560 78 us with 256, 75 with 224, 84 with 144.
-// (Few tiles split over K by the CTAs of a cluster were quicker, 100 tokens x 2560 x 6912 25 us for 43, but sums of parts are other bits
-// than one accumulator's, and a token's result then depends on how many others are in its block.)
+// Columns of a tile.  Measured: a slice takes 0.28 us with 32 columns (both matrices together), 0.29 with 64 and 0.31 with 128; 0.05 us more
+// where tiles cross blocks of 128 rows of W and need two copies of it; with every SM at work 0.355 with 144, 0.40 with 192 and 0.46 with
+// 256; an epilogue behind the last MMA 0.015 us a column.  Wide tiles leave a last wave of few of them: 2048 x 2560 x 6912 takes 96 us as
+// 160 tiles of 256, 83 as 224 of 192 and 78 as 288 of 144 (100 before residual rows were asked for ahead); 2048 x 7696 x 2560 78 us with
+// 256, 75 with 224, 84 with 144.  100 tokens x 2560 x 6912: 30 us with 32 columns, 31 with 64, 34 with 128, 38 with 96, 55 (two waves) with 16.
+// (Few tiles split over K by the CTAs of a cluster took 25 us there, but sums of parts are other bits than one accumulator's, and a
+// token's result then depends on how many others are in its block.)
 Plan plan(const loom_b200_ctx* ctx, const LbDenseGemm& p, bool dual) {
     const int blocks = p.nblocks ? p.max_blocks : lb_ceil_div(p.tokens, kImgRows), most = dual ? 128 : 256, rows = lb_round_up(p.rows, kImgRows);  // (the padding's zeros too)
     Plan best = {};
     double best_us = 1e30;
-    for (int n = most < rows ? most : rows; n >= 48; n -= 16) {
+    for (int n = most < rows ? most : rows; n >= 32; n -= 16) {
         const int tiles = lb_ceil_div(rows, n) * blocks, cols = dual ? 2 * n : n;
-        const double slice = cols <= 106 ? 0.32 : 0.22 + cols * 0.00094;
+        const double slice = cols > 128 ? 0.22 + cols * 0.00094 : 0.27 + cols * 0.00035 + (kImgRows % n ? 0.05 : 0.0);
         const double us = lb_ceil_div(tiles, ctx->sm_count) * p.slices * slice + cols * 0.015;
         if (us < 0.98 * best_us) {
             best_us = us;
