@@ -719,9 +719,9 @@ def batch_measure(args, torch, dist, rank, world, local, shape_name, B, n_prompt
         dist.all_reduce(t, op=dist.ReduceOp.MAX)
         dev_s = float(t[0].item())
     tern_b, kv_b, head_b = algorithmic_bytes(shape, n_prompt + warmup + steps // 2)
-    passes = (B + 7) // 8
-    # per GPU: weights once per pass of eight, KV of every sequence, head once per head pass of two rows
-    moved = (passes * tern_b + B * kv_b + ((B + 1) // 2) * head_b) / world
+    passes, heads = -(-B // (24 if world == 1 else 8)), -(-B // 8)
+    # per GPU: weights once per pass of 24 sequences (eight under a group), KV of every sequence, head once per pass of eight rows
+    moved = (passes * tern_b + B * kv_b + heads * head_b) / world
     res = {"shape": shape_name, "layers": shape["layers"], "world": world, "batch": B, "prompt": n_prompt, "steps": steps,
            "tok_per_s": B * steps / dev_s, "ms_per_step": 1e3 * dev_s / steps, "per_sequence_tok_per_s": steps / dev_s,
            "prefill_seconds_all_sequences": prefill_s, "prefill_tok_per_s": B * n_prompt / prefill_s, "clocks": clocks,
@@ -737,8 +737,8 @@ def batch_measure(args, torch, dist, rank, world, local, shape_name, B, n_prompt
 
 
 def batch_mode(args):
-    """Decode with `--batch` independent sequences (configs[3]: 8B shape, batch 16, 2048-token prompts): up to eight
-    sequences per pass over every packed matrix and several hidden rows per pass over the LM head.  value = sequences x
+    """Decode with `--batch` independent sequences (configs[3]: 8B shape, batch 16, 2048-token prompts): up to 24
+    sequences per pass over every packed matrix (eight in a tensor-parallel group) and eight hidden rows per pass over the LM head.  value = sequences x
     steps / time.  Under torchrun the decoder is tensor-parallel over the ranks (column-sharded Q/K/V/gate/up, row-sharded
     O/down, vocabulary-sharded head whose tail exchanges (maximum, index) pairs; peer-memory exchange) and `scaling` is
     "strong"."""
@@ -770,7 +770,7 @@ def batch_mode(args):
             "prefill_tok_per_s": r["prefill_tok_per_s"], "clocks": r["clocks"],
             "roofline": {"bound": "hbm", "achieved": r["bytes_per_gpu_per_step"] / step_s / 1e9, "peak": peak, "unit": "GB/s",
                          "frac": r["bytes_per_gpu_per_step"] / step_s / 1e9 / peak, "traffic": None, "peak_kind": peak_kind,
-                         "kernel": "whole batch step, per GPU: packed weights once per pass of eight sequences, KV of every sequence, fp32 head once per head pass"}}))
+                         "kernel": "whole batch step, per GPU: packed weights once per pass of 24 sequences (eight under a group), KV of every sequence, fp32 head once per pass of eight rows"}}))
     if world > 1:
         dist.barrier()
         dist.destroy_process_group()

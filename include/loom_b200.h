@@ -99,8 +99,8 @@ void loom_b200_graph_free(loom_b200_ctx* ctx, loom_b200_graph* graph);
 void* loom_b200_ctx_stream(loom_b200_ctx* ctx);
 /* Tuning knobs, the counterpart of the tileSize argument the WGSL dispatchers take
  * (poly/wgpu_kernels.go:416-427): "gemv_variant" 0 = integer-MMA inner loop, 1 = dp4a inner loop;
- * "gemv_ctas_per_sm" 1..8; "gemv_partition" 0 = choose, 1 = stream-K over tiles with the int32 fix-up,
- * 2 = whole strips per CTA; "pdl" 0/1 = programmatic dependent launch; "tp_graph" 0/1 = record the
+ * "gemv_ctas_per_sm" 1..8 (passes of one and two tokens; more have a kernel with a grid of its own); "gemv_partition" 0 = choose,
+ * 1 = stream-K over tiles with the int32 fix-up, 2 = whole strips per CTA (1 and 2 also keep three to eight tokens on that kernel); "pdl" 0/1 = programmatic dependent launch; "tp_graph" 0/1 = record the
  * tensor-parallel decode step, collectives included, as a graph; "gemm_tile" 0 / 128 / 256 = tokens per CTA of the
  * token-block GEMM (0 = choose); "gemm_splitk" 0/1 = let several CTAs share the K range of an output tile;
  * "fold_rope" 0/1 = one-token decoder steps apply RoPE inside the attention kernel (one launch less per block);
@@ -114,7 +114,7 @@ void* loom_b200_ctx_stream(loom_b200_ctx* ctx);
  * exchange of the partial sums in the GEMV's epilogue (1, default);
  * "dense_tc" 0/1 = token blocks of bf16 layer stacks run on the tensor cores (1, default) or as plain fused multiply-adds (0);
  * "prefill_gemm" 0/1 = prompts of 32 or more tokens
- * run their projections as token-block GEMMs on the tensor cores (1) or eight tokens at a time through the GEMV (0).  "gemm_cache" 0/1 = the token-block GEMM reads pre-expanded int8 codes (one byte per weight, built per
+ * run their projections as token-block GEMMs on the tensor cores (1) or up to 24 tokens at a time through the GEMV (0).  "gemm_cache" 0/1 = the token-block GEMM reads pre-expanded int8 codes (one byte per weight, built per
  * matrix the first time it meets the GEMM, four times its packed bytes; the device twin of ensureBitNetCodes,
  * poly/bitnet_cpu.go:700-729) and fuses the SwiGLU gate product into the gate/up GEMM (1), or expands the 2-bit tiles
  * inside the kernel (0); "head_stream" 0/1 = the fp32 LM head streams
@@ -217,8 +217,8 @@ int loom_b200_ternary_gemm(loom_b200_ctx* ctx, const loom_b200_weight* w, int to
  * 1.02 MiB array inside the library image (held by every GPU that loads the library until the process exits)
  * and calls no cudaMalloc, cudaFree or allocating routine.
  *   Limits: rows <= 65,536 and 16*ceil(rows/16)*tokens_per_pass <= 262,144, where tokens_per_pass is
- *   min(batch, 8) for inputs of up to about 19,000 columns and fewer beyond (5 at 28,672 columns: the same
- *   rule as loom_b200_ternary_linear); beyond them the call fails with LOOM_B200_ERR_UNSUPPORTED and a message
+ *   min(batch, 8) for inputs of up to about 19,000 columns and fewer beyond (5 at 28,672 columns);
+ *   beyond them the call fails with LOOM_B200_ERR_UNSUPPORTED and a message
  *   naming loom_b200_ternary_linear.  A bounded device-side wait that runs out inside this call is reported
  *   by loom_b200_sync like one inside the regular call (the context's own status word is used).
  *   The first call on a device looks the array's address up (cudaGetSymbolAddress); make that call before

@@ -62,7 +62,7 @@ struct loom_b200_ctx {
     // device status word written by kernels with bounded waits (0 = ok)
     int* status_dev = nullptr;
     int* status_host = nullptr;    // pinned mirror, refreshed by lb_sync_checked
-    void* quant_scratch = nullptr;   // int8 row and absmax of the stand-alone GEMV prologue (wide inputs)
+    void* quant_scratch = nullptr;   // rows quantized in front of a GEMV: fragments, largest values and sums of up to 24 tokens, or int8 rows and largest values
     size_t quant_scratch_bytes = 0;
     void* tp_rows = nullptr;         // this rank's int8 slices of the rows of a row-parallel product (their GEMV may use quant_scratch)
     size_t tp_rows_bytes = 0;

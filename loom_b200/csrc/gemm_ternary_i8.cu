@@ -456,17 +456,19 @@ __global__ void __launch_bounds__(kGemmThreads, 1) lb_gemm_ternary_i8_kernel(con
 // ------------------------------------------------------------------------------------------------------------------
 // Persistent variant over pre-expanded codes.  One CTA per SM walks output tiles (row tile fastest, so the CTAs that run
 // together share a token tile's activations in L2); the shared-memory ring runs on across tile boundaries, and tensor
-// memory holds TWO accumulator buffers, so the epilogue warps drain tile i (tcgen05.ld, float64 rescale, stores)
+// memory holds TWO accumulator buffers, so the epilogue warps drain tile i (tcgen05.ld, rescale, stores)
 // while the MMA warp already accumulates tile i+1.  In the one-shot kernel above the epilogue of a 128 x 256 tile costs
 // about as long as its twenty k-slices of MMAs, and two co-resident CTAs ran in lockstep instead of overlapping.
-// What bounds it (operands replaced by 16-byte copies change nothing): the epilogue, whose float64 instructions take 2.4 times
-// as long while the tensor core is at work (18,500 clocks for a 128 x 256 tile against 7,700 behind the last MMA, twenty slices of MMAs
-// 11,000), and how fast one thread can issue (lb_elect).  Sixteen epilogue warps instead of eight, statistics fetched a tile ahead,
-// a token's scale and correction in one 16-byte load, copies and MMAs from elected threads: 2048 x 6912 x 2560 43 -> 36 us,
-// 512 x 2560 x 6912 25 -> 17.5, 2999 x 14336 x 4096 164 -> 147; gate and up of 1024 x 6912 x 2560 67 -> 53.
+// What bounds it (operands replaced by 16-byte copies change little): how fast one thread can issue (lb_elect), the last wave of tiles, and
+// the epilogue where it is float64 (a bias, raw sums, float64 outputs, gate products): those instructions take 2.4 times as long while
+// the tensor core is at work (18,500 clocks for a 128 x 256 tile against 7,700 behind the last MMA, twenty slices of MMAs 11,000).
+// Plain outputs are rescaled in float arithmetic (gemm_scaled32).  us, the product alone, float / float64 epilogue: 512 x 6912 x 2560
+// 13.6 / 15.4, 512 x 2560 x 6912 16.7 / 17.8, 2048 x 6912 x 2560 30.8 / 41.8, 2048 x 2560 x 6912 32.8 / 34.7, 2999 x 14336 x 4096 135 / 194;
+// gate and up of 1024 x 6912 x 2560 47.  With eight epilogue warps, float64 throughout, a branch on the lane around copies and MMAs and tiles
+// of 128 or 256 tokens: 2048 x 6912 x 2560 43, 512 x 2560 x 6912 25, 2999 x 14336 x 4096 164, that gate and up 67.
 // A launch takes up to three products of the same activations (Q, K and V), whose row tiles follow one another.  Tiles are `ntok`
 // tokens wide, a multiple of 16 (gemm_stream_tokens has the rule), and of a group of token tiles the token runs fastest, so that the
-// CTAs at work together read few rows and few tokens: 2999 x 14336 x 4096 147 -> 142 us against rows first, 2048 x 2560 x 6912 52 -> 48.6.
+// CTAs at work together read few rows and few tokens (against rows first 3 % of 2999 x 14336 x 4096, 6 % of 2048 x 2560 x 6912).
 // DUAL: a gate / up pair that shares the activations -- both code blocks ride in one stage, two accumulators per buffer
 // (gate at column 0, up at column 128), and the epilogue writes float32(gateProduct(yg + bg, yu + bu)) only
 // (poly/swiglu.go:299-310): the two int32 accumulator planes never travel through memory.
@@ -1375,9 +1377,9 @@ static int gemm_launch(loom_b200_ctx* ctx, const GemmParams& p, dim3 grid, unsig
 // Tokens per tile of the persistent kernel: the widest, or what is five percent better in the time until the busiest CTA is done plus the
 // time all SMs together are kept from other streams' work.  Measured: a k-slice takes 0.25 us with up to 128 tokens and 0.39 with 256; an
 // epilogue beside MMAs 2 us and 0.036 us a token (a gate / up pair: twice the slice, 0.11 us a token), the last one 0.02.  Wide tiles
-// leave a last wave of few of them: 2048 tokens of 20 row tiles, K = 6912, take 42 us as 160 tiles of 256 and 32 us as 260 of 160;
-// 700 x 4096 x 4096 29 us with 256 tokens and 24 with 176.  Narrow ones load the codes more often: three streams that each multiply 512
-// tokens by both 2B projections take 30 us a pass with 256, 33 with 128, 36 with 112 and 80.
+// leave a last wave of few of them: 2048 tokens of 20 row tiles, K = 6912, take 40.6 us as 160 tiles of 256 and 32.8 as 260 of 160;
+// 700 x 4096 x 4096 17.1 us with 256 tokens and 13.6 with 176.  Narrow ones load the codes more often: three streams that each multiply 512
+// tokens by both 2B projections take 28.2 us a pass and stream with 256 or the rule's choice, 30.6 with 128 (with the float64 rescale 36 with 112 and 80).
 static int gemm_stream_tokens(const loom_b200_ctx* ctx, int row_tiles, int tokens, int kblocks, bool dual) {
     const int most = dual ? 128 : 256;
     if (ctx->opt_gemm_tile) return ctx->opt_gemm_tile < most ? ctx->opt_gemm_tile : most;

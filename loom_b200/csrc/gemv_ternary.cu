@@ -566,8 +566,8 @@ int lb_launch_gemv(loom_b200_ctx* ctx, const LbGemvParams& pin) {
     if (lb_gemv_tokens_takes(ctx, pin)) return lb_launch_gemv_tokens(ctx, pin);
     LB_REQUIRE(ctx, pin.M <= kMaxM, "gemv: %d tokens per pass (max %d)", pin.M, kMaxM);
     LbGemvParams p = pin;
-    // Wide inputs, or three and more tokens: normalise and quantize once in a launch of its own (one CTA per token), then
-    // stream the weights against the int8 rows.  The fused prologue is repeated by every CTA and costs it 4-6 us per token:
+    // Wide inputs, or three and more tokens that lb_gemv_tokens_takes leaves here: normalise and quantize once in a launch of its own (one CTA
+    // per token), then stream the weights against the int8 rows.  The fused prologue is repeated by every CTA and costs it 4-6 us per token:
     // right for one or two tokens on the critical path of a decode step, wrong for a pass of eight.
     if (p.pro != LB_PRO_Q8 && (p.K >= kSplitQuantK || p.M >= kSplitQuantTokens) && (p.K & 3) == 0 && (((uintptr_t)p.x) & 15) == 0 &&
         (!p.norm_w || (((uintptr_t)p.norm_w) & 15) == 0) && (!p.norm_out || (((uintptr_t)p.norm_out) & 15) == 0) &&

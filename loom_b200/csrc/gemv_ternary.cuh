@@ -46,7 +46,7 @@ struct LbGemvSeg {
     long long seq_stride;
 };
 
-// Tokens one pass can carry for K input columns: the int8 activations of all tokens sit in shared memory beside a
+// Tokens one pass of the one-token kernel can carry for K input columns: the int8 activations of all tokens sit in shared memory beside a
 // weight ring of at least two stages.  8 for every K up to ~19,000; 5 for K = 28,672.
 int lb_gemv_max_tokens(int K);
 // Passes of 3 to kPassTokens tokens over inputs of at most kGtMaxColumns columns have a kernel of their own (gemv_tokens.cu).
@@ -118,7 +118,7 @@ __device__ __forceinline__ double lb_pro_value(double x, double root, double rr,
 // Inputs at least this wide are normalised and quantized by one stand-alone launch (lb_launch_norm_quantize)
 // instead of inside every CTA of the GEMV.
 constexpr int kSplitQuantK = 8192;
-constexpr int kSplitQuantTokens = 3;  // ... and so are passes of at least this many tokens
+constexpr int kSplitQuantTokens = 3;  // ... and so are passes of at least this many tokens, in gemv_tokens.cu or, where that kernel does not take them, here
 bool lb_gemv_tokens_takes(const loom_b200_ctx* ctx, const LbGemvParams& p);
 int lb_launch_gemv_tokens(loom_b200_ctx* ctx, const LbGemvParams& p);
 // tokens a caller should put into one pass over inputs of K columns

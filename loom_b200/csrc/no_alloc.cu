@@ -59,7 +59,7 @@ extern "C" int loom_b200_ternary_linear_no_alloc(loom_b200_ctx* ctx, const loom_
     if (batch == 0) return 0;
     LB_REQUIRE(ctx, q && amax && out, "ternary_linear_no_alloc: NULL buffer");
     LB_REQUIRE(ctx, w->device == ctx->device, "ternary_linear_no_alloc: weight lives on device %d, context on %d", w->device, ctx->device);
-    // tokens one pass carries: the same rule as the regular entry point (8, fewer for very wide inputs)
+    // tokens a pass of the one-token kernel carries (8, fewer for very wide inputs); the kernel of more needs scratch of its own
     const int pass = lb_gemv_max_tokens(w->cols);
     const int per_pass = batch < pass ? batch : pass;
     // the fixed scratch bounds the shapes this entry point takes
