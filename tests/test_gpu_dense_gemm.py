@@ -50,7 +50,8 @@ def test_prompts_over_few_tiles(ctx, dtype, tensor_cores, width, ff, tokens):
 @pytest.mark.parametrize("width,ff,tokens", [(1300, 2100, 1500), (2560, 700, 600), (640, 5000, 2100), (330, 1000, 1030)])
 def test_tiles_of_any_width(ctx, width, ff, tokens):
     """Prompts of many tiles, whose columns are cut where the waves of CTAs come out even: across blocks of 128 rows of a matrix, with
-    ragged last ones; against the plain multiply-adds, with the tolerances to the oracle above (each side is within them)."""
+    ragged last ones; whole models against the plain multiply-adds, with the tolerances to the oracle above (each side is within them).
+    A wrong group of columns may hide in such a row's error: test_gpu_gemm_bf16.py has the products column by column."""
     for cfg, weights, tol in (
             (dk.config(width, 96, [dk.mlstm(2, 40, 136, 9.0, ff), dk.attention(4, 2, 48, 40, 512, 90.0, 0.15, ff)]), dk.random_weights, 0.02),
             (kit.config(width, 96, [kit.latent(3, 48, 56, 72, 0.14, kit.dense(ff)), kit.gla(2, 40, 136, 8.0, kit.dense(ff))]), kit.random_weights, 0.06)):
